@@ -9,6 +9,7 @@
 #include <cstring>
 
 #include "ernn.h"
+#include "ernn_block.h"
 #include "ernn_launch.h"
 #include "ernn_resident.h"
 #include "ernn_tma.h"
@@ -20,6 +21,7 @@ constexpr size_t kAlign = 256;
 constexpr double kPi = 3.14159265358979323846;
 // segment length of the resident reverse pass when the tape keeps every state
 constexpr int kResStoreAllSegment = 128;
+constexpr int kBlockMinCols = 40;
 inline size_t align_up(size_t v) { return (v + kAlign - 1) / kAlign * kAlign; }
 
 // Workspace plan of one problem.
@@ -34,14 +36,33 @@ struct Plan {
   size_t s_coef, s_LA, s_LB, s_seg, s_lbuf, s_gacc, s_part, s_tflags, s_total;
   // instances on a canvas: tile table (tape and scratch), a zero state (scratch)
   bool inst;
-  size_t inst_bytes, t_inst, s_inst, s_zero;
+  size_t inst_bytes, t_inst, s_inst;
+  // time-blocked tile kernels: the problem is theirs (given aligned buffers),
+  // floats between rows of a state, two more working levels in the tape and
+  // the scratch
+  bool block;
+  int pitch, geo;
+  size_t t_C, t_D, t_rec, s_LC, s_LD, s_rec;
 };
+
+// Problems of the time-blocked tile kernels, from sizes alone (the workspace
+// queries, the forward and the adjoint agree).  ERNN_PATH_AUTO takes rows of
+// any length from kBlockMinCols up (a warp spans 120 columns, so narrower
+// grids leave most lanes idle; the plain kernels take those); their states
+// are padded to 16-byte rows.  Where the cluster-resident path can run it
+// comes first.
+bool block_rule(const ErnnProblem& p) {
+  if (p.mode != kModeScalar) return false;
+  if (p.flags & ERNN_FLAG_INSTANCES) return true;
+  if (p.path == ERNN_PATH_TILED) return p.ny % 4 == 0;
+  return p.path == ERNN_PATH_AUTO && p.ny >= kBlockMinCols && !resident_possible(p.mode, p.nx, p.ny);
+}
 
 // Upper bound of the tile-table entries of any placement of S instances on
 // an nx x ny canvas (each instance's tiling has at most one partial tile row
 // and column).
 inline size_t inst_table_bound(int nx, int ny, int S) {
-  return ((size_t)(nx + kInstTileRows - 1) / kInstTileRows + S) * ((size_t)(ny + 63) / 64 + S);
+  return ((size_t)(nx + blk_tile_rows(kBlkTall) - 1) / blk_tile_rows(kBlkTall) + S) * ((size_t)(ny + kBlkCols - 1) / kBlkCols + S);
 }
 
 Plan make_plan(const ErnnProblem& p) {
@@ -54,7 +75,10 @@ Plan make_plan(const ErnnProblem& p) {
   pl.N = (size_t)p.nx * p.ny;
   pl.inst = (p.flags & ERNN_FLAG_INSTANCES) != 0;
   // instances share the canvas's one state plane
-  pl.state_bytes = align_up((size_t)(pl.inst ? 1 : p.nshots) * 2 * pl.N * sizeof(float));
+  pl.block = block_rule(p);
+  pl.geo = pl.inst ? kBlkTall : blk_geometry(p.nx, p.ny, p.nshots);
+  pl.pitch = pl.block ? (p.ny + 3) / 4 * 4 : p.ny;
+  pl.state_bytes = align_up((size_t)(pl.inst ? 1 : p.nshots) * 2 * p.nx * pl.pitch * sizeof(float));
   const dim3 g = step_grid(p.nx, p.ny, pl.inst ? 1 : p.nshots);
   pl.nblocks = (int)(g.x * g.y * g.z);
   pl.ncoef = (p.flags & (ERNN_FLAG_SHOT_CONSTANTS | ERNN_FLAG_INSTANCES)) ? p.nshots : 1;
@@ -66,6 +90,15 @@ Plan make_plan(const ErnnProblem& p) {
   pl.t_inst = off; off += pl.inst_bytes;
   pl.t_A = off; off += pl.state_bytes;
   pl.t_B = off; off += pl.state_bytes;
+  pl.t_C = off; if (pl.block) off += pl.state_bytes;
+  pl.t_D = off; if (pl.block) off += pl.state_bytes;
+  // receivers of the tiles
+  const size_t rec_bytes =
+      pl.block && p.record == kRecordReceivers
+          ? align_up(blk_rec_bytes(pl.inst ? inst_table_bound(p.nx, p.ny, p.nshots)
+                                           : (size_t)p.nshots * blk_tiles(pl.geo, p.nx, p.ny), p.nshots, p.nrec))
+          : 0;
+  pl.t_rec = off; off += rec_bytes;
   pl.t_total_notape = off;
   pl.t_store = off;
   if (pl.store_all) off += (size_t)p.nt * pl.state_bytes;           // u^1..u^nt
@@ -74,17 +107,20 @@ Plan make_plan(const ErnnProblem& p) {
   off = 0;
   pl.s_coef = off; off += align_up((size_t)pl.ncoef * sizeof(Coef));
   pl.s_inst = off; off += pl.inst_bytes;
-  pl.s_zero = off; if (pl.inst) off += pl.state_bytes;  // u^0 = u^{-1} = 0 of the first segment
   pl.s_LA = off; off += pl.state_bytes;
   pl.s_LB = off; off += pl.state_bytes;
+  pl.s_LC = off; if (pl.block) off += pl.state_bytes;
+  pl.s_LD = off; if (pl.block) off += pl.state_bytes;
+  pl.s_rec = off; off += rec_bytes;
   // two recompute segments: the cluster-resident path recomputes segment j-1
   // while the adjoint consumes segment j
-  // (instances: the tiled path only, one segment)
-  pl.s_seg = off; if (!pl.store_all) off += (size_t)(pl.inst ? 1 : 2) * pl.k * pl.state_bytes;
+  // (one segment where that path cannot run)
+  const bool res = resident_possible(p.mode, p.nx, p.ny) && !pl.inst;
+  pl.s_seg = off; if (!pl.store_all) off += (size_t)(pl.block && !res ? 1 : 2) * pl.k * pl.state_bytes;
   // lam buffers of the resident reverse pass: two segments of kres steps,
   // only where that path can run
   pl.kres = pl.store_all ? (p.nt < kResStoreAllSegment ? p.nt : kResStoreAllSegment) : pl.k;
-  if (!resident_possible(p.mode, p.nx, p.ny) || pl.inst) pl.kres = 0;
+  if (!res) pl.kres = 0;
   pl.s_lbuf = off; off += (size_t)2 * pl.kres * pl.state_bytes;
   pl.s_gacc = off;
   if (p.mode == kModeDField) off += align_up((size_t)p.nshots * pl.N * sizeof(float));
@@ -99,8 +135,8 @@ Plan make_plan(const ErnnProblem& p) {
   // receiver table of the tiled adjoint: one byte per (shot, tile), sized for
   // its smallest tiles (64 x 16)
   pl.s_tflags = off;
-  if (p.record == kRecordReceivers)
-    off += align_up(pl.inst ? inst_table_bound(p.nx, p.ny, p.nshots) : tma_tiles(p.nx, p.ny, p.nshots, 16));
+  if (p.record == kRecordReceivers && !pl.inst) off += align_up(tma_tiles(p.nx, p.ny, p.nshots, 16));
+  if (pl.block) off += 16;  // the scratch starts at its first 16-byte boundary
   pl.s_total = off;
   return pl;
 }
@@ -145,6 +181,14 @@ int validate_inputs(const ErnnProblem* p, const ErnnInputs* in) {
     return ERNN_ERR_INVALID;
   if (p->record == kRecordReceivers && in->rec_idx == nullptr) return ERNN_ERR_INVALID;
   return ERNN_OK;
+}
+
+inline bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+// The scratch of a time-blocked problem is used from its first 16-byte
+// boundary (states that TMA reads).
+inline void* scratch_base(const Plan& pl, void* scratch) {
+  const uintptr_t v = reinterpret_cast<uintptr_t>(scratch);
+  return pl.block ? reinterpret_cast<void*>((v + 15u) & ~(uintptr_t)15u) : scratch;
 }
 
 inline char* at(void* base, size_t off) { return static_cast<char*>(base) + off; }
@@ -356,6 +400,8 @@ int plan_instances(const ErnnProblem& p, const ErnnInstances* in, InstPlan* ip) 
   for (int k = 0; k < S; ++k) order[k] = k;
   std::stable_sort(order, order + S, [&](int u, int v) { return in->nt[u] > in->nt[v]; });
   ip->d.count = S;
+  ip->d.tile_rows = blk_tile_rows(kBlkTall);
+  ip->d.tile_cols = kBlkCols;
   ip->upto[0] = 0;
   for (int g = 0; g < S; ++g) {
     const int k = order[g];
@@ -366,7 +412,158 @@ int plan_instances(const ErnnProblem& p, const ErnnInstances* in, InstPlan* ip) 
     ip->d.ny[g] = in->ny[k];
     ip->d.nt[g] = in->nt[k];
     ip->d.base[g] = ip->upto[g];
-    ip->upto[g + 1] = ip->upto[g] + inst_tiles(in->nx[k], in->ny[k]);
+    ip->upto[g + 1] = ip->upto[g] + (int)blk_tiles(kBlkTall, in->nx[k], in->ny[k]);
+  }
+  return ERNN_OK;
+}
+
+// Steps of the next launch of a run of n: four at a time, the rest in
+// launches of two or three (one only where the run has one step: a launch
+// of one step leaves its older level behind in the buffer it read).
+inline int block_steps(int n) { return n <= kBlkSteps ? n : (n == kBlkSteps + 1 ? kBlkSteps - 1 : kBlkSteps); }
+
+// Of four working states, one that is neither x, y nor z.
+inline float* free_state(float* const pool[4], const float* x, const float* y, const float* z) {
+  for (int k = 0; k < 4; ++k)
+    if (pool[k] != x && pool[k] != y && pool[k] != z) return pool[k];
+  return nullptr;
+}
+
+BlkFwd base_blk_fwd(const ErnnProblem& p, const Plan& pl, const ErnnInputs& in, const Coef* coef, const InstTiles& it) {
+  BlkFwd a;
+  std::memset(&a, 0, sizeof(a));
+  a.geo = pl.geo;
+  // grids below four 64 x 32 tiles per SM, and odd ones, keep the plain
+  // kernels' rounding order: their states agree with those bit for bit
+  a.swap = p.path == ERNN_PATH_AUTO && !pl.inst && (p.ny % 4 != 0 || tma_tiles(p.nx, p.ny, p.nshots) < 608);
+  a.nx = p.nx; a.ny = p.ny; a.pitch = pl.pitch; a.S = p.nshots; a.nt = p.nt;
+  a.nt_out = pl.nt_out; a.record = p.record; a.nrec = p.nrec;
+  a.coef = coef; a.coef_stride = pl.ncoef > 1 ? 1 : 0;
+  a.src_signal = in.src_signal; a.src_map = in.src_map; a.src_origin = in.src_origin;
+  a.bx = p.src_bx; a.by = p.src_by; a.src_comp = p.src_comp;
+  a.inst = it;
+  for (int t = 0; t <= kBlkSteps; ++t) a.frame[t] = -1;
+  return a;
+}
+
+// Tiles of a time-blocked call.
+size_t block_tiles(const ErnnProblem& p, const Plan& pl, const InstPlan* ip) {
+  return ip != nullptr ? (size_t)ip->upto[ip->d.count] : (size_t)p.nshots * blk_tiles(pl.geo, p.nx, p.ny);
+}
+
+// Forward time loop on the time-blocked kernels: launches of up to four
+// steps, ending at the checkpoints, whose pair of levels is what a launch
+// leaves behind.
+int block_forward(const ErnnProblem& p, const Plan& pl, const ErnnInputs& in, const InstPlan* ip, InstTiles itab,
+                  Coef* coef, float* out_ux, float* out_uy, void* tape, int with_tape, cudaStream_t st) {
+  BlkFwd a = base_blk_fwd(p, pl, in, coef, itab);
+  if (p.record == kRecordReceivers)
+    ERNN_CUDA(launch_rec_tiles(pl.geo, in.rec_idx, p.nshots, p.nrec, p.nx, p.ny, itab.box, block_tiles(p, pl, ip),
+                               at(tape, pl.t_rec), &a.rec_tile, &a.rec_ent, st));
+  a.rec_x = out_ux;
+  a.rec_y = out_uy;
+  a.vec = p.ny % 4 == 0 && al16(out_ux) && al16(out_uy);
+  float* const pool[4] = {fat(tape, pl.t_A), fat(tape, pl.t_B), fat(tape, pl.t_C), fat(tape, pl.t_D)};
+  const bool store_all = with_tape && pl.store_all;
+  const int seg = with_tape && !pl.store_all ? pl.k : p.nt;
+  const float *cur = nullptr, *prev = nullptr;
+  for (int i = 0; i < p.nt;) {
+    const int end = (i / seg + 1) * seg < p.nt ? (i / seg + 1) * seg : p.nt;
+    const int T = block_steps(end - i);
+    a.i = i;
+    a.T = T;
+    a.cur = cur;
+    a.prev = prev;
+    for (int t = 0; t <= kBlkSteps; ++t) {
+      a.out[t] = nullptr;
+      a.frame[t] = t >= 1 && t <= T && (i + t - 1) % p.stride == 0 ? (i + t - 1) / p.stride : -1;
+    }
+    if (store_all) {
+      for (int t = 1; t <= T; ++t) a.out[t] = fat(tape, pl.t_store + (size_t)(i + t - 1) * pl.state_bytes);
+    } else {
+      a.out[T] = free_state(pool, cur, prev, nullptr);
+      if (T > 1) a.out[T - 1] = free_state(pool, cur, prev, a.out[T]);
+      if (with_tape && end < p.nt && i + T == end) {  // checkpoint j: (u^{jk}, u^{jk-1})
+        const int j = end / seg;
+        a.out[T] = fat(tape, pl.t_store + (size_t)(j - 1) * 2 * pl.state_bytes);
+        if (T > 1 || cur != nullptr) a.out[T - 1] = fat(tape, pl.t_store + ((size_t)(j - 1) * 2 + 1) * pl.state_bytes);
+      }
+    }
+    if (ip != nullptr) a.inst.ntiles = ip->fwd_tiles(i);
+    a.chained = i > 0;
+    ERNN_CUDA(launch_blk_fwd(a, &coef->err, st));
+    prev = T > 1 ? a.out[T - 1] : cur;
+    cur = a.out[T];
+    i += T;
+  }
+  return ERNN_OK;
+}
+
+// Adjoint on the time-blocked kernels: per segment from the last, the
+// recomputation of its states (when the tape does not hold them), then the
+// reverse steps over it.
+int block_adjoint(const ErnnProblem& p, const Plan& pl, const ErnnInputs& in, const InstPlan* ip, InstTiles itab,
+                  Coef* coef, const float* g_ux, const float* g_uy, void* tape, void* scratch, double* partials,
+                  cudaStream_t st) {
+  BlkFwd a = base_blk_fwd(p, pl, in, coef, itab);
+  BlkAdj b;
+  std::memset(&b, 0, sizeof(b));
+  b.geo = pl.geo;
+  b.nx = p.nx; b.ny = p.ny; b.pitch = pl.pitch; b.S = p.nshots; b.nt = p.nt;
+  b.u_stride = pl.state_bytes / sizeof(float);
+  b.g_x = g_ux; b.g_y = g_uy;
+  b.stride = p.stride; b.nt_out = pl.nt_out; b.record = p.record; b.nrec = p.nrec;
+  if (p.record == kRecordReceivers)
+    ERNN_CUDA(launch_rec_tiles(pl.geo, in.rec_idx, p.nshots, p.nrec, p.nx, p.ny, itab.box, block_tiles(p, pl, ip),
+                               at(scratch, pl.s_rec), &b.rec_tile, &b.rec_ent, st));
+  b.coef = coef;
+  b.coef_stride = a.coef_stride;
+  b.partials = partials;
+  b.inst = itab;
+  float* const pool[4] = {fat(scratch, pl.s_LA), fat(scratch, pl.s_LB), fat(scratch, pl.s_LC), fat(scratch, pl.s_LD)};
+  bool chained = false;  // every launch after the first follows one of the loop's
+  const int seg = pl.store_all ? p.nt : pl.k, nseg = pl.store_all ? 1 : pl.nseg;
+  for (int j = nseg - 1; j >= 0; --j) {
+    const int i0 = j * seg, i1 = (j + 1) * seg < p.nt ? (j + 1) * seg : p.nt;
+    if (pl.store_all) {
+      b.u_base = fat(tape, pl.t_store);
+    } else {
+      // u^{i0+1} .. u^{i1} into the segment buffer (u^{nt} is never imaged)
+      const int iend = i1 < p.nt ? i1 : p.nt - 1;
+      const float* ck0 = j == 0 ? nullptr : fat(tape, pl.t_store + (size_t)(j - 1) * 2 * pl.state_bytes);
+      const float* ck1 = j == 0 || j * pl.k - 1 == 0 ? nullptr  // u^0 = 0
+                                                     : fat(tape, pl.t_store + ((size_t)(j - 1) * 2 + 1) * pl.state_bytes);
+      auto slot = [&](int n) { return fat(scratch, pl.s_seg + (size_t)n * pl.state_bytes); };
+      for (int i = i0; i < iend;) {
+        const int T = block_steps(iend - i);
+        a.i = i;
+        a.T = T;
+        a.cur = i == i0 ? ck0 : slot(i - i0 - 1);
+        a.prev = i == i0 ? ck1 : (i == i0 + 1 ? ck0 : slot(i - i0 - 2));
+        for (int t = 0; t <= kBlkSteps; ++t) a.out[t] = t >= 1 && t <= T ? slot(i - i0 + t - 1) : nullptr;
+        if (ip != nullptr) a.inst.ntiles = ip->fwd_tiles(i);
+        a.chained = chained ? 1 : 0;
+        chained = true;
+        ERNN_CUDA(launch_blk_fwd(a, &coef->err, st));
+        i += T;
+      }
+      b.u_base = slot(0);
+    }
+    b.m_base = i0 + 1;
+    for (int m = i1; m > i0;) {
+      const int T = block_steps(m - i0);
+      b.m_hi = m;
+      b.T = T;
+      b.out_last = free_state(pool, b.cur, b.prev, nullptr);
+      b.out_before = T > 1 ? free_state(pool, b.cur, b.prev, b.out_last) : nullptr;
+      if (ip != nullptr) b.inst.ntiles = ip->adj_tiles(m - T + 1);
+      b.chained = chained ? 1 : 0;
+      chained = true;
+      ERNN_CUDA(launch_blk_adj(b, &coef->err, st));
+      b.prev = T > 1 ? b.out_before : b.cur;
+      b.cur = b.out_last;
+      m -= T;
+    }
   }
   return ERNN_OK;
 }
@@ -477,24 +674,18 @@ static int forward_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPl
   ERNN_CUDA(launch_coef(p->mode, in->C, in->rho, p->h, p->dt, coef, st, pl.ncoef));
 
   InstTiles itab{nullptr, nullptr, 0};
+  const bool block = pl.block && al16(tape) && blk_available();
   if (ip != nullptr) {
-    // instances: the tiled kernels over the tile table only.  A and B start
-    // at zero (B stands for u^0); the stored states need only the instances'
-    // ghost rings zeroed (the cells between the regions are never written,
-    // and outside the regions the kernels read only the rings); trace frames
-    // past an instance's steps are zero
+    // instances: the time-blocked kernels over the tile table only, which
+    // read and write a state inside the instances' regions alone; trace
+    // frames past an instance's steps are zero
     if (p->path != ERNN_PATH_AUTO && p->path != ERNN_PATH_TILED) return ERNN_ERR_UNSUPPORTED;
-    if (!tma_eligible(p->mode, p->nx, p->ny, 1)) return ERNN_ERR_UNSUPPORTED;
+    if (p->ny % 4 != 0) return ERNN_ERR_UNSUPPORTED;
+    if (!block) return blk_available() ? ERNN_ERR_CUDA : ERNN_ERR_UNSUPPORTED;
     itab.tiles = reinterpret_cast<int4*>(at(tape, pl.t_inst));
     itab.box = reinterpret_cast<int4*>(at(tape, pl.t_inst + align_up(inst_table_bound(p->nx, p->ny, p->nshots) *
                                                                        sizeof(int4))));
     ERNN_CUDA(launch_inst_table(ip->d, const_cast<int4*>(itab.tiles), const_cast<int4*>(itab.box), st));
-    ERNN_CUDA(cudaMemsetAsync(at(tape, pl.t_A), 0, 2 * pl.state_bytes, st));  // A and B are adjacent
-    if (with_tape) {
-      const int nstore = pl.store_all ? p->nt : 2 * (pl.nseg - 1);
-      ERNN_CUDA(launch_inst_ring_zero(fat(tape, pl.t_store), pl.state_bytes / sizeof(float), nstore, p->nx, p->ny,
-                                      itab.box, p->nshots, st));
-    }
     const size_t tr_bytes = (size_t)p->nshots * pl.nt_out * p->nrec * sizeof(float);
     ERNN_CUDA(cudaMemsetAsync(out_ux, 0, tr_bytes, st));
     ERNN_CUDA(cudaMemsetAsync(out_uy, 0, tr_bytes, st));
@@ -508,9 +699,12 @@ static int forward_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPl
     }
     if (p->path == ERNN_PATH_RESIDENT) return ERNN_ERR_UNSUPPORTED;
   }
+  if (block) {
+    g_last_path.store(ERNN_PATH_TILED, std::memory_order_relaxed);
+    return block_forward(*p, pl, *in, ip, itab, coef, out_ux, out_uy, tape, with_tape, st);
+  }
   int tiled = 0;
-  if (ip != nullptr) tiled = 1;
-  else if ((rc = use_tiled(*p, &tiled))) return rc;
+  if ((rc = use_tiled(*p, &tiled))) return rc;
   g_last_path.store(tiled ? ERNN_PATH_TILED : ERNN_PATH_STEP, std::memory_order_relaxed);
   auto fwd_step = [&](const FwdStep& s) {
     return tiled ? launch_tma_fwd(p->mode, s, &coef->err, st) : launch_fwd_step(p->mode, s, st);
@@ -525,7 +719,6 @@ static int forward_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPl
   };
   const bool receivers = (p->record == kRecordReceivers);
   FwdStep a = base_fwd(*p, *in, coef, pl.nt_out);
-  a.inst = itab;
   a.tile_rows = tile_rows_of(*p);
   const float* last = nullptr;
   for (int i = 0; i < p->nt; ++i) {
@@ -537,11 +730,6 @@ static int forward_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPl
       a.out = (i % 2 == 0) ? A : B;
       a.cur = i == 0 ? nullptr : ((i % 2 == 0) ? B : A);
       a.prev = i <= 1 ? nullptr : a.out;
-    }
-    if (ip != nullptr) {
-      // u^0 = 0: B (zeroed, first written at step 1) stands for it
-      if (a.cur == nullptr) a.cur = B;
-      a.inst.ntiles = ip->fwd_tiles(i);
     }
     a.i = i;
     a.copy0 = a.copy1 = nullptr;
@@ -562,7 +750,7 @@ static int forward_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPl
   }
   if (receivers && (p->nt - 1) % p->stride == 0) {
     ERNN_CUDA(launch_gather(last, p->nx, p->ny, p->nshots, in->rec_idx, p->nrec,
-                            (p->nt - 1) / p->stride, pl.nt_out, out_ux, out_uy, st, itab.box, p->nt));
+                            (p->nt - 1) / p->stride, pl.nt_out, out_ux, out_uy, st));
   }
   return ERNN_OK;
 }
@@ -599,6 +787,8 @@ static int adjoint_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPl
   if (tape_bytes < pl.t_total_tape || scratch_bytes < pl.s_total) return ERNN_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
   void* tape = const_cast<void*>(tape_c);  // read only below
+  scratch = scratch_base(pl, scratch);
+  const bool block = pl.block && al16(tape) && blk_available();
 
   Coef* coef = reinterpret_cast<Coef*>(at(scratch, pl.s_coef));
   ERNN_CUDA(launch_coef(p->mode, in->C, in->rho, p->h, p->dt, coef, st, pl.ncoef));
@@ -607,7 +797,7 @@ static int adjoint_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPl
   ERNN_CUDA(launch_gscale(g_ux, g_uy, gcount, coef, st, pl.ncoef));
   float* LA = fat(scratch, pl.s_LA);
   float* LB = fat(scratch, pl.s_LB);
-  ERNN_CUDA(cudaMemsetAsync(LA, 0, 2 * pl.state_bytes, st));  // LA and LB are adjacent
+  if (!block) ERNN_CUDA(cudaMemsetAsync(LA, 0, 2 * pl.state_bytes, st));  // LA and LB are adjacent
   float* gacc = fat(scratch, pl.s_gacc);
   double* partials = reinterpret_cast<double*>(at(scratch, pl.s_part));
   if (p->mode != kModeScalar) ERNN_CUDA(cudaMemsetAsync(gacc, 0, pl.s_part - pl.s_gacc, st));
@@ -615,19 +805,13 @@ static int adjoint_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPl
 
   InstTiles itab{nullptr, nullptr, 0};
   if (ip != nullptr) {
-    // instances: the tiled kernels over the tile table only; the zero state
-    // starts at zero, the recompute segment's states need only the
-    // instances' ghost rings zeroed (as the stored states of the forward)
     if (p->path != ERNN_PATH_AUTO && p->path != ERNN_PATH_TILED) return ERNN_ERR_UNSUPPORTED;
-    if (!tma_eligible(p->mode, p->nx, p->ny, 1)) return ERNN_ERR_UNSUPPORTED;
+    if (p->ny % 4 != 0) return ERNN_ERR_UNSUPPORTED;
+    if (!block) return blk_available() ? ERNN_ERR_CUDA : ERNN_ERR_UNSUPPORTED;
     itab.tiles = reinterpret_cast<int4*>(at(scratch, pl.s_inst));
     itab.box = reinterpret_cast<int4*>(at(scratch, pl.s_inst + align_up(inst_table_bound(p->nx, p->ny, p->nshots) *
                                                                           sizeof(int4))));
     ERNN_CUDA(launch_inst_table(ip->d, const_cast<int4*>(itab.tiles), const_cast<int4*>(itab.box), st));
-    ERNN_CUDA(cudaMemsetAsync(at(scratch, pl.s_zero), 0, pl.state_bytes, st));
-    if (!pl.store_all)
-      ERNN_CUDA(launch_inst_ring_zero(fat(scratch, pl.s_seg), pl.state_bytes / sizeof(float), pl.k, p->nx, p->ny,
-                                      itab.box, p->nshots, st));
   }
 
   if (ip == nullptr && (p->path == ERNN_PATH_AUTO || p->path == ERNN_PATH_RESIDENT)) {
@@ -645,15 +829,22 @@ static int adjoint_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPl
     }
     if (p->path == ERNN_PATH_RESIDENT) return ERNN_ERR_UNSUPPORTED;
   }
+  if (block) {
+    g_last_path.store(ERNN_PATH_TILED, std::memory_order_relaxed);
+    if ((rc = block_adjoint(*p, pl, *in, ip, itab, coef, g_ux, g_uy, tape, scratch, partials, st))) return rc;
+    if (pl.ncoef > 1)
+      ERNN_CUDA(launch_finalize_scalar(partials, kTiledRowsPerShot, coef, grad_C, st, p->nshots, 1));
+    else
+      ERNN_CUDA(launch_finalize_scalar(partials, pl.npart, coef, grad_C, st));
+    return ERNN_OK;
+  }
   int tiled = 0;
-  if (ip != nullptr) tiled = 1;
-  else if ((rc = use_tiled(*p, &tiled))) return rc;
+  if ((rc = use_tiled(*p, &tiled))) return rc;
   g_last_path.store(tiled ? ERNN_PATH_TILED : ERNN_PATH_STEP, std::memory_order_relaxed);
 
   auto stored = [&](int n) { return fat(tape, pl.t_store + (size_t)(n - 1) * pl.state_bytes); };
-  const float* zero_state = ip != nullptr ? fat(scratch, pl.s_zero) : nullptr;
   auto ck = [&](int j, int lev) -> const float* {
-    if (j == 0) return lev == 0 ? zero_state : nullptr;  // u^0 = 0 (given as a state with instances)
+    if (j == 0) return nullptr;
     if (lev == 1 && j * pl.k - 1 == 0) return nullptr;  // u^0 = 0 (k == 1)
     return fat(tape, pl.t_store + ((size_t)(j - 1) * 2 + lev) * pl.state_bytes);
   };
@@ -670,16 +861,10 @@ static int adjoint_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPl
   b.partials = partials;
   b.gacc = gacc;
   b.tile_flags = nullptr;
-  b.inst = itab;
   b.tile_rows = tile_rows_of(*p);
   if (tiled && p->record == kRecordReceivers) {
     uint8_t* flags = reinterpret_cast<uint8_t*>(at(scratch, pl.s_tflags));
-    if (ip != nullptr)
-      ERNN_CUDA(launch_inst_tile_flags(in->rec_idx, p->nshots, p->nrec, p->ny, itab.box, flags,
-                                       ip->upto[ip->d.count], st));
-    else
-      ERNN_CUDA(launch_tile_flags(p->mode, in->rec_idx, p->nshots, p->nrec, p->nx, p->ny, flags, st,
-                                  b.tile_rows));
+    ERNN_CUDA(launch_tile_flags(p->mode, in->rec_idx, p->nshots, p->nrec, p->nx, p->ny, flags, st, b.tile_rows));
     b.tile_flags = flags;
   }
 
@@ -700,7 +885,6 @@ static int adjoint_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPl
   auto adj_step = [&](int m, const float* um) -> int {
     const int idx = p->nt - m;
     b.m = m;
-    if (ip != nullptr) b.inst.ntiles = ip->adj_tiles(m);
     b.out = (idx % 2 == 0) ? LA : LB;
     b.cur = (idx % 2 == 0) ? LB : LA;
     b.prev = b.out;
@@ -717,7 +901,6 @@ static int adjoint_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPl
       if ((rc = adj_step(m, stored(m)))) return rc;
   } else {
     FwdStep a = base_fwd(*p, *in, coef, pl.nt_out);
-    a.inst = itab;
     a.tile_rows = b.tile_rows;
     for (int j = pl.nseg - 1; j >= 0; --j) {
       const int i0 = j * pl.k, i1 = (j + 1) * pl.k < p->nt ? (j + 1) * pl.k : p->nt;
@@ -732,13 +915,7 @@ static int adjoint_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPl
         a.prev = (i == i0) ? ck(j, 1) : (i == i0 + 1 ? ck(j, 0) : seg(i - i0 - 2));
         a.chained = chained ? 1 : 0;
         chained = true;
-        if (ip != nullptr) a.inst.ntiles = ip->fwd_tiles(i);
-        // (a pair of steps takes the tiles of the first step: an instance
-        // ending after step i runs both of them, one ending at i + 1 takes
-        // the pair only when it has step i + 1)
-        a.out2 = (tiled && i + 1 < iend && (ip == nullptr || ip->fwd_tiles(i + 1) == a.inst.ntiles))
-                     ? seg(i + 1 - i0)
-                     : nullptr;
+        a.out2 = (tiled && i + 1 < iend) ? seg(i + 1 - i0) : nullptr;
         if (a.out2 != nullptr && tma_fwd2_would_run(p->mode, a)) {
           ERNN_CUDA(launch_tma_fwd2(p->mode, a, &coef->err, st));
           i += 2;
@@ -792,8 +969,8 @@ int ernn_device_status(const ErnnProblem* p, const void* workspace, int is_scrat
   if (workspace == nullptr || status_host == nullptr || (is_scratch != 0 && is_scratch != 1))
     return ERNN_ERR_INVALID;
   const Plan pl = make_plan(*p);
-  const char* w = static_cast<const char*>(workspace) + (is_scratch ? pl.s_coef : pl.t_coef) +
-                  offsetof(Coef, err);
+  const void* base = is_scratch ? scratch_base(pl, const_cast<void*>(workspace)) : workspace;
+  const char* w = static_cast<const char*>(base) + (is_scratch ? pl.s_coef : pl.t_coef) + offsetof(Coef, err);
   ERNN_CUDA(cudaMemcpyAsync(status_host, w, sizeof(int32_t), cudaMemcpyDeviceToHost,
                             (cudaStream_t)stream));
   return ERNN_OK;

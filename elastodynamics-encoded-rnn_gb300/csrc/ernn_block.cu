@@ -1,0 +1,833 @@
+// Time-blocked tile kernels (sm_103a): up to four time steps of a tile per
+// launch, the tile's state in registers.
+//
+// One step of the scheme on a large grid moves 24 bytes of state per cell
+// (adjoint 32) through HBM for some 60 FP32 operations: a launch per step is
+// bound by the memory, and on grids of a few hundred cells a side by the
+// launches.  Here a CTA loads a tile of both levels with a halo of four
+// cells once (TMA, zeros outside the grid), advances it up to four steps,
+// and writes the last two levels: 24 -> 8 bytes per cell and step.
+//
+// Layout: a warp holds RW rows of 128 columns, each lane one quad of four
+// columns, both levels of its cells in registers for all steps; the new
+// level overwrites the older one.  A step needs from other threads only
+// the columns beside a quad (lane shuffles) and the rows above and below the
+// warp's (exchanged through shared memory, one CTA barrier per step); there
+// are no window loads.  The valid region shrinks by one cell per step, so
+// the outer quad and the outer four rows of the tile are not stored: 120
+// columns x (W RW - 8) rows are.  The loads of the CTA's next tile run
+// while the current one is advanced.
+//
+// Every cell's update is the same sequence of rounded operations as in the
+// per-step kernels, so the states agree with theirs bit for bit.
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
+#include <cmath>
+#include <mutex>
+
+#include "ernn_block.h"
+#include "ernn_launch.h"
+#include "ernn_tile.cuh"
+
+namespace ernn {
+
+namespace {
+
+constexpr int kBox = 128;  // columns of a tile with its halo: 32 lanes x 4
+constexpr int kH = kBlkSteps;
+constexpr unsigned kFull = 0xffffffffu;
+
+// A tile: state plane, instance, first row and column, and the region
+// [xs, xe) x [ys, ye) of its instance (the whole grid without instances).
+struct BTile {
+  int plane, inst, x0, y0, xs, ys, xe, ye;
+};
+
+// The tiles first, first + step, ... of a CTA.  Grid: walked in (shot, row
+// block, column block) digits, an addition with carries per tile; instances:
+// entries of the tile table.
+template <bool INST, int H>
+struct BWalk {
+  int t, step, shot, xt, yt, ds, dx, dy, tiles_x, tiles_y, nx, ny;
+  __device__ __forceinline__ void init(int first, int step_, int tx, int ty, int nx_, int ny_) {
+    t = first;
+    step = step_;
+    if constexpr (!INST) {
+      tiles_x = tx;
+      tiles_y = ty;
+      nx = nx_;
+      ny = ny_;
+      const int per = tx * ty;
+      shot = first / per;
+      int r = first - shot * per;
+      xt = r / ty;
+      yt = r - xt * ty;
+      ds = step / per;
+      r = step - ds * per;
+      dx = r / ty;
+      dy = r - dx * ty;
+    }
+  }
+  __device__ __forceinline__ BTile tile(const InstTiles& in) const {
+    if constexpr (INST) {
+      const int4 e = __ldg(&in.tiles[t]);
+      return BTile{0, e.x, (int)((unsigned)e.y & 0xffffu), (int)((unsigned)e.y >> 16), (int)((unsigned)e.z & 0xffffu),
+                   (int)((unsigned)e.z >> 16), (int)((unsigned)e.w & 0xffffu), (int)((unsigned)e.w >> 16)};
+    } else {
+      return BTile{shot, shot, xt * H, yt * kBlkCols, 0, 0, nx, ny};
+    }
+  }
+  __device__ __forceinline__ void next() {
+    t += step;
+    if constexpr (!INST) {
+      yt += dy;
+      if (yt >= tiles_y) { yt -= tiles_y; ++xt; }
+      xt += dx;
+      if (xt >= tiles_x) { xt -= tiles_x; ++shot; }
+      shot += ds;
+    }
+  }
+};
+
+// Four cells of a row.
+struct Q4 {
+  float v[4];
+};
+__device__ __forceinline__ Q4 q4(const float4 v) { return Q4{{v.x, v.y, v.z, v.w}}; }
+__device__ __forceinline__ float4 f4(const Q4& q) { return make_float4(q.v[0], q.v[1], q.v[2], q.v[3]); }
+__device__ __forceinline__ Q4 zero_q4() { return Q4{{0.f, 0.f, 0.f, 0.f}}; }
+
+// One row of a component: the quad (w[1] .. w[4]) and the cells beside it.
+struct Row {
+  float w[6];
+};
+__device__ __forceinline__ Row row_of(const Q4& q) {
+  return Row{{__shfl_up_sync(kFull, q.v[3], 1), q.v[0], q.v[1], q.v[2], q.v[3], __shfl_down_sync(kFull, q.v[0], 1)}};
+}
+
+// The constants in the order of Coef; zero for a lane whose quad lies outside
+// the region (its levels are zero, and stay so).
+__device__ __forceinline__ Coefs coefs_in(const float* k, bool in) {
+  return Coefs{in ? k[0] : 0.f, in ? k[1] : 0.f, in ? k[2] : 0.f, in ? k[3] : 0.f,
+               in ? k[4] : 0.f, in ? k[5] : 0.f, in ? k[6] : 0.f, in ? k[7] : 0.f};
+}
+
+// Second differences at cell q of the quad of row m, with the rows t above
+// and b below:
+//   xx = (t + b) - 2 m,  yy = (left + right) - 2 m,
+//   xy = (b[+1] + t[-1]) - (b[-1] + t[+1]),
+// each with the association and rounding of the per-step kernels.  Scalar
+// operations: a packed one (two cells) takes the FP32 pipe twice as long, and
+// a scalar one between packed ones as long as they (measured: 3.9 scalar,
+// 1.8 packed, 1.9 mixed warp instructions per cycle and SM).
+struct Sums {
+  float xx, yy, xy;
+};
+__device__ __forceinline__ Sums sums_of(const Row& t, const Row& m, const Row& b, int q) {
+  const int k = q + 1;
+  return Sums{fmaf(-2.f, m.w[k], t.w[k] + b.w[k]), fmaf(-2.f, m.w[k], m.w[k - 1] + m.w[k + 1]),
+              (b.w[k + 1] + t.w[k - 1]) - (b.w[k - 1] + t.w[k + 1])};
+}
+
+// The operator at a cell from the sums of both components.  The first two
+// terms are one rounded product and one fused multiply-add: SWAP = false
+// rounds the first product (as the tiled per-step kernels), true the second
+// (as the plain ones).
+template <bool SWAP>
+__device__ __forceinline__ void oper(const Coefs& k, const Sums& x, const Sums& y, float& lx, float& ly) {
+  lx = SWAP ? fmaf(k.k11, x.xx, __fmul_rn(k.k66, x.yy)) : fmaf(k.k66, x.yy, __fmul_rn(k.k11, x.xx));
+  lx = fmaf(k.kq12, y.xy, lx);
+  lx = fmaf(k.k16h, x.xy, lx);
+  lx = fmaf(k.k16, y.xx, lx);
+  lx = fmaf(k.k26, y.yy, lx);
+  ly = SWAP ? fmaf(k.k66, y.xx, __fmul_rn(k.k22, y.yy)) : fmaf(k.k22, y.yy, __fmul_rn(k.k66, y.xx));
+  ly = fmaf(k.kq12, x.xy, ly);
+  ly = fmaf(k.k16, x.xx, ly);
+  ly = fmaf(k.k26, x.yy, ly);
+  ly = fmaf(k.k26h, y.xy, ly);
+}
+// (2 c - p) + l
+__device__ __forceinline__ float leap(float c, float p, float l) { return fmaf(2.f, c, -p) + l; }
+
+// A CTA's tile: both levels of W RW rows of 128 columns, both components,
+// with a guard row on either side (read for rows that are never stored).
+template <int W, int RW>
+struct BlkTile {
+  static constexpr int kThreads = 32 * W;
+  static constexpr int kRows = W * RW;
+  static constexpr int kUse = kRows - 2 * kH;        // rows stored
+  static constexpr int kPlane = kRows * kBox;        // floats of a component
+  static constexpr int kLevel = 2 * kPlane;
+  static constexpr int kFloats = 2 * kLevel + 2 * kBox;
+  static constexpr int kMeta = 16;
+  static constexpr size_t kBytes = (size_t)(kFloats + kMeta) * 4 + 8 + 128;
+};
+
+template <bool V>
+struct BoolC {
+  static constexpr bool value = V;
+};
+
+// Zeroes the cells n .. 3 of a quad.
+__device__ __forceinline__ void mask_q(float (&v)[4], int n) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) v[q] = n > q ? v[q] : 0.f;
+}
+
+__device__ __forceinline__ Row load_row(const float* p) {  // a row of the tile at the lane's quad
+  return row_of(q4(*reinterpret_cast<const float4*>(p)));
+}
+
+// Rows of a warp's share that lie in [lo, hi) of the tile, as bits.
+template <int RW>
+__device__ __forceinline__ uint32_t rows_in(int rr0, int lo, int hi) {
+  lo = max(lo - rr0, 0);
+  hi = min(hi - rr0, RW);
+  return hi > lo ? ((1u << hi) - 1u) & ~((1u << lo) - 1u) : 0u;
+}
+
+// Zeroes the tile's cells outside its instance's region (on a canvas they
+// belong to other instances), or all of a level that is a zero state.
+template <int W, int RW>
+__device__ __forceinline__ void clear_cells(float* lev, bool all, const BTile& t) {
+  using B = BlkTile<W, RW>;
+  for (int e = threadIdx.x; e < B::kPlane / 4; e += B::kThreads) {
+    const int gi = t.x0 - kH + (e >> 5), gj = t.y0 - kH + 4 * (e & 31);
+    if (!all && gi >= t.xs && gi < t.xe && gj >= t.ys && gj < t.ye) continue;
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    *reinterpret_cast<float4*>(lev + 4 * e) = z;
+    *reinterpret_cast<float4*>(lev + B::kPlane + 4 * e) = z;
+  }
+}
+
+// Both levels of a tile into shared memory: c (u^i, or lam^{m+1}) and p (the
+// level before it); a level that is not used is zero.  Every thread calls it;
+// the tile is complete after the caller's next CTA barrier.
+template <int W, int RW, bool INST>
+__device__ __forceinline__ void load_tile(float* lev0, float* lev1, const CUtensorMap* cm, const CUtensorMap* pm,
+                                          bool has_c, bool has_p, bool use_c, bool use_p, const BTile& t, int k,
+                                          uint64_t* bar, PipeGuard* guard, int* err) {
+  using B = BlkTile<W, RW>;
+  const uint32_t bytes = (uint32_t)((has_c ? B::kLevel : 0) + (has_p ? B::kLevel : 0)) * 4u;
+  if (bytes != 0) {
+    if (threadIdx.x == 0 && !pipe_failed(guard)) {
+      pipe_issued(guard, k);
+      fence_async();
+      bar_expect(bar, bytes);
+      if (has_c) tma_load3(lev0, cm, t.y0 - kH, t.x0 - kH, 2 * t.plane, bar);
+      if (has_p) tma_load3(lev1, pm, t.y0 - kH, t.x0 - kH, 2 * t.plane, bar);
+    }
+    bar_wait_ok(bar, (uint32_t)k & 1u, err, guard);
+  }
+  if (INST || !use_c) clear_cells<W, RW>(lev0, !use_c, t);
+  if (INST || !use_p) clear_cells<W, RW>(lev1, !use_p, t);
+}
+
+// ----------------------------------------------------------------- forward
+template <int W, int RW, bool INST, bool SWAP, int CTAS>
+__global__ void __launch_bounds__(32 * W, CTAS)
+    blk_fwd_kernel(const BlkFwd a, const __grid_constant__ CUtensorMap cur_map,
+                   const __grid_constant__ CUtensorMap prev_map, int tiles_x, int tiles_y, int ntiles, int* err) {
+  extern __shared__ float sm_raw[];
+  float* sm = aligned128(sm_raw);
+  using B = BlkTile<W, RW>;
+  constexpr int NT = B::kThreads;
+  float* lev0 = sm + kBox;  // (a guard row before and after the levels)
+  float* lev1 = lev0 + B::kLevel;
+  float* meta = sm + B::kFloats;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(meta + B::kMeta);
+  __shared__ PipeGuard guard;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int nx = a.nx, ny = a.ny;
+  const size_t N = (size_t)nx * ny, Np = (size_t)nx * a.pitch;
+  const bool has_src = a.bx > 0 && a.by > 0;
+  grid_dep_trigger();
+  if (tid == 0) {
+    prefetch_map(&cur_map);
+    prefetch_map(&prev_map);
+    bar_init(bar);
+    pipe_init(&guard);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  // (zeros: what rows without a neighbour read stays finite)
+  if (tid < kBox) sm[tid] = sm[B::kFloats - kBox + tid] = 0.f;
+  BWalk<INST, B::kUse> walk;
+  walk.init((int)blockIdx.x, (int)gridDim.x, tiles_x, tiles_y, nx, ny);
+  __syncthreads();
+  grid_dep_wait();  // the states of the previous launch are complete from here on
+
+  const int rr0 = w * RW;  // first row of the warp in the tile
+  const int o0 = rr0 * kBox + 4 * lane;
+  for (int k = 0; walk.t < ntiles; ++k, walk.next()) {
+    const BTile tile = walk.tile(a.inst);
+    // per-tile scalars: coefficients, amplitudes of the steps, source origin
+    if (w == 0) {
+      const Coef* K = a.coef + (size_t)tile.inst * a.coef_stride;
+      if (lane < 8) meta[lane] = (&K->k11)[lane];
+      if (lane >= 8 && lane < 8 + kBlkSteps && a.i + lane - 8 < a.nt)
+        meta[lane] = a.src_signal[(size_t)tile.inst * a.nt + a.i + lane - 8] * K->kappa;
+      if (lane >= 12 && lane < 14 && has_src) meta[lane] = __int_as_float(a.src_origin[2 * tile.inst + lane - 12]);
+    }
+    load_tile<W, RW, INST>(lev0, lev1, &cur_map, &prev_map, a.cur != nullptr, a.prev != nullptr, a.cur != nullptr,
+                           a.prev != nullptr, tile, k, bar, &guard, err);
+    __syncthreads();
+    const int gj = tile.y0 - kH + 4 * lane, gi0 = tile.x0 - kH + rr0;
+    // cells of the quad inside the region's columns; rows of the warp inside
+    // its rows, and those this lane stores
+    const int nq = gj >= tile.ys ? max(0, min(4, tile.ye - gj)) : 0;
+    const uint32_t region = rows_in<RW>(rr0, tile.xs - tile.x0 + kH, tile.xe - tile.x0 + kH);
+    const uint32_t stored = lane >= 1 && lane <= 30 && nq > 0 ? region & rows_in<RW>(rr0, kH, B::kRows - kH) : 0u;
+    const Coefs ks = coefs_in(meta, nq > 0);
+    const int ox = __float_as_int(meta[12]), oy = __float_as_int(meta[13]);
+    const bool src = has_src && tile.x0 - kH < ox + a.bx && tile.x0 - kH + B::kRows > ox &&
+                     tile.y0 - kH < oy + a.by && tile.y0 - kH + kBox > oy;
+    const bool ragged = ((tile.ye - tile.ys) & 3) != 0 && tile.y0 - kH + kBox > tile.ye;
+    const int2 recs = a.rec_tile != nullptr ? a.rec_tile[walk.t] : make_int2(0, 0);
+    int T = a.T;
+    if (INST) T = min(T, a.inst.box[2 * tile.inst + 1].z - a.i);
+    const ptrdiff_t off = (ptrdiff_t)tile.plane * 2 * (ptrdiff_t)Np + (ptrdiff_t)gi0 * a.pitch + gj;
+    if (a.out[0] != nullptr) {
+#pragma unroll
+      for (int r = 0; r < RW; ++r)
+        if ((stored >> r) & 1u) {
+          float* o = a.out[0] + off + (ptrdiff_t)r * a.pitch;
+          *reinterpret_cast<float4*>(o) = *reinterpret_cast<const float4*>(lev0 + o0 + r * kBox);
+          *reinterpret_cast<float4*>(o + Np) = *reinterpret_cast<const float4*>(lev0 + B::kPlane + o0 + r * kBox);
+        }
+    }
+    for (int t = 1; t <= T; ++t) {
+      const float* c0 = ((t & 1) ? lev0 : lev1) + o0;  // u^{i+t-1}
+      float* p0 = ((t & 1) ? lev1 : lev0) + o0;        // u^{i+t-2}, becomes u^{i+t}
+      const int frame = a.frame[t];
+      const bool dense = frame >= 0 && a.record == kRecordFields;
+      float* out0 = a.out[t] + off;
+      float* out1 = out0 + Np;
+      const uint32_t st = a.out[t] != nullptr ? stored : 0u;
+      auto rows = [&](auto plain) {
+        constexpr bool PLAIN = decltype(plain)::value;
+        Row t0 = load_row(c0 - kBox), t1 = load_row(c0 + B::kPlane - kBox);
+        Row m0 = load_row(c0), m1 = load_row(c0 + B::kPlane);
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+          const Row b0 = load_row(c0 + (r + 1) * kBox), b1 = load_row(c0 + B::kPlane + (r + 1) * kBox);
+          if (PLAIN || ((region >> r) & 1u)) {  // (rows outside the region stay zero)
+            const float4 pv0 = *reinterpret_cast<const float4*>(p0 + r * kBox);
+            const float4 pv1 = *reinterpret_cast<const float4*>(p0 + B::kPlane + r * kBox);
+            const float q0[4] = {pv0.x, pv0.y, pv0.z, pv0.w}, q1[4] = {pv1.x, pv1.y, pv1.z, pv1.w};
+            float v0[4], v1[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) oper<SWAP>(ks, sums_of(t0, m0, b0, q), sums_of(t1, m1, b1, q), v0[q], v1[q]);
+            if (!PLAIN && src && (unsigned)(gi0 + r - ox) < (unsigned)a.bx) {
+              // the load joins the operator sum before the update, as in the
+              // reference's (A u + f) / rho
+              const float amp = meta[7 + t];
+              const float* f = a.src_map + ((size_t)tile.inst * a.bx + (gi0 + r - ox)) * a.by;
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                const int sb = gj + q - oy;
+                if ((unsigned)sb < (unsigned)a.by && q < nq) {
+                  float& l = a.src_comp == 0 ? v0[q] : v1[q];
+                  l = fmaf(amp, f[sb], l);  // L + amp f, one rounding
+                }
+              }
+            }
+            // (quads outside the region stay zero: their lanes' coefficients are)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              v0[q] = leap(m0.w[q + 1], q0[q], v0[q]);
+              v1[q] = leap(m1.w[q + 1], q1[q], v1[q]);
+            }
+            if (!PLAIN && ragged) {  // the region's last column is inside a quad
+              mask_q(v0, nq);
+              mask_q(v1, nq);
+            }
+            const float4 n0 = make_float4(v0[0], v0[1], v0[2], v0[3]), n1 = make_float4(v1[0], v1[1], v1[2], v1[3]);
+            *reinterpret_cast<float4*>(p0 + r * kBox) = n0;
+            *reinterpret_cast<float4*>(p0 + B::kPlane + r * kBox) = n1;
+            if ((st >> r) & 1u) {
+              *reinterpret_cast<float4*>(out0) = n0;
+              *reinterpret_cast<float4*>(out1) = n1;
+            }
+            if (!PLAIN && dense && ((stored >> r) & 1u)) {
+              const size_t o = ((size_t)tile.plane * a.nt_out + frame) * N + (size_t)(gi0 + r) * ny + gj;
+              if (a.vec) {
+                *reinterpret_cast<float4*>(a.rec_x + o) = n0;
+                *reinterpret_cast<float4*>(a.rec_y + o) = n1;
+              } else {
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                  if (q < nq) {
+                    a.rec_x[o + q] = v0[q];
+                    a.rec_y[o + q] = v1[q];
+                  }
+              }
+            }
+          }
+          out0 += a.pitch;
+          out1 += a.pitch;
+          t0 = m0; t1 = m1; m0 = b0; m1 = b1;
+        }
+      };
+      // (warps none of whose rows a later step reads have nothing to do)
+      if (region != 0 && rows_in<RW>(rr0, t, B::kRows - t) != 0) {
+        if (region == (1u << RW) - 1u && !src && !ragged && !dense) rows(BoolC<true>{});
+        else rows(BoolC<false>{});
+      }
+      __syncthreads();  // u^{i+t} is complete; its receivers are read beside the next step
+      if (frame >= 0 && recs.y > 0) {
+        const float* lv = (t & 1) ? lev1 : lev0;
+        const size_t o = ((size_t)tile.inst * a.nt_out + frame) * a.nrec;
+        for (int e = tid; e < recs.y; e += NT) {
+          const int2 v = a.rec_ent[recs.x + e];
+          const int rr = v.x / kBox, cc = v.x % kBox;
+          if (rr < kH || rr >= B::kRows - kH || cc < kH || cc >= kBox - kH) continue;  // another tile's
+          a.rec_x[o + v.y] = lv[v.x];
+          a.rec_y[o + v.y] = lv[B::kPlane + v.x];
+        }
+      }
+    }
+    __syncthreads();  // the levels and scalars are read: the next tile's may arrive
+  }
+  if (tid == 0 && pipe_failed(&guard)) pipe_drain(bar, 1, &guard);
+}
+
+// ----------------------------------------------------------------- adjoint
+// As the forward, with lam^{m+1}, lam^{m+2} in the levels' place and no
+// load: the recorded residuals enter at the receivers' cells (subtracted
+// from lam^{m+2} before the update) or at every cell (dense history).  The
+// six imaging sums sum_cells lam . (dA/dC_k u) are formed in the transposed
+// form sum_cells u . (dA/dC_k lam) (the second differences with zero ghosts
+// are symmetric), which needs u^m only at the cell itself, read from global
+// memory one row ahead.
+template <int W, int RW, bool INST, int CTAS>
+__global__ void __launch_bounds__(32 * W, CTAS)
+    blk_adj_kernel(const BlkAdj a, const __grid_constant__ CUtensorMap cur_map,
+                   const __grid_constant__ CUtensorMap prev_map, int tiles_x, int tiles_y, int ntiles, int* err) {
+  extern __shared__ float sm_raw[];
+  float* sm = aligned128(sm_raw);
+  using B = BlkTile<W, RW>;
+  constexpr int NT = B::kThreads;
+  float* lev0 = sm + kBox;
+  float* lev1 = lev0 + B::kLevel;
+  float* meta = sm + B::kFloats;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(meta + B::kMeta);
+  __shared__ PipeGuard guard;
+  __shared__ float2 red[W][6];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int nx = a.nx, ny = a.ny;
+  const size_t N = (size_t)nx * ny, Np = (size_t)nx * a.pitch;
+  grid_dep_trigger();
+  if (tid == 0) {
+    prefetch_map(&cur_map);
+    prefetch_map(&prev_map);
+    bar_init(bar);
+    pipe_init(&guard);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  // This CTA's tiles: strided over the grid, or with per-shot constants a
+  // contiguous chunk (its sums are flushed whenever it enters another shot)
+  const bool per_shot = a.coef_stride != 0;
+  const int b = (int)blockIdx.x, nb = (int)gridDim.x;
+  const int t_end = per_shot ? (int)((long long)(b + 1) * ntiles / nb) : ntiles;
+  // (zeros: what rows without a neighbour read stays finite)
+  if (tid < kBox) sm[tid] = sm[B::kFloats - kBox + tid] = 0.f;
+  BWalk<INST, B::kUse> walk;
+  walk.init(per_shot ? (int)((long long)b * ntiles / nb) : b, per_shot ? 1 : nb, tiles_x, tiles_y, nx, ny);
+  __syncthreads();
+  grid_dep_wait();  // the states of the previous launch are complete from here on
+  const float gs = a.coef->gscale;  // one scale for every shot
+
+  // Imaging sums: FP32 over a thread's cells of one step, over steps and
+  // tiles as FP32 pairs (TwoSum; the sum does not depend on how the steps
+  // are split over launches), FP64 across warps and launches.
+  float hi[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, lo[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  // (the lanes' pairs are added as pairs: a warp's FP64 addition occupies
+  // this part's FP64 pipe for 16 cycles and more, and thirty per warp took
+  // longer than a step of a small tile)
+  auto flush = [&](int shot) {  // CTA-uniform
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+      float h = hi[q], l = lo[q];
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) {
+        const float h2 = __shfl_down_sync(kFull, h, off), l2 = __shfl_down_sync(kFull, l, off);
+        const float s = h + h2, bp = s - h;
+        l = (l + l2) + ((h - (s - bp)) + (h2 - bp));
+        h = s;
+      }
+      if (lane == 0) red[w][q] = make_float2(h, l);
+      hi[q] = 0.f;
+      lo[q] = 0.f;
+    }
+    __syncthreads();
+    if (tid < 6) {
+      double v = 0.0;
+      for (int x = 0; x < W; ++x) v += (double)red[x][tid].x + (double)red[x][tid].y;
+      const size_t row = per_shot ? (size_t)shot * kTiledRowsPerShot + b : (size_t)b;
+      a.partials[row * 8 + tid] += v;
+    }
+    __syncthreads();  // red is free again
+  };
+  int acc_shot = -1;
+
+  const int rr0 = w * RW;  // first row of the warp in the tile
+  const int o0 = rr0 * kBox + 4 * lane;
+  for (int k = 0; walk.t < t_end; ++k, walk.next()) {
+    const BTile tile = walk.tile(a.inst);
+    if (per_shot && tile.inst != acc_shot) {
+      if (acc_shot >= 0) flush(acc_shot);
+      acc_shot = tile.inst;
+    }
+    // steps of the tile's instance; lam beyond the last is zero, and its
+    // imaging pairs are m <= steps - 1
+    const int steps = INST ? min(a.inst.box[2 * tile.inst + 1].z, a.nt) : a.nt;
+    if (w == 0 && lane < 8) meta[lane] = (&(a.coef + (size_t)tile.inst * a.coef_stride)->k11)[lane];
+    load_tile<W, RW, INST>(lev0, lev1, &cur_map, &prev_map, a.cur != nullptr, a.prev != nullptr,
+                           a.cur != nullptr && steps >= a.m_hi + 1, a.prev != nullptr && steps >= a.m_hi + 2, tile, k,
+                           bar, &guard, err);
+    __syncthreads();
+    const int gj = tile.y0 - kH + 4 * lane, gi0 = tile.x0 - kH + rr0;
+    const int nq = gj >= tile.ys ? max(0, min(4, tile.ye - gj)) : 0;
+    const uint32_t region = rows_in<RW>(rr0, tile.xs - tile.x0 + kH, tile.xe - tile.x0 + kH);
+    const uint32_t stored = lane >= 1 && lane <= 30 && nq > 0 ? region & rows_in<RW>(rr0, kH, B::kRows - kH) : 0u;
+    const Coefs ks = coefs_in(meta, nq > 0);
+    const bool ragged = ((tile.ye - tile.ys) & 3) != 0 && tile.y0 - kH + kBox > tile.ye;
+    const int2 recs = a.rec_tile != nullptr ? a.rec_tile[walk.t] : make_int2(0, 0);
+    const ptrdiff_t off = (ptrdiff_t)tile.plane * 2 * (ptrdiff_t)Np + (ptrdiff_t)gi0 * a.pitch + gj;
+    for (int t = max(1, a.m_hi - steps + 1); t <= a.T; ++t) {
+      const int m = a.m_hi - t + 1;
+      // the frame whose residuals enter lam^m
+      const int frame = (m - 1) % a.stride == 0 ? (m - 1) / a.stride : -1;
+      const bool dense = frame >= 0 && a.record == kRecordFields;
+      float* lc = (t & 1) ? lev0 : lev1;
+      float* lp = (t & 1) ? lev1 : lev0;
+      if (frame >= 0 && recs.y > 0) {  // lam^m = ... - (lam^{m+2} - g) + ...
+        const size_t o = ((size_t)tile.inst * a.nt_out + frame) * a.nrec;
+        for (int e = tid; e < recs.y; e += NT) {
+          const int2 v = a.rec_ent[recs.x + e];
+          atomicAdd(&lp[v.x], -gs * a.g_x[o + v.y]);
+          atomicAdd(&lp[B::kPlane + v.x], -gs * a.g_y[o + v.y]);
+        }
+        __syncthreads();
+      }
+      const float* c0 = lc + o0;  // lam^{m+1}
+      float* p0 = lp + o0;        // lam^{m+2}, becomes lam^m
+      float* out = t == a.T ? a.out_last : (t == a.T - 1 ? a.out_before : nullptr);
+      const uint32_t st = out != nullptr ? stored : 0u;
+      // cells with an imaging pair; the others' u is taken as zero
+      const uint32_t im = m <= steps - 1 ? stored : 0u;
+      float* out0 = out + off;
+      float* out1 = out0 + Np;
+      const float* u0 = a.u_base + (ptrdiff_t)(m - a.m_base) * (ptrdiff_t)a.u_stride + off;
+      const float* u1 = u0 + Np;
+      float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      auto rows = [&](auto plain) {
+        constexpr bool PLAIN = decltype(plain)::value;
+        auto load_u = [&](int r, float4& x, float4& y) {
+          x = y = make_float4(0.f, 0.f, 0.f, 0.f);
+          if ((im >> r) & 1u) {
+            x = __ldcg(reinterpret_cast<const float4*>(u0));
+            y = __ldcg(reinterpret_cast<const float4*>(u1));
+          }
+          u0 += a.pitch;
+          u1 += a.pitch;
+        };
+        float4 ux4, uy4, nx4, ny4;
+        load_u(0, nx4, ny4);
+        Row t0 = load_row(c0 - kBox), t1 = load_row(c0 + B::kPlane - kBox);
+        Row m0 = load_row(c0), m1 = load_row(c0 + B::kPlane);
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+          ux4 = nx4;
+          uy4 = ny4;
+          if (r + 1 < RW) load_u(r + 1, nx4, ny4);
+          const Row b0 = load_row(c0 + (r + 1) * kBox), b1 = load_row(c0 + B::kPlane + (r + 1) * kBox);
+          if (PLAIN || ((region >> r) & 1u)) {  // (rows outside the region stay zero)
+            const float4 pv0 = *reinterpret_cast<const float4*>(p0 + r * kBox);
+            const float4 pv1 = *reinterpret_cast<const float4*>(p0 + B::kPlane + r * kBox);
+            const float q0[4] = {pv0.x, pv0.y, pv0.z, pv0.w}, q1[4] = {pv1.x, pv1.y, pv1.z, pv1.w};
+            const float ux[4] = {ux4.x, ux4.y, ux4.z, ux4.w}, uy[4] = {uy4.x, uy4.y, uy4.z, uy4.w};
+            float v0[4], v1[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const Sums sx = sums_of(t0, m0, b0, q), sy = sums_of(t1, m1, b1, q);
+              oper<false>(ks, sx, sy, v0[q], v1[q]);
+              acc[0] = fmaf(ux[q], sx.xx, acc[0]);
+              acc[1] = fmaf(uy[q], sy.yy, acc[1]);
+              acc[2] = fmaf(ux[q], sy.xy, fmaf(uy[q], sx.xy, acc[2]));
+              acc[3] = fmaf(uy[q], sx.xx, fmaf(ux[q], fmaf(0.5f, sx.xy, sy.xx), acc[3]));
+              acc[4] = fmaf(ux[q], sy.yy, fmaf(uy[q], fmaf(0.5f, sy.xy, sx.yy), acc[4]));
+              acc[5] = fmaf(uy[q], sy.xx, fmaf(ux[q], sx.yy, acc[5]));
+              // (quads outside the region stay zero: their lanes' coefficients are)
+              v0[q] = leap(m0.w[q + 1], q0[q], v0[q]);
+              v1[q] = leap(m1.w[q + 1], q1[q], v1[q]);
+            }
+            if (!PLAIN && dense) {
+              const size_t o = ((size_t)tile.plane * a.nt_out + frame) * N + (size_t)(gi0 + r) * ny + gj;
+#pragma unroll
+              for (int q = 0; q < 4; ++q)
+                if (q < nq) {
+                  v0[q] = fmaf(gs, a.g_x[o + q], v0[q]);
+                  v1[q] = fmaf(gs, a.g_y[o + q], v1[q]);
+                }
+            }
+            if (!PLAIN && ragged) {  // the region's last column is inside a quad
+              mask_q(v0, nq);
+              mask_q(v1, nq);
+            }
+            const float4 n0 = make_float4(v0[0], v0[1], v0[2], v0[3]), n1 = make_float4(v1[0], v1[1], v1[2], v1[3]);
+            *reinterpret_cast<float4*>(p0 + r * kBox) = n0;
+            *reinterpret_cast<float4*>(p0 + B::kPlane + r * kBox) = n1;
+            if ((st >> r) & 1u) {
+              *reinterpret_cast<float4*>(out0) = n0;
+              *reinterpret_cast<float4*>(out1) = n1;
+            }
+          }
+          out0 += a.pitch;
+          out1 += a.pitch;
+          t0 = m0; t1 = m1; m0 = b0; m1 = b1;
+        }
+      };
+      if (region != 0 && rows_in<RW>(rr0, t, B::kRows - t) != 0) {
+        if (region == (1u << RW) - 1u && !ragged && !dense) rows(BoolC<true>{});
+        else rows(BoolC<false>{});
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {  // TwoSum(hi, acc)
+          const float s = hi[q] + acc[q];
+          const float bp = s - hi[q];
+          lo[q] += (hi[q] - (s - bp)) + (acc[q] - bp);
+          hi[q] = s;
+        }
+      }
+      __syncthreads();  // lam^m is complete
+    }
+  }
+  if (tid == 0 && pipe_failed(&guard)) pipe_drain(bar, 1, &guard);
+  flush(per_shot ? acc_shot : 0);
+}
+
+// ------------------------------------------------- receivers of the tiles
+// The receivers whose cells lie in a tile with its halo, for every tile of a
+// call: tile[t] = (first entry, entries), an entry = (cell in the tile's
+// planes, receiver number).  Counted, given room and filled by three small
+// kernels (the order inside a tile does not matter).
+struct RecPlace {  // the tiles (at most 2 x 2) around a cell
+  int x0, x1, y0, y1, base, tiles_y, oi, oj;
+  __device__ __forceinline__ bool find(int idx, int s, int nx, int ny, int H, int tiles_x, int ty, const int4* box) {
+    if (idx < 0 || (int64_t)idx >= (int64_t)nx * ny) return false;  // out of range: ignored
+    int gi = idx / ny, gj = idx - gi * ny;
+    if (box != nullptr) {
+      const int4 r = box[2 * s], m = box[2 * s + 1];
+      if (gi < r.x || gi >= r.z || gj < r.y || gj >= r.w) return false;
+      gi -= r.x;
+      gj -= r.y;
+      base = m.x;
+      tiles_y = m.y;
+      tiles_x = (r.z - r.x + H - 1) / H;
+    } else {
+      base = s * tiles_x * ty;
+      tiles_y = ty;
+    }
+    oi = gi + kH;
+    oj = gj + kH;
+    x1 = min(oi / H, tiles_x - 1);
+    x0 = max((oi - (H + 2 * kH) + H) / H, 0);  // first tile whose last row reaches the cell
+    y1 = min(oj / kBlkCols, tiles_y - 1);
+    y0 = max((oj - kBox + kBlkCols) / kBlkCols, 0);
+    return true;
+  }
+};
+
+template <bool FILL>
+__global__ void rec_tiles_kernel(const int32_t* __restrict__ rec_idx, int S, int nrec, int nx, int ny, int H,
+                                 int tiles_x, int tiles_y, const int4* __restrict__ box, int* __restrict__ count,
+                                 int2* __restrict__ tile, int2* __restrict__ ent) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= S * nrec) return;
+  const int s = e / nrec;
+  RecPlace p;
+  if (!p.find(rec_idx[e], s, nx, ny, H, tiles_x, tiles_y, box)) return;
+  for (int xt = p.x0; xt <= p.x1; ++xt)
+    for (int yt = p.y0; yt <= p.y1; ++yt) {
+      const int rr = p.oi - xt * H, cc = p.oj - yt * kBlkCols;
+      if (rr < 0 || rr >= H + 2 * kH || cc < 0 || cc >= kBox) continue;
+      const int t = p.base + xt * p.tiles_y + yt;
+      if (FILL) ent[tile[t].x + atomicAdd(&tile[t].y, 1)] = make_int2(rr * kBox + cc, e - s * nrec);
+      else atomicAdd(&count[t], 1);
+    }
+}
+
+__global__ void rec_base_kernel(int* __restrict__ count, int ntiles, int2* __restrict__ tile) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= ntiles) return;
+  const int n = count[t];
+  tile[t] = make_int2(n > 0 ? atomicAdd(&count[ntiles], n) : 0, 0);
+}
+
+// ----------------------------------------------------------------- host
+PFN_cuTensorMapEncodeTiled_v12000 blk_encode_fn() {
+  static std::mutex mu;
+  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
+  std::lock_guard<std::mutex> lock(mu);
+  if (fn == nullptr) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
+            cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
+  }
+  return fn;
+}
+
+// Tensor map over S shots of [comp][nx][pitch] floats, columns ny .. pitch - 1
+// read as zeros: dims (ny, nx, 2 S).
+bool blk_map(CUtensorMap* m, const float* base, int nx, int ny, int pitch, int S, int bw, int bh) {
+  auto fn = blk_encode_fn();
+  if (fn == nullptr || base == nullptr) return false;
+  const cuuint64_t dims[3] = {(cuuint64_t)ny, (cuuint64_t)nx, (cuuint64_t)2 * S};
+  const cuuint64_t strides[2] = {(cuuint64_t)pitch * 4, (cuuint64_t)nx * pitch * 4};
+  const cuuint32_t box[3] = {(cuuint32_t)bw, (cuuint32_t)bh, 2};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+int blk_sms() {
+  static int n = [] {
+    int dev = 0, v = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0)
+      return 1;
+    return v;
+  }();
+  return n;
+}
+
+
+template <int W, int RW, int CTAS, bool INST, bool SWAP>
+cudaError_t fwd_t(const BlkFwd& a, int* err, cudaStream_t st) {
+  using B = BlkTile<W, RW>;
+  constexpr size_t smem = B::kBytes;
+  static std::once_flag once;
+  static cudaError_t ready = cudaSuccess;
+  std::call_once(once, [] {
+    ready = cudaFuncSetAttribute(blk_fwd_kernel<W, RW, INST, SWAP, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  });
+  if (ready != cudaSuccess) return ready;
+  const int planes = INST ? 1 : a.S;
+  const float* any = a.cur ? a.cur : a.out[a.T];  // (a level that is zero is not loaded)
+  CUtensorMap cm, pm;
+  if (!blk_map(&cm, any, a.nx, a.ny, a.pitch, planes, kBox, B::kRows) ||
+      !blk_map(&pm, a.prev ? a.prev : any, a.nx, a.ny, a.pitch, planes, kBox, B::kRows))
+    return cudaErrorNotSupported;
+  const int tiles_x = (a.nx + B::kUse - 1) / B::kUse, tiles_y = (a.ny + kBlkCols - 1) / kBlkCols;
+  const int ntiles = INST ? a.inst.ntiles : a.S * tiles_x * tiles_y;
+  const int grid = ntiles < CTAS * blk_sms() ? ntiles : CTAS * blk_sms();
+  const double cells = INST ? (double)ntiles * B::kUse * kBlkCols : (double)a.S * a.nx * a.ny;
+  int stores = 0;
+  for (int t = 0; t <= a.T; ++t) stores += a.out[t] != nullptr ? 1 : 0;
+  return tracked_launch(kProfForward, st, [&] {
+    launch_step_kernel(blk_fwd_kernel<W, RW, INST, SWAP, CTAS>, dim3(grid), dim3(32 * W), smem, st, a.chained != 0, a, cm, pm,
+                       tiles_x, tiles_y, ntiles, err);
+  }, cells * 8.0 * (stores + (a.cur ? 1 : 0) + (a.prev ? 1 : 0)));
+}
+
+template <int W, int RW, int CTAS, bool INST>
+cudaError_t adj_t(const BlkAdj& a, int* err, cudaStream_t st) {
+  using B = BlkTile<W, RW>;
+  constexpr size_t smem = B::kBytes;
+  static std::once_flag once;
+  static cudaError_t ready = cudaSuccess;
+  std::call_once(once, [] {
+    ready = cudaFuncSetAttribute(blk_adj_kernel<W, RW, INST, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  });
+  if (ready != cudaSuccess) return ready;
+  const int planes = INST ? 1 : a.S;
+  const float* any = a.cur ? a.cur : a.out_last;  // (a level that is zero is not loaded)
+  CUtensorMap cm, pm;
+  if (!blk_map(&cm, any, a.nx, a.ny, a.pitch, planes, kBox, B::kRows) ||
+      !blk_map(&pm, a.prev ? a.prev : any, a.nx, a.ny, a.pitch, planes, kBox, B::kRows))
+    return cudaErrorNotSupported;
+  const int tiles_x = (a.nx + B::kUse - 1) / B::kUse, tiles_y = (a.ny + kBlkCols - 1) / kBlkCols;
+  const int ntiles = INST ? a.inst.ntiles : a.S * tiles_x * tiles_y;
+  const int all = CTAS * blk_sms(), slots = all < kTiledRowsPerShot ? all : kTiledRowsPerShot;  // a partial row each
+  const int grid = ntiles < slots ? ntiles : slots;
+  const double cells = INST ? (double)ntiles * B::kUse * kBlkCols : (double)a.S * a.nx * a.ny;
+  return tracked_launch(kProfAdjoint, st, [&] {
+    launch_step_kernel(blk_adj_kernel<W, RW, INST, CTAS>, dim3(grid), dim3(32 * W), smem, st, a.chained != 0, a, cm, pm,
+                       tiles_x, tiles_y, ntiles, err);
+  }, cells * 8.0 * (a.T + (a.T > 1 ? 2 : 1) + (a.cur ? 1 : 0) + (a.prev ? 1 : 0)));
+}
+
+}  // namespace
+
+// Tile geometries.  kBlkTall: eight warps of six rows, two CTAs per SM (one
+// loads its tile while the other computes), 40 of 48 rows stored; the best
+// use of the FP32 pipe, for grids of several tiles per SM.  kBlkShort:
+// sixteen warps of two rows, one CTA per SM, 24 of 32 rows stored: a tile
+// takes half as long, for grids whose tall tiles would leave SMs idle or a
+// last wave nearly empty.  (Measured, 8 x 640 x 720 forward: 50 us per
+// launch of four steps tall, 66 short; 512^2, one shot, forward and adjoint
+// launch together: 50 us tall, 31 short.)
+int blk_tile_rows(int geo) { return geo == kBlkTall ? 8 * 6 - 2 * kH : 16 * 2 - 2 * kH; }
+
+size_t blk_tiles(int geo, int nx, int ny) {
+  const int h = blk_tile_rows(geo);
+  return (size_t)((nx + h - 1) / h) * ((ny + kBlkCols - 1) / kBlkCols);
+}
+
+// The geometry whose waves of tiles take less time (measured us per wave of
+// 152 SMs; from sizes alone, as the workspace layout depends on it).
+int blk_geometry(int nx, int ny, int S) {
+  const double sms = 152.0;
+  const double tall = S * (double)blk_tiles(kBlkTall, nx, ny), low = S * (double)blk_tiles(kBlkShort, nx, ny);
+  const double t_tall = tall <= sms ? 11.0 : 15.0 * std::ceil(tall / (2.0 * sms));
+  return t_tall <= 7.2 * std::ceil(low / sms) ? kBlkTall : kBlkShort;
+}
+
+bool blk_available() { return blk_encode_fn() != nullptr; }
+
+size_t blk_rec_bytes(size_t ntiles, int S, int nrec) {
+  return (ntiles + 2) / 2 * 8 + ntiles * sizeof(int2) + 4 * (size_t)S * nrec * sizeof(int2);
+}
+
+cudaError_t launch_rec_tiles(int geo, const int32_t* rec_idx, int S, int nrec, int nx, int ny, const int4* box,
+                             size_t ntiles, void* ws, const int2** tile, const int2** ent, cudaStream_t st) {
+  const int H = blk_tile_rows(geo);
+  int* count = static_cast<int*>(ws);
+  int2* tl = reinterpret_cast<int2*>(static_cast<char*>(ws) + (ntiles + 2) / 2 * 8);
+  int2* en = tl + ntiles;
+  *tile = tl;
+  *ent = en;
+  cudaError_t e = cudaMemsetAsync(count, 0, (ntiles + 1) * sizeof(int), st);
+  if (e != cudaSuccess) return e;
+  const int n = S * nrec, tx = (nx + H - 1) / H, ty = (ny + kBlkCols - 1) / kBlkCols;
+  const int nt = (int)ntiles;
+  e = tracked_launch(kProfOther, st, [&] {
+    rec_tiles_kernel<false><<<(n + 255) / 256, 256, 0, st>>>(rec_idx, S, nrec, nx, ny, H, tx, ty, box, count, tl, en);
+  });
+  if (e != cudaSuccess) return e;
+  e = tracked_launch(kProfOther, st, [&] { rec_base_kernel<<<(nt + 255) / 256, 256, 0, st>>>(count, nt, tl); });
+  if (e != cudaSuccess) return e;
+  return tracked_launch(kProfOther, st, [&] {
+    rec_tiles_kernel<true><<<(n + 255) / 256, 256, 0, st>>>(rec_idx, S, nrec, nx, ny, H, tx, ty, box, count, tl, en);
+  });
+}
+
+cudaError_t launch_blk_fwd(const BlkFwd& a, int* err, cudaStream_t st) {
+  if (a.inst.tiles != nullptr) return fwd_t<8, 6, 2, true, false>(a, err, st);
+  if (a.geo == kBlkShort)
+    return a.swap ? fwd_t<16, 2, 1, false, true>(a, err, st) : fwd_t<16, 2, 1, false, false>(a, err, st);
+  return a.swap ? fwd_t<8, 6, 2, false, true>(a, err, st) : fwd_t<8, 6, 2, false, false>(a, err, st);
+}
+
+cudaError_t launch_blk_adj(const BlkAdj& a, int* err, cudaStream_t st) {
+  if (a.inst.tiles != nullptr) return adj_t<8, 6, 2, true>(a, err, st);
+  if (a.geo == kBlkShort) return adj_t<16, 2, 1, false>(a, err, st);
+  return adj_t<8, 6, 2, false>(a, err, st);
+}
+
+}  // namespace ernn

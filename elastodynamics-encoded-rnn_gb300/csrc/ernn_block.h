@@ -1,0 +1,79 @@
+// Time-blocked tile kernels (ernn_block.cu): up to four time steps per launch.
+// Internal to the library.
+#pragma once
+
+#include "ernn_launch.h"
+#include "ernn_tma.h"
+
+namespace ernn {
+
+constexpr int kBlkSteps = 4;       // most time steps of one launch (and halo rows / columns of a tile)
+constexpr int kBlkCols = 120;      // columns of a tile (a warp's 128 less one quad each side)
+
+// Forward: u^{i+1} .. u^{i+T} from (u^i, u^{i-1}).
+struct BlkFwd {
+  int geo;                         // tile geometry (blk_geometry)
+  int swap;                        // rounding order of the operator's first two terms (oper)
+  int nx, ny, pitch, S, nt, i, T;  // pitch: floats between rows of a state (ny rounded up to 4)
+  const float* cur;                // u^i, nullptr: zero
+  const float* prev;               // u^{i-1}, nullptr: zero
+  float* out[kBlkSteps + 1];       // where u^{i+t} goes (t = 0: a copy of u^i), or nullptr
+  // dense history or receiver traces: frame of u^{i+t} in frame[t], or -1
+  float* rec_x;
+  float* rec_y;
+  int frame[kBlkSteps + 1];
+  int nt_out, record, nrec;
+  int vec;                         // dense history rows start on 16-byte boundaries
+  const int2* rec_tile;            // receivers of every tile (launch_rec_tiles), or nullptr
+  const int2* rec_ent;
+  const Coef* coef;
+  int coef_stride;
+  const float* src_signal;
+  const float* src_map;
+  const int32_t* src_origin;
+  int bx, by, src_comp;
+  int chained;
+  InstTiles inst;
+};
+
+// Adjoint: lam^m, m = m_hi down to m_hi - T + 1, from (lam^{m_hi+1},
+// lam^{m_hi+2}), and the imaging sums of the pairs (lam^{m+1}, u^m).
+struct BlkAdj {
+  int geo;
+  int nx, ny, pitch, S, nt, m_hi, T;
+  const float* cur;     // lam^{m_hi+1}, nullptr: zero
+  const float* prev;    // lam^{m_hi+2}, nullptr: zero
+  float* out_last;      // lam^{m_hi-T+1}
+  float* out_before;    // lam^{m_hi-T+2} (T >= 2)
+  // u^m = u_base + (m - m_base) u_stride floats; the pair of m == nt vanishes
+  const float* u_base;
+  size_t u_stride;
+  int m_base;
+  const float* g_x;
+  const float* g_y;
+  int stride, nt_out, record, nrec;
+  const int2* rec_tile;
+  const int2* rec_ent;
+  const Coef* coef;
+  int coef_stride;
+  double* partials;
+  int chained;
+  InstTiles inst;
+};
+
+// Tile geometry of a grid problem (instances: kBlkTall), rows it stores,
+// tiles of an nx x ny grid.
+constexpr int kBlkTall = 0, kBlkShort = 1;
+int blk_geometry(int nx, int ny, int S);
+int blk_tile_rows(int geo);
+size_t blk_tiles(int geo, int nx, int ny);
+// Receivers of the tiles of a call: room for `ntiles` tiles, and the table
+// (box: instances, else nullptr).
+size_t blk_rec_bytes(size_t ntiles, int S, int nrec);
+cudaError_t launch_rec_tiles(int geo, const int32_t* rec_idx, int S, int nrec, int nx, int ny, const int4* box,
+                             size_t ntiles, void* ws, const int2** tile, const int2** ent, cudaStream_t st);
+bool blk_available();  // the driver exposes the tensor-map encoder
+cudaError_t launch_blk_fwd(const BlkFwd& a, int* err, cudaStream_t st);
+cudaError_t launch_blk_adj(const BlkAdj& a, int* err, cudaStream_t st);
+
+}  // namespace ernn

@@ -41,7 +41,7 @@ cudaError_t launch_tile_flags(int mode, const int32_t* rec_idx, int S, int nrec,
 constexpr int kMaxInstances = 256;
 constexpr int kInstTileRows = 16;  // tile rows of every instance kernel (scalar constants)
 struct InstDesc {
-  int count;
+  int count, tile_rows, tile_cols;
   int id[kMaxInstances], x0[kMaxInstances], y0[kMaxInstances], nx[kMaxInstances];
   int ny[kMaxInstances], nt[kMaxInstances], base[kMaxInstances];
 };

@@ -1,0 +1,65 @@
+"""Time-blocked tile kernels (up to four steps per launch) against the plain
+per-step kernels at the sizes where a tile ends: stored rows of a tile (24 and
+40), its 120 columns, halo columns, quads cut by the grid's last column, step
+counts that leave launches of one to three steps, checkpoints on and off them.
+
+Both evaluate the same sequence of rounded operations per cell, so the
+recorded fields are equal bit for bit; the gradient's six sums group their
+FP32 partial sums differently (relative 2^-24 sqrt(cells per partial sum),
+below 1e-5).  GPU only."""
+import numpy as np
+import pytest
+import torch
+
+import ernn_gb300 as E
+from cases import random_case, rel
+from oracle import oracle as O
+from test_gpu_parity import DEV, GRAD_TOL, run_oracle, to_geometry, weights
+
+pytestmark = pytest.mark.gpu
+
+
+def run(case, wx, wy, path, ckpt_k):
+    geom = to_geometry(case, path=path, ckpt_k=ckpt_k)
+    C = torch.tensor(case.C, dtype=torch.float32, device=DEV, requires_grad=True)
+    ux, uy = E.propagate(C, torch.tensor(case.rho, dtype=torch.float32, device=DEV), geom)
+    used = E.load_library().ernn_last_path()
+    ((ux.double() * torch.as_tensor(wx, device=DEV)).sum() + (uy.double() * torch.as_tensor(wy, device=DEV)).sum()).backward()
+    return ux.detach().cpu().numpy(), uy.detach().cpu().numpy(), C.grad.double().cpu().numpy(), used
+
+
+SIZES = [(24, 41), (25, 119), (23, 121), (40, 122), (41, 127), (48, 129), (3, 243), (97, 250), (130, 361)]
+
+
+@pytest.mark.parametrize("nx,ny", SIZES)
+@pytest.mark.parametrize("record", [O.RECORD_FIELDS, O.RECORD_RECEIVERS])
+@pytest.mark.parametrize("nt,ckpt_k", [(41, None), (42, 7), (30, 1), (33, 6)])
+def test_same_fields_as_the_plain_kernels(nx, ny, record, nt, ckpt_k):
+    case = random_case(nx=nx, ny=ny, nt=nt, S=2, stride=1 + nt % 2, record=record, nrec=min(40, nx * ny),
+                       src_comp=nx % 2)
+    wx, wy = weights(case)
+    ax, ay, ag, used = run(case, wx, wy, E.PATH_AUTO, ckpt_k)
+    assert used == E.PATH_TILED  # ny % 4 != 0: not the resident path's
+    bx, by, bg, _ = run(case, wx, wy, E.PATH_STEP, ckpt_k)
+    assert np.array_equal(ax, bx) and np.array_equal(ay, by)
+    assert rel(ag, bg) <= 1e-5, rel(ag, bg)
+
+
+def test_every_cell_a_receiver():
+    case = random_case(nx=50, ny=126, nt=20, S=2, record=O.RECORD_RECEIVERS, nrec=50 * 126, stride=2)
+    wx, wy = weights(case)
+    ax, ay, ag, used = run(case, wx, wy, E.PATH_AUTO, 6)
+    bx, by, bg, _ = run(case, wx, wy, E.PATH_STEP, 6)
+    assert used == E.PATH_TILED
+    assert np.array_equal(ax, bx) and np.array_equal(ay, by)
+    assert rel(ag, bg) <= 1e-5, rel(ag, bg)
+
+
+def test_large_odd_grid_vs_fp64_oracle():
+    case = random_case(nx=330, ny=437, nt=60, S=5, record=O.RECORD_RECEIVERS, nrec=60)
+    wx, wy = weights(case)
+    ax, ay, ag, used = run(case, wx, wy, E.PATH_AUTO, 9)
+    assert used == E.PATH_TILED
+    ox, oy, og = run_oracle(case, wx, wy)
+    assert rel(ax, ox) <= 1e-5 and rel(ay, oy) <= 1e-5
+    assert rel(ag, og) <= GRAD_TOL, rel(ag, og)
