@@ -442,24 +442,40 @@ __global__ void __launch_bounds__(32 * W, CTAS)
   // tiles as FP32 pairs (TwoSum; the sum does not depend on how the steps
   // are split over launches), FP64 across warps and launches.
   float hi[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, lo[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  // (the lanes' pairs are added as pairs: a warp's FP64 addition occupies
-  // this part's FP64 pipe for 16 cycles and more, and thirty per warp took
-  // longer than a step of a small tile)
+  // The lanes' pairs are added as pairs (a warp's FP64 addition occupies this
+  // part's FP64 pipe for 16 cycles and more, and thirty of them took longer
+  // than a step of a small tile), and each exchange halves the values a lane
+  // still carries: 4 + 2 + 1 additions leave one value in every group of four
+  // lanes, two more sum it over the group.
   auto flush = [&](int shot) {  // CTA-uniform
+    float h[8], l[8];
 #pragma unroll
-    for (int q = 0; q < 6; ++q) {
-      float h = hi[q], l = lo[q];
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        const float h2 = __shfl_down_sync(kFull, h, off), l2 = __shfl_down_sync(kFull, l, off);
-        const float s = h + h2, bp = s - h;
-        l = (l + l2) + ((h - (s - bp)) + (h2 - bp));
-        h = s;
-      }
-      if (lane == 0) red[w][q] = make_float2(h, l);
-      hi[q] = 0.f;
-      lo[q] = 0.f;
+    for (int q = 0; q < 8; ++q) {
+      h[q] = q < 6 ? hi[q < 6 ? q : 0] : 0.f;
+      l[q] = q < 6 ? lo[q < 6 ? q : 0] : 0.f;
     }
+    auto add = [&](int q, float h2, float l2) {
+      const float s = h[q] + h2, bp = s - h[q];
+      l[q] = (l[q] + l2) + ((h[q] - (s - bp)) + (h2 - bp));
+      h[q] = s;
+    };
+#pragma unroll
+    for (int n = 4; n >= 1; n >>= 1) {  // lanes with bit 4 n set keep values n .. 2 n - 1
+      const bool up = (lane & (4 * n)) != 0;
+#pragma unroll
+      for (int q = 0; q < n; ++q) {
+        const float sh = up ? h[q] : h[q + n], sl = up ? l[q] : l[q + n];
+        h[q] = up ? h[q + n] : h[q];
+        l[q] = up ? l[q + n] : l[q];
+        add(q, __shfl_xor_sync(kFull, sh, 4 * n), __shfl_xor_sync(kFull, sl, 4 * n));
+      }
+    }
+    add(0, __shfl_xor_sync(kFull, h[0], 2), __shfl_xor_sync(kFull, l[0], 2));
+    add(0, __shfl_xor_sync(kFull, h[0], 1), __shfl_xor_sync(kFull, l[0], 1));
+    // (bits 4, 3, 2 of the lane: bits 2, 1, 0 of the value)
+    if ((lane & 3) == 0 && lane < 24) red[w][lane >> 2] = make_float2(h[0], l[0]);
+#pragma unroll
+    for (int q = 0; q < 6; ++q) hi[q] = lo[q] = 0.f;
     __syncthreads();
     if (tid < 6) {
       double v = 0.0;
@@ -765,27 +781,29 @@ cudaError_t adj_t(const BlkAdj& a, int* err, cudaStream_t st) {
 }  // namespace
 
 // Tile geometries.  kBlkTall: eight warps of six rows, two CTAs per SM (one
-// loads its tile while the other computes), 40 of 48 rows stored; the best
+// loads its tile while the other computes), 40 of 48 rows stored: the best
 // use of the FP32 pipe, for grids of several tiles per SM.  kBlkShort:
-// sixteen warps of two rows, one CTA per SM, 24 of 32 rows stored: a tile
-// takes half as long, for grids whose tall tiles would leave SMs idle or a
-// last wave nearly empty.  (Measured, 8 x 640 x 720 forward: 50 us per
-// launch of four steps tall, 66 short; 512^2, one shot, forward and adjoint
-// launch together: 50 us tall, 31 short.)
-int blk_tile_rows(int geo) { return geo == kBlkTall ? 8 * 6 - 2 * kH : 16 * 2 - 2 * kH; }
+// sixteen warps of two rows, one CTA per SM, 24 of 32 rows stored, and
+// kBlkFlat: sixteen warps of one row, 8 of 16 stored, whose tiles take a half
+// and a quarter as long, for grids that would leave SMs idle.
+int blk_tile_rows(int geo) { return (geo == kBlkTall ? 8 * 6 : geo == kBlkShort ? 16 * 2 : 16) - 2 * kH; }
 
 size_t blk_tiles(int geo, int nx, int ny) {
   const int h = blk_tile_rows(geo);
   return (size_t)((nx + h - 1) / h) * ((ny + kBlkCols - 1) / kBlkCols);
 }
 
-// The geometry whose waves of tiles take less time (measured us per wave of
-// 152 SMs; from sizes alone, as the workspace layout depends on it).
+// The geometry whose waves of tiles take the least time: us per wave on 152
+// SMs, mean of a forward and an adjoint launch of four steps (measured at
+// one shot of 301^2 and 512^2, three of 501 x 389, eight of 640 x 720).  From
+// sizes alone, as the workspace layout depends on it.
 int blk_geometry(int nx, int ny, int S) {
   const double sms = 152.0;
-  const double tall = S * (double)blk_tiles(kBlkTall, nx, ny), low = S * (double)blk_tiles(kBlkShort, nx, ny);
-  const double t_tall = tall <= sms ? 11.0 : 15.0 * std::ceil(tall / (2.0 * sms));
-  return t_tall <= 7.2 * std::ceil(low / sms) ? kBlkTall : kBlkShort;
+  auto tiles = [&](int geo) { return S * (double)blk_tiles(geo, nx, ny); };
+  const double tall = tiles(kBlkTall) <= sms ? 21.0 : 20.0 * std::ceil(tiles(kBlkTall) / (2.0 * sms));
+  const double low = 9.4 * std::ceil(tiles(kBlkShort) / sms), flat = 5.0 * std::ceil(tiles(kBlkFlat) / sms);
+  if (flat < low && flat < tall) return kBlkFlat;
+  return low < tall ? kBlkShort : kBlkTall;
 }
 
 bool blk_available() { return blk_encode_fn() != nullptr; }
@@ -819,6 +837,8 @@ cudaError_t launch_rec_tiles(int geo, const int32_t* rec_idx, int S, int nrec, i
 
 cudaError_t launch_blk_fwd(const BlkFwd& a, int* err, cudaStream_t st) {
   if (a.inst.tiles != nullptr) return fwd_t<8, 6, 2, true, false>(a, err, st);
+  if (a.geo == kBlkFlat)
+    return a.swap ? fwd_t<16, 1, 1, false, true>(a, err, st) : fwd_t<16, 1, 1, false, false>(a, err, st);
   if (a.geo == kBlkShort)
     return a.swap ? fwd_t<16, 2, 1, false, true>(a, err, st) : fwd_t<16, 2, 1, false, false>(a, err, st);
   return a.swap ? fwd_t<8, 6, 2, false, true>(a, err, st) : fwd_t<8, 6, 2, false, false>(a, err, st);
@@ -826,6 +846,7 @@ cudaError_t launch_blk_fwd(const BlkFwd& a, int* err, cudaStream_t st) {
 
 cudaError_t launch_blk_adj(const BlkAdj& a, int* err, cudaStream_t st) {
   if (a.inst.tiles != nullptr) return adj_t<8, 6, 2, true>(a, err, st);
+  if (a.geo == kBlkFlat) return adj_t<16, 1, 1, false>(a, err, st);
   if (a.geo == kBlkShort) return adj_t<16, 2, 1, false>(a, err, st);
   return adj_t<8, 6, 2, false>(a, err, st);
 }

@@ -63,7 +63,7 @@ struct BlkAdj {
 
 // Tile geometry of a grid problem (instances: kBlkTall), rows it stores,
 // tiles of an nx x ny grid.
-constexpr int kBlkTall = 0, kBlkShort = 1;
+constexpr int kBlkTall = 0, kBlkShort = 1, kBlkFlat = 2;
 int blk_geometry(int nx, int ny, int S);
 int blk_tile_rows(int geo);
 size_t blk_tiles(int geo, int nx, int ny);

@@ -28,7 +28,7 @@ def run(case, wx, wy, path, ckpt_k):
     return ux.detach().cpu().numpy(), uy.detach().cpu().numpy(), C.grad.double().cpu().numpy(), used
 
 
-SIZES = [(24, 41), (25, 119), (23, 121), (40, 122), (41, 127), (48, 129), (3, 243), (97, 250), (130, 361)]
+SIZES = [(8, 41), (17, 40 + 3), (24, 41), (25, 119), (23, 121), (40, 122), (41, 127), (48, 129), (3, 243), (97, 250), (130, 361)]
 
 
 @pytest.mark.parametrize("nx,ny", SIZES)
