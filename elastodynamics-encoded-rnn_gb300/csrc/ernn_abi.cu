@@ -22,6 +22,7 @@ constexpr double kPi = 3.14159265358979323846;
 // segment length of the resident reverse pass when the tape keeps every state
 constexpr int kResStoreAllSegment = 128;
 constexpr int kBlockMinCols = 40;
+constexpr double kBlockMaxFields = 1e6;
 inline size_t align_up(size_t v) { return (v + kAlign - 1) / kAlign * kAlign; }
 
 // Workspace plan of one problem.
@@ -45,17 +46,33 @@ struct Plan {
   size_t t_C, t_D, t_rec, s_LC, s_LD, s_rec;
 };
 
+// Grids that the plain per-step kernels took before the time-blocked ones:
+// odd rows, or a step of fewer than four 64 x 32 tiles per SM.
+inline bool plain_size(const ErnnProblem& p) {
+  return p.path == ERNN_PATH_AUTO && !(p.flags & ERNN_FLAG_INSTANCES) &&
+         (p.ny % 4 != 0 || tma_tiles(p.nx, p.ny, p.nshots) < 608);
+}
+
 // Problems of the time-blocked tile kernels, from sizes alone (the workspace
-// queries, the forward and the adjoint agree).  ERNN_PATH_AUTO takes rows of
-// any length from kBlockMinCols up (a warp spans 120 columns, so narrower
-// grids leave most lanes idle; the plain kernels take those); their states
-// are padded to 16-byte rows.  Where the cluster-resident path can run it
-// comes first.
+// queries, the forward and the adjoint agree).
+//  - Instances, and scalar constants on the tiled path: all of them.
+//  - ERNN_PATH_AUTO takes rows of any length from kBlockMinCols up (a warp
+//    spans 120 columns: narrower grids leave most lanes idle, the plain
+//    kernels take those); states of odd rows are padded to 16-byte rows.
+//    Where the cluster-resident path can run it comes first.
+//  - A degradation map: grids of the plain kernels' size.  On larger ones the
+//    TMA-fed kernels of one step are faster (8 x 512^2: 29 against 33 us per
+//    forward and adjoint step): the map, u's rows and the running gradient
+//    are read at every step either way, here from L2 by the threads.
+//  - Six constant planes: up to kBlockMaxFields cells, where launches set the
+//    time (301^2: 36.1 against 21.9 ms per 4001-step iteration).
 bool block_rule(const ErnnProblem& p) {
-  if (p.mode != kModeScalar) return false;
   if (p.flags & ERNN_FLAG_INSTANCES) return true;
-  if (p.path == ERNN_PATH_TILED) return p.ny % 4 == 0;
-  return p.path == ERNN_PATH_AUTO && p.ny >= kBlockMinCols && !resident_possible(p.mode, p.nx, p.ny);
+  if (p.path == ERNN_PATH_TILED) return p.mode == kModeScalar && p.ny % 4 == 0;
+  if (p.path != ERNN_PATH_AUTO || p.ny < kBlockMinCols) return false;
+  if (p.mode == kModeFields) return (double)p.nshots * p.nx * p.ny <= kBlockMaxFields;
+  if (p.mode == kModeDField) return plain_size(p);
+  return !resident_possible(p.mode, p.nx, p.ny);
 }
 
 // Upper bound of the tile-table entries of any placement of S instances on
@@ -76,7 +93,7 @@ Plan make_plan(const ErnnProblem& p) {
   pl.inst = (p.flags & ERNN_FLAG_INSTANCES) != 0;
   // instances share the canvas's one state plane
   pl.block = block_rule(p);
-  pl.geo = pl.inst ? kBlkTall : blk_geometry(p.nx, p.ny, p.nshots);
+  pl.geo = pl.inst ? kBlkTall : p.mode == kModeFields ? kBlkFlat : blk_geometry(p.nx, p.ny, p.nshots);
   pl.pitch = pl.block ? (p.ny + 3) / 4 * 4 : p.ny;
   pl.state_bytes = align_up((size_t)(pl.inst ? 1 : p.nshots) * 2 * p.nx * pl.pitch * sizeof(float));
   const dim3 g = step_grid(p.nx, p.ny, pl.inst ? 1 : p.nshots);
@@ -433,12 +450,12 @@ BlkFwd base_blk_fwd(const ErnnProblem& p, const Plan& pl, const ErnnInputs& in, 
   BlkFwd a;
   std::memset(&a, 0, sizeof(a));
   a.geo = pl.geo;
-  // grids below four 64 x 32 tiles per SM, and odd ones, keep the plain
-  // kernels' rounding order: their states agree with those bit for bit
-  a.swap = p.path == ERNN_PATH_AUTO && !pl.inst && (p.ny % 4 != 0 || tma_tiles(p.nx, p.ny, p.nshots) < 608);
+  a.plain_order = plain_size(p) ? 1 : 0;
   a.nx = p.nx; a.ny = p.ny; a.pitch = pl.pitch; a.S = p.nshots; a.nt = p.nt;
   a.nt_out = pl.nt_out; a.record = p.record; a.nrec = p.nrec;
   a.coef = coef; a.coef_stride = pl.ncoef > 1 ? 1 : 0;
+  a.field = p.mode == kModeFields ? in.C : in.D;
+  a.vec_field = p.ny % 4 == 0 && al16(a.field);
   a.src_signal = in.src_signal; a.src_map = in.src_map; a.src_origin = in.src_origin;
   a.bx = p.src_bx; a.by = p.src_by; a.src_comp = p.src_comp;
   a.inst = it;
@@ -491,7 +508,7 @@ int block_forward(const ErnnProblem& p, const Plan& pl, const ErnnInputs& in, co
     }
     if (ip != nullptr) a.inst.ntiles = ip->fwd_tiles(i);
     a.chained = i > 0;
-    ERNN_CUDA(launch_blk_fwd(a, &coef->err, st));
+    ERNN_CUDA(launch_blk_fwd(p.mode, a, &coef->err, st));
     prev = T > 1 ? a.out[T - 1] : cur;
     cur = a.out[T];
     i += T;
@@ -518,6 +535,9 @@ int block_adjoint(const ErnnProblem& p, const Plan& pl, const ErnnInputs& in, co
                                at(scratch, pl.s_rec), &b.rec_tile, &b.rec_ent, st));
   b.coef = coef;
   b.coef_stride = a.coef_stride;
+  b.field = a.field;
+  b.vec_field = a.vec_field;
+  b.gacc = fat(scratch, pl.s_gacc);
   b.partials = partials;
   b.inst = itab;
   float* const pool[4] = {fat(scratch, pl.s_LA), fat(scratch, pl.s_LB), fat(scratch, pl.s_LC), fat(scratch, pl.s_LD)};
@@ -544,7 +564,7 @@ int block_adjoint(const ErnnProblem& p, const Plan& pl, const ErnnInputs& in, co
         if (ip != nullptr) a.inst.ntiles = ip->fwd_tiles(i);
         a.chained = chained ? 1 : 0;
         chained = true;
-        ERNN_CUDA(launch_blk_fwd(a, &coef->err, st));
+        ERNN_CUDA(launch_blk_fwd(p.mode, a, &coef->err, st));
         i += T;
       }
       b.u_base = slot(0);
@@ -559,7 +579,7 @@ int block_adjoint(const ErnnProblem& p, const Plan& pl, const ErnnInputs& in, co
       if (ip != nullptr) b.inst.ntiles = ip->adj_tiles(m - T + 1);
       b.chained = chained ? 1 : 0;
       chained = true;
-      ERNN_CUDA(launch_blk_adj(b, &coef->err, st));
+      ERNN_CUDA(launch_blk_adj(p.mode, b, &coef->err, st));
       b.prev = T > 1 ? b.out_before : b.cur;
       b.cur = b.out_last;
       m -= T;
@@ -832,6 +852,10 @@ static int adjoint_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPl
   if (block) {
     g_last_path.store(ERNN_PATH_TILED, std::memory_order_relaxed);
     if ((rc = block_adjoint(*p, pl, *in, ip, itab, coef, g_ux, g_uy, tape, scratch, partials, st))) return rc;
+    if (p->mode != kModeScalar) {
+      ERNN_CUDA(launch_finalize_fields(p->mode, gacc, p->nshots, (int)pl.N, coef, grad_field, st));
+      return ERNN_OK;
+    }
     if (pl.ncoef > 1)
       ERNN_CUDA(launch_finalize_scalar(partials, kTiledRowsPerShot, coef, grad_C, st, p->nshots, 1));
     else

@@ -131,21 +131,41 @@ __device__ __forceinline__ Sums sums_of(const Row& t, const Row& m, const Row& b
 }
 
 // The operator at a cell from the sums of both components.  The first two
-// terms are one rounded product and one fused multiply-add: SWAP = false
-// rounds the first product (as the tiled per-step kernels), true the second
-// (as the plain ones).
-template <bool SWAP>
+// terms of each row are one rounded product and one fused multiply-add; which
+// product is rounded is an argument (kOrder*), so that a problem's states
+// agree bit for bit with those of the per-step kernels of its size and mode:
+// the first in the tiled ones, the second in the plain ones (with constant
+// planes: the second of the x row, the first of the y row).
+constexpr int kOrderTiled = 0, kOrderPlain = 3, kOrderFields = 1;
+template <int ORDER>
 __device__ __forceinline__ void oper(const Coefs& k, const Sums& x, const Sums& y, float& lx, float& ly) {
-  lx = SWAP ? fmaf(k.k11, x.xx, __fmul_rn(k.k66, x.yy)) : fmaf(k.k66, x.yy, __fmul_rn(k.k11, x.xx));
+  lx = (ORDER & 1) ? fmaf(k.k11, x.xx, __fmul_rn(k.k66, x.yy)) : fmaf(k.k66, x.yy, __fmul_rn(k.k11, x.xx));
   lx = fmaf(k.kq12, y.xy, lx);
   lx = fmaf(k.k16h, x.xy, lx);
   lx = fmaf(k.k16, y.xx, lx);
   lx = fmaf(k.k26, y.yy, lx);
-  ly = SWAP ? fmaf(k.k66, y.xx, __fmul_rn(k.k22, y.yy)) : fmaf(k.k22, y.yy, __fmul_rn(k.k66, y.xx));
+  ly = (ORDER & 2) ? fmaf(k.k66, y.xx, __fmul_rn(k.k22, y.yy)) : fmaf(k.k22, y.yy, __fmul_rn(k.k66, y.xx));
   ly = fmaf(k.kq12, x.xy, ly);
   ly = fmaf(k.k16, x.xx, ly);
   ly = fmaf(k.k26, x.yy, ly);
   ly = fmaf(k.k26h, y.xy, ly);
+}
+// The scaled constants of a cell (C11, C22, C12, C16, C26, C66 planes of n
+// cells), zero when it is not `in`.
+__device__ __forceinline__ Coefs cell_coefs(const float* f, size_t n, size_t o, bool in, float q) {
+  float c[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) c[k] = in ? __ldg(f + k * n + o) : 0.f;
+  Coefs r;
+  r.k11 = c[0] * q;
+  r.k22 = c[1] * q;
+  r.k66 = c[5] * q;
+  r.k16 = c[3] * q;
+  r.k26 = c[4] * q;
+  r.k16h = 0.5f * r.k16;
+  r.k26h = 0.5f * r.k26;
+  r.kq12 = (c[2] + c[5]) * q * 0.25f;
+  return r;
 }
 // (2 c - p) + l
 __device__ __forceinline__ float leap(float c, float p, float l) { return fmaf(2.f, c, -p) + l; }
@@ -225,7 +245,10 @@ __device__ __forceinline__ void load_tile(float* lev0, float* lev1, const CUtens
 }
 
 // ----------------------------------------------------------------- forward
-template <int W, int RW, bool INST, bool SWAP, int CTAS>
+// Per-cell modes: FIELDS keeps the constants of the thread's cells in registers
+// for the launch (one row per thread); DFIELD reads the weights 1 - D of a row
+// one row ahead.
+template <int MODE, int W, int RW, bool INST, int ORDER, int CTAS>
 __global__ void __launch_bounds__(32 * W, CTAS)
     blk_fwd_kernel(const BlkFwd a, const __grid_constant__ CUtensorMap cur_map,
                    const __grid_constant__ CUtensorMap prev_map, int tiles_x, int tiles_y, int ntiles, int* err) {
@@ -279,6 +302,25 @@ __global__ void __launch_bounds__(32 * W, CTAS)
     const uint32_t region = rows_in<RW>(rr0, tile.xs - tile.x0 + kH, tile.xe - tile.x0 + kH);
     const uint32_t stored = lane >= 1 && lane <= 30 && nq > 0 ? region & rows_in<RW>(rr0, kH, B::kRows - kH) : 0u;
     const Coefs ks = coefs_in(meta, nq > 0);
+    Coefs kc[MODE == kModeFields ? 4 : 1];
+    if constexpr (MODE == kModeFields) {
+      static_assert(RW == 1, "one row of constants in registers");
+      const float q = a.coef->q;
+      const size_t o = (size_t)gi0 * ny + gj;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) kc[c] = cell_coefs(a.field, N, o + c, region != 0 && c < nq, q);
+    }
+    auto weights = [&](int r, float(&wv)[4]) {  // 1 - D at the warp's row r (zero outside the grid)
+      const float* d = a.field + (ptrdiff_t)(gi0 + r) * ny + gj;
+      const bool in = (region >> r) & 1u;
+      if (a.vec_field) {
+        const float4 v = in && nq > 0 ? __ldg(reinterpret_cast<const float4*>(d)) : make_float4(1.f, 1.f, 1.f, 1.f);
+        wv[0] = 1.f - v.x; wv[1] = 1.f - v.y; wv[2] = 1.f - v.z; wv[3] = 1.f - v.w;
+      } else {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) wv[c] = in && c < nq ? 1.f - __ldg(d + c) : 0.f;
+      }
+    };
     const int ox = __float_as_int(meta[12]), oy = __float_as_int(meta[13]);
     const bool src = has_src && tile.x0 - kH < ox + a.bx && tile.x0 - kH + B::kRows > ox &&
                      tile.y0 - kH < oy + a.by && tile.y0 - kH + kBox > oy;
@@ -306,10 +348,17 @@ __global__ void __launch_bounds__(32 * W, CTAS)
       const uint32_t st = a.out[t] != nullptr ? stored : 0u;
       auto rows = [&](auto plain) {
         constexpr bool PLAIN = decltype(plain)::value;
+        float wn[4], wv[4];
+        if constexpr (MODE == kModeDField) weights(0, wn);
         Row t0 = load_row(c0 - kBox), t1 = load_row(c0 + B::kPlane - kBox);
         Row m0 = load_row(c0), m1 = load_row(c0 + B::kPlane);
 #pragma unroll
         for (int r = 0; r < RW; ++r) {
+          if constexpr (MODE == kModeDField) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) wv[q] = wn[q];
+            if (r + 1 < RW) weights(r + 1, wn);
+          }
           const Row b0 = load_row(c0 + (r + 1) * kBox), b1 = load_row(c0 + B::kPlane + (r + 1) * kBox);
           if (PLAIN || ((region >> r) & 1u)) {  // (rows outside the region stay zero)
             const float4 pv0 = *reinterpret_cast<const float4*>(p0 + r * kBox);
@@ -317,7 +366,14 @@ __global__ void __launch_bounds__(32 * W, CTAS)
             const float q0[4] = {pv0.x, pv0.y, pv0.z, pv0.w}, q1[4] = {pv1.x, pv1.y, pv1.z, pv1.w};
             float v0[4], v1[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) oper<SWAP>(ks, sums_of(t0, m0, b0, q), sums_of(t1, m1, b1, q), v0[q], v1[q]);
+            for (int q = 0; q < 4; ++q) {
+              oper<ORDER>(MODE == kModeFields ? kc[MODE == kModeFields ? q : 0] : ks, sums_of(t0, m0, b0, q),
+                         sums_of(t1, m1, b1, q), v0[q], v1[q]);
+              if constexpr (MODE == kModeDField) {
+                v0[q] = __fmul_rn(v0[q], wv[q]);
+                v1[q] = __fmul_rn(v1[q], wv[q]);
+              }
+            }
             if (!PLAIN && src && (unsigned)(gi0 + r - ox) < (unsigned)a.bx) {
               // the load joins the operator sum before the update, as in the
               // reference's (A u + f) / rho
@@ -568,7 +624,7 @@ __global__ void __launch_bounds__(32 * W, CTAS)
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               const Sums sx = sums_of(t0, m0, b0, q), sy = sums_of(t1, m1, b1, q);
-              oper<false>(ks, sx, sy, v0[q], v1[q]);
+              oper<kOrderTiled>(ks, sx, sy, v0[q], v1[q]);
               acc[0] = fmaf(ux[q], sx.xx, acc[0]);
               acc[1] = fmaf(uy[q], sy.yy, acc[1]);
               acc[2] = fmaf(ux[q], sy.xy, fmaf(uy[q], sx.xy, acc[2]));
@@ -621,6 +677,393 @@ __global__ void __launch_bounds__(32 * W, CTAS)
   }
   if (tid == 0 && pipe_failed(&guard)) pipe_drain(bar, 1, &guard);
   flush(per_shot ? acc_shot : 0);
+}
+
+// ------------------------------------------- adjoint, degradation map
+// A^T lam = A0((1 - D) lam): the update's stencils run over the weighted
+// lam^{m+1}, its centre stays unweighted.  The imaging sum is kept per cell,
+// lam^{m+1} . (A0 u^m), so u's own stencils are needed: a second pass over the
+// warp's rows, with u's rows read from global memory (halo columns by the
+// outer lanes) one row ahead.
+template <int W, int RW, int CTAS>
+__global__ void __launch_bounds__(32 * W, CTAS)
+    blk_adj_d_kernel(const BlkAdj a, const __grid_constant__ CUtensorMap cur_map,
+                     const __grid_constant__ CUtensorMap prev_map, int tiles_x, int tiles_y, int ntiles, int* err) {
+  extern __shared__ float sm_raw[];
+  float* sm = aligned128(sm_raw);
+  using B = BlkTile<W, RW>;
+  constexpr int NT = B::kThreads;
+  float* lev0 = sm + kBox;
+  float* lev1 = lev0 + B::kLevel;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + B::kFloats + B::kMeta);
+  __shared__ PipeGuard guard;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int nx = a.nx, ny = a.ny;
+  const size_t N = (size_t)nx * ny, Np = (size_t)nx * a.pitch;
+  grid_dep_trigger();
+  if (tid == 0) {
+    prefetch_map(&cur_map);
+    prefetch_map(&prev_map);
+    bar_init(bar);
+    pipe_init(&guard);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (tid < kBox) sm[tid] = sm[B::kFloats - kBox + tid] = 0.f;
+  BWalk<false, B::kUse> walk;
+  walk.init((int)blockIdx.x, (int)gridDim.x, tiles_x, tiles_y, nx, ny);
+  __syncthreads();
+  grid_dep_wait();  // the states of the previous launch are complete from here on
+  const float gs = a.coef->gscale;
+  const int rr0 = w * RW;  // first row of the warp in the tile
+  const int o0 = rr0 * kBox + 4 * lane;
+  for (int k = 0; walk.t < ntiles; ++k, walk.next()) {
+    const BTile tile = walk.tile(a.inst);
+    const int2 recs = a.rec_tile != nullptr ? a.rec_tile[walk.t] : make_int2(0, 0);
+    load_tile<W, RW, false>(lev0, lev1, &cur_map, &prev_map, a.cur != nullptr, a.prev != nullptr, a.cur != nullptr,
+                            a.prev != nullptr, tile, k, bar, &guard, err);
+    __syncthreads();
+    const int gj = tile.y0 - kH + 4 * lane, gi0 = tile.x0 - kH + rr0;
+    const int nq = gj >= 0 ? max(0, min(4, ny - gj)) : 0;
+    const uint32_t region = rows_in<RW>(rr0, kH - tile.x0, nx - tile.x0 + kH);
+    const uint32_t rows_st = region & rows_in<RW>(rr0, kH, B::kRows - kH);
+    const uint32_t stored = lane >= 1 && lane <= 30 && nq > 0 ? rows_st : 0u;
+    const Coefs ks = coefs_in(&a.coef->k11, nq > 0);
+    const bool ragged = (ny & 3) != 0 && tile.y0 - kH + kBox > ny;
+    const ptrdiff_t off = (ptrdiff_t)tile.plane * 2 * (ptrdiff_t)Np + (ptrdiff_t)gi0 * a.pitch + gj;
+    auto weights = [&](int gi, float(&wv)[4]) {  // 1 - D (zero outside the grid)
+      const float* d = a.field + (ptrdiff_t)gi * ny + gj;
+      const bool in = gi >= 0 && gi < nx;
+      if (a.vec_field) {
+        const float4 v = in && nq > 0 ? __ldg(reinterpret_cast<const float4*>(d)) : make_float4(1.f, 1.f, 1.f, 1.f);
+        wv[0] = 1.f - v.x; wv[1] = 1.f - v.y; wv[2] = 1.f - v.z; wv[3] = 1.f - v.w;
+      } else {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) wv[c] = in && c < nq ? 1.f - __ldg(d + c) : 0.f;
+      }
+    };
+    for (int t = 1; t <= a.T; ++t) {
+      const int m = a.m_hi - t + 1;
+      const int frame = (m - 1) % a.stride == 0 ? (m - 1) / a.stride : -1;
+      const bool dense = frame >= 0 && a.record == kRecordFields;
+      float* lc = (t & 1) ? lev0 : lev1;
+      float* lp = (t & 1) ? lev1 : lev0;
+      if (frame >= 0 && recs.y > 0) {  // lam^m = ... - (lam^{m+2} - g) + ...
+        const size_t o = ((size_t)tile.inst * a.nt_out + frame) * a.nrec;
+        for (int e = tid; e < recs.y; e += NT) {
+          const int2 v = a.rec_ent[recs.x + e];
+          atomicAdd(&lp[v.x], -gs * a.g_x[o + v.y]);
+          atomicAdd(&lp[B::kPlane + v.x], -gs * a.g_y[o + v.y]);
+        }
+        __syncthreads();
+      }
+      const float* c0 = lc + o0;  // lam^{m+1}
+      float* p0 = lp + o0;        // lam^{m+2}, becomes lam^m
+      float* out = t == a.T ? a.out_last : (t == a.T - 1 ? a.out_before : nullptr);
+      const uint32_t st = out != nullptr ? stored : 0u;
+      if (region != 0 && rows_in<RW>(rr0, t, B::kRows - t) != 0) {
+        float* out0 = out + off;
+        float* out1 = out0 + Np;
+        // a row of lam^{m+1}: the quads, and their weighted windows
+        struct LRow {
+          Q4 x, y;
+          Row wx, wy;
+        };
+        float wn[4];
+        auto lam_row = [&](int r) {
+          LRow l;
+          l.x = q4(*reinterpret_cast<const float4*>(c0 + r * kBox));
+          l.y = q4(*reinterpret_cast<const float4*>(c0 + B::kPlane + r * kBox));
+          Q4 vx, vy;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            vx.v[q] = __fmul_rn(wn[q], l.x.v[q]);
+            vy.v[q] = __fmul_rn(wn[q], l.y.v[q]);
+          }
+          l.wx = row_of(vx);
+          l.wy = row_of(vy);
+          return l;
+        };
+        weights(gi0 - 1, wn);
+        LRow tr = lam_row(-1);
+        weights(gi0, wn);
+        LRow mr = lam_row(0);
+        weights(gi0 + 1, wn);
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+          const LRow br = lam_row(r + 1);
+          if (r + 1 < RW) weights(gi0 + r + 2, wn);
+          if ((region >> r) & 1u) {
+            const float4 pv0 = *reinterpret_cast<const float4*>(p0 + r * kBox);
+            const float4 pv1 = *reinterpret_cast<const float4*>(p0 + B::kPlane + r * kBox);
+            const float q0[4] = {pv0.x, pv0.y, pv0.z, pv0.w}, q1[4] = {pv1.x, pv1.y, pv1.z, pv1.w};
+            float v0[4], v1[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              oper<kOrderTiled>(ks, sums_of(tr.wx, mr.wx, br.wx, q), sums_of(tr.wy, mr.wy, br.wy, q), v0[q], v1[q]);
+              v0[q] = leap(mr.x.v[q], q0[q], v0[q]);
+              v1[q] = leap(mr.y.v[q], q1[q], v1[q]);
+            }
+            if (dense) {
+              const size_t o = ((size_t)tile.plane * a.nt_out + frame) * N + (size_t)(gi0 + r) * ny + gj;
+#pragma unroll
+              for (int q = 0; q < 4; ++q)
+                if (q < nq) {
+                  v0[q] = fmaf(gs, a.g_x[o + q], v0[q]);
+                  v1[q] = fmaf(gs, a.g_y[o + q], v1[q]);
+                }
+            }
+            if (ragged) {  // the grid's last column is inside a quad
+              mask_q(v0, nq);
+              mask_q(v1, nq);
+            }
+            const float4 n0 = make_float4(v0[0], v0[1], v0[2], v0[3]), n1 = make_float4(v1[0], v1[1], v1[2], v1[3]);
+            *reinterpret_cast<float4*>(p0 + r * kBox) = n0;
+            *reinterpret_cast<float4*>(p0 + B::kPlane + r * kBox) = n1;
+            if ((st >> r) & 1u) {
+              *reinterpret_cast<float4*>(out0) = n0;
+              *reinterpret_cast<float4*>(out1) = n1;
+            }
+          }
+          out0 += a.pitch;
+          out1 += a.pitch;
+          tr = mr;
+          mr = br;
+        }
+      }
+      if (m <= a.nt - 1 && rows_st != 0) {
+        const float* u0 = a.u_base + (ptrdiff_t)(m - a.m_base) * (ptrdiff_t)a.u_stride + off;
+        auto load_u = [&](int r, float4& x, float4& y) {
+          x = y = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (gi0 + r >= 0 && gi0 + r < nx && nq > 0) {
+            const float* u = u0 + (ptrdiff_t)r * a.pitch;
+            x = __ldcg(reinterpret_cast<const float4*>(u));
+            y = __ldcg(reinterpret_cast<const float4*>(u + Np));
+          }
+        };
+        float* ga = a.gacc + (size_t)tile.plane * N + (ptrdiff_t)gi0 * ny + gj;
+        float4 nx4, ny4, tx4, ty4;
+        load_u(-1, tx4, ty4);
+        load_u(0, nx4, ny4);
+        Row t0 = row_of(q4(tx4)), t1 = row_of(q4(ty4));
+        load_u(1, tx4, ty4);
+        Row m0 = row_of(q4(nx4)), m1 = row_of(q4(ny4));
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+          const Row b0 = row_of(q4(tx4)), b1 = row_of(q4(ty4));
+          if (r + 1 < RW) load_u(r + 2, tx4, ty4);
+          if ((stored >> r) & 1u) {
+            const float4 lx = *reinterpret_cast<const float4*>(c0 + r * kBox);
+            const float4 ly = *reinterpret_cast<const float4*>(c0 + B::kPlane + r * kBox);
+            const float l0[4] = {lx.x, lx.y, lx.z, lx.w}, l1[4] = {ly.x, ly.y, ly.z, ly.w};
+            float gv[4];
+            if (a.vec_field) {
+              const float4 g = *reinterpret_cast<const float4*>(ga);
+              gv[0] = g.x; gv[1] = g.y; gv[2] = g.z; gv[3] = g.w;
+            } else {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) gv[q] = q < nq ? ga[q] : 0.f;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              float Lx, Ly;
+              oper<kOrderPlain>(ks, sums_of(t0, m0, b0, q), sums_of(t1, m1, b1, q), Lx, Ly);
+              gv[q] += fmaf(l0[q], Lx, __fmul_rn(l1[q], Ly));
+            }
+            if (a.vec_field) {
+              *reinterpret_cast<float4*>(ga) = make_float4(gv[0], gv[1], gv[2], gv[3]);
+            } else {
+#pragma unroll
+              for (int q = 0; q < 4; ++q)
+                if (q < nq) ga[q] = gv[q];
+            }
+          }
+          ga += ny;
+          t0 = m0; t1 = m1; m0 = b0; m1 = b1;
+        }
+      }
+      __syncthreads();  // lam^m is complete
+    }
+  }
+  if (tid == 0 && pipe_failed(&guard)) pipe_drain(bar, 1, &guard);
+}
+
+// ------------------------------------------- adjoint, six constant planes
+// One row of 128 columns per warp; the thread keeps its cells' two levels,
+// constants and six running gradients in registers for the launch.  A^T
+// applies the stencils to products of each cell's own constants with lam:
+// the four products whose vertical or diagonal neighbours are needed go
+// through shared memory (one CTA barrier per step), the others' column
+// neighbours come by lane shuffles.
+template <int W>
+__global__ void __launch_bounds__(32 * W, 1)
+    blk_adj_f_kernel(const BlkAdj a, int tiles_x, int tiles_y, int ntiles) {
+  extern __shared__ float sm_raw[];
+  float* ex = aligned128(sm_raw);  // [parity][product][row][128]
+  constexpr int kRows = W, kUse = W - 2 * kH;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int nx = a.nx, ny = a.ny;
+  const size_t N = (size_t)nx * ny, Np = (size_t)nx * a.pitch;
+  grid_dep_trigger();
+  BWalk<false, kUse> walk;
+  walk.init((int)blockIdx.x, (int)gridDim.x, tiles_x, tiles_y, nx, ny);
+  const float qf = a.coef->q;
+  for (; walk.t < ntiles; walk.next()) {
+    const BTile tile = walk.tile(a.inst);
+    const int2 recs = a.rec_tile != nullptr ? a.rec_tile[walk.t] : make_int2(0, 0);
+    const int gj = tile.y0 - kH + 4 * lane, gi = tile.x0 - kH + w;
+    const bool row_in = gi >= 0 && gi < nx;
+    const int nq = row_in && gj >= 0 ? max(0, min(4, ny - gj)) : 0;
+    const bool stored = w >= kH && w < kRows - kH && lane >= 1 && lane <= 30 && nq > 0;
+    float C[6][4];
+#pragma unroll
+    for (int c = 0; c < 6; ++c)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) C[c][q] = q < nq ? __ldg(a.field + c * N + (size_t)gi * ny + gj + q) : 0.f;
+    grid_dep_wait();  // the states of the previous launch are complete from here on
+    const float gs = a.coef->gscale;
+    const ptrdiff_t off = (ptrdiff_t)tile.plane * 2 * (ptrdiff_t)Np + (ptrdiff_t)gi * a.pitch + gj;
+    auto load_state = [&](const float* s, ptrdiff_t o, bool in, float(&x)[4], float(&y)[4]) {
+      const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 vx = in ? __ldcg(reinterpret_cast<const float4*>(s + o)) : z;
+      const float4 vy = in ? __ldcg(reinterpret_cast<const float4*>(s + o + Np)) : z;
+      x[0] = vx.x; x[1] = vx.y; x[2] = vx.z; x[3] = vx.w;
+      y[0] = vy.x; y[1] = vy.y; y[2] = vy.z; y[3] = vy.w;
+    };
+    float cx[4], cy[4], px[4], py[4], ga[6][4];
+    load_state(a.cur, off, a.cur != nullptr && nq > 0, cx, cy);
+    load_state(a.prev, off, a.prev != nullptr && nq > 0, px, py);
+#pragma unroll
+    for (int c = 0; c < 6; ++c)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) ga[c][q] = 0.f;
+    for (int t = 1; t <= a.T; ++t) {
+      const int m = a.m_hi - t + 1;
+      const int frame = (m - 1) % a.stride == 0 ? (m - 1) / a.stride : -1;
+      // the products of this row, those the rows above and below need in
+      // shared memory
+      Q4 s0, s1, s2, s3, s4, s5;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float lx = cx[q], ly = cy[q], c1266 = C[2][q] + C[5][q];
+        s0.v[q] = fmaf(C[0][q], lx, __fmul_rn(C[3][q], ly));
+        s1.v[q] = fmaf(C[5][q], lx, __fmul_rn(C[4][q], ly));
+        s2.v[q] = fmaf(2.f * C[3][q], lx, __fmul_rn(c1266, ly));
+        s3.v[q] = fmaf(C[3][q], lx, __fmul_rn(C[5][q], ly));
+        s4.v[q] = fmaf(C[4][q], lx, __fmul_rn(C[1][q], ly));
+        s5.v[q] = fmaf(c1266, lx, __fmul_rn(2.f * C[4][q], ly));
+      }
+      float* e = ex + (t & 1) * (4 * kRows * kBox) + w * kBox + 4 * lane;
+      *reinterpret_cast<float4*>(e) = f4(s0);
+      *reinterpret_cast<float4*>(e + kRows * kBox) = f4(s2);
+      *reinterpret_cast<float4*>(e + 2 * kRows * kBox) = f4(s3);
+      *reinterpret_cast<float4*>(e + 3 * kRows * kBox) = f4(s5);
+      // (the u rows of the imaging sums, in flight over the barrier)
+      const bool im = m <= a.nt - 1 && w >= kH && w < kRows - kH && row_in;
+      float ux[3][4], uy[3][4];
+      if (im) {
+        const float* u = a.u_base + (ptrdiff_t)(m - a.m_base) * (ptrdiff_t)a.u_stride;
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+          load_state(u, off + (ptrdiff_t)(d - 1) * a.pitch, nq > 0 && gi + d - 1 >= 0 && gi + d - 1 < nx, ux[d], uy[d]);
+      }
+      __syncthreads();
+      if (row_in && w >= t && w < kRows - t) {
+        const float* up = e - (w > 0 ? kBox : 0);
+        const float* dn = e + (w < kRows - 1 ? kBox : 0);
+        auto quad = [](const float* p) { return q4(*reinterpret_cast<const float4*>(p)); };
+        const Row r1 = row_of(s1), r4 = row_of(s4);
+        float vx[4], vy[4];
+        {
+          const Q4 t0 = quad(up), b0 = quad(dn);
+          const Row t2 = row_of(quad(up + kRows * kBox)), b2 = row_of(quad(dn + kRows * kBox));
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float xx = fmaf(-2.f, s0.v[q], t0.v[q] + b0.v[q]);
+            const float yy = fmaf(-2.f, s1.v[q], r1.w[q] + r1.w[q + 2]);
+            const float xy = (b2.w[q + 2] + t2.w[q]) - (b2.w[q] + t2.w[q + 2]);
+            vx[q] = fmaf(qf, fmaf(0.25f, xy, xx + yy), fmaf(2.f, cx[q], -px[q]));
+          }
+        }
+        {
+          const Q4 t3 = quad(up + 2 * kRows * kBox), b3 = quad(dn + 2 * kRows * kBox);
+          const Row t5 = row_of(quad(up + 3 * kRows * kBox)), b5 = row_of(quad(dn + 3 * kRows * kBox));
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float xx = fmaf(-2.f, s3.v[q], t3.v[q] + b3.v[q]);
+            const float yy = fmaf(-2.f, s4.v[q], r4.w[q] + r4.w[q + 2]);
+            const float xy = (b5.w[q + 2] + t5.w[q]) - (b5.w[q] + t5.w[q + 2]);
+            vy[q] = fmaf(qf, fmaf(0.25f, xy, xx + yy), fmaf(2.f, cy[q], -py[q]));
+          }
+        }
+        if (frame >= 0 && a.record == kRecordFields) {
+          const size_t o = ((size_t)tile.plane * a.nt_out + frame) * N + (size_t)gi * ny + gj;
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (q < nq) {
+              vx[q] = fmaf(gs, a.g_x[o + q], vx[q]);
+              vy[q] = fmaf(gs, a.g_y[o + q], vy[q]);
+            }
+        }
+        if (frame >= 0 && recs.y > 0) {
+          const size_t o = ((size_t)tile.inst * a.nt_out + frame) * a.nrec;
+          for (int n = 0; n < recs.y; ++n) {
+            const int2 v = a.rec_ent[recs.x + n];
+            if (v.x / 4 != w * (kBox / 4) + lane) continue;  // another thread's cell
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              if ((v.x & 3) == q) {
+                vx[q] = fmaf(gs, a.g_x[o + v.y], vx[q]);
+                vy[q] = fmaf(gs, a.g_y[o + v.y], vy[q]);
+              }
+          }
+        }
+        mask_q(vx, nq);  // cells outside the grid stay zero
+        mask_q(vy, nq);
+        if (im) {  // lam^{m+1} against the derivatives of A u^m
+          const Row t0 = row_of(Q4{{ux[0][0], ux[0][1], ux[0][2], ux[0][3]}});
+          const Row m0 = row_of(Q4{{ux[1][0], ux[1][1], ux[1][2], ux[1][3]}});
+          const Row b0 = row_of(Q4{{ux[2][0], ux[2][1], ux[2][2], ux[2][3]}});
+          const Row t1 = row_of(Q4{{uy[0][0], uy[0][1], uy[0][2], uy[0][3]}});
+          const Row m1 = row_of(Q4{{uy[1][0], uy[1][1], uy[1][2], uy[1][3]}});
+          const Row b1 = row_of(Q4{{uy[2][0], uy[2][1], uy[2][2], uy[2][3]}});
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const Sums sx = sums_of(t0, m0, b0, q), sy = sums_of(t1, m1, b1, q);
+            const float lx = cx[q], ly = cy[q];
+            ga[0][q] = fmaf(lx, sx.xx, ga[0][q]);
+            ga[1][q] = fmaf(ly, sy.yy, ga[1][q]);
+            ga[2][q] += fmaf(lx, sy.xy, __fmul_rn(ly, sx.xy));
+            ga[3][q] += fmaf(lx, fmaf(0.5f, sx.xy, sy.xx), __fmul_rn(ly, sx.xx));
+            ga[4][q] += fmaf(lx, sy.yy, __fmul_rn(ly, fmaf(0.5f, sy.xy, sx.yy)));
+            ga[5][q] += fmaf(lx, sx.yy, __fmul_rn(ly, sy.xx));
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          px[q] = cx[q];
+          py[q] = cy[q];
+          cx[q] = vx[q];
+          cy[q] = vy[q];
+        }
+      }
+    }
+    if (stored) {
+      // cur holds lam of the last step, prev of the one before
+      *reinterpret_cast<float4*>(a.out_last + off) = make_float4(cx[0], cx[1], cx[2], cx[3]);
+      *reinterpret_cast<float4*>(a.out_last + off + Np) = make_float4(cy[0], cy[1], cy[2], cy[3]);
+      if (a.out_before != nullptr) {
+        *reinterpret_cast<float4*>(a.out_before + off) = make_float4(px[0], px[1], px[2], px[3]);
+        *reinterpret_cast<float4*>(a.out_before + off + Np) = make_float4(py[0], py[1], py[2], py[3]);
+      }
+      float* g = a.gacc + (size_t)tile.plane * 6 * N + (size_t)gi * ny + gj;
+#pragma unroll
+      for (int c = 0; c < 6; ++c)
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (q < nq) g[c * N + q] += ga[c][q];
+    }
+    __syncthreads();  // the products are read: the next tile's may be written
+  }
 }
 
 // ------------------------------------------------- receivers of the tiles
@@ -723,14 +1166,14 @@ int blk_sms() {
 }
 
 
-template <int W, int RW, int CTAS, bool INST, bool SWAP>
+template <int MODE, int W, int RW, int CTAS, bool INST, int ORDER>
 cudaError_t fwd_t(const BlkFwd& a, int* err, cudaStream_t st) {
   using B = BlkTile<W, RW>;
   constexpr size_t smem = B::kBytes;
   static std::once_flag once;
   static cudaError_t ready = cudaSuccess;
   std::call_once(once, [] {
-    ready = cudaFuncSetAttribute(blk_fwd_kernel<W, RW, INST, SWAP, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    ready = cudaFuncSetAttribute(blk_fwd_kernel<MODE, W, RW, INST, ORDER, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
   if (ready != cudaSuccess) return ready;
   const int planes = INST ? 1 : a.S;
@@ -746,7 +1189,7 @@ cudaError_t fwd_t(const BlkFwd& a, int* err, cudaStream_t st) {
   int stores = 0;
   for (int t = 0; t <= a.T; ++t) stores += a.out[t] != nullptr ? 1 : 0;
   return tracked_launch(kProfForward, st, [&] {
-    launch_step_kernel(blk_fwd_kernel<W, RW, INST, SWAP, CTAS>, dim3(grid), dim3(32 * W), smem, st, a.chained != 0, a, cm, pm,
+    launch_step_kernel(blk_fwd_kernel<MODE, W, RW, INST, ORDER, CTAS>, dim3(grid), dim3(32 * W), smem, st, a.chained != 0, a, cm, pm,
                        tiles_x, tiles_y, ntiles, err);
   }, cells * 8.0 * (stores + (a.cur ? 1 : 0) + (a.prev ? 1 : 0)));
 }
@@ -776,6 +1219,47 @@ cudaError_t adj_t(const BlkAdj& a, int* err, cudaStream_t st) {
     launch_step_kernel(blk_adj_kernel<W, RW, INST, CTAS>, dim3(grid), dim3(32 * W), smem, st, a.chained != 0, a, cm, pm,
                        tiles_x, tiles_y, ntiles, err);
   }, cells * 8.0 * (a.T + (a.T > 1 ? 2 : 1) + (a.cur ? 1 : 0) + (a.prev ? 1 : 0)));
+}
+
+// The per-cell modes' adjoint launches.
+template <int W, int RW, int CTAS>
+cudaError_t adj_d_t(const BlkAdj& a, int* err, cudaStream_t st) {
+  using B = BlkTile<W, RW>;
+  static std::once_flag once;
+  static cudaError_t ready = cudaSuccess;
+  std::call_once(once, [] {
+    ready = cudaFuncSetAttribute(blk_adj_d_kernel<W, RW, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)B::kBytes);
+  });
+  if (ready != cudaSuccess) return ready;
+  const float* any = a.cur ? a.cur : a.out_last;  // (a level that is zero is not loaded)
+  CUtensorMap cm, pm;
+  if (!blk_map(&cm, any, a.nx, a.ny, a.pitch, a.S, kBox, B::kRows) ||
+      !blk_map(&pm, a.prev ? a.prev : any, a.nx, a.ny, a.pitch, a.S, kBox, B::kRows))
+    return cudaErrorNotSupported;
+  const int tiles_x = (a.nx + B::kUse - 1) / B::kUse, tiles_y = (a.ny + kBlkCols - 1) / kBlkCols;
+  const int ntiles = a.S * tiles_x * tiles_y, slots = CTAS * blk_sms();
+  return tracked_launch(kProfAdjoint, st, [&] {
+    launch_step_kernel(blk_adj_d_kernel<W, RW, CTAS>, dim3(ntiles < slots ? ntiles : slots), dim3(32 * W), B::kBytes,
+                       st, a.chained != 0, a, cm, pm, tiles_x, tiles_y, ntiles, err);
+  }, (double)a.S * a.nx * a.ny * (16.0 * a.T + 32.0 + 4.0));
+}
+
+cudaError_t adj_f(const BlkAdj& a, cudaStream_t st) {
+  constexpr int W = 16, H = W - 2 * kH;
+  constexpr size_t smem = (size_t)2 * 4 * W * kBox * 4 + 128;
+  static std::once_flag once;
+  static cudaError_t ready = cudaSuccess;
+  std::call_once(once, [] {
+    ready = cudaFuncSetAttribute(blk_adj_f_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  });
+  if (ready != cudaSuccess) return ready;
+  const int tiles_x = (a.nx + H - 1) / H, tiles_y = (a.ny + kBlkCols - 1) / kBlkCols;
+  const int ntiles = a.S * tiles_x * tiles_y;
+  return tracked_launch(kProfAdjoint, st, [&] {
+    launch_step_kernel(blk_adj_f_kernel<W>, dim3(ntiles < blk_sms() ? ntiles : blk_sms()), dim3(32 * W), smem, st,
+                       a.chained != 0, a, tiles_x, tiles_y, ntiles);
+  }, (double)a.S * a.nx * a.ny * (8.0 * a.T + 32.0 + 72.0));
 }
 
 }  // namespace
@@ -835,16 +1319,29 @@ cudaError_t launch_rec_tiles(int geo, const int32_t* rec_idx, int S, int nrec, i
   });
 }
 
-cudaError_t launch_blk_fwd(const BlkFwd& a, int* err, cudaStream_t st) {
-  if (a.inst.tiles != nullptr) return fwd_t<8, 6, 2, true, false>(a, err, st);
-  if (a.geo == kBlkFlat)
-    return a.swap ? fwd_t<16, 1, 1, false, true>(a, err, st) : fwd_t<16, 1, 1, false, false>(a, err, st);
-  if (a.geo == kBlkShort)
-    return a.swap ? fwd_t<16, 2, 1, false, true>(a, err, st) : fwd_t<16, 2, 1, false, false>(a, err, st);
-  return a.swap ? fwd_t<8, 6, 2, false, true>(a, err, st) : fwd_t<8, 6, 2, false, false>(a, err, st);
+namespace {
+template <int MODE, int ORDER>
+cudaError_t fwd_geo(const BlkFwd& a, int* err, cudaStream_t st) {
+  if (a.geo == kBlkFlat) return fwd_t<MODE, 16, 1, 1, false, ORDER>(a, err, st);
+  if (a.geo == kBlkShort) return fwd_t<MODE, 16, 2, 1, false, ORDER>(a, err, st);
+  return fwd_t<MODE, 8, 6, 2, false, ORDER>(a, err, st);
+}
+}  // namespace
+
+cudaError_t launch_blk_fwd(int mode, const BlkFwd& a, int* err, cudaStream_t st) {
+  if (a.inst.tiles != nullptr) return fwd_t<kModeScalar, 8, 6, 2, true, kOrderTiled>(a, err, st);
+  if (mode == kModeFields) return fwd_t<kModeFields, 16, 1, 1, false, kOrderFields>(a, err, st);
+  if (mode == kModeDField) return fwd_geo<kModeDField, kOrderPlain>(a, err, st);
+  return a.plain_order ? fwd_geo<kModeScalar, kOrderPlain>(a, err, st) : fwd_geo<kModeScalar, kOrderTiled>(a, err, st);
 }
 
-cudaError_t launch_blk_adj(const BlkAdj& a, int* err, cudaStream_t st) {
+cudaError_t launch_blk_adj(int mode, const BlkAdj& a, int* err, cudaStream_t st) {
+  if (mode == kModeFields) return adj_f(a, st);
+  if (mode == kModeDField) {
+    if (a.geo == kBlkFlat) return adj_d_t<16, 1, 1>(a, err, st);
+    if (a.geo == kBlkShort) return adj_d_t<16, 2, 1>(a, err, st);
+    return adj_d_t<8, 6, 2>(a, err, st);
+  }
   if (a.inst.tiles != nullptr) return adj_t<8, 6, 2, true>(a, err, st);
   if (a.geo == kBlkFlat) return adj_t<16, 1, 1, false>(a, err, st);
   if (a.geo == kBlkShort) return adj_t<16, 2, 1, false>(a, err, st);

@@ -13,7 +13,7 @@ constexpr int kBlkCols = 120;      // columns of a tile (a warp's 128 less one q
 // Forward: u^{i+1} .. u^{i+T} from (u^i, u^{i-1}).
 struct BlkFwd {
   int geo;                         // tile geometry (blk_geometry)
-  int swap;                        // rounding order of the operator's first two terms (oper)
+  int plain_order;                 // SCALAR: rounding order of the plain kernels (oper), else the tiled ones'
   int nx, ny, pitch, S, nt, i, T;  // pitch: floats between rows of a state (ny rounded up to 4)
   const float* cur;                // u^i, nullptr: zero
   const float* prev;               // u^{i-1}, nullptr: zero
@@ -28,6 +28,8 @@ struct BlkFwd {
   const int2* rec_ent;
   const Coef* coef;
   int coef_stride;
+  const float* field;              // FIELDS: 6 planes of C; DFIELD: D plane (rows of ny floats)
+  int vec_field;                   // the plane's rows start on 16-byte boundaries
   const float* src_signal;
   const float* src_map;
   const int32_t* src_origin;
@@ -56,7 +58,10 @@ struct BlkAdj {
   const int2* rec_ent;
   const Coef* coef;
   int coef_stride;
-  double* partials;
+  const float* field;   // as in BlkFwd (vec_field: gacc's rows too)
+  int vec_field;
+  float* gacc;          // DFIELD: [S][N]; FIELDS: [S][6][N] running sums
+  double* partials;     // SCALAR
   int chained;
   InstTiles inst;
 };
@@ -73,7 +78,7 @@ size_t blk_rec_bytes(size_t ntiles, int S, int nrec);
 cudaError_t launch_rec_tiles(int geo, const int32_t* rec_idx, int S, int nrec, int nx, int ny, const int4* box,
                              size_t ntiles, void* ws, const int2** tile, const int2** ent, cudaStream_t st);
 bool blk_available();  // the driver exposes the tensor-map encoder
-cudaError_t launch_blk_fwd(const BlkFwd& a, int* err, cudaStream_t st);
-cudaError_t launch_blk_adj(const BlkAdj& a, int* err, cudaStream_t st);
+cudaError_t launch_blk_fwd(int mode, const BlkFwd& a, int* err, cudaStream_t st);
+cudaError_t launch_blk_adj(int mode, const BlkAdj& a, int* err, cudaStream_t st);
 
 }  // namespace ernn

@@ -4,9 +4,9 @@ per-step kernels at the sizes where a tile ends: stored rows of a tile (24 and
 counts that leave launches of one to three steps, checkpoints on and off them.
 
 Both evaluate the same sequence of rounded operations per cell, so the
-recorded fields are equal bit for bit; the gradient's six sums group their
-FP32 partial sums differently (relative 2^-24 sqrt(cells per partial sum),
-below 1e-5).  GPU only."""
+recorded fields are equal bit for bit; the gradient's sums group their FP32
+partial sums differently (relative 2^-24 sqrt(terms of a partial sum), below
+1e-5).  GPU only."""
 import numpy as np
 import pytest
 import torch
@@ -21,11 +21,12 @@ pytestmark = pytest.mark.gpu
 
 def run(case, wx, wy, path, ckpt_k):
     geom = to_geometry(case, path=path, ckpt_k=ckpt_k)
-    C = torch.tensor(case.C, dtype=torch.float32, device=DEV, requires_grad=True)
-    ux, uy = E.propagate(C, torch.tensor(case.rho, dtype=torch.float32, device=DEV), geom)
+    C = torch.tensor(case.C, dtype=torch.float32, device=DEV, requires_grad=case.D is None)
+    D = None if case.D is None else torch.tensor(case.D, dtype=torch.float32, device=DEV, requires_grad=True)
+    ux, uy = E.propagate(C, torch.tensor(case.rho, dtype=torch.float32, device=DEV), geom, D=D)
     used = E.load_library().ernn_last_path()
     ((ux.double() * torch.as_tensor(wx, device=DEV)).sum() + (uy.double() * torch.as_tensor(wy, device=DEV)).sum()).backward()
-    return ux.detach().cpu().numpy(), uy.detach().cpu().numpy(), C.grad.double().cpu().numpy(), used
+    return ux.detach().cpu().numpy(), uy.detach().cpu().numpy(), (C if D is None else D).grad.double().cpu().numpy(), used
 
 
 SIZES = [(8, 41), (17, 40 + 3), (24, 41), (25, 119), (23, 121), (40, 122), (41, 127), (48, 129), (3, 243), (97, 250), (130, 361)]
@@ -45,8 +46,23 @@ def test_same_fields_as_the_plain_kernels(nx, ny, record, nt, ckpt_k):
     assert rel(ag, bg) <= 1e-5, rel(ag, bg)
 
 
-def test_every_cell_a_receiver():
-    case = random_case(nx=50, ny=126, nt=20, S=2, record=O.RECORD_RECEIVERS, nrec=50 * 126, stride=2)
+@pytest.mark.parametrize("mode", [O.MODE_DFIELD, O.MODE_FIELDS])
+@pytest.mark.parametrize("nx,ny", [(8, 41), (25, 119), (23, 124), (61, 76), (97, 250)])
+@pytest.mark.parametrize("record", [O.RECORD_FIELDS, O.RECORD_RECEIVERS])
+@pytest.mark.parametrize("nt,ckpt_k", [(37, None), (30, 1), (33, 6)])
+def test_per_cell_modes_same_fields_as_the_plain_kernels(mode, nx, ny, record, nt, ckpt_k):
+    case = random_case(nx=nx, ny=ny, nt=nt, S=2, stride=1 + nt % 2, mode=mode, record=record, nrec=40, src_comp=nx % 2)
+    wx, wy = weights(case)
+    ax, ay, ag, used = run(case, wx, wy, E.PATH_AUTO, ckpt_k)
+    assert used == E.PATH_TILED
+    bx, by, bg, _ = run(case, wx, wy, E.PATH_STEP, ckpt_k)
+    assert np.array_equal(ax, bx) and np.array_equal(ay, by)
+    assert rel(ag, bg) <= 1e-5, rel(ag, bg)
+
+
+@pytest.mark.parametrize("mode", [O.MODE_SCALAR, O.MODE_DFIELD, O.MODE_FIELDS])
+def test_every_cell_a_receiver(mode):
+    case = random_case(nx=50, ny=126, nt=20, S=2, mode=mode, record=O.RECORD_RECEIVERS, nrec=50 * 126, stride=2)
     wx, wy = weights(case)
     ax, ay, ag, used = run(case, wx, wy, E.PATH_AUTO, 6)
     bx, by, bg, _ = run(case, wx, wy, E.PATH_STEP, 6)
