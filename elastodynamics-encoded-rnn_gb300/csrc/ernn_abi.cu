@@ -149,10 +149,9 @@ Plan make_plan(const ErnnProblem& p) {
   pl.npart = pl.nblocks > p.nshots * 16 * 8 ? pl.nblocks : p.nshots * 16 * 8;
   if (pl.ncoef > 1 && pl.npart < p.nshots * kTiledRowsPerShot) pl.npart = p.nshots * kTiledRowsPerShot;
   if (p.mode == kModeScalar) off += align_up((size_t)pl.npart * 8 * sizeof(double));
-  // receiver table of the tiled adjoint: one byte per (shot, tile), sized for
-  // its smallest tiles (64 x 16)
+  // receiver table of the tiled per-step adjoint: one byte per (shot, tile)
   pl.s_tflags = off;
-  if (p.record == kRecordReceivers && !pl.inst) off += align_up(tma_tiles(p.nx, p.ny, p.nshots, 16));
+  if (p.record == kRecordReceivers && !pl.block) off += align_up(tma_tiles(p.nx, p.ny, p.nshots));
   if (pl.block) off += 16;  // the scratch starts at its first 16-byte boundary
   pl.s_total = off;
   return pl;
@@ -236,21 +235,19 @@ FwdStep base_fwd(const ErnnProblem& p, const ErnnInputs& in, const Coef* coef, i
 
 std::atomic<int32_t> g_last_path{ERNN_PATH_AUTO};
 
-// Tiled per-step kernels: requested (ERNN_PATH_TILED, an error when the
-// problem is not eligible) or chosen by ERNN_PATH_AUTO when eligible and one
-// step has at least four 64 x 32 tiles per SM.  The tiled kernels are
+// Tiled per-step kernels (degradation maps): requested (ERNN_PATH_TILED, an
+// error when the problem is not eligible) or chosen by ERNN_PATH_AUTO when
+// eligible and one step has at least four 64 x 32 tiles per SM.  They are
 // persistent (2-3 CTAs of 72-111 KB shared memory per SM, each streaming
-// several tiles); below that size the plain per-step kernels, many small
-// CTAs per SM, hide latency better and share the GPU better with other
-// streams' work.
+// several tiles).  Scalar problems of the tiled path get here only with a
+// tape that is not on a 16-byte boundary: the plain kernels take those.
 int use_tiled(const ErnnProblem& p, int* tiled) {
   *tiled = 0;
   if (p.path == ERNN_PATH_STEP) return ERNN_OK;
-  const bool ok = tma_eligible(p.mode, p.nx, p.ny, p.nshots);
+  const bool ok = tma_eligible(p.mode, p.ny);
   if (p.path == ERNN_PATH_TILED) {
-    if (!ok) return ERNN_ERR_UNSUPPORTED;
-    *tiled = 1;
-    return ERNN_OK;
+    *tiled = ok;
+    return ok || (p.mode == kModeScalar && p.ny % 4 == 0 && blk_available()) ? ERNN_OK : ERNN_ERR_UNSUPPORTED;
   }
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -671,13 +668,6 @@ int ernn_operator(int32_t nshots, int32_t nx, int32_t ny, int32_t mode, double h
   return ERNN_OK;
 }
 
-// Tile rows of the tiled kernels: 32 with ERNN_FLAG_TALL_TILES and always in
-// the D-field mode (its forward measured faster with them: 8 x 512^2 shots,
-// 81.3 -> 75.6 ms per inversion iteration), else 16.
-static int tile_rows_of(const ErnnProblem& p) {
-  return ((p.flags & ERNN_FLAG_TALL_TILES) || p.mode == kModeDField) ? 32 : 16;
-}
-
 // The forward time loop of ernn_forward and, with an instance plan `ip`, of
 // ernn_forward_instances.
 static int forward_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPlan* ip, float* out_ux,
@@ -727,7 +717,7 @@ static int forward_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPl
   if ((rc = use_tiled(*p, &tiled))) return rc;
   g_last_path.store(tiled ? ERNN_PATH_TILED : ERNN_PATH_STEP, std::memory_order_relaxed);
   auto fwd_step = [&](const FwdStep& s) {
-    return tiled ? launch_tma_fwd(p->mode, s, &coef->err, st) : launch_fwd_step(p->mode, s, st);
+    return tiled ? launch_tma_fwd(s, &coef->err, st) : launch_fwd_step(p->mode, s, st);
   };
 
   const bool store_all = with_tape && pl.store_all;
@@ -739,7 +729,6 @@ static int forward_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPl
   };
   const bool receivers = (p->record == kRecordReceivers);
   FwdStep a = base_fwd(*p, *in, coef, pl.nt_out);
-  a.tile_rows = tile_rows_of(*p);
   const float* last = nullptr;
   for (int i = 0; i < p->nt; ++i) {
     if (store_all) {
@@ -885,25 +874,12 @@ static int adjoint_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPl
   b.partials = partials;
   b.gacc = gacc;
   b.tile_flags = nullptr;
-  b.tile_rows = tile_rows_of(*p);
   if (tiled && p->record == kRecordReceivers) {
     uint8_t* flags = reinterpret_cast<uint8_t*>(at(scratch, pl.s_tflags));
-    ERNN_CUDA(launch_tile_flags(p->mode, in->rec_idx, p->nshots, p->nrec, p->nx, p->ny, flags, st, b.tile_rows));
+    ERNN_CUDA(launch_tile_flags(in->rec_idx, p->nshots, p->nrec, p->nx, p->ny, flags, st));
     b.tile_flags = flags;
   }
 
-  // per-shot gradients need one row layout for the whole call: the tiled
-  // kernel only if every step takes it (same buffers every step)
-  if (tiled && pl.ncoef > 1) {
-    AdjStep probe = b;
-    probe.out = LA; probe.cur = LB; probe.prev = LA;
-    probe.u = pl.store_all ? stored(1) : seg(0);
-    if (!tma_adj_would_run(p->mode, probe)) {
-      tiled = 0;
-      g_last_path.store(ERNN_PATH_STEP, std::memory_order_relaxed);
-    }
-  }
-  const bool tiled_adj = tiled != 0;
   // every step launch after the first of the loop below follows a step kernel
   bool chained = false;
   auto adj_step = [&](int m, const float* um) -> int {
@@ -916,7 +892,7 @@ static int adjoint_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPl
     b.frame = ((m - 1) % p->stride == 0) ? (m - 1) / p->stride : -1;
     b.chained = chained ? 1 : 0;
     chained = true;
-    const cudaError_t e = tiled ? launch_tma_adj(p->mode, b, &coef->err, st) : launch_adj_step(p->mode, b, st);
+    const cudaError_t e = tiled ? launch_tma_adj(b, &coef->err, st) : launch_adj_step(p->mode, b, st);
     return e == cudaSuccess ? ERNN_OK : ERNN_ERR_CUDA;
   };
 
@@ -925,39 +901,27 @@ static int adjoint_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPl
       if ((rc = adj_step(m, stored(m)))) return rc;
   } else {
     FwdStep a = base_fwd(*p, *in, coef, pl.nt_out);
-    a.tile_rows = b.tile_rows;
     for (int j = pl.nseg - 1; j >= 0; --j) {
       const int i0 = j * pl.k, i1 = (j + 1) * pl.k < p->nt ? (j + 1) * pl.k : p->nt;
       // recompute u^{i0+1} .. u^{i1} into the segment buffer; u^{nt} is never
       // imaged, so the last segment stops one step short
       const int iend = i1 < p->nt ? i1 : p->nt - 1;
-      // on the tiled path, pairs of steps go through the two-step kernel
-      for (int i = i0; i < iend;) {
+      for (int i = i0; i < iend; ++i) {
         a.i = i;
         a.out = seg(i - i0);
         a.cur = (i == i0) ? ck(j, 0) : seg(i - i0 - 1);
         a.prev = (i == i0) ? ck(j, 1) : (i == i0 + 1 ? ck(j, 0) : seg(i - i0 - 2));
         a.chained = chained ? 1 : 0;
         chained = true;
-        a.out2 = (tiled && i + 1 < iend) ? seg(i + 1 - i0) : nullptr;
-        if (a.out2 != nullptr && tma_fwd2_would_run(p->mode, a)) {
-          ERNN_CUDA(launch_tma_fwd2(p->mode, a, &coef->err, st));
-          i += 2;
-          continue;
-        }
-        a.out2 = nullptr;
-        ERNN_CUDA(tiled ? launch_tma_fwd(p->mode, a, &coef->err, st) : launch_fwd_step(p->mode, a, st));
-        ++i;
+        ERNN_CUDA(tiled ? launch_tma_fwd(a, &coef->err, st) : launch_fwd_step(p->mode, a, st));
       }
       for (int m = i1; m >= i0 + 1; --m)
         if ((rc = adj_step(m, seg(m - 1 - i0)))) return rc;
     }
   }
   if (p->mode == kModeScalar && pl.ncoef > 1) {
-    // per-shot gradients: the tiled kernel keeps kTiledRowsPerShot rows per
-    // shot, the plain kernel one row per block (blocks of a shot contiguous)
-    const int rows = tiled_adj ? kTiledRowsPerShot : pl.nblocks / p->nshots;
-    ERNN_CUDA(launch_finalize_scalar(partials, rows, coef, grad_C, st, p->nshots, 1));
+    // per-shot gradients: one row per block, blocks of a shot contiguous
+    ERNN_CUDA(launch_finalize_scalar(partials, pl.nblocks / p->nshots, coef, grad_C, st, p->nshots, 1));
   } else if (p->mode == kModeScalar) {
     ERNN_CUDA(launch_finalize_scalar(partials, pl.nblocks, coef, grad_C, st));
   } else {

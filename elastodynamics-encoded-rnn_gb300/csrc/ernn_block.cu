@@ -96,7 +96,6 @@ struct Q4 {
 };
 __device__ __forceinline__ Q4 q4(const float4 v) { return Q4{{v.x, v.y, v.z, v.w}}; }
 __device__ __forceinline__ float4 f4(const Q4& q) { return make_float4(q.v[0], q.v[1], q.v[2], q.v[3]); }
-__device__ __forceinline__ Q4 zero_q4() { return Q4{{0.f, 0.f, 0.f, 0.f}}; }
 
 // One row of a component: the quad (w[1] .. w[4]) and the cells beside it.
 struct Row {
@@ -348,7 +347,7 @@ __global__ void __launch_bounds__(32 * W, CTAS)
       const uint32_t st = a.out[t] != nullptr ? stored : 0u;
       auto rows = [&](auto plain) {
         constexpr bool PLAIN = decltype(plain)::value;
-        float wn[4], wv[4];
+        [[maybe_unused]] float wn[4], wv[4];
         if constexpr (MODE == kModeDField) weights(0, wn);
         Row t0 = load_row(c0 - kBox), t1 = load_row(c0 + B::kPlane - kBox);
         Row m0 = load_row(c0), m1 = load_row(c0 + B::kPlane);
@@ -1066,6 +1065,28 @@ __global__ void __launch_bounds__(32 * W, 1)
   }
 }
 
+// ------------------------------------------------------- instance tiles
+// Block b writes the tiles of instance d.id[b] (entry base[b] + xt * tiles_y
+// + yt for the tile at rows x0 + 16 xt, columns y0 + 64 yt) and its box.
+__global__ void inst_table_kernel(const InstDesc d, int4* __restrict__ tiles, int4* __restrict__ box) {
+  const int b = blockIdx.x;
+  const int k = d.id[b];
+  const int tiles_y = (d.ny[b] + d.tile_cols - 1) / d.tile_cols;
+  const int n = tiles_y * ((d.nx[b] + d.tile_rows - 1) / d.tile_rows);
+  for (int t = threadIdx.x; t < n; t += blockDim.x) {
+    const int xt = t / tiles_y, yt = t - xt * tiles_y;
+    // the entry: instance, tile origin, instance region (16-bit pairs)
+    const unsigned rx = (unsigned)(d.x0[b] + d.tile_rows * xt), ry = (unsigned)(d.y0[b] + d.tile_cols * yt);
+    const unsigned xs = (unsigned)d.x0[b], ys = (unsigned)d.y0[b];
+    const unsigned xe = xs + (unsigned)d.nx[b], ye = ys + (unsigned)d.ny[b];
+    tiles[d.base[b] + t] = make_int4(k, (int)(rx | (ry << 16)), (int)(xs | (ys << 16)), (int)(xe | (ye << 16)));
+  }
+  if (threadIdx.x == 0) {
+    box[2 * k] = make_int4(d.x0[b], d.y0[b], d.x0[b] + d.nx[b], d.y0[b] + d.ny[b]);
+    box[2 * k + 1] = make_int4(d.base[b], tiles_y, d.nt[b], 0);
+  }
+}
+
 // ------------------------------------------------- receivers of the tiles
 // The receivers whose cells lie in a tile with its halo, for every tile of a
 // call: tile[t] = (first entry, entries), an entry = (cell in the tile's
@@ -1291,6 +1312,11 @@ int blk_geometry(int nx, int ny, int S) {
 }
 
 bool blk_available() { return blk_encode_fn() != nullptr; }
+
+cudaError_t launch_inst_table(const InstDesc& d, int4* tiles, int4* box, cudaStream_t st) {
+  if (d.count < 1) return cudaSuccess;
+  return tracked_launch(kProfOther, st, [&] { inst_table_kernel<<<d.count, 256, 0, st>>>(d, tiles, box); });
+}
 
 size_t blk_rec_bytes(size_t ntiles, int S, int nrec) {
   return (ntiles + 2) / 2 * 8 + ntiles * sizeof(int2) + 4 * (size_t)S * nrec * sizeof(int2);

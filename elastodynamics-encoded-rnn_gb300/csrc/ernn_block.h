@@ -10,6 +10,17 @@ namespace ernn {
 constexpr int kBlkSteps = 4;       // most time steps of one launch (and halo rows / columns of a tile)
 constexpr int kBlkCols = 120;      // columns of a tile (a warp's 128 less one quad each side)
 
+// Instances on one canvas (ERNN_FLAG_INSTANCES): the kernels walk a tile
+// table instead of the grid's tiling.  Entry t of the table is one tile's
+// instance, origin and instance region (16-bit pairs); per instance k, box[2k] =
+// (x0, y0, x1, y1) of its region and box[2k + 1] = (first table entry of its
+// tiles, tiles per tile row, steps, 0).
+struct InstTiles {
+  const int4* tiles;   // the table, instances ordered by decreasing step count
+  const int4* box;     // per instance (region, tiling and step count)
+  int ntiles;          // entries of this launch: the prefix of running instances
+};
+
 // Forward: u^{i+1} .. u^{i+T} from (u^i, u^{i-1}).
 struct BlkFwd {
   int geo;                         // tile geometry (blk_geometry)
@@ -72,6 +83,21 @@ constexpr int kBlkTall = 0, kBlkShort = 1, kBlkFlat = 2;
 int blk_geometry(int nx, int ny, int S);
 int blk_tile_rows(int geo);
 size_t blk_tiles(int geo, int nx, int ny);
+// Partial-sum rows reserved per shot with per-shot constants (an adjoint grid
+// never exceeds this many CTAs).
+constexpr int kTiledRowsPerShot = 1024;
+// Instances on a canvas (ERNN_FLAG_INSTANCES), passed by value to the kernel
+// that writes the tile table: in the order of decreasing step count, each
+// with its caller-side index.
+constexpr int kMaxInstances = 256;
+struct InstDesc {
+  int count, tile_rows, tile_cols;
+  int id[kMaxInstances], x0[kMaxInstances], y0[kMaxInstances], nx[kMaxInstances];
+  int ny[kMaxInstances], nt[kMaxInstances], base[kMaxInstances];
+};
+// Writes the tile table (in the order of d) and the per-instance boxes
+// (2 x S int4) described in InstTiles.
+cudaError_t launch_inst_table(const InstDesc& d, int4* tiles, int4* box, cudaStream_t st);
 // Receivers of the tiles of a call: room for `ntiles` tiles, and the table
 // (box: instances, else nullptr).
 size_t blk_rec_bytes(size_t ntiles, int S, int nrec);
