@@ -523,6 +523,7 @@ int block_adjoint(const ErnnProblem& p, const Plan& pl, const ErnnInputs& in, co
   BlkAdj b;
   std::memset(&b, 0, sizeof(b));
   b.geo = pl.geo;
+  b.plain_order = a.plain_order;
   b.nx = p.nx; b.ny = p.ny; b.pitch = pl.pitch; b.S = p.nshots; b.nt = p.nt;
   b.u_stride = pl.state_bytes / sizeof(float);
   b.g_x = g_ux; b.g_y = g_uy;

@@ -134,7 +134,10 @@ __device__ __forceinline__ Sums sums_of(const Row& t, const Row& m, const Row& b
 // product is rounded is an argument (kOrder*), so that a problem's states
 // agree bit for bit with those of the per-step kernels of its size and mode:
 // the first in the tiled ones, the second in the plain ones (with constant
-// planes: the second of the x row, the first of the y row).
+// planes: the second of the x row, the first of the y row).  The same for the
+// adjoint: its constants' sums cancel to a small part of their terms, and a
+// lam of another rounding moved single constants' gradients by up to 3e-5 of
+// their value (the plain kernels' own distance from 64 bits is as large).
 constexpr int kOrderTiled = 0, kOrderPlain = 3, kOrderFields = 1;
 template <int ORDER>
 __device__ __forceinline__ void oper(const Coefs& k, const Sums& x, const Sums& y, float& lx, float& ly) {
@@ -450,12 +453,14 @@ __global__ void __launch_bounds__(32 * W, CTAS)
 // ----------------------------------------------------------------- adjoint
 // As the forward, with lam^{m+1}, lam^{m+2} in the levels' place and no
 // load: the recorded residuals enter at the receivers' cells (subtracted
-// from lam^{m+2} before the update) or at every cell (dense history).  The
+// from lam^{m+2} before the update, as the tiled per-step kernels do; added
+// to lam^m after it in the plain kernels' order) or at every cell (dense
+// history).  The
 // six imaging sums sum_cells lam . (dA/dC_k u) are formed in the transposed
 // form sum_cells u . (dA/dC_k lam) (the second differences with zero ghosts
 // are symmetric), which needs u^m only at the cell itself, read from global
 // memory one row ahead.
-template <int W, int RW, bool INST, int CTAS>
+template <int W, int RW, bool INST, int ORDER, int CTAS>
 __global__ void __launch_bounds__(32 * W, CTAS)
     blk_adj_kernel(const BlkAdj a, const __grid_constant__ CUtensorMap cur_map,
                    const __grid_constant__ CUtensorMap prev_map, int tiles_x, int tiles_y, int ntiles, int* err) {
@@ -573,15 +578,17 @@ __global__ void __launch_bounds__(32 * W, CTAS)
       const bool dense = frame >= 0 && a.record == kRecordFields;
       float* lc = (t & 1) ? lev0 : lev1;
       float* lp = (t & 1) ? lev1 : lev0;
-      if (frame >= 0 && recs.y > 0) {  // lam^m = ... - (lam^{m+2} - g) + ...
+      const bool inject = frame >= 0 && recs.y > 0;
+      auto add_residuals = [&](float gss) {
         const size_t o = ((size_t)tile.inst * a.nt_out + frame) * a.nrec;
         for (int e = tid; e < recs.y; e += NT) {
           const int2 v = a.rec_ent[recs.x + e];
-          atomicAdd(&lp[v.x], -gs * a.g_x[o + v.y]);
-          atomicAdd(&lp[B::kPlane + v.x], -gs * a.g_y[o + v.y]);
+          atomicAdd(&lp[v.x], gss * a.g_x[o + v.y]);
+          atomicAdd(&lp[B::kPlane + v.x], gss * a.g_y[o + v.y]);
         }
         __syncthreads();
-      }
+      };
+      if (ORDER == kOrderTiled && inject) add_residuals(-gs);  // lam^m = ... - (lam^{m+2} - g) + ...
       const float* c0 = lc + o0;  // lam^{m+1}
       float* p0 = lp + o0;        // lam^{m+2}, becomes lam^m
       float* out = t == a.T ? a.out_last : (t == a.T - 1 ? a.out_before : nullptr);
@@ -623,7 +630,7 @@ __global__ void __launch_bounds__(32 * W, CTAS)
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               const Sums sx = sums_of(t0, m0, b0, q), sy = sums_of(t1, m1, b1, q);
-              oper<kOrderTiled>(ks, sx, sy, v0[q], v1[q]);
+              oper<ORDER>(ks, sx, sy, v0[q], v1[q]);
               acc[0] = fmaf(ux[q], sx.xx, acc[0]);
               acc[1] = fmaf(uy[q], sy.yy, acc[1]);
               acc[2] = fmaf(ux[q], sy.xy, fmaf(uy[q], sx.xy, acc[2]));
@@ -672,7 +679,21 @@ __global__ void __launch_bounds__(32 * W, CTAS)
         }
       }
       __syncthreads();  // lam^m is complete
+      if (ORDER != kOrderTiled && inject) {  // ... but for the residuals: lam^m = (...) + g
+        add_residuals(gs);
+        if (out != nullptr) {
+          for (int e = tid; e < recs.y; e += NT) {
+            const int c = a.rec_ent[recs.x + e].x, rr = c / kBox, cc = c % kBox;
+            if (rr < kH || rr >= B::kRows - kH || cc < kH || cc >= kBox - kH) continue;  // another tile's
+            float* o = out + (ptrdiff_t)tile.plane * 2 * (ptrdiff_t)Np + (ptrdiff_t)(tile.x0 - kH + rr) * a.pitch +
+                       (tile.y0 - kH + cc);
+            o[0] = lp[c];
+            o[Np] = lp[B::kPlane + c];
+          }
+        }
+      }
     }
+    if (ORDER != kOrderTiled) __syncthreads();  // the stored receivers' cells are read: the next tile may arrive
   }
   if (tid == 0 && pipe_failed(&guard)) pipe_drain(bar, 1, &guard);
   flush(per_shot ? acc_shot : 0);
@@ -1215,14 +1236,14 @@ cudaError_t fwd_t(const BlkFwd& a, int* err, cudaStream_t st) {
   }, cells * 8.0 * (stores + (a.cur ? 1 : 0) + (a.prev ? 1 : 0)));
 }
 
-template <int W, int RW, int CTAS, bool INST>
+template <int W, int RW, int CTAS, bool INST, int ORDER>
 cudaError_t adj_t(const BlkAdj& a, int* err, cudaStream_t st) {
   using B = BlkTile<W, RW>;
   constexpr size_t smem = B::kBytes;
   static std::once_flag once;
   static cudaError_t ready = cudaSuccess;
   std::call_once(once, [] {
-    ready = cudaFuncSetAttribute(blk_adj_kernel<W, RW, INST, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    ready = cudaFuncSetAttribute(blk_adj_kernel<W, RW, INST, ORDER, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
   if (ready != cudaSuccess) return ready;
   const int planes = INST ? 1 : a.S;
@@ -1237,7 +1258,7 @@ cudaError_t adj_t(const BlkAdj& a, int* err, cudaStream_t st) {
   const int grid = ntiles < slots ? ntiles : slots;
   const double cells = INST ? (double)ntiles * B::kUse * kBlkCols : (double)a.S * a.nx * a.ny;
   return tracked_launch(kProfAdjoint, st, [&] {
-    launch_step_kernel(blk_adj_kernel<W, RW, INST, CTAS>, dim3(grid), dim3(32 * W), smem, st, a.chained != 0, a, cm, pm,
+    launch_step_kernel(blk_adj_kernel<W, RW, INST, ORDER, CTAS>, dim3(grid), dim3(32 * W), smem, st, a.chained != 0, a, cm, pm,
                        tiles_x, tiles_y, ntiles, err);
   }, cells * 8.0 * (a.T + (a.T > 1 ? 2 : 1) + (a.cur ? 1 : 0) + (a.prev ? 1 : 0)));
 }
@@ -1352,6 +1373,13 @@ cudaError_t fwd_geo(const BlkFwd& a, int* err, cudaStream_t st) {
   if (a.geo == kBlkShort) return fwd_t<MODE, 16, 2, 1, false, ORDER>(a, err, st);
   return fwd_t<MODE, 8, 6, 2, false, ORDER>(a, err, st);
 }
+
+template <int ORDER>
+cudaError_t adj_geo(const BlkAdj& a, int* err, cudaStream_t st) {
+  if (a.geo == kBlkFlat) return adj_t<16, 1, 1, false, ORDER>(a, err, st);
+  if (a.geo == kBlkShort) return adj_t<16, 2, 1, false, ORDER>(a, err, st);
+  return adj_t<8, 6, 2, false, ORDER>(a, err, st);
+}
 }  // namespace
 
 cudaError_t launch_blk_fwd(int mode, const BlkFwd& a, int* err, cudaStream_t st) {
@@ -1368,10 +1396,8 @@ cudaError_t launch_blk_adj(int mode, const BlkAdj& a, int* err, cudaStream_t st)
     if (a.geo == kBlkShort) return adj_d_t<16, 2, 1>(a, err, st);
     return adj_d_t<8, 6, 2>(a, err, st);
   }
-  if (a.inst.tiles != nullptr) return adj_t<8, 6, 2, true>(a, err, st);
-  if (a.geo == kBlkFlat) return adj_t<16, 1, 1, false>(a, err, st);
-  if (a.geo == kBlkShort) return adj_t<16, 2, 1, false>(a, err, st);
-  return adj_t<8, 6, 2, false>(a, err, st);
+  if (a.inst.tiles != nullptr) return adj_t<8, 6, 2, true, kOrderTiled>(a, err, st);
+  return a.plain_order ? adj_geo<kOrderPlain>(a, err, st) : adj_geo<kOrderTiled>(a, err, st);
 }
 
 }  // namespace ernn

@@ -53,6 +53,7 @@ struct BlkFwd {
 // lam^{m_hi+2}), and the imaging sums of the pairs (lam^{m+1}, u^m).
 struct BlkAdj {
   int geo;
+  int plain_order;      // as in BlkFwd
   int nx, ny, pitch, S, nt, m_hi, T;
   const float* cur;     // lam^{m_hi+1}, nullptr: zero
   const float* prev;    // lam^{m_hi+2}, nullptr: zero

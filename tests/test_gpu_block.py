@@ -71,6 +71,24 @@ def test_every_cell_a_receiver(mode):
     assert rel(ag, bg) <= 1e-5, rel(ag, bg)
 
 
+@pytest.mark.parametrize("kw,ckpt_k", [
+    (dict(nx=170, ny=133, nt=300, S=3, record=O.RECORD_RECEIVERS, nrec=40), 9),
+    (dict(nx=130, ny=361, nt=250, stride=3, record=O.RECORD_RECEIVERS, nrec=1500), None),
+    (dict(nx=145, ny=79, nt=400, stride=2), None),
+    (dict(nx=330, ny=437, nt=120, S=9, record=O.RECORD_RECEIVERS, nrec=60), 20),  # several tiles per CTA
+])
+def test_gradient_of_each_constant_follows_the_plain_kernels(kw, ckpt_k):
+    """The adjoint states are the plain kernels' bit for bit, so only the order
+    of the imaging sums differs: FP32 over a thread's cells of one step (24 at
+    most: 2^-24 sqrt(24) = 3e-7 of the terms, averaged over the steps)."""
+    case = random_case(**kw)
+    wx, wy = weights(case)
+    ax, ay, ag, used = run(case, wx, wy, E.PATH_AUTO, ckpt_k)
+    bx, by, bg, _ = run(case, wx, wy, E.PATH_STEP, ckpt_k)
+    assert used == E.PATH_TILED
+    assert np.all(np.abs(ag - bg) <= 1e-6 * np.abs(bg) + 1e-7 * np.abs(bg).max()), (ag, bg)
+
+
 def test_large_odd_grid_vs_fp64_oracle():
     case = random_case(nx=330, ny=437, nt=60, S=5, record=O.RECORD_RECEIVERS, nrec=60)
     wx, wy = weights(case)
