@@ -59,11 +59,17 @@ inline bool plain_size(const ErnnProblem& p) {
 //  - ERNN_PATH_AUTO takes rows of any length from kBlockMinCols up (a warp
 //    spans 120 columns: narrower grids leave most lanes idle, the plain
 //    kernels take those); states of odd rows are padded to 16-byte rows.
+//    (16 x 941x41, 200 steps: 5.11 ms there, 4.98 here; 5 x 1000x41: 3.05, 2.52.)
 //    Where the cluster-resident path can run it comes first.
 //  - A degradation map: grids of the plain kernels' size.  On larger ones the
 //    TMA-fed kernels of one step are faster (8 x 512^2: 29 against 33 us per
 //    forward and adjoint step): the map, u's rows and the running gradient
 //    are read at every step either way, here from L2 by the threads.
+//    Tiles that a narrow grid leaves half empty cost more than the plain
+//    kernels' step: a forward and an adjoint step take about 2 us + 0.7 of
+//    the cost of the launch here, 6 us + 20 us per million cells there
+//    (measured, us per iteration, plain -> here: 7 x 563x51 1516 -> 2022, 7 x
+//    595x72 2684 -> 2721, 8 x 98x560 3267 -> 2644, 1 x 563x51 1468 -> 1055).
 //  - Six constant planes: up to kBlockMaxFields cells, where launches set the
 //    time (301^2: 36.1 against 21.9 ms per 4001-step iteration).
 bool block_rule(const ErnnProblem& p) {
@@ -71,7 +77,10 @@ bool block_rule(const ErnnProblem& p) {
   if (p.path == ERNN_PATH_TILED) return p.mode == kModeScalar && p.ny % 4 == 0;
   if (p.path != ERNN_PATH_AUTO || p.ny < kBlockMinCols) return false;
   if (p.mode == kModeFields) return (double)p.nshots * p.nx * p.ny <= kBlockMaxFields;
-  if (p.mode == kModeDField) return plain_size(p);
+  if (p.mode == kModeDField) {
+    const double cost = blk_cost(blk_geometry(p.nx, p.ny, p.nshots), p.nx, p.ny, p.nshots);
+    return plain_size(p) && (cost <= 10.0 || cost <= 6.0 + 31e-6 * p.nshots * p.nx * p.ny);
+  }
   return !resident_possible(p.mode, p.nx, p.ny);
 }
 

@@ -1323,11 +1323,15 @@ size_t blk_tiles(int geo, int nx, int ny) {
 // SMs, mean of a forward and an adjoint launch of four steps (measured at
 // one shot of 301^2 and 512^2, three of 501 x 389, eight of 640 x 720).  From
 // sizes alone, as the workspace layout depends on it.
+double blk_cost(int geo, int nx, int ny, int S) {
+  const double sms = 152.0, tiles = S * (double)blk_tiles(geo, nx, ny);
+  if (geo == kBlkTall) return tiles <= sms ? 21.0 : 20.0 * std::ceil(tiles / (2.0 * sms));
+  return (geo == kBlkShort ? 9.4 : 5.0) * std::ceil(tiles / sms);
+}
+
 int blk_geometry(int nx, int ny, int S) {
-  const double sms = 152.0;
-  auto tiles = [&](int geo) { return S * (double)blk_tiles(geo, nx, ny); };
-  const double tall = tiles(kBlkTall) <= sms ? 21.0 : 20.0 * std::ceil(tiles(kBlkTall) / (2.0 * sms));
-  const double low = 9.4 * std::ceil(tiles(kBlkShort) / sms), flat = 5.0 * std::ceil(tiles(kBlkFlat) / sms);
+  const double tall = blk_cost(kBlkTall, nx, ny, S), low = blk_cost(kBlkShort, nx, ny, S);
+  const double flat = blk_cost(kBlkFlat, nx, ny, S);
   if (flat < low && flat < tall) return kBlkFlat;
   return low < tall ? kBlkShort : kBlkTall;
 }

@@ -82,6 +82,7 @@ struct BlkAdj {
 // tiles of an nx x ny grid.
 constexpr int kBlkTall = 0, kBlkShort = 1, kBlkFlat = 2;
 int blk_geometry(int nx, int ny, int S);
+double blk_cost(int geo, int nx, int ny, int S);  // us of a launch of four steps (scalar constants)
 int blk_tile_rows(int geo);
 size_t blk_tiles(int geo, int nx, int ny);
 // Partial-sum rows reserved per shot with per-shot constants (an adjoint grid

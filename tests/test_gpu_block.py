@@ -89,6 +89,20 @@ def test_gradient_of_each_constant_follows_the_plain_kernels(kw, ckpt_k):
     assert np.all(np.abs(ag - bg) <= 1e-6 * np.abs(bg) + 1e-7 * np.abs(bg).max()), (ag, bg)
 
 
+@pytest.mark.parametrize("mode,S,nx,ny,path", [
+    (O.MODE_SCALAR, 16, 941, 41, E.PATH_TILED), (O.MODE_DFIELD, 8, 98, 559, E.PATH_TILED),
+    (O.MODE_DFIELD, 7, 563, 51, E.PATH_STEP), (O.MODE_DFIELD, 1, 563, 51, E.PATH_TILED),
+])
+def test_narrow_grids_on_either_side_of_the_cost_rule(mode, S, nx, ny, path):
+    case = random_case(nx=nx, ny=ny, nt=9, S=S, mode=mode, record=O.RECORD_RECEIVERS, nrec=12)
+    wx, wy = weights(case)
+    ax, ay, ag, used = run(case, wx, wy, E.PATH_AUTO, 4)
+    bx, by, bg, _ = run(case, wx, wy, E.PATH_STEP, 4)
+    assert used == path
+    assert np.array_equal(ax, bx) and np.array_equal(ay, by)
+    assert rel(ag, bg) <= 1e-5, rel(ag, bg)
+
+
 def test_large_odd_grid_vs_fp64_oracle():
     case = random_case(nx=330, ny=437, nt=60, S=5, record=O.RECORD_RECEIVERS, nrec=60)
     wx, wy = weights(case)
