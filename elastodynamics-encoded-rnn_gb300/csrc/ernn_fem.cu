@@ -18,6 +18,7 @@
 // State layout: [i][j] with j (y) fastest, the layout of the saved frames
 // (nt_out, nx, ny); node (i, j) is the generator's node j*nx + i.
 #include <cmath>
+#include <cstdint>
 #include <cstring>
 
 #include "ernn.h"
@@ -186,6 +187,212 @@ FemConsts fem_consts(const ErnnFemProblem& p) {
   return k;
 }
 
+// ------------------------------------------- several levels per launch
+// Uniform constants: the force on a node is one linear stencil per node
+// parity, sum over its neighbours of K_b (u_b - u), with K summed over the
+// node's triangles on the host in double (an odd node's triangles reach its
+// four edge neighbours, an even one's all eight; the rows of K sum to zero, so
+// the centre enters through the differences).  16 to 32 multiply-adds a node
+// instead of 120 to 240 operations and two divisions of the element form, and
+// no divergence: a warp holds a row of 128 nodes, a lane four columns, whose
+// parities are the same in every lane.  With so little arithmetic a level is
+// bound by its launch, so a launch advances a tile up to H levels, the state
+// of a thread's nodes in registers, rows exchanged through shared memory (one
+// CTA barrier per level), H outer rows and columns of the tile not stored.
+// 2001 levels of 301^2 nodes: 10.2 ms with one level a launch, 2.4 ms here
+// (4.8 us a launch of four levels; 16 rows with H = 4 against 24 with 8: 2.5
+// ms, 24 with 4: 3.7, 14 with 3 and 20 with 4 slower).
+//
+// The state is u^n and its difference to u^{n-1}, not the two levels: a
+// rounding of u then moves u once, where in 2 u^n - u^{n-1} it would enter
+// every later level.  Error against 64 bits after 2001 levels: 1e-6 (the one-
+// level kernel: 1e-5 on 301^2 nodes, 4e-5 on 61^2).
+struct FemStencil {
+  float e[8][4];  // even nodes: (-1,-1) (-1,0) (-1,1) (0,-1) (0,1) (1,-1) (1,0) (1,1); xx, xy, yx, yy
+  float o[4][4];  // odd nodes: (-1,0) (0,-1) (0,1) (1,0)
+  float dt2, rho_inv, scale;
+};
+
+struct FemBlock {
+  int nx, ny, pitch, n, T;   // levels n + 1 .. n + T from u^n and its difference to u^{n-1}
+  const float* cur;          // [2][nx][pitch], nullptr: zero
+  const float* diff;         // u^n - u^{n-1}
+  float* out;                // u^{n+T} and the difference to the level before it
+  float* out_diff;
+  const float* load;
+  const float* signal;
+  float* frames_x;
+  float* frames_y;
+  int stride;
+};
+
+template <int W, int H>
+__global__ void __launch_bounds__(32 * W) fem_block_kernel(const FemBlock a, const FemStencil k) {
+  constexpr int kCols = 128 - 8 * ((H + 3) / 4), kLeft = 4 * ((H + 3) / 4);  // stored columns, halo columns
+  __shared__ float4 ex[2][2][W][32];  // [parity][component][row][quad]
+  grid_dep_trigger();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int gi = (int)blockIdx.y * (W - 2 * H) + w - H;
+  const int gj = (int)blockIdx.x * kCols - kLeft + 4 * lane;
+  const int nx = a.nx, ny = a.ny;
+  const size_t N = (size_t)nx * ny, Np = (size_t)nx * a.pitch;
+  const bool row_in = gi >= 0 && gi < nx;
+  const int nq = row_in && gj >= 0 ? max(0, min(4, ny - gj)) : 0;
+  const bool stored = w >= H && w < W - H && 4 * lane >= kLeft && 4 * lane < kLeft + kCols && nq > 0;
+  bool inside[4];  // nodes that move: the edges are fixed at zero
+  float ld[4], cx[4], cy[4], dx_[4], dy_[4];  // u^n and u^n - u^{n-1}
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    inside[q] = gi > 0 && gi < nx - 1 && gj + q > 0 && gj + q < ny - 1;
+    ld[q] = inside[q] ? a.load[(size_t)gi * ny + gj + q] : 0.f;  // (written by no launch: before the wait)
+  }
+  grid_dep_wait();  // levels of the previous launch complete from here on
+  const ptrdiff_t off = (ptrdiff_t)gi * a.pitch + gj;
+  auto load_level = [&](const float* s, float(&x)[4], float(&y)[4]) {
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool in = s != nullptr && nq > 0;
+    const float4 vx = in ? __ldcg(reinterpret_cast<const float4*>(s + off)) : z;
+    const float4 vy = in ? __ldcg(reinterpret_cast<const float4*>(s + off + Np)) : z;
+    x[0] = vx.x; x[1] = vx.y; x[2] = vx.z; x[3] = vx.w;
+    y[0] = vy.x; y[1] = vy.y; y[2] = vy.z; y[3] = vy.w;
+  };
+  load_level(a.cur, cx, cy);
+  load_level(a.diff, dx_, dy_);
+  const bool even_row = (gi & 1) == 0;  // node (gi, gj + q) has the parity of gi + q
+  for (int t = 1; t <= a.T; ++t) {
+    ex[t & 1][0][w][lane] = make_float4(cx[0], cx[1], cx[2], cx[3]);
+    ex[t & 1][1][w][lane] = make_float4(cy[0], cy[1], cy[2], cy[3]);
+    __syncthreads();
+    if (row_in && w >= t && w < W - t) {
+      // windows of rows gi - 1, gi, gi + 1: columns gj - 1 .. gj + 4
+      float ux[3][6], uy[3][6];
+      auto window = [&](const float4& v, float(&u)[6]) {
+        u[0] = __shfl_up_sync(0xffffffffu, v.w, 1);
+        u[1] = v.x; u[2] = v.y; u[3] = v.z; u[4] = v.w;
+        u[5] = __shfl_down_sync(0xffffffffu, v.x, 1);
+      };
+      window(ex[t & 1][0][w - 1][lane], ux[0]);
+      window(ex[t & 1][1][w - 1][lane], uy[0]);
+      window(make_float4(cx[0], cx[1], cx[2], cx[3]), ux[1]);
+      window(make_float4(cy[0], cy[1], cy[2], cy[3]), uy[1]);
+      window(ex[t & 1][0][w + 1][lane], ux[2]);
+      window(ex[t & 1][1][w + 1][lane], uy[2]);
+      const int n = a.n + t - 1;  // this level makes u^{n+1}
+      const float amp = a.signal[n];
+      auto node = [&](int q, bool even) {
+        const float x = cx[q], y = cy[q];
+        float fx = 0.f, fy = 0.f;
+        auto add = [&](const float(&c)[4], int di, int dj) {
+          const float dx = ux[1 + di][q + 1 + dj] - x, dy = uy[1 + di][q + 1 + dj] - y;
+          fx = fmaf(c[0], dx, fmaf(c[1], dy, fx));
+          fy = fmaf(c[2], dx, fmaf(c[3], dy, fy));
+        };
+        if (even) {
+          add(k.e[0], -1, -1); add(k.e[1], -1, 0); add(k.e[2], -1, 1); add(k.e[3], 0, -1);
+          add(k.e[4], 0, 1);   add(k.e[5], 1, -1); add(k.e[6], 1, 0);  add(k.e[7], 1, 1);
+        } else {
+          add(k.o[0], -1, 0); add(k.o[1], 0, -1); add(k.o[2], 0, 1); add(k.o[3], 1, 0);
+        }
+        const float f = k.dt2 * (amp * ld[q] * k.rho_inv);
+        dx_[q] = inside[q] ? dx_[q] - fx : 0.f;
+        dy_[q] = inside[q] ? dy_[q] + (f - fy) : 0.f;
+      };
+      if (even_row) {
+        node(0, true); node(1, false); node(2, true); node(3, false);
+      } else {
+        node(0, false); node(1, true); node(2, false); node(3, true);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        cx[q] += dx_[q];
+        cy[q] += dy_[q];
+      }
+      if (stored && (n + 1) % a.stride == 0) {
+        const size_t o = (size_t)((n + 1) / a.stride) * N + (size_t)gi * ny + gj;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (q < nq) {
+            a.frames_x[o + q] = k.scale * cx[q];
+            a.frames_y[o + q] = k.scale * cy[q];
+          }
+      }
+    }
+  }
+  if (stored) {
+    *reinterpret_cast<float4*>(a.out + off) = make_float4(cx[0], cx[1], cx[2], cx[3]);
+    *reinterpret_cast<float4*>(a.out + off + Np) = make_float4(cy[0], cy[1], cy[2], cy[3]);
+    *reinterpret_cast<float4*>(a.out_diff + off) = make_float4(dx_[0], dx_[1], dx_[2], dx_[3]);
+    *reinterpret_cast<float4*>(a.out_diff + off + Np) = make_float4(dy_[0], dy_[1], dy_[2], dy_[3]);
+  }
+}
+
+// The stencils of both parities: every triangle adjacent to the node adds
+// |J| / 2 (B_a^T C B_b), scaled by dt^2 / m.
+FemStencil fem_stencil(const ErnnFemProblem& p) {
+  const int vi[4][3] = {{0, 1, 1}, {0, 1, 0}, {0, 1, 0}, {1, 1, 0}};
+  const int vj[4][3] = {{0, 0, 1}, {0, 1, 1}, {0, 0, 1}, {0, 1, 1}};
+  // (shape, cell offset, vertex) of the triangles around an even and an odd node
+  const int even[8][4] = {{0, -1, -1, 2}, {1, -1, -1, 1}, {2, 0, -1, 2}, {3, 0, -1, 2},
+                          {2, -1, 0, 1}, {3, -1, 0, 0}, {0, 0, 0, 0}, {1, 0, 0, 0}};
+  const int odd[4][4] = {{3, -1, -1, 1}, {1, 0, -1, 2}, {0, -1, 0, 1}, {2, 0, 0, 0}};
+  const double* C = p.C;  // C11, C22, C12, C16, C26, C66
+  auto build = [&](const int (*tri)[4], int ntri, double K[3][3][4]) {
+    std::memset(K, 0, sizeof(double) * 36);
+    const double m = ntri * p.rho * (p.dx * p.dy / 2.0) / 3.0;
+    for (int t = 0; t < ntri; ++t) {
+      const int T = tri[t][0], A = tri[t][3];
+      const double J00 = (vi[T][1] - vi[T][0]) * p.dx, J01 = (vi[T][2] - vi[T][0]) * p.dx;
+      const double J10 = (vj[T][1] - vj[T][0]) * p.dy, J11 = (vj[T][2] - vj[T][0]) * p.dy;
+      const double det = J00 * J11 - J01 * J10;
+      const double dxi[3] = {-1.0, 1.0, 0.0}, deta[3] = {-1.0, 0.0, 1.0};
+      double bx[3], by[3];
+      for (int b = 0; b < 3; ++b) {
+        bx[b] = (J11 * dxi[b] - J10 * deta[b]) / det;
+        by[b] = (-J01 * dxi[b] + J00 * deta[b]) / det;
+      }
+      const double f = std::fabs(det) / 2.0 * p.dt * p.dt / m;
+      for (int b = 0; b < 3; ++b) {
+        // stresses of a unit x, y displacement of vertex b
+        const double sx[3] = {C[0] * bx[b] + C[3] * by[b], C[2] * bx[b] + C[4] * by[b], C[3] * bx[b] + C[5] * by[b]};
+        const double sy[3] = {C[2] * by[b] + C[3] * bx[b], C[1] * by[b] + C[4] * bx[b], C[4] * by[b] + C[5] * bx[b]};
+        double* c = K[1 + tri[t][1] + vi[T][b]][1 + tri[t][2] + vj[T][b]];
+        c[0] += f * (bx[A] * sx[0] + by[A] * sx[2]);
+        c[1] += f * (bx[A] * sy[0] + by[A] * sy[2]);
+        c[2] += f * (by[A] * sx[1] + bx[A] * sx[2]);
+        c[3] += f * (by[A] * sy[1] + bx[A] * sy[2]);
+      }
+    }
+  };
+  FemStencil s;
+  double K[3][3][4];
+  build(even, 8, K);
+  for (int n = 0, b = 0; n < 9; ++n) {
+    if (n == 4) continue;
+    for (int c = 0; c < 4; ++c) s.e[b][c] = (float)K[n / 3][n % 3][c];
+    ++b;
+  }
+  build(odd, 4, K);
+  const int at[4][2] = {{0, 1}, {1, 0}, {1, 2}, {2, 1}};
+  for (int b = 0; b < 4; ++b)
+    for (int c = 0; c < 4; ++c) s.o[b][c] = (float)K[at[b][0]][at[b][1]][c];
+  s.dt2 = (float)(p.dt * p.dt);
+  s.rho_inv = (float)(1.0 / p.rho);
+  s.scale = (float)p.out_scale;
+  return s;
+}
+
+// Which uniform runs take several levels per launch: those of up to seven
+// levels per node across the grid's narrower side.  The one-level kernel's
+// rounding noise grows with the crossings of the grid, about 1.5e-6 of the
+// field per (levels / nodes across) (61^2, 120^2, 200^2, 301^2 nodes, 430 to
+// 2001 levels), and the two kernels' frames part by as much: up to this line
+// by 1.6e-5 at most in what was measured.  Longer runs on small grids keep the
+// element form, and with it their frames.
+constexpr int kFemCrossings = 7;
+inline bool fem_block_rule(const ErnnFemProblem& p) {
+  return p.nt <= (int64_t)kFemCrossings * (p.nx < p.ny ? p.nx : p.ny);
+}
+
 constexpr size_t kFemAlign = 256;
 inline size_t fem_align(size_t v) { return (v + kFemAlign - 1) / kFemAlign * kFemAlign; }
 
@@ -196,7 +403,9 @@ using namespace ernn;
 
 extern "C" size_t ernn_fem_workspace_bytes(const ErnnFemProblem* p) {
   if (p == nullptr || p->nx < 2 || p->ny < 2) return 0;
-  return 6 * fem_align((size_t)p->nx * p->ny * sizeof(float));
+  // four levels of both components with rows padded to 16 bytes (several
+  // levels per launch), at least three unpadded ones
+  return 8 * fem_align((size_t)p->nx * ((p->ny + 3) / 4 * 4) * sizeof(float));
 }
 
 extern "C" int ernn_fem_forward(const ErnnFemProblem* p, const float* load, const float* signal,
@@ -216,6 +425,49 @@ extern "C" int ernn_fem_forward(const ErnnFemProblem* p, const float* load, cons
   if (workspace_bytes < ernn_fem_workspace_bytes(p)) return ERNN_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
   const size_t N = (size_t)p->nx * p->ny;
+  const int nt_out = (p->nt + p->stride - 1) / p->stride;
+  // frames of the levels that are never computed (0, and 1 when stride is 1)
+  for (int f = 0; f < nt_out && f * p->stride <= 1; ++f) {
+    if (cudaMemsetAsync(frames_x + (size_t)f * N, 0, N * sizeof(float), st) != cudaSuccess ||
+        cudaMemsetAsync(frames_y + (size_t)f * N, 0, N * sizeof(float), st) != cudaSuccess)
+      return ERNN_ERR_CUDA;
+  }
+  if (C_fields == nullptr && fem_block_rule(*p) && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0) {
+    // uniform constants: kH levels per launch, each from one pair of working
+    // states into the other (levels 0 and 1 are zero)
+    constexpr int kW = 16, kH = 4, kCols = 128 - 8 * ((kH + 3) / 4);
+    const int pitch = (p->ny + 3) / 4 * 4;
+    const size_t lev = fem_align((size_t)p->nx * pitch * sizeof(float)) / sizeof(float);
+    float* w = static_cast<float*>(workspace);
+    FemBlock a;
+    std::memset(&a, 0, sizeof(a));
+    a.nx = p->nx; a.ny = p->ny; a.pitch = pitch;
+    a.load = load;
+    a.signal = signal;
+    a.frames_x = frames_x;
+    a.frames_y = frames_y;
+    a.stride = p->stride;
+    const FemStencil k = fem_stencil(*p);
+    const dim3 grid((p->ny + kCols - 1) / kCols, (p->nx + kW - 2 * kH - 1) / (kW - 2 * kH), 1);
+    int pair = 0;
+    for (int n = 1; n < p->nt - 1;) {
+      const int left = p->nt - 1 - n;
+      a.n = n;
+      a.T = left < kH ? left : kH;
+      a.out = w + (size_t)(4 * pair) * lev;
+      a.out_diff = a.out + 2 * lev;
+      const bool chained = n > 1;  // the previous launch is the previous levels'
+      const cudaError_t e = tracked_launch(kProfForward, st, [&] {
+        launch_step_kernel(fem_block_kernel<kW, kH>, grid, dim3(32 * kW), 0, st, chained, a, k);
+      }, (double)N * 28.0 * a.T);
+      if (e != cudaSuccess) return ERNN_ERR_CUDA;
+      a.cur = a.out;
+      a.diff = a.out_diff;
+      pair ^= 1;
+      n += a.T;
+    }
+    return ERNN_OK;
+  }
   const size_t lev = fem_align(N * sizeof(float));
   char* w = static_cast<char*>(workspace);
   float* ux[3];
@@ -226,13 +478,6 @@ extern "C" int ernn_fem_forward(const ErnnFemProblem* p, const float* load, cons
   }
   // levels 0 and 1 are zero (slot n % 3 holds u^n)
   if (cudaMemsetAsync(w, 0, 4 * lev, st) != cudaSuccess) return ERNN_ERR_CUDA;
-  const int nt_out = (p->nt + p->stride - 1) / p->stride;
-  // frames of the levels that are never computed (0, and 1 when stride is 1)
-  for (int f = 0; f < nt_out && f * p->stride <= 1; ++f) {
-    if (cudaMemsetAsync(frames_x + (size_t)f * N, 0, N * sizeof(float), st) != cudaSuccess ||
-        cudaMemsetAsync(frames_y + (size_t)f * N, 0, N * sizeof(float), st) != cudaSuccess)
-      return ERNN_ERR_CUDA;
-  }
   const FemConsts k = fem_consts(*p);
   const dim3 block(32, 8, 1);
   const dim3 grid((p->ny + 31) / 32, (p->nx + 7) / 8, 1);

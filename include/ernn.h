@@ -258,7 +258,8 @@ typedef struct ErnnFemProblem {
   double out_scale; /* factor applied to the frames */
 } ErnnFemProblem;
 
-/* Device workspace of ernn_fem_forward: three time levels of two components. */
+/* Device workspace of ernn_fem_forward: four time levels of two components,
+ * rows padded to 16 bytes. */
 size_t ernn_fem_workspace_bytes(const ErnnFemProblem* p);
 
 /* load: (nx, ny) nodal Gaussian (y fastest), signal: (nt) time factors,

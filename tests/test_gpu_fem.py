@@ -114,3 +114,25 @@ def test_fem_frames_match_fp64_oracle_generator_grid():
     ox, oy = OF.fem_forward(*args, stride=5)
     ex, ey = rel(fx.cpu().numpy(), ox), rel(fy.cpu().numpy(), oy)
     assert ex <= TOL and ey <= TOL, (ex, ey)
+
+
+@pytest.mark.parametrize("nx,ny", [(2, 9), (5, 3), (8, 121), (9, 120), (17, 124), (24, 243)])
+@pytest.mark.parametrize("nt,stride", [(2, 1), (3, 1), (4, 2), (9, 1), (14, 1), (55, 3), (63, 5), (169, 12)])
+def test_fem_frames_at_tile_edges(nx, ny, nt, stride):
+    """Grids that end inside a tile's stored rows (8), columns (120), halo or a
+    quad of nodes, level counts that leave launches of one to four levels, and
+    both sides of the line (seven levels per node across the narrower side)
+    between several levels per launch and one; the error of a level is a few
+    roundings of the displacement, far below the bound after 169 of them."""
+    dx, dy = 1e-3, 1.25e-3
+    x = np.linspace(-(nx - 1) * dx / 2, (nx - 1) * dx / 2, nx)
+    y = np.linspace(-(ny - 1) * dy / 2, (ny - 1) * dy / 2, ny)
+    X, Y = np.meshgrid(x, y, indexing="ij")
+    load = EF.gaussian_point_load(X, Y, 0.0, (ny // 4) * dy, 1e5).astype(np.float32)
+    sig = EF.ricker_wavelet(np.arange(nt) * 5e-8, 1e6, 5e-7, 1e10).astype(np.float32)
+    C = (130.74e9, 11.5e9, 10.49e9, 30.67e9, 3.75e9, 14.77e9)
+    fx, fy = EF.fem_frames(nx, ny, nt, dx, dy, 5e-8, 1610.0, C, load, sig, stride=stride)
+    ox, oy = OF.fem_forward(nx, ny, nt, dx, dy, 5e-8, 1610.0, C, load, sig, stride=stride)
+    assert fx.shape == ox.shape
+    for a, b in ((fx, ox), (fy, oy)):
+        assert np.linalg.norm(a.double().cpu().numpy() - b) <= TOL * max(np.linalg.norm(ox), np.linalg.norm(oy))
