@@ -1,5 +1,5 @@
 // Time-blocked tile kernels (sm_103a): up to four time steps of a tile per
-// launch, the tile's state in registers.
+// launch, the tile's state in shared memory.
 //
 // One step of the scheme on a large grid moves 24 bytes of state per cell
 // (adjoint 32) through HBM for some 60 FP32 operations: a launch per step is
@@ -8,15 +8,20 @@
 // cells once (TMA, zeros outside the grid), advances it up to four steps,
 // and writes the last two levels: 24 -> 8 bytes per cell and step.
 //
-// Layout: a warp holds RW rows of 128 columns, each lane one quad of four
-// columns, both levels of its cells in registers for all steps; the new
-// level overwrites the older one.  A step needs from other threads only
-// the columns beside a quad (lane shuffles) and the rows above and below the
-// warp's (exchanged through shared memory, one CTA barrier per step); there
-// are no window loads.  The valid region shrinks by one cell per step, so
-// the outer quad and the outer four rows of the tile are not stored: 120
-// columns x (W RW - 8) rows are.  The loads of the CTA's next tile run
-// while the current one is advanced.
+// Layout: a warp owns RW rows of 128 columns, each lane one quad of four
+// columns; a new level overwrites the older one in place.  A row is read once
+// per step and kept in registers while it is the upper, middle and lower row
+// of the window; the columns beside a quad come by lane shuffles, rows of
+// other warps from shared memory (one CTA barrier per step).  The valid region
+// shrinks by one cell per step, so the outer quad and the outer four rows of
+// the tile are not stored: 120 columns x (W RW - 8) rows are.  Two CTAs per SM
+// (tall tiles): one loads its tile while the other computes.
+//
+// Measured (16 x 1024^2, us per launch of four steps against four launches of
+// the one-step kernels before): forward 173 against 264, adjoint 290 against
+// 456.  What bounds it is the FP32 pipe's issue: 40 warp instructions per
+// four cells and step, 30 of them the scheme's, at 55-60 % of the issue rate;
+// HBM runs at half its measured rate.
 //
 // Every cell's update is the same sequence of rounded operations as in the
 // per-step kernels, so the states agree with theirs bit for bit.
@@ -24,7 +29,9 @@
 #include <cudaTypedefs.h>
 
 #include <cmath>
+#include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "ernn_block.h"
 #include "ernn_launch.h"
@@ -450,6 +457,74 @@ __global__ void __launch_bounds__(32 * W, CTAS)
   if (tid == 0 && pipe_failed(&guard)) pipe_drain(bar, 1, &guard);
 }
 
+// Adds the threads' imaging sums (FP32 pairs) to a row of partials and clears
+// them; every thread of the CTA calls it.
+// The lanes' pairs are added as pairs (a warp's FP64 addition occupies this
+// part's FP64 pipe for 16 cycles and more, and thirty of them took longer
+// than a step of a small tile), and each exchange halves the values a lane
+// still carries: 4 + 2 + 1 additions leave one value in every group of four
+// lanes, two more sum it over the group.
+template <int W>
+__device__ __forceinline__ void flush_sums(float (&hi)[6], float (&lo)[6], float2 (*red)[6], double* row) {
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  float h[8], l[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    h[q] = q < 6 ? hi[q < 6 ? q : 0] : 0.f;
+    l[q] = q < 6 ? lo[q < 6 ? q : 0] : 0.f;
+  }
+  auto add = [&](int q, float h2, float l2) {
+    const float s = h[q] + h2, bp = s - h[q];
+    l[q] = (l[q] + l2) + ((h[q] - (s - bp)) + (h2 - bp));
+    h[q] = s;
+  };
+#pragma unroll
+  for (int n = 4; n >= 1; n >>= 1) {  // lanes with bit 4 n set keep values n .. 2 n - 1
+    const bool up = (lane & (4 * n)) != 0;
+#pragma unroll
+    for (int q = 0; q < n; ++q) {
+      const float sh = up ? h[q] : h[q + n], sl = up ? l[q] : l[q + n];
+      h[q] = up ? h[q + n] : h[q];
+      l[q] = up ? l[q + n] : l[q];
+      add(q, __shfl_xor_sync(kFull, sh, 4 * n), __shfl_xor_sync(kFull, sl, 4 * n));
+    }
+  }
+  add(0, __shfl_xor_sync(kFull, h[0], 2), __shfl_xor_sync(kFull, l[0], 2));
+  add(0, __shfl_xor_sync(kFull, h[0], 1), __shfl_xor_sync(kFull, l[0], 1));
+  // (bits 4, 3, 2 of the lane: bits 2, 1, 0 of the value)
+  if ((lane & 3) == 0 && lane < 24) red[w][lane >> 2] = make_float2(h[0], l[0]);
+#pragma unroll
+  for (int q = 0; q < 6; ++q) hi[q] = lo[q] = 0.f;
+  __syncthreads();
+  if (tid < 6) {
+    double v = 0.0;
+    for (int x = 0; x < W; ++x) v += (double)red[x][tid].x + (double)red[x][tid].y;
+    row[tid] += v;
+  }
+  __syncthreads();  // red is free again
+}
+
+// TwoSum(hi, acc)
+__device__ __forceinline__ void fold_sums(float (&hi)[6], float (&lo)[6], const float (&acc)[6]) {
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+    const float s = hi[q] + acc[q];
+    const float bp = s - hi[q];
+    lo[q] += (hi[q] - (s - bp)) + (acc[q] - bp);
+    hi[q] = s;
+  }
+}
+
+// The six sums' terms of a cell.
+__device__ __forceinline__ void image(float (&acc)[6], float ux, float uy, const Sums& sx, const Sums& sy) {
+  acc[0] = fmaf(ux, sx.xx, acc[0]);
+  acc[1] = fmaf(uy, sy.yy, acc[1]);
+  acc[2] = fmaf(ux, sy.xy, fmaf(uy, sx.xy, acc[2]));
+  acc[3] = fmaf(uy, sx.xx, fmaf(ux, fmaf(0.5f, sx.xy, sy.xx), acc[3]));
+  acc[4] = fmaf(ux, sy.yy, fmaf(uy, fmaf(0.5f, sy.xy, sx.yy), acc[4]));
+  acc[5] = fmaf(uy, sy.xx, fmaf(ux, sx.yy, acc[5]));
+}
+
 // ----------------------------------------------------------------- adjoint
 // As the forward, with lam^{m+1}, lam^{m+2} in the levels' place and no
 // load: the recorded residuals enter at the receivers' cells (subtracted
@@ -502,48 +577,8 @@ __global__ void __launch_bounds__(32 * W, CTAS)
   // tiles as FP32 pairs (TwoSum; the sum does not depend on how the steps
   // are split over launches), FP64 across warps and launches.
   float hi[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, lo[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  // The lanes' pairs are added as pairs (a warp's FP64 addition occupies this
-  // part's FP64 pipe for 16 cycles and more, and thirty of them took longer
-  // than a step of a small tile), and each exchange halves the values a lane
-  // still carries: 4 + 2 + 1 additions leave one value in every group of four
-  // lanes, two more sum it over the group.
   auto flush = [&](int shot) {  // CTA-uniform
-    float h[8], l[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      h[q] = q < 6 ? hi[q < 6 ? q : 0] : 0.f;
-      l[q] = q < 6 ? lo[q < 6 ? q : 0] : 0.f;
-    }
-    auto add = [&](int q, float h2, float l2) {
-      const float s = h[q] + h2, bp = s - h[q];
-      l[q] = (l[q] + l2) + ((h[q] - (s - bp)) + (h2 - bp));
-      h[q] = s;
-    };
-#pragma unroll
-    for (int n = 4; n >= 1; n >>= 1) {  // lanes with bit 4 n set keep values n .. 2 n - 1
-      const bool up = (lane & (4 * n)) != 0;
-#pragma unroll
-      for (int q = 0; q < n; ++q) {
-        const float sh = up ? h[q] : h[q + n], sl = up ? l[q] : l[q + n];
-        h[q] = up ? h[q + n] : h[q];
-        l[q] = up ? l[q + n] : l[q];
-        add(q, __shfl_xor_sync(kFull, sh, 4 * n), __shfl_xor_sync(kFull, sl, 4 * n));
-      }
-    }
-    add(0, __shfl_xor_sync(kFull, h[0], 2), __shfl_xor_sync(kFull, l[0], 2));
-    add(0, __shfl_xor_sync(kFull, h[0], 1), __shfl_xor_sync(kFull, l[0], 1));
-    // (bits 4, 3, 2 of the lane: bits 2, 1, 0 of the value)
-    if ((lane & 3) == 0 && lane < 24) red[w][lane >> 2] = make_float2(h[0], l[0]);
-#pragma unroll
-    for (int q = 0; q < 6; ++q) hi[q] = lo[q] = 0.f;
-    __syncthreads();
-    if (tid < 6) {
-      double v = 0.0;
-      for (int x = 0; x < W; ++x) v += (double)red[x][tid].x + (double)red[x][tid].y;
-      const size_t row = per_shot ? (size_t)shot * kTiledRowsPerShot + b : (size_t)b;
-      a.partials[row * 8 + tid] += v;
-    }
-    __syncthreads();  // red is free again
+    flush_sums<W>(hi, lo, red, a.partials + (per_shot ? (size_t)shot * kTiledRowsPerShot + b : (size_t)b) * 8);
   };
   int acc_shot = -1;
 
@@ -631,12 +666,7 @@ __global__ void __launch_bounds__(32 * W, CTAS)
             for (int q = 0; q < 4; ++q) {
               const Sums sx = sums_of(t0, m0, b0, q), sy = sums_of(t1, m1, b1, q);
               oper<ORDER>(ks, sx, sy, v0[q], v1[q]);
-              acc[0] = fmaf(ux[q], sx.xx, acc[0]);
-              acc[1] = fmaf(uy[q], sy.yy, acc[1]);
-              acc[2] = fmaf(ux[q], sy.xy, fmaf(uy[q], sx.xy, acc[2]));
-              acc[3] = fmaf(uy[q], sx.xx, fmaf(ux[q], fmaf(0.5f, sx.xy, sy.xx), acc[3]));
-              acc[4] = fmaf(ux[q], sy.yy, fmaf(uy[q], fmaf(0.5f, sy.xy, sx.yy), acc[4]));
-              acc[5] = fmaf(uy[q], sy.xx, fmaf(ux[q], sx.yy, acc[5]));
+              image(acc, ux[q], uy[q], sx, sy);
               // (quads outside the region stay zero: their lanes' coefficients are)
               v0[q] = leap(m0.w[q + 1], q0[q], v0[q]);
               v1[q] = leap(m1.w[q + 1], q1[q], v1[q]);
@@ -670,13 +700,7 @@ __global__ void __launch_bounds__(32 * W, CTAS)
       if (region != 0 && rows_in<RW>(rr0, t, B::kRows - t) != 0) {
         if (region == (1u << RW) - 1u && !ragged && !dense) rows(BoolC<true>{});
         else rows(BoolC<false>{});
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {  // TwoSum(hi, acc)
-          const float s = hi[q] + acc[q];
-          const float bp = s - hi[q];
-          lo[q] += (hi[q] - (s - bp)) + (acc[q] - bp);
-          hi[q] = s;
-        }
+        fold_sums(hi, lo, acc);
       }
       __syncthreads();  // lam^m is complete
       if (ORDER != kOrderTiled && inject) {  // ... but for the residuals: lam^m = (...) + g
@@ -697,6 +721,447 @@ __global__ void __launch_bounds__(32 * W, CTAS)
   }
   if (tid == 0 && pipe_failed(&guard)) pipe_drain(bar, 1, &guard);
   flush(per_shot ? acc_shot : 0);
+}
+
+// ------------------------------------------------------------ runs of passes
+// Grids whose tiles fit the chip, one per CTA: one cooperative launch makes
+// several passes of up to four steps.  A launch per pass costs such a grid as
+// much as its arithmetic (a CTA of 512 threads cannot start before the
+// previous launch's has left).  Here a tile's state stays in registers: a warp holds RW rows, a lane
+// four columns of them; rows beside another warp's go through shared memory
+// (one barrier per step), and between passes a CTA waits only for the tiles
+// around it, by a flag per tile that counts passes, and reloads its halo.
+// A neighbour is at most one pass ahead, and a pass never writes the states
+// that the pass before it has read.
+// Measured, us per pass of four steps, forward / adjoint: 301^2 (8-row tiles)
+// 6.0 / 7.5 against 7.5 / 11 with a launch each, 512^2 (24-row tiles) 7.0 /
+// 11.1 against 9.4 / 14.  Without waiting for neighbours, halo loads and
+// stores a forward pass of 301^2 takes 4.2: what bounds it is the chain of a
+// step (exchange, barrier, window, operator) with four warps per scheduler.
+struct NoRun {};
+__device__ __forceinline__ int passes_of(const NoRun&) { return 1; }
+template <class R>
+__device__ __forceinline__ int passes_of(const R& r) { return r.n; }
+
+// The passes of a run, copied to shared memory at its start: read from the
+// kernel's arguments, every pass would begin with misses of the constant
+// cache.  Without a run the launch's arguments are the pass.
+template <class R>
+struct Passes {
+  decltype(R::p) p;
+};
+template <>
+struct Passes<NoRun> {};
+template <class A>
+__device__ __forceinline__ const A& pass_of(const A& a, const Passes<NoRun>&, int) { return a; }
+template <class A, class R>
+__device__ __forceinline__ const auto& pass_of(const A&, const Passes<R>& s, int k) { return s.p[k]; }
+__device__ __forceinline__ void copy_passes(Passes<NoRun>&, const NoRun&) {}
+template <class R>
+__device__ __forceinline__ void copy_passes(Passes<R>& s, const R& r) {  // (visible after the next CTA barrier)
+  static_assert(sizeof(r.p[0]) % 8 == 0, "copied by words of 8 bytes");
+  const uint64_t* src = reinterpret_cast<const uint64_t*>(r.p);
+  uint64_t* dst = reinterpret_cast<uint64_t*>(s.p);
+  for (int e = threadIdx.x; e < (int)(r.n * sizeof(r.p[0]) / 8); e += blockDim.x) dst[e] = src[e];
+}
+
+// A neighbour that has not started yet is waited for (its SM may still be
+// busy with another stream's kernel), but not for ever.
+constexpr long long kRunWaitCycles = 1ll << 34;
+
+// Waits until the tiles around tile t of a shot's tiles_x x tiles_y have
+// counted k passes of this run.  Every thread of the CTA calls it.
+template <class R>
+__device__ __forceinline__ void wait_neighbours(const R& run, int k, int t, int tiles_x, int tiles_y, int* err) {
+  if (k > 0 && threadIdx.x < 9) {
+    const int r = t % (tiles_x * tiles_y), xt = r / tiles_y, yt = r - xt * tiles_y;
+    const int i = (int)threadIdx.x / 3 - 1, j = (int)threadIdx.x % 3 - 1;
+    if (xt + i >= 0 && xt + i < tiles_x && yt + j >= 0 && yt + j < tiles_y) {
+      const int* f = run.flags + t + i * tiles_y + j;
+      const long long t0 = clock64();
+      for (bool done = false; !done;) {
+        for (int n = 0; n < 64 && !done; ++n) {
+          int v;
+          asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
+          done = v >= run.epoch + k;
+        }
+        if (done || *(volatile int*)err != 0) break;
+        if (clock64() - t0 > kRunWaitCycles) {
+          atomicExch(err, kDeviceTimeout);
+          break;
+        }
+      }
+    }
+  }
+  __syncthreads();
+}
+__device__ __forceinline__ void wait_neighbours(const NoRun&, int, int, int, int, int*) {}
+
+// Counts the pass once every thread's stores are made.
+template <class R>
+__device__ __forceinline__ void count_pass(const R& run, int k, int t) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(run.flags + t), "r"(run.epoch + k + 1) : "memory");
+  }
+}
+__device__ __forceinline__ void count_pass(const NoRun&, int, int) {}
+
+constexpr int kRunW = 16;  // warps of a run's CTA
+
+// A warp's part of a run's tile.
+template <int RW>
+struct RunTile {
+  static constexpr int kRows = kRunW * RW;
+  static constexpr int kUse = kRows - 2 * kH;
+  static constexpr int kPlane = kRows * kBox;
+  static constexpr size_t kBytes = (size_t)2 * 2 * kPlane * 4 + 128;  // [parity][component][row][column]
+  BTile tile;
+  int lane, w, rr0, gi0, gj, nq, pitch;
+  uint32_t region, stored;
+  bool ragged;
+  ptrdiff_t off;
+  size_t Np;
+  float* ex;  // the lane's quad of the warp's first row, parity 0
+
+  template <class A>
+  __device__ __forceinline__ RunTile(const A& a, int t, int tiles_x, int tiles_y, float* sm) {
+    lane = threadIdx.x & 31;
+    w = threadIdx.x >> 5;
+    const int per = tiles_x * tiles_y, shot = t / per, r = t - shot * per, xt = r / tiles_y;
+    tile = BTile{shot, shot, xt * kUse, (r - xt * tiles_y) * kBlkCols, 0, 0, a.nx, a.ny};
+    rr0 = w * RW;
+    gi0 = tile.x0 - kH + rr0;
+    gj = tile.y0 - kH + 4 * lane;
+    nq = gj >= 0 ? max(0, min(4, a.ny - gj)) : 0;
+    region = rows_in<RW>(rr0, kH - tile.x0, a.nx - tile.x0 + kH);
+    stored = lane >= 1 && lane <= 30 && nq > 0 ? region & rows_in<RW>(rr0, kH, kRows - kH) : 0u;
+    ragged = (a.ny & 3) != 0 && tile.y0 - kH + kBox > a.ny;
+    pitch = a.pitch;
+    Np = (size_t)a.nx * a.pitch;
+    off = (ptrdiff_t)tile.plane * 2 * (ptrdiff_t)Np + (ptrdiff_t)gi0 * a.pitch + gj;
+    ex = sm + rr0 * kBox + 4 * lane;
+  }
+  // Whether a step t later still reads one of the warp's rows.
+  __device__ __forceinline__ bool active(int t) const {
+    return region != 0 && rr0 + RW > t && rr0 < kRows - t;
+  }
+  __device__ __forceinline__ float* row(int parity, int c, int r) const {  // r: -1 .. RW
+    return ex + parity * 2 * kPlane + c * kPlane + r * kBox;
+  }
+  // Cells of a state that the tile does not store itself (all: every cell).
+  __device__ __forceinline__ void load(const float* s, bool all, Q4 (&x)[RW], Q4 (&y)[RW]) const {
+#pragma unroll
+    for (int r = 0; r < RW; ++r) {
+      if (!all && ((stored >> r) & 1u)) continue;
+      const bool on = s != nullptr && nq > 0 && ((region >> r) & 1u);
+      const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+      x[r] = q4(on ? __ldcg(reinterpret_cast<const float4*>(s + off + (ptrdiff_t)r * pitch)) : z);
+      y[r] = q4(on ? __ldcg(reinterpret_cast<const float4*>(s + off + (ptrdiff_t)r * pitch + Np)) : z);
+    }
+  }
+  // The rows that other warps read (or every row) to shared memory.
+  __device__ __forceinline__ void put(int parity, bool all, const Q4 (&x)[RW], const Q4 (&y)[RW]) const {
+#pragma unroll
+    for (int r = 0; r < RW; ++r) {
+      if (r != 0 && r != RW - 1 && !all) continue;
+      *reinterpret_cast<float4*>(row(parity, 0, r)) = f4(x[r]);
+      *reinterpret_cast<float4*>(row(parity, 1, r)) = f4(y[r]);
+    }
+  }
+  __device__ __forceinline__ Row above(int parity, int c) const {
+    return w > 0 ? load_row(row(parity, c, -1)) : Row{{0.f, 0.f, 0.f, 0.f, 0.f, 0.f}};
+  }
+  __device__ __forceinline__ Row below(int parity, int c) const {
+    return w < kRunW - 1 ? load_row(row(parity, c, RW)) : Row{{0.f, 0.f, 0.f, 0.f, 0.f, 0.f}};
+  }
+  __device__ __forceinline__ void store(float* s, int r, const Q4& x, const Q4& y) const {
+    *reinterpret_cast<float4*>(s + off + (ptrdiff_t)r * pitch) = f4(x);
+    *reinterpret_cast<float4*>(s + off + (ptrdiff_t)r * pitch + Np) = f4(y);
+  }
+};
+
+template <int MODE, int RW, int ORDER>
+__global__ void __launch_bounds__(32 * kRunW, 1)
+    run_fwd_kernel(const BlkFwd a, const __grid_constant__ FwdRun run, int tiles_x, int tiles_y, int* err) {
+  extern __shared__ float sm_raw[];
+  using R = RunTile<RW>;
+  __shared__ Passes<FwdRun> pass;
+  copy_passes(pass, run);
+  const int t0 = (int)blockIdx.x, ny = a.ny;
+  const R g(a, t0, tiles_x, tiles_y, aligned128(sm_raw));
+  const size_t N = (size_t)a.nx * ny;
+  const Coef* K = a.coef + (size_t)g.tile.inst * a.coef_stride;
+  const Coefs ks = coefs_in(&K->k11, g.nq > 0);
+  Coefs kc[MODE == kModeFields ? 4 : 1];
+  if constexpr (MODE == kModeFields) {
+    static_assert(RW == 1, "one row of constants in registers");
+    const float q = K->q;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      kc[c] = cell_coefs(a.field, N, (size_t)g.gi0 * ny + g.gj + c, g.region != 0 && c < g.nq, q);
+  }
+  const bool has_src = a.bx > 0 && a.by > 0;
+  const int ox = has_src ? a.src_origin[2 * g.tile.inst] : 0, oy = has_src ? a.src_origin[2 * g.tile.inst + 1] : 0;
+  const bool src = has_src && g.gi0 < ox + a.bx && g.gi0 + RW > ox && g.tile.y0 - kH < oy + a.by &&
+                   g.tile.y0 - kH + kBox > oy;
+  const float kappa = K->kappa;
+  const int2 recs = a.rec_tile != nullptr ? a.rec_tile[t0] : make_int2(0, 0);
+  Q4 cx[RW], cy[RW], px[RW], py[RW];
+  int pending = -1;  // the frame of the newest level, whose receivers are not read yet
+  float fs[RW][4];     // the load of the thread's cells
+  uint32_t loaded = 0;  // cells inside the load's box, bit 4 r + q
+#pragma unroll
+  for (int r = 0; r < RW; ++r)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int sa = g.gi0 + r - ox, sb = g.gj + q - oy;
+      const bool in = src && q < g.nq && (unsigned)sa < (unsigned)a.bx && (unsigned)sb < (unsigned)a.by;
+      fs[r][q] = in ? a.src_map[((size_t)g.tile.inst * a.bx + sa) * a.by + sb] : 0.f;
+      loaded |= (in ? 1u : 0u) << (4 * r + q);
+    }
+  auto receivers = [&](int parity) {  // of the level in ex[parity]
+    const float* lv = aligned128(sm_raw) + parity * 2 * R::kPlane;
+    const size_t o = ((size_t)g.tile.inst * a.nt_out + pending) * a.nrec;
+    for (int e = threadIdx.x; e < recs.y; e += 32 * kRunW) {
+      const int2 v = a.rec_ent[recs.x + e];
+      const int rr = v.x / kBox, cc = v.x % kBox;
+      if (rr < kH || rr >= R::kRows - kH || cc < kH || cc >= kBox - kH) continue;  // another tile's
+      a.rec_x[o + v.y] = lv[v.x];
+      a.rec_y[o + v.y] = lv[R::kPlane + v.x];
+    }
+  };
+  __syncthreads();  // the passes are copied
+  for (int k = 0; k < run.n; ++k) {
+    const FwdPass& ps = pass.p[k];
+    float amp[kBlkSteps];
+#pragma unroll
+    for (int t = 0; t < kBlkSteps; ++t)  // (in flight over the wait)
+      amp[t] = src && t < ps.T ? a.src_signal[(size_t)g.tile.inst * a.nt + ps.i + t] * kappa : 0.f;
+    wait_neighbours(run, k, t0, tiles_x, tiles_y, err);
+    g.load(ps.cur, k == 0, cx, cy);
+    g.load(ps.prev, k == 0, px, py);
+    if (ps.out[0] != nullptr) {
+#pragma unroll
+      for (int r = 0; r < RW; ++r)
+        if ((g.stored >> r) & 1u) g.store(ps.out[0], r, cx[r], cy[r]);
+    }
+    // one step: the new level into the older one's registers
+    auto step = [&](int t, float am, const Q4(&ux)[RW], const Q4(&uy)[RW], Q4(&vx)[RW], Q4(&vy)[RW]) {
+      const int e = (t - 1) & 1;
+      const bool read = pending >= 0 && recs.y > 0;
+      g.put(e, read, ux, uy);
+      __syncthreads();
+      if (read) receivers(e);
+      const int frame = ps.frame[t];
+      const bool dense = frame >= 0 && a.record == kRecordFields;
+      float* out = ps.out[t];
+      if (g.active(t)) {
+        Row tx = g.above(e, 0), ty = g.above(e, 1), mx = row_of(ux[0]), my = row_of(uy[0]);
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+          const Row bx = r + 1 < RW ? row_of(ux[r + 1 < RW ? r + 1 : r]) : g.below(e, 0);
+          const Row by = r + 1 < RW ? row_of(uy[r + 1 < RW ? r + 1 : r]) : g.below(e, 1);
+          if ((g.region >> r) & 1u) {  // (rows outside the grid stay zero)
+            float lx[4], ly[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              oper<ORDER>(MODE == kModeFields ? kc[MODE == kModeFields ? q : 0] : ks, sums_of(tx, mx, bx, q),
+                          sums_of(ty, my, by, q), lx[q], ly[q]);
+            if (src) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                float& l = a.src_comp == 0 ? lx[q] : ly[q];
+                if ((loaded >> (4 * r + q)) & 1u) l = fmaf(am, fs[r][q], l);  // L + amp f, one rounding
+              }
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              vx[r].v[q] = leap(ux[r].v[q], vx[r].v[q], lx[q]);
+              vy[r].v[q] = leap(uy[r].v[q], vy[r].v[q], ly[q]);
+            }
+            if (g.ragged) {  // the grid's last column is inside a quad
+              mask_q(vx[r].v, g.nq);
+              mask_q(vy[r].v, g.nq);
+            }
+            if ((g.stored >> r) & 1u) {
+              if (out != nullptr) g.store(out, r, vx[r], vy[r]);
+              if (dense) {
+                const size_t o = ((size_t)g.tile.plane * a.nt_out + frame) * N + (size_t)(g.gi0 + r) * ny + g.gj;
+                if (a.vec) {
+                  *reinterpret_cast<float4*>(a.rec_x + o) = f4(vx[r]);
+                  *reinterpret_cast<float4*>(a.rec_y + o) = f4(vy[r]);
+                } else {
+#pragma unroll
+                  for (int q = 0; q < 4; ++q)
+                    if (q < g.nq) {
+                      a.rec_x[o + q] = vx[r].v[q];
+                      a.rec_y[o + q] = vy[r].v[q];
+                    }
+                }
+              }
+            }
+          }
+          tx = mx; ty = my; mx = bx; my = by;
+        }
+      }
+      pending = frame;
+    };
+#pragma unroll
+    for (int t = 1; t <= kBlkSteps; t += 2) {
+      if (t > ps.T) break;
+      step(t, amp[t - 1], cx, cy, px, py);
+      if (t == ps.T) {  // (odd: the newest level goes to c)
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+          Q4 s = cx[r]; cx[r] = px[r]; px[r] = s;
+          s = cy[r]; cy[r] = py[r]; py[r] = s;
+        }
+        break;
+      }
+      step(t + 1, amp[t], px, py, cx, cy);
+    }
+    count_pass(run, k, t0);
+  }
+  if (pending >= 0 && recs.y > 0) {
+    g.put(0, true, cx, cy);
+    __syncthreads();
+    receivers(0);
+  }
+}
+
+// As the forward run; the imaging pairs' u is read a step ahead.  The sums
+// leave the registers once, at the end of the run.
+template <int RW, int ORDER>
+__global__ void __launch_bounds__(32 * kRunW, 1)
+    run_adj_kernel(const BlkAdj a, const __grid_constant__ AdjRun run, int tiles_x, int tiles_y, int* err) {
+  extern __shared__ float sm_raw[];
+  using R = RunTile<RW>;
+  __shared__ Passes<AdjRun> pass;
+  __shared__ float2 red[kRunW][6];
+  copy_passes(pass, run);
+  const int t0 = (int)blockIdx.x, ny = a.ny;
+  const R g(a, t0, tiles_x, tiles_y, aligned128(sm_raw));
+  const size_t N = (size_t)a.nx * ny;
+  const Coefs ks = coefs_in(&(a.coef + (size_t)g.tile.inst * a.coef_stride)->k11, g.nq > 0);
+  const float gs = a.coef->gscale;
+  const int2 recs = a.rec_tile != nullptr ? a.rec_tile[t0] : make_int2(0, 0);
+  Q4 cx[RW], cy[RW], px[RW], py[RW], ux[RW], uy[RW];
+  float hi[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, lo[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  // u^m of the cells with an imaging pair, zero for the others; read from
+  // m_base on (what a run's last step would read next is not used)
+#pragma unroll
+  for (int r = 0; r < RW; ++r) ux[r] = uy[r] = Q4{{0.f, 0.f, 0.f, 0.f}};
+  const float* up = nullptr;
+  auto load_u = [&](int m, int r) {
+    if (m >= a.m_base && ((g.stored >> r) & 1u)) {
+      ux[r] = q4(__ldcg(reinterpret_cast<const float4*>(up + (ptrdiff_t)r * g.pitch)));
+      uy[r] = q4(__ldcg(reinterpret_cast<const float4*>(up + (ptrdiff_t)r * g.pitch + g.Np)));
+    }
+  };
+  __syncthreads();  // the passes are copied
+  {
+    const int m = pass.p[0].m_hi;
+    up = a.u_base + (ptrdiff_t)(m - a.m_base) * (ptrdiff_t)a.u_stride + g.off;
+    if (m <= a.nt - 1) {
+#pragma unroll
+      for (int r = 0; r < RW; ++r) load_u(m, r);
+    }
+  }
+  for (int k = 0; k < run.n; ++k) {
+    const AdjPass& ps = pass.p[k];
+    wait_neighbours(run, k, t0, tiles_x, tiles_y, err);
+    g.load(ps.cur, k == 0, cx, cy);
+    g.load(ps.prev, k == 0, px, py);
+    auto step = [&](int t, const Q4(&lx)[RW], const Q4(&ly)[RW], Q4(&vx)[RW], Q4(&vy)[RW]) {
+      const int m = ps.m_hi - t + 1, e = (t - 1) & 1;
+      const int frame = (m - 1) % a.stride == 0 ? (m - 1) / a.stride : -1;
+      const bool dense = frame >= 0 && a.record == kRecordFields;
+      g.put(e, false, lx, ly);
+      up -= a.u_stride;  // u^{m-1}
+      __syncthreads();
+      float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      if (g.active(t)) {
+        Row tx = g.above(e, 0), ty = g.above(e, 1), mx = row_of(lx[0]), my = row_of(ly[0]);
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+          const Row bx = r + 1 < RW ? row_of(lx[r + 1 < RW ? r + 1 : r]) : g.below(e, 0);
+          const Row by = r + 1 < RW ? row_of(ly[r + 1 < RW ? r + 1 : r]) : g.below(e, 1);
+          if ((g.region >> r) & 1u) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const Sums sx = sums_of(tx, mx, bx, q), sy = sums_of(ty, my, by, q);
+              float ax, ay;
+              oper<ORDER>(ks, sx, sy, ax, ay);
+              image(acc, ux[r].v[q], uy[r].v[q], sx, sy);
+              vx[r].v[q] = leap(lx[r].v[q], vx[r].v[q], ax);
+              vy[r].v[q] = leap(ly[r].v[q], vy[r].v[q], ay);
+            }
+            if (dense) {
+              const size_t o = ((size_t)g.tile.plane * a.nt_out + frame) * N + (size_t)(g.gi0 + r) * ny + g.gj;
+#pragma unroll
+              for (int q = 0; q < 4; ++q)
+                if (q < g.nq) {
+                  vx[r].v[q] = fmaf(gs, a.g_x[o + q], vx[r].v[q]);
+                  vy[r].v[q] = fmaf(gs, a.g_y[o + q], vy[r].v[q]);
+                }
+            }
+            if (g.ragged) {  // the grid's last column is inside a quad
+              mask_q(vx[r].v, g.nq);
+              mask_q(vy[r].v, g.nq);
+            }
+          }
+          load_u(m - 1, r);
+          tx = mx; ty = my; mx = bx; my = by;
+        }
+        fold_sums(hi, lo, acc);
+      } else {
+#pragma unroll
+        for (int r = 0; r < RW; ++r) load_u(m - 1, r);
+      }
+      if (frame >= 0 && recs.y > 0) {  // lam^m = (...) + g at the receivers' cells
+        g.put(e ^ 1, true, vx, vy);
+        __syncthreads();
+        float* lv = aligned128(sm_raw) + (e ^ 1) * 2 * R::kPlane;
+        const size_t o = ((size_t)g.tile.inst * a.nt_out + frame) * a.nrec;
+        for (int i = threadIdx.x; i < recs.y; i += 32 * kRunW) {
+          const int2 v = a.rec_ent[recs.x + i];
+          atomicAdd(&lv[v.x], gs * a.g_x[o + v.y]);
+          atomicAdd(&lv[R::kPlane + v.x], gs * a.g_y[o + v.y]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+          vx[r] = q4(*reinterpret_cast<const float4*>(g.row(e ^ 1, 0, r)));
+          vy[r] = q4(*reinterpret_cast<const float4*>(g.row(e ^ 1, 1, r)));
+        }
+      }
+      float* out = t == ps.T ? ps.out_last : (t == ps.T - 1 ? ps.out_before : nullptr);
+      if (out != nullptr) {
+#pragma unroll
+        for (int r = 0; r < RW; ++r)
+          if ((g.stored >> r) & 1u) g.store(out, r, vx[r], vy[r]);
+      }
+    };
+#pragma unroll
+    for (int t = 1; t <= kBlkSteps; t += 2) {
+      if (t > ps.T) break;
+      step(t, cx, cy, px, py);
+      if (t == ps.T) {
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+          Q4 s = cx[r]; cx[r] = px[r]; px[r] = s;
+          s = cy[r]; cy[r] = py[r]; py[r] = s;
+        }
+        break;
+      }
+      step(t + 1, px, py, cx, cy);
+    }
+    count_pass(run, k, t0);
+  }
+  const size_t row = a.coef_stride != 0 ? (size_t)g.tile.inst * kTiledRowsPerShot + blockIdx.x : (size_t)blockIdx.x;
+  flush_sums<kRunW>(hi, lo, red, a.partials + row * 8);
 }
 
 // ------------------------------------------- adjoint, degradation map
@@ -914,9 +1379,10 @@ __global__ void __launch_bounds__(32 * W, CTAS)
 // the four products whose vertical or diagonal neighbours are needed go
 // through shared memory (one CTA barrier per step), the others' column
 // neighbours come by lane shuffles.
-template <int W>
+template <int W, bool RUN>
 __global__ void __launch_bounds__(32 * W, 1)
-    blk_adj_f_kernel(const BlkAdj a, int tiles_x, int tiles_y, int ntiles) {
+    blk_adj_f_kernel(const BlkAdj a, const __grid_constant__ std::conditional_t<RUN, AdjRun, NoRun> run, int tiles_x,
+                     int tiles_y, int ntiles, int* err) {
   extern __shared__ float sm_raw[];
   float* ex = aligned128(sm_raw);  // [parity][product][row][128]
   constexpr int kRows = W, kUse = W - 2 * kH;
@@ -927,6 +1393,8 @@ __global__ void __launch_bounds__(32 * W, 1)
   BWalk<false, kUse> walk;
   walk.init((int)blockIdx.x, (int)gridDim.x, tiles_x, tiles_y, nx, ny);
   const float qf = a.coef->q;
+  __shared__ Passes<std::conditional_t<RUN, AdjRun, NoRun>> pass;
+  copy_passes(pass, run);
   for (; walk.t < ntiles; walk.next()) {
     const BTile tile = walk.tile(a.inst);
     const int2 recs = a.rec_tile != nullptr ? a.rec_tile[walk.t] : make_int2(0, 0);
@@ -950,29 +1418,39 @@ __global__ void __launch_bounds__(32 * W, 1)
       y[0] = vy.x; y[1] = vy.y; y[2] = vy.z; y[3] = vy.w;
     };
     float cx[4], cy[4], px[4], py[4], ga[6][4];
-    load_state(a.cur, off, a.cur != nullptr && nq > 0, cx, cy);
-    load_state(a.prev, off, a.prev != nullptr && nq > 0, px, py);
+    // the running sums of the thread's cells, a step's terms added to them one
+    // by one as in the per-step kernels
+    float* const gc = a.gacc + (size_t)tile.plane * 6 * N + (size_t)gi * ny + gj;
 #pragma unroll
     for (int c = 0; c < 6; ++c)
 #pragma unroll
-      for (int q = 0; q < 4; ++q) ga[c][q] = 0.f;
-    for (int t = 1; t <= a.T; ++t) {
-      const int m = a.m_hi - t + 1;
+      for (int q = 0; q < 4; ++q) ga[c][q] = stored && q < nq ? gc[c * N + q] : 0.f;
+    int n = 0;  // steps so far
+    for (int k = 0; k < passes_of(run); ++k) {
+    if (RUN) wait_neighbours(run, k, walk.t, tiles_x, tiles_y, err);
+    const auto& ps = pass_of(a, pass, k);
+    if (!(k > 0 && stored)) {
+      load_state(ps.cur, off, ps.cur != nullptr && nq > 0, cx, cy);
+      load_state(ps.prev, off, ps.prev != nullptr && nq > 0, px, py);
+    }
+    for (int t = 1; t <= ps.T; ++t, ++n) {
+      const int m = ps.m_hi - t + 1;
       const int frame = (m - 1) % a.stride == 0 ? (m - 1) / a.stride : -1;
       // the products of this row, those the rows above and below need in
-      // shared memory
+      // shared memory (which of a sum's products is rounded is as in the plain
+      // kernels: the states are theirs bit for bit)
       Q4 s0, s1, s2, s3, s4, s5;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const float lx = cx[q], ly = cy[q], c1266 = C[2][q] + C[5][q];
         s0.v[q] = fmaf(C[0][q], lx, __fmul_rn(C[3][q], ly));
-        s1.v[q] = fmaf(C[5][q], lx, __fmul_rn(C[4][q], ly));
+        s1.v[q] = fmaf(C[4][q], ly, __fmul_rn(C[5][q], lx));
         s2.v[q] = fmaf(2.f * C[3][q], lx, __fmul_rn(c1266, ly));
         s3.v[q] = fmaf(C[3][q], lx, __fmul_rn(C[5][q], ly));
-        s4.v[q] = fmaf(C[4][q], lx, __fmul_rn(C[1][q], ly));
-        s5.v[q] = fmaf(c1266, lx, __fmul_rn(2.f * C[4][q], ly));
+        s4.v[q] = fmaf(C[1][q], ly, __fmul_rn(C[4][q], lx));
+        s5.v[q] = fmaf(2.f * C[4][q], ly, __fmul_rn(c1266, lx));
       }
-      float* e = ex + (t & 1) * (4 * kRows * kBox) + w * kBox + 4 * lane;
+      float* e = ex + (n & 1) * (4 * kRows * kBox) + w * kBox + 4 * lane;
       *reinterpret_cast<float4*>(e) = f4(s0);
       *reinterpret_cast<float4*>(e + kRows * kBox) = f4(s2);
       *reinterpret_cast<float4*>(e + 2 * kRows * kBox) = f4(s3);
@@ -1026,8 +1504,8 @@ __global__ void __launch_bounds__(32 * W, 1)
         }
         if (frame >= 0 && recs.y > 0) {
           const size_t o = ((size_t)tile.inst * a.nt_out + frame) * a.nrec;
-          for (int n = 0; n < recs.y; ++n) {
-            const int2 v = a.rec_ent[recs.x + n];
+          for (int r = 0; r < recs.y; ++r) {
+            const int2 v = a.rec_ent[recs.x + r];
             if (v.x / 4 != w * (kBox / 4) + lane) continue;  // another thread's cell
 #pragma unroll
             for (int q = 0; q < 4; ++q)
@@ -1052,8 +1530,8 @@ __global__ void __launch_bounds__(32 * W, 1)
             const float lx = cx[q], ly = cy[q];
             ga[0][q] = fmaf(lx, sx.xx, ga[0][q]);
             ga[1][q] = fmaf(ly, sy.yy, ga[1][q]);
-            ga[2][q] += fmaf(lx, sy.xy, __fmul_rn(ly, sx.xy));
-            ga[3][q] += fmaf(lx, fmaf(0.5f, sx.xy, sy.xx), __fmul_rn(ly, sx.xx));
+            ga[2][q] += fmaf(ly, sx.xy, __fmul_rn(lx, sy.xy));
+            ga[3][q] += fmaf(ly, sx.xx, __fmul_rn(lx, fmaf(0.5f, sx.xy, sy.xx)));
             ga[4][q] += fmaf(lx, sy.yy, __fmul_rn(ly, fmaf(0.5f, sy.xy, sx.yy)));
             ga[5][q] += fmaf(lx, sx.yy, __fmul_rn(ly, sy.xx));
           }
@@ -1069,18 +1547,21 @@ __global__ void __launch_bounds__(32 * W, 1)
     }
     if (stored) {
       // cur holds lam of the last step, prev of the one before
-      *reinterpret_cast<float4*>(a.out_last + off) = make_float4(cx[0], cx[1], cx[2], cx[3]);
-      *reinterpret_cast<float4*>(a.out_last + off + Np) = make_float4(cy[0], cy[1], cy[2], cy[3]);
-      if (a.out_before != nullptr) {
-        *reinterpret_cast<float4*>(a.out_before + off) = make_float4(px[0], px[1], px[2], px[3]);
-        *reinterpret_cast<float4*>(a.out_before + off + Np) = make_float4(py[0], py[1], py[2], py[3]);
+      *reinterpret_cast<float4*>(ps.out_last + off) = make_float4(cx[0], cx[1], cx[2], cx[3]);
+      *reinterpret_cast<float4*>(ps.out_last + off + Np) = make_float4(cy[0], cy[1], cy[2], cy[3]);
+      if (ps.out_before != nullptr) {
+        *reinterpret_cast<float4*>(ps.out_before + off) = make_float4(px[0], px[1], px[2], px[3]);
+        *reinterpret_cast<float4*>(ps.out_before + off + Np) = make_float4(py[0], py[1], py[2], py[3]);
       }
-      float* g = a.gacc + (size_t)tile.plane * 6 * N + (size_t)gi * ny + gj;
+    }
+    if (RUN) count_pass(run, k, walk.t);
+    }
+    if (stored) {
 #pragma unroll
       for (int c = 0; c < 6; ++c)
 #pragma unroll
         for (int q = 0; q < 4; ++q)
-          if (q < nq) g[c * N + q] += ga[c][q];
+          if (q < nq) gc[c * N + q] = ga[c][q];
     }
     __syncthreads();  // the products are read: the next tile's may be written
   }
@@ -1287,21 +1768,76 @@ cudaError_t adj_d_t(const BlkAdj& a, int* err, cudaStream_t st) {
   }, (double)a.S * a.nx * a.ny * (16.0 * a.T + 32.0 + 4.0));
 }
 
-cudaError_t adj_f(const BlkAdj& a, cudaStream_t st) {
-  constexpr int W = 16, H = W - 2 * kH;
+// A run: one CTA per tile, launched cooperatively.
+template <class Kernel, class... Args>
+cudaError_t launch_run(int cls, Kernel kernel, int ntiles, size_t smem, double bytes, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ntiles);
+  cfg.blockDim = dim3(32 * kRunW);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaSuccess;
+  const cudaError_t l = tracked_launch(cls, st, [&] { e = cudaLaunchKernelEx(&cfg, kernel, args...); }, bytes);
+  return e != cudaSuccess ? e : l;
+}
+
+template <int MODE, int RW, int ORDER>
+cudaError_t fwd_run(const BlkFwd& a, const FwdRun& r, int* err, cudaStream_t st) {
+  using R = RunTile<RW>;
+  static std::once_flag once;
+  static cudaError_t ready = cudaSuccess;
+  std::call_once(once, [] {
+    ready = cudaFuncSetAttribute(run_fwd_kernel<MODE, RW, ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)R::kBytes);
+  });
+  if (ready != cudaSuccess) return ready;
+  const int tiles_x = (a.nx + R::kUse - 1) / R::kUse, tiles_y = (a.ny + kBlkCols - 1) / kBlkCols;
+  return launch_run(kProfForward, run_fwd_kernel<MODE, RW, ORDER>, a.S * tiles_x * tiles_y, R::kBytes,
+                    (double)a.S * a.nx * a.ny * 8.0 * kBlkSteps * r.n, st, a, r, tiles_x, tiles_y, err);
+}
+
+template <int RW, int ORDER>
+cudaError_t adj_run(const BlkAdj& a, const AdjRun& r, int* err, cudaStream_t st) {
+  using R = RunTile<RW>;
+  static std::once_flag once;
+  static cudaError_t ready = cudaSuccess;
+  std::call_once(once, [] {
+    ready = cudaFuncSetAttribute(run_adj_kernel<RW, ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)R::kBytes);
+  });
+  if (ready != cudaSuccess) return ready;
+  const int tiles_x = (a.nx + R::kUse - 1) / R::kUse, tiles_y = (a.ny + kBlkCols - 1) / kBlkCols;
+  return launch_run(kProfAdjoint, run_adj_kernel<RW, ORDER>, a.S * tiles_x * tiles_y, R::kBytes,
+                    (double)a.S * a.nx * a.ny * 8.0 * (kBlkSteps + 2) * r.n, st, a, r, tiles_x, tiles_y, err);
+}
+
+template <bool RUN>
+cudaError_t adj_f(const BlkAdj& a, const std::conditional_t<RUN, AdjRun, NoRun>& r, int* err, cudaStream_t st) {
+  constexpr int W = kRunW, H = W - 2 * kH;
   constexpr size_t smem = (size_t)2 * 4 * W * kBox * 4 + 128;
   static std::once_flag once;
   static cudaError_t ready = cudaSuccess;
   std::call_once(once, [] {
-    ready = cudaFuncSetAttribute(blk_adj_f_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    ready = cudaFuncSetAttribute(blk_adj_f_kernel<W, RUN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
   if (ready != cudaSuccess) return ready;
   const int tiles_x = (a.nx + H - 1) / H, tiles_y = (a.ny + kBlkCols - 1) / kBlkCols;
   const int ntiles = a.S * tiles_x * tiles_y;
-  return tracked_launch(kProfAdjoint, st, [&] {
-    launch_step_kernel(blk_adj_f_kernel<W>, dim3(ntiles < blk_sms() ? ntiles : blk_sms()), dim3(32 * W), smem, st,
-                       a.chained != 0, a, tiles_x, tiles_y, ntiles);
-  }, (double)a.S * a.nx * a.ny * (8.0 * a.T + 32.0 + 72.0));
+  if constexpr (RUN) {
+    return launch_run(kProfAdjoint, blk_adj_f_kernel<W, true>, ntiles, smem,
+                      (double)a.S * a.nx * a.ny * (8.0 * (kBlkSteps + 2) * r.n + 72.0), st, a, r, tiles_x, tiles_y,
+                      ntiles, err);
+  } else {
+    return tracked_launch(kProfAdjoint, st, [&] {
+      launch_step_kernel(blk_adj_f_kernel<W, false>, dim3(ntiles < blk_sms() ? ntiles : blk_sms()), dim3(32 * W), smem,
+                         st, a.chained != 0, a, r, tiles_x, tiles_y, ntiles, err);
+    }, (double)a.S * a.nx * a.ny * (8.0 * a.T + 32.0 + 72.0));
+  }
 }
 
 }  // namespace
@@ -1394,7 +1930,7 @@ cudaError_t launch_blk_fwd(int mode, const BlkFwd& a, int* err, cudaStream_t st)
 }
 
 cudaError_t launch_blk_adj(int mode, const BlkAdj& a, int* err, cudaStream_t st) {
-  if (mode == kModeFields) return adj_f(a, st);
+  if (mode == kModeFields) return adj_f<false>(a, NoRun{}, err, st);
   if (mode == kModeDField) {
     if (a.geo == kBlkFlat) return adj_d_t<16, 1, 1>(a, err, st);
     if (a.geo == kBlkShort) return adj_d_t<16, 2, 1>(a, err, st);
@@ -1402,6 +1938,30 @@ cudaError_t launch_blk_adj(int mode, const BlkAdj& a, int* err, cudaStream_t st)
   }
   if (a.inst.tiles != nullptr) return adj_t<8, 6, 2, true, kOrderTiled>(a, err, st);
   return a.plain_order ? adj_geo<kOrderPlain>(a, err, st) : adj_geo<kOrderTiled>(a, err, st);
+}
+
+// Runs: the tiles of a flat or short geometry that are resident at the same
+// time, one per SM, scalar constants in the plain kernels' order and constant
+// planes.
+bool blk_run_fits(int mode, int geo, int nx, int ny, int S) {
+  if (mode == kModeDField || geo == kBlkTall) return false;
+  static const bool coop = [] {
+    int dev = 0, v = 0;
+    return cudaGetDevice(&dev) == cudaSuccess &&
+           cudaDeviceGetAttribute(&v, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && v != 0;
+  }();
+  return coop && S * blk_tiles(geo, nx, ny) <= (size_t)blk_sms();
+}
+
+cudaError_t launch_blk_fwd_run(int mode, const BlkFwd& a, const FwdRun& r, int* err, cudaStream_t st) {
+  if (mode == kModeFields) return fwd_run<kModeFields, 1, kOrderFields>(a, r, err, st);
+  return a.geo == kBlkFlat ? fwd_run<kModeScalar, 1, kOrderPlain>(a, r, err, st)
+                           : fwd_run<kModeScalar, 2, kOrderPlain>(a, r, err, st);
+}
+
+cudaError_t launch_blk_adj_run(int mode, const BlkAdj& a, const AdjRun& r, int* err, cudaStream_t st) {
+  if (mode == kModeFields) return adj_f<true>(a, r, err, st);
+  return a.geo == kBlkFlat ? adj_run<1, kOrderPlain>(a, r, err, st) : adj_run<2, kOrderPlain>(a, r, err, st);
 }
 
 }  // namespace ernn

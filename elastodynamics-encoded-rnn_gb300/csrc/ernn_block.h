@@ -78,6 +78,38 @@ struct BlkAdj {
   InstTiles inst;
 };
 
+// A run: several passes (launches' worth of steps) in one cooperative launch,
+// each over the state the one before left.  24 passes take 140 to 270 us, of
+// which the launch is 3 to 4 (and their arguments 2 KB).
+constexpr int kRunPasses = 24;
+struct FwdPass {
+  int i, T;
+  const float* cur;
+  const float* prev;
+  float* out[kBlkSteps + 1];
+  int frame[kBlkSteps + 1];
+};
+struct AdjPass {
+  int m_hi, T;
+  const float* cur;
+  const float* prev;
+  float* out_last;
+  float* out_before;
+};
+struct FwdRun {
+  int n, epoch;  // passes; passes that the flags have counted before
+  int* flags;    // one per tile
+  FwdPass p[kRunPasses];
+};
+struct AdjRun {
+  int n, epoch;
+  int* flags;
+  AdjPass p[kRunPasses];
+};
+bool blk_run_fits(int mode, int geo, int nx, int ny, int S);
+cudaError_t launch_blk_fwd_run(int mode, const BlkFwd& a, const FwdRun& r, int* err, cudaStream_t st);
+cudaError_t launch_blk_adj_run(int mode, const BlkAdj& a, const AdjRun& r, int* err, cudaStream_t st);
+
 // Tile geometry of a grid problem (instances: kBlkTall), rows it stores,
 // tiles of an nx x ny grid.
 constexpr int kBlkTall = 0, kBlkShort = 1, kBlkFlat = 2;

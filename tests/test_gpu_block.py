@@ -103,6 +103,58 @@ def test_narrow_grids_on_either_side_of_the_cost_rule(mode, S, nx, ny, path):
     assert rel(ag, bg) <= 1e-5, rel(ag, bg)
 
 
+@pytest.mark.parametrize("mode,S,nx,ny", [
+    (O.MODE_SCALAR, 1, 41, 242), (O.MODE_FIELDS, 2, 41, 122),    # 8-row tiles, one per SM
+    (O.MODE_SCALAR, 5, 121, 361), (O.MODE_SCALAR, 9, 49, 241),   # 24-row tiles
+    (O.MODE_SCALAR, 3, 313, 389), (O.MODE_SCALAR, 13, 105, 243), # more tiles than SMs: a launch per pass
+])
+@pytest.mark.parametrize("record,nrec", [(O.RECORD_FIELDS, 0), (O.RECORD_RECEIVERS, 70)])
+@pytest.mark.parametrize("nt,ckpt_k,stride", [(102, None, 1), (205, 103, 3), (61, 17, 1)])
+def test_runs_of_passes(mode, S, nx, ny, record, nrec, nt, ckpt_k, stride):
+    """Several passes per launch, tiles kept in registers between them: step
+    counts over one launch (24 passes of four steps), odd last passes, segments
+    that are no multiple of four."""
+    case = random_case(nx=nx, ny=ny, nt=nt, S=S, stride=stride, mode=mode, record=record, nrec=nrec, src_comp=nx % 2)
+    wx, wy = weights(case)
+    ax, ay, ag, used = run(case, wx, wy, E.PATH_AUTO, ckpt_k)
+    assert used == E.PATH_TILED
+    bx, by, bg, _ = run(case, wx, wy, E.PATH_STEP, ckpt_k)
+    assert np.array_equal(ax, bx) and np.array_equal(ay, by)
+    assert rel(ag, bg) <= 1e-5, rel(ag, bg)
+
+
+def test_run_in_a_captured_graph_and_on_two_streams():
+    """A run replayed from a graph, and two at once on two streams (together
+    more tiles than SMs), give the results of a plain call."""
+    cases = [random_case(nx=nx, ny=241, nt=130, S=1, record=O.RECORD_RECEIVERS, nrec=30) for nx in (301, 290)]
+    want, calls = [], []
+    for c in cases:
+        geom = to_geometry(c, path=E.PATH_AUTO)
+        C = torch.tensor(c.C, dtype=torch.float32, device=DEV)
+        r = torch.tensor(c.rho, dtype=torch.float32, device=DEV)
+        calls.append(lambda C=C, r=r, geom=geom: E.propagate(C, r, geom))
+        with torch.no_grad():
+            want.append([v.clone() for v in calls[-1]()])
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in cases]
+    with torch.no_grad():
+        for _ in range(3):
+            got = []
+            for st, call in zip(streams, calls):
+                with torch.cuda.stream(st):
+                    got.append(call())
+            torch.cuda.synchronize()
+            for g, w in zip(got, want):
+                assert torch.equal(g[0], w[0]) and torch.equal(g[1], w[1])
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = calls[0]()
+        for _ in range(2):
+            graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out[0], want[0][0]) and torch.equal(out[1], want[0][1])
+
+
 def test_large_odd_grid_vs_fp64_oracle():
     case = random_case(nx=330, ny=437, nt=60, S=5, record=O.RECORD_RECEIVERS, nrec=60)
     wx, wy = weights(case)
