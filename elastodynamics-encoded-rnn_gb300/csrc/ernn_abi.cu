@@ -78,7 +78,7 @@ bool block_rule(const ErnnProblem& p) {
   if (p.path != ERNN_PATH_AUTO || p.ny < kBlockMinCols) return false;
   if (p.mode == kModeFields) return (double)p.nshots * p.nx * p.ny <= kBlockMaxFields;
   if (p.mode == kModeDField) {
-    const double cost = blk_cost(blk_geometry(p.nx, p.ny, p.nshots), p.nx, p.ny, p.nshots);
+    const double cost = blk_cost(blk_geometry(p.mode, p.nx, p.ny, p.nshots), p.nx, p.ny, p.nshots);
     return plain_size(p) && (cost <= 10.0 || cost <= 6.0 + 31e-6 * p.nshots * p.nx * p.ny);
   }
   return !resident_possible(p.mode, p.nx, p.ny);
@@ -102,7 +102,7 @@ Plan make_plan(const ErnnProblem& p) {
   pl.inst = (p.flags & ERNN_FLAG_INSTANCES) != 0;
   // instances share the canvas's one state plane
   pl.block = block_rule(p);
-  pl.geo = pl.inst ? kBlkTall : p.mode == kModeFields ? kBlkFlat : blk_geometry(p.nx, p.ny, p.nshots);
+  pl.geo = pl.inst ? kBlkTall : p.mode == kModeFields ? kBlkFlat : blk_geometry(p.mode, p.nx, p.ny, p.nshots);
   pl.pitch = pl.block ? (p.ny + 3) / 4 * 4 : p.ny;
   pl.state_bytes = align_up((size_t)(pl.inst ? 1 : p.nshots) * 2 * p.nx * pl.pitch * sizeof(float));
   const dim3 g = step_grid(p.nx, p.ny, pl.inst ? 1 : p.nshots);

@@ -1844,11 +1844,16 @@ cudaError_t adj_f(const BlkAdj& a, const std::conditional_t<RUN, AdjRun, NoRun>&
 
 // Tile geometries.  kBlkTall: eight warps of six rows, two CTAs per SM (one
 // loads its tile while the other computes), 40 of 48 rows stored: the best
-// use of the FP32 pipe, for grids of several tiles per SM.  kBlkShort:
-// sixteen warps of two rows, one CTA per SM, 24 of 32 rows stored, and
-// kBlkFlat: sixteen warps of one row, 8 of 16 stored, whose tiles take a half
-// and a quarter as long, for grids that would leave SMs idle.
-int blk_tile_rows(int geo) { return (geo == kBlkTall ? 8 * 6 : geo == kBlkShort ? 16 * 2 : 16) - 2 * kH; }
+// use of the FP32 pipe, for grids of several tiles per SM; kBlkTall5 and
+// kBlkTall4, with five and four rows a warp, where these fill their last wave
+// of tiles better.  kBlkShort: sixteen warps of two rows, one CTA per SM, 24
+// of 32 rows stored, and kBlkFlat: sixteen warps of one row, 8 of 16 stored,
+// whose tiles take a half and a quarter as long, for grids that would leave
+// SMs idle.
+int blk_tile_rows(int geo) {
+  const int rows[] = {8 * 6, 16 * 2, 16, 8 * 5, 8 * 4};
+  return rows[geo] - 2 * kH;
+}
 
 size_t blk_tiles(int geo, int nx, int ny) {
   const int h = blk_tile_rows(geo);
@@ -1862,14 +1867,16 @@ size_t blk_tiles(int geo, int nx, int ny) {
 double blk_cost(int geo, int nx, int ny, int S) {
   const double sms = 152.0, tiles = S * (double)blk_tiles(geo, nx, ny);
   if (geo == kBlkTall) return tiles <= sms ? 21.0 : 20.0 * std::ceil(tiles / (2.0 * sms));
+  if (geo == kBlkTall5 || geo == kBlkTall4) return (geo == kBlkTall5 ? 17.3 : 14.6) * std::ceil(tiles / (2.0 * sms));
   return (geo == kBlkShort ? 9.4 : 5.0) * std::ceil(tiles / sms);
 }
 
-int blk_geometry(int nx, int ny, int S) {
-  const double tall = blk_cost(kBlkTall, nx, ny, S), low = blk_cost(kBlkShort, nx, ny, S);
-  const double flat = blk_cost(kBlkFlat, nx, ny, S);
-  if (flat < low && flat < tall) return kBlkFlat;
-  return low < tall ? kBlkShort : kBlkTall;
+int blk_geometry(int mode, int nx, int ny, int S) {
+  int best = kBlkTall;
+  // (the five- and four-row tiles: scalar constants)
+  for (int geo : {kBlkShort, kBlkFlat, kBlkTall5, kBlkTall4})
+    if ((mode == kModeScalar || geo < kBlkTall5) && blk_cost(geo, nx, ny, S) < blk_cost(best, nx, ny, S)) best = geo;
+  return best;
 }
 
 bool blk_available() { return blk_encode_fn() != nullptr; }
@@ -1911,6 +1918,10 @@ template <int MODE, int ORDER>
 cudaError_t fwd_geo(const BlkFwd& a, int* err, cudaStream_t st) {
   if (a.geo == kBlkFlat) return fwd_t<MODE, 16, 1, 1, false, ORDER>(a, err, st);
   if (a.geo == kBlkShort) return fwd_t<MODE, 16, 2, 1, false, ORDER>(a, err, st);
+  if constexpr (MODE == kModeScalar) {
+    if (a.geo == kBlkTall5) return fwd_t<MODE, 8, 5, 2, false, ORDER>(a, err, st);
+    if (a.geo == kBlkTall4) return fwd_t<MODE, 8, 4, 2, false, ORDER>(a, err, st);
+  }
   return fwd_t<MODE, 8, 6, 2, false, ORDER>(a, err, st);
 }
 
@@ -1918,6 +1929,8 @@ template <int ORDER>
 cudaError_t adj_geo(const BlkAdj& a, int* err, cudaStream_t st) {
   if (a.geo == kBlkFlat) return adj_t<16, 1, 1, false, ORDER>(a, err, st);
   if (a.geo == kBlkShort) return adj_t<16, 2, 1, false, ORDER>(a, err, st);
+  if (a.geo == kBlkTall5) return adj_t<8, 5, 2, false, ORDER>(a, err, st);
+  if (a.geo == kBlkTall4) return adj_t<8, 4, 2, false, ORDER>(a, err, st);
   return adj_t<8, 6, 2, false, ORDER>(a, err, st);
 }
 }  // namespace
@@ -1944,7 +1957,7 @@ cudaError_t launch_blk_adj(int mode, const BlkAdj& a, int* err, cudaStream_t st)
 // time, one per SM, scalar constants in the plain kernels' order and constant
 // planes.
 bool blk_run_fits(int mode, int geo, int nx, int ny, int S) {
-  if (mode == kModeDField || geo == kBlkTall) return false;
+  if (mode == kModeDField || (geo != kBlkFlat && geo != kBlkShort)) return false;
   static const bool coop = [] {
     int dev = 0, v = 0;
     return cudaGetDevice(&dev) == cudaSuccess &&

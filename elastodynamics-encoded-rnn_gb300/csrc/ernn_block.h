@@ -112,8 +112,8 @@ cudaError_t launch_blk_adj_run(int mode, const BlkAdj& a, const AdjRun& r, int* 
 
 // Tile geometry of a grid problem (instances: kBlkTall), rows it stores,
 // tiles of an nx x ny grid.
-constexpr int kBlkTall = 0, kBlkShort = 1, kBlkFlat = 2;
-int blk_geometry(int nx, int ny, int S);
+constexpr int kBlkTall = 0, kBlkShort = 1, kBlkFlat = 2, kBlkTall5 = 3, kBlkTall4 = 4;
+int blk_geometry(int mode, int nx, int ny, int S);
 double blk_cost(int geo, int nx, int ny, int S);  // us of a launch of four steps (scalar constants)
 int blk_tile_rows(int geo);
 size_t blk_tiles(int geo, int nx, int ny);
