@@ -449,7 +449,8 @@ def run_ernn(args, dist):
     peak, peak_kind = peaks()
     used = int(lib.ernn_last_path())
     kernel_name = {E.PATH_RESIDENT: {"forward": "resident_kernel", "adjoint": "resident_kernel"},
-                   E.PATH_TILED: {"forward": "tma_fwd_kernel", "adjoint": "tma_adj_kernel"}}.get(
+                   E.PATH_TILED: {"forward": "tma_fwd_kernel", "adjoint": "tma_adj_kernel"} if w.D_true is not None
+                   else {"forward": "blk_fwd_kernel", "adjoint": "blk_adj_kernel"}}.get(
         used, {"forward": "fwd_step_kernel", "adjoint": "adj_step_kernel"})[cls]
     traffic = profiled_traffic(kernel_name, args.workload)
     state_mb = w.nshots * 2 * w.nx * w.ny * 4 / 2**20
@@ -477,8 +478,7 @@ def run_ernn(args, dist):
                    "kernel_path": {0: "auto", 1: "step", 2: "resident", 3: "tiled"}[int(lib.ernn_last_path())],
                    "launch": ("one CUDA graph per iteration" if inv.graph is not None else "eager") +
                              ("" if args.no_overlap else ", step kernels overlapped (programmatic dependent launch)"),
-                   "path_choice": (f"measured (autotune): tiles 64x{inv.geom.tile_rows}" if tuned
-                                   else args.path),
+                   "path_choice": "measured (autotune)" if tuned else args.path,
                    "l2": "flushed between timed iterations (256 MiB write)",
                    **({"iterations": "each restarts from the initial guess (outside the timed region)"}
                       if w.extra.get("restart") else {}),
@@ -728,7 +728,7 @@ def run_multi(args, dist):
         inv = Hn.MultiInversion(ws, dev, tuned=tuned, path=None if tuned else PATHS[args.path])
     else:
         # configuration 5 as one propagation: every instance a region of one
-        # canvas, one launch per time step over the running instances' tiles
+        # canvas, one launch per four time steps over the running instances' tiles
         inv = (Hn.CanvasInversion(ws, dev, nt=args.nt) if args.canvas_parts <= 1 else
                Hn.CanvasSet(ws, dev, parts=args.canvas_parts, nt=args.nt))
     setup_s = time.perf_counter() - t0
@@ -809,12 +809,12 @@ def run_multi(args, dist):
                                f"one CUDA-graph-captured Adam iteration over all instances; " +
                                (f"{len(inv.groups)} groups of equal instances, each one call with "
                                 f"per-shot constants, on 8 streams" if args.grouped else
-                                f"one {inv.canvas[0]}x{inv.canvas[1]} canvas, one launch per step over "
+                                f"one {inv.canvas[0]}x{inv.canvas[1]} canvas, one launch per four steps over "
                                 f"a tile table of the running instances (checkpoint every "
                                 f"{inv.geom.ckpt_k})" if args.canvas_parts <= 1 else
                                 f"{len(inv.parts)} canvases (" + ", ".join(f"{c.canvas[0]}x{c.canvas[1]}"
                                                                          for c in inv.parts) +
-                                "), each one launch per step over its running instances' tiles, "
+                                "), each one launch per four steps over its running instances' tiles, "
                                 "on their own streams"),
                    "cell_steps_per_iter": inv.cell_steps,
                    "path_choice": "measured per group (autotune)" if tuned else args.path,

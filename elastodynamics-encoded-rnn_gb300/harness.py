@@ -590,7 +590,7 @@ class CanvasSet(_GraphedIteration):
     """The instances split into `parts` canvases of about equal work
     (cell-steps, largest first to the lightest part), each a CanvasInversion
     advanced on its own CUDA stream, the whole iteration one graph.  Each
-    canvas is one launch per step; the canvases' launches overlap, so one
+    canvas is one launch per four steps; the canvases' launches overlap, so one
     canvas's last partial wave of tiles runs beside the other's work."""
 
     def __init__(self, ws, device, parts=2, lr=1e-2, seed=0, graph=True, nt=None):

@@ -65,11 +65,11 @@ class Geometry:
     rec_idx:    (S, R) int32 flat receiver cells (i*ny + j), or None for the
                 dense history of the reference.
     ckpt_k:     checkpoint interval in steps (>= nt keeps every state).
-    path:       PATH_AUTO (cluster-resident when the problem fits, else the
-                tiled TMA kernels when eligible, else one plain kernel per
-                step), PATH_STEP, PATH_RESIDENT or PATH_TILED.
-    tile_rows:  tile rows of the tiled kernels, 16 or 32 (autotune.tune
-                measures both).
+    path:       PATH_AUTO (cluster-resident when the problem fits, else
+                time-blocked tiles, else one kernel per step), PATH_STEP,
+                PATH_RESIDENT or PATH_TILED.
+    tile_rows:  16 or 32; the tiled kernels choose their own tiles, so both
+                run the same kernels.
     """
     nx: int
     ny: int
@@ -85,7 +85,7 @@ class Geometry:
     ckpt_k: int | None = None
     path: int = _lib.PATH_AUTO
     instances: Instances | None = None
-    tile_rows: int = 16  # tiled kernels: 16 (64 x 16 tiles) or 32 (64 x 32, ERNN_FLAG_TALL_TILES)
+    tile_rows: int = 16  # 32 sets ERNN_FLAG_TALL_TILES
     _checked: bool = field(default=False, repr=False)
 
     @property

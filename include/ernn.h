@@ -56,17 +56,19 @@ enum {
 };
 
 enum {
-  ERNN_PATH_AUTO = 0,     /* cluster-resident when the problem fits, else tiled when
-                             eligible, else per-step */
+  ERNN_PATH_AUTO = 0,     /* cluster-resident when the problem fits, else time-blocked
+                             tiles (scalar constants and constant planes with rows of
+                             any length from 40 cells; degradation maps of moderate
+                             size), else tiled or per-step launches */
   ERNN_PATH_STEP = 1,     /* one fused kernel launch per time step (any size, any mode) */
   ERNN_PATH_RESIDENT = 2, /* one thread-block cluster per shot holds the state in
                              distributed shared memory for all steps (scalar constants,
                              ny % 4 == 0, state small enough); ERNN_ERR_UNSUPPORTED otherwise */
-  ERNN_PATH_TILED = 3     /* one launch per time step of persistent CTAs that stream
-                             64-column tiles (16 rows; 32 for the degradation-map
-                             adjoint) through TMA loads (scalar constants or a
-                             degradation map, ny % 4 == 0); ERNN_ERR_UNSUPPORTED
-                             otherwise */
+  ERNN_PATH_TILED = 3     /* persistent CTAs that stream tiles through TMA loads, ny %
+                             4 == 0: scalar constants in time-blocked tiles of 120
+                             columns, up to four steps per launch; a degradation map
+                             in 64 x 32 tiles, one launch per step.
+                             ERNN_ERR_UNSUPPORTED otherwise */
 };
 
 /* Problem flags. */
@@ -81,16 +83,11 @@ enum {
    * a rectangular region of the canvas with its own constants (C nshots x 6,
    * rho nshots, as ERNN_FLAG_SHOT_CONSTANTS), source (src_signal nshots x nt,
    * src_map, src_origin in canvas cells), receivers (rec_idx: canvas cell
-   * indices) and step count; nt is the largest step count.  SCALAR mode,
+   * indices; one outside its instance's region records zeros) and step count; nt is the largest step count.  SCALAR mode,
    * RECORD_RECEIVERS, tiled kernels (ERNN_PATH_AUTO or _TILED). */
   ERNN_FLAG_INSTANCES = 2,
-  /* Tiled kernels: 64 x 32 tiles for the forward steps and the scalar
-   * adjoint instead of 64 x 16 (a tenth fewer halo rows per cell, one CTA
-   * fewer per SM); a tile geometry the autotuner measures.  Results are the
-   * same up to FP32 rounding of the imaging sums' grouping.  The D-field
-   * mode takes 64 x 32 tiles with or without the flag (its adjoint always
-   * did; its forward measured faster so: 8 x 512^2 shots, 81.3 -> 75.6 ms
-   * per inversion iteration). */
+  /* Accepted and without effect: the tiled kernels choose their tiles from
+   * the grid (it once chose 64 x 32 over 64 x 16 tiles). */
   ERNN_FLAG_TALL_TILES = 4
 };
 
@@ -167,7 +164,8 @@ int ernn_operator(int32_t nshots, int32_t nx, int32_t ny, int32_t mode, double h
  * out_ux, out_uy: (nshots, nt_out, nx, ny) for RECORD_FIELDS or
  * (nshots, nt_out, nrec) for RECORD_RECEIVERS, nt_out = ceil(nt / stride).
  * tape: ernn_tape_bytes(p, with_tape) bytes; keep it unchanged until
- * ernn_adjoint when with_tape != 0. */
+ * ernn_adjoint when with_tape != 0 (a tape copied elsewhere keeps its address
+ * modulo 16: its layout depends on it). */
 int ernn_forward(const ErnnProblem* p, const ErnnInputs* in, float* out_ux, float* out_uy,
                  void* tape, size_t tape_bytes, int with_tape, void* stream);
 
