@@ -155,6 +155,16 @@ def test_run_in_a_captured_graph_and_on_two_streams():
         assert torch.equal(out[0], want[0][0]) and torch.equal(out[1], want[0][1])
 
 
+def test_autotune_measures_the_kernels_that_no_path_names():
+    from ernn_gb300 import autotune
+    case = random_case(nx=90, ny=243, nt=120, S=1, record=O.RECORD_RECEIVERS, nrec=8)
+    geom = to_geometry(case, None, E.PATH_AUTO)
+    C = torch.tensor(case.C, dtype=torch.float32, device=DEV)
+    rho = torch.tensor(case.rho, dtype=torch.float32, device=DEV)
+    path, k, rows = autotune.tune(geom, C, rho, probe_steps=96)  # ny % 4 != 0: neither RESIDENT nor TILED
+    assert path in (E.PATH_AUTO, E.PATH_STEP) and 1 <= k <= case.nt and rows == 16
+
+
 def test_large_odd_grid_vs_fp64_oracle():
     case = random_case(nx=330, ny=437, nt=60, S=5, record=O.RECORD_RECEIVERS, nrec=60)
     wx, wy = weights(case)
