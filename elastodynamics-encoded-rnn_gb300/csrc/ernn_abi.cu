@@ -537,6 +537,17 @@ struct PassRunner {
       f.flags = flags;
       epoch += f.n;
       e = launch_blk_fwd_run(mode, *fa, f, err, st);
+      if (e == cudaErrorCooperativeLaunchTooLarge) {  // a context with fewer SMs: a launch per pass
+        on = false;
+        e = cudaSuccess;
+        BlkFwd a = *fa;
+        for (int k = 0; k < f.n && e == cudaSuccess; ++k) {
+          const FwdPass& q = f.p[k];
+          a.i = q.i; a.T = q.T; a.cur = q.cur; a.prev = q.prev;
+          for (int t = 0; t <= kBlkSteps; ++t) { a.out[t] = q.out[t]; a.frame[t] = q.frame[t]; }
+          e = add(a);
+        }
+      }
       f.n = 0;
     }
     if (e == cudaSuccess && r.n > 0) {
@@ -544,6 +555,16 @@ struct PassRunner {
       r.flags = flags;
       epoch += r.n;
       e = launch_blk_adj_run(mode, *ra, r, err, st);
+      if (e == cudaErrorCooperativeLaunchTooLarge) {
+        on = false;
+        e = cudaSuccess;
+        BlkAdj b = *ra;
+        for (int k = 0; k < r.n && e == cudaSuccess; ++k) {
+          const AdjPass& q = r.p[k];
+          b.m_hi = q.m_hi; b.T = q.T; b.cur = q.cur; b.prev = q.prev; b.out_last = q.out_last; b.out_before = q.out_before;
+          e = add(b);
+        }
+      }
       r.n = 0;
     }
     return e;
