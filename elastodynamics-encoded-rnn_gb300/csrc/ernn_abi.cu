@@ -579,7 +579,7 @@ int block_forward(const ErnnProblem& p, const Plan& pl, const ErnnInputs& in, co
   BlkFwd a = base_blk_fwd(p, pl, in, coef, itab);
   if (p.record == kRecordReceivers)
     ERNN_CUDA(launch_rec_tiles(pl.geo, in.rec_idx, p.nshots, p.nrec, p.nx, p.ny, itab.box, block_tiles(p, pl, ip),
-                               at(tape, pl.t_rec), &a.rec_tile, &a.rec_ent, st));
+                               at(tape, pl.t_rec), &a.rec_tile, &a.rec_ent, out_ux, out_uy, pl.nt_out, st));
   a.rec_x = out_ux;
   a.rec_y = out_uy;
   a.vec = p.ny % 4 == 0 && al16(out_ux) && al16(out_uy);
@@ -638,7 +638,7 @@ int block_adjoint(const ErnnProblem& p, const Plan& pl, const ErnnInputs& in, co
   b.stride = p.stride; b.nt_out = pl.nt_out; b.record = p.record; b.nrec = p.nrec;
   if (p.record == kRecordReceivers)
     ERNN_CUDA(launch_rec_tiles(pl.geo, in.rec_idx, p.nshots, p.nrec, p.nx, p.ny, itab.box, block_tiles(p, pl, ip),
-                               at(scratch, pl.s_rec), &b.rec_tile, &b.rec_ent, st));
+                               at(scratch, pl.s_rec), &b.rec_tile, &b.rec_ent, nullptr, nullptr, 0, st));
   b.coef = coef;
   b.coef_stride = a.coef_stride;
   b.field = a.field;

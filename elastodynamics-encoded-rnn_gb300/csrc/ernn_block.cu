@@ -1593,7 +1593,8 @@ __global__ void inst_table_kernel(const InstDesc d, int4* __restrict__ tiles, in
 // The receivers whose cells lie in a tile with its halo, for every tile of a
 // call: tile[t] = (first entry, entries), an entry = (cell in the tile's
 // planes, receiver number).  Counted, given room and filled by three small
-// kernels (the order inside a tile does not matter).
+// kernels (the order inside a tile does not matter).  A receiver outside the
+// grid is in no tile: the counting kernel writes its nt_out frames (zeros).
 struct RecPlace {  // the tiles (at most 2 x 2) around a cell
   int x0, x1, y0, y1, base, tiles_y, oi, oj;
   __device__ __forceinline__ bool find(int idx, int s, int nx, int ny, int H, int tiles_x, int ty, const int4* box) {
@@ -1624,12 +1625,20 @@ struct RecPlace {  // the tiles (at most 2 x 2) around a cell
 template <bool FILL>
 __global__ void rec_tiles_kernel(const int32_t* __restrict__ rec_idx, int S, int nrec, int nx, int ny, int H,
                                  int tiles_x, int tiles_y, const int4* __restrict__ box, int* __restrict__ count,
-                                 int2* __restrict__ tile, int2* __restrict__ ent) {
+                                 int2* __restrict__ tile, int2* __restrict__ ent, float* __restrict__ tr_x,
+                                 float* __restrict__ tr_y, int nt_out) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= S * nrec) return;
   const int s = e / nrec;
   RecPlace p;
-  if (!p.find(rec_idx[e], s, nx, ny, H, tiles_x, tiles_y, box)) return;
+  if (!p.find(rec_idx[e], s, nx, ny, H, tiles_x, tiles_y, box)) {
+    if (!FILL && tr_x != nullptr)
+      for (int k = 0; k < nt_out; ++k) {
+        const size_t o = ((size_t)s * nt_out + k) * nrec + (e - s * nrec);
+        tr_x[o] = tr_y[o] = 0.f;
+      }
+    return;
+  }
   for (int xt = p.x0; xt <= p.x1; ++xt)
     for (int yt = p.y0; yt <= p.y1; ++yt) {
       const int rr = p.oi - xt * H, cc = p.oj - yt * kBlkCols;
@@ -1891,7 +1900,8 @@ size_t blk_rec_bytes(size_t ntiles, int S, int nrec) {
 }
 
 cudaError_t launch_rec_tiles(int geo, const int32_t* rec_idx, int S, int nrec, int nx, int ny, const int4* box,
-                             size_t ntiles, void* ws, const int2** tile, const int2** ent, cudaStream_t st) {
+                             size_t ntiles, void* ws, const int2** tile, const int2** ent, float* tr_x, float* tr_y,
+                             int nt_out, cudaStream_t st) {
   const int H = blk_tile_rows(geo);
   int* count = static_cast<int*>(ws);
   int2* tl = reinterpret_cast<int2*>(static_cast<char*>(ws) + (ntiles + 2) / 2 * 8);
@@ -1903,13 +1913,15 @@ cudaError_t launch_rec_tiles(int geo, const int32_t* rec_idx, int S, int nrec, i
   const int n = S * nrec, tx = (nx + H - 1) / H, ty = (ny + kBlkCols - 1) / kBlkCols;
   const int nt = (int)ntiles;
   e = tracked_launch(kProfOther, st, [&] {
-    rec_tiles_kernel<false><<<(n + 255) / 256, 256, 0, st>>>(rec_idx, S, nrec, nx, ny, H, tx, ty, box, count, tl, en);
+    rec_tiles_kernel<false><<<(n + 255) / 256, 256, 0, st>>>(rec_idx, S, nrec, nx, ny, H, tx, ty, box, count, tl, en, tr_x,
+                                                             tr_y, nt_out);
   });
   if (e != cudaSuccess) return e;
   e = tracked_launch(kProfOther, st, [&] { rec_base_kernel<<<(nt + 255) / 256, 256, 0, st>>>(count, nt, tl); });
   if (e != cudaSuccess) return e;
   return tracked_launch(kProfOther, st, [&] {
-    rec_tiles_kernel<true><<<(n + 255) / 256, 256, 0, st>>>(rec_idx, S, nrec, nx, ny, H, tx, ty, box, count, tl, en);
+    rec_tiles_kernel<true><<<(n + 255) / 256, 256, 0, st>>>(rec_idx, S, nrec, nx, ny, H, tx, ty, box, count, tl, en, tr_x,
+                                                            tr_y, nt_out);
   });
 }
 

@@ -133,10 +133,12 @@ struct InstDesc {
 // (2 x S int4) described in InstTiles.
 cudaError_t launch_inst_table(const InstDesc& d, int4* tiles, int4* box, cudaStream_t st);
 // Receivers of the tiles of a call: room for `ntiles` tiles, and the table
-// (box: instances, else nullptr).
+// (box: instances, else nullptr).  The traces of receivers outside the grid
+// (tr_x, tr_y; nullptr: not recorded here) become zeros.
 size_t blk_rec_bytes(size_t ntiles, int S, int nrec);
 cudaError_t launch_rec_tiles(int geo, const int32_t* rec_idx, int S, int nrec, int nx, int ny, const int4* box,
-                             size_t ntiles, void* ws, const int2** tile, const int2** ent, cudaStream_t st);
+                             size_t ntiles, void* ws, const int2** tile, const int2** ent, float* tr_x, float* tr_y,
+                             int nt_out, cudaStream_t st);
 bool blk_available();  // the driver exposes the tensor-map encoder
 cudaError_t launch_blk_fwd(int mode, const BlkFwd& a, int* err, cudaStream_t st);
 cudaError_t launch_blk_adj(int mode, const BlkAdj& a, int* err, cudaStream_t st);

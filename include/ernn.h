@@ -118,7 +118,8 @@ typedef struct ErnnInputs {
   const float* src_signal;   /* nshots*nt: force amplitude of step i */
   const float* src_map;      /* nshots*src_bx*src_by: spatial load inside the box */
   const int32_t* src_origin; /* nshots*2: (x0, y0) of each shot's box; may lie partly outside */
-  const int32_t* rec_idx;    /* nshots*nrec flat cell indices; NULL unless RECEIVERS */
+  const int32_t* rec_idx;    /* nshots*nrec flat cell indices; NULL unless RECEIVERS.  One outside the
+                              * grid records zeros and injects nothing in the adjoint */
 } ErnnInputs;
 
 /* ABI version of the loaded library (ERNN_ABI_VERSION). */

@@ -1,0 +1,58 @@
+"""Calls at the edges of the rules that choose the kernels give on every route
+what the plain per-step kernels give.  GPU only."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+import ernn_gb300 as E
+from cases import random_case, rel
+from oracle import oracle as O
+from test_gpu_parity import DEV, to_geometry
+
+pytestmark = pytest.mark.gpu
+
+
+def forward_into_poison(case, path):
+    """ernn_forward through the C ABI, whose receiver indices are device data
+    that no host check sees, into outputs full of NaN."""
+    geom = to_geometry(case, path=path)
+    lib = E.load_library()
+    prob = geom.problem(case.mode)
+    C = torch.tensor(case.C, dtype=torch.float32, device=DEV)
+    D = None if case.D is None else torch.tensor(case.D, dtype=torch.float32, device=DEV)
+    rho = torch.tensor([case.rho], dtype=torch.float32, device=DEV)
+    out = torch.full((2,) + geom.out_shape(), float("nan"), device=DEV)
+    ptr = lambda t: ctypes.c_void_p(None if t is None else t.data_ptr())
+    ins = E._lib.ErnnInputs(ptr(C), ptr(D), ptr(rho), ptr(geom.src_signal), ptr(geom.src_map), ptr(geom.src_origin),
+                            ptr(geom.rec_idx))
+    n = lib.ernn_tape_bytes(ctypes.byref(prob), 1)
+    tape = torch.empty(n, dtype=torch.uint8, device=DEV)
+    rc = lib.ernn_forward(ctypes.byref(prob), ctypes.byref(ins), ptr(out[0]), ptr(out[1]), ptr(tape),
+                          ctypes.c_size_t(n), 1, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    torch.cuda.synchronize()
+    return out.cpu().numpy(), lib.ernn_last_path()
+
+
+@pytest.mark.parametrize("kw,path", [
+    (dict(nx=61, ny=243), E.PATH_TILED),                              # passes of one launch
+    (dict(nx=313, ny=389, S=3), E.PATH_TILED),                        # a launch per pass
+    (dict(nx=61, ny=243, mode=O.MODE_DFIELD), E.PATH_TILED),
+    (dict(nx=61, ny=243, mode=O.MODE_FIELDS), E.PATH_TILED),
+    (dict(nx=64, ny=64, S=2), E.PATH_RESIDENT),
+    (dict(nx=61, ny=33), E.PATH_STEP),
+])
+def test_receivers_outside_the_grid_record_zeros(kw, path):
+    case = random_case(nt=23, stride=2, record=O.RECORD_RECEIVERS, nrec=12, **kw)
+    inside = case.rec_idx.copy()
+    case.rec_idx[:, [0, 5, 11]] = [-1, case.nx * case.ny, -2 ** 31]
+    case.rec_idx[0, 7] = 2 ** 31 - 1
+    got, used = forward_into_poison(case, E.PATH_AUTO)
+    assert used == path
+    want, _ = forward_into_poison(case, E.PATH_STEP)
+    out = case.rec_idx != inside  # (S, nrec)
+    shot, rec = np.nonzero(out)
+    assert np.all(got[:, shot, :, rec] == 0) and np.all(want[:, shot, :, rec] == 0)
+    assert np.all(np.isfinite(got)) and rel(got, want) <= 1e-5
