@@ -1686,26 +1686,13 @@ bool blk_map(CUtensorMap* m, const float* base, int nx, int ny, int pitch, int S
             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-int blk_sms() {
-  static int n = [] {
-    int dev = 0, v = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0)
-      return 1;
-    return v;
-  }();
-  return n;
-}
-
-
 template <int MODE, int W, int RW, int CTAS, bool INST, int ORDER>
 cudaError_t fwd_t(const BlkFwd& a, int* err, cudaStream_t st) {
   using B = BlkTile<W, RW>;
   constexpr size_t smem = B::kBytes;
-  static std::once_flag once;
-  static cudaError_t ready = cudaSuccess;
-  std::call_once(once, [] {
-    ready = cudaFuncSetAttribute(blk_fwd_kernel<MODE, W, RW, INST, ORDER, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static OncePerDevice once;
+  const cudaError_t ready = once([] {
+    return cudaFuncSetAttribute(blk_fwd_kernel<MODE, W, RW, INST, ORDER, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
   if (ready != cudaSuccess) return ready;
   const int planes = INST ? 1 : a.S;
@@ -1716,7 +1703,7 @@ cudaError_t fwd_t(const BlkFwd& a, int* err, cudaStream_t st) {
     return cudaErrorNotSupported;
   const int tiles_x = (a.nx + B::kUse - 1) / B::kUse, tiles_y = (a.ny + kBlkCols - 1) / kBlkCols;
   const int ntiles = INST ? a.inst.ntiles : a.S * tiles_x * tiles_y;
-  const int grid = ntiles < CTAS * blk_sms() ? ntiles : CTAS * blk_sms();
+  const int grid = ntiles < CTAS * device_info().sms ? ntiles : CTAS * device_info().sms;
   const double cells = INST ? (double)ntiles * B::kUse * kBlkCols : (double)a.S * a.nx * a.ny;
   int stores = 0;
   for (int t = 0; t <= a.T; ++t) stores += a.out[t] != nullptr ? 1 : 0;
@@ -1730,10 +1717,9 @@ template <int W, int RW, int CTAS, bool INST, int ORDER>
 cudaError_t adj_t(const BlkAdj& a, int* err, cudaStream_t st) {
   using B = BlkTile<W, RW>;
   constexpr size_t smem = B::kBytes;
-  static std::once_flag once;
-  static cudaError_t ready = cudaSuccess;
-  std::call_once(once, [] {
-    ready = cudaFuncSetAttribute(blk_adj_kernel<W, RW, INST, ORDER, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static OncePerDevice once;
+  const cudaError_t ready = once([] {
+    return cudaFuncSetAttribute(blk_adj_kernel<W, RW, INST, ORDER, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
   if (ready != cudaSuccess) return ready;
   const int planes = INST ? 1 : a.S;
@@ -1744,7 +1730,7 @@ cudaError_t adj_t(const BlkAdj& a, int* err, cudaStream_t st) {
     return cudaErrorNotSupported;
   const int tiles_x = (a.nx + B::kUse - 1) / B::kUse, tiles_y = (a.ny + kBlkCols - 1) / kBlkCols;
   const int ntiles = INST ? a.inst.ntiles : a.S * tiles_x * tiles_y;
-  const int all = CTAS * blk_sms(), slots = all < kTiledRowsPerShot ? all : kTiledRowsPerShot;  // a partial row each
+  const int all = CTAS * device_info().sms, slots = all < kTiledRowsPerShot ? all : kTiledRowsPerShot;  // a partial row each
   const int grid = ntiles < slots ? ntiles : slots;
   const double cells = INST ? (double)ntiles * B::kUse * kBlkCols : (double)a.S * a.nx * a.ny;
   return tracked_launch(kProfAdjoint, st, [&] {
@@ -1757,11 +1743,10 @@ cudaError_t adj_t(const BlkAdj& a, int* err, cudaStream_t st) {
 template <int W, int RW, int CTAS>
 cudaError_t adj_d_t(const BlkAdj& a, int* err, cudaStream_t st) {
   using B = BlkTile<W, RW>;
-  static std::once_flag once;
-  static cudaError_t ready = cudaSuccess;
-  std::call_once(once, [] {
-    ready = cudaFuncSetAttribute(blk_adj_d_kernel<W, RW, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)B::kBytes);
+  static OncePerDevice once;
+  const cudaError_t ready = once([] {
+    return cudaFuncSetAttribute(blk_adj_d_kernel<W, RW, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)B::kBytes);
   });
   if (ready != cudaSuccess) return ready;
   const float* any = a.cur ? a.cur : a.out_last;  // (a level that is zero is not loaded)
@@ -1770,7 +1755,7 @@ cudaError_t adj_d_t(const BlkAdj& a, int* err, cudaStream_t st) {
       !blk_map(&pm, a.prev ? a.prev : any, a.nx, a.ny, a.pitch, a.S, kBox, B::kRows))
     return cudaErrorNotSupported;
   const int tiles_x = (a.nx + B::kUse - 1) / B::kUse, tiles_y = (a.ny + kBlkCols - 1) / kBlkCols;
-  const int ntiles = a.S * tiles_x * tiles_y, slots = CTAS * blk_sms();
+  const int ntiles = a.S * tiles_x * tiles_y, slots = CTAS * device_info().sms;
   return tracked_launch(kProfAdjoint, st, [&] {
     launch_step_kernel(blk_adj_d_kernel<W, RW, CTAS>, dim3(ntiles < slots ? ntiles : slots), dim3(32 * W), B::kBytes,
                        st, a.chained != 0, a, cm, pm, tiles_x, tiles_y, ntiles, err);
@@ -1798,11 +1783,10 @@ cudaError_t launch_run(int cls, Kernel kernel, int ntiles, size_t smem, double b
 template <int MODE, int RW, int ORDER>
 cudaError_t fwd_run(const BlkFwd& a, const FwdRun& r, int* err, cudaStream_t st) {
   using R = RunTile<RW>;
-  static std::once_flag once;
-  static cudaError_t ready = cudaSuccess;
-  std::call_once(once, [] {
-    ready = cudaFuncSetAttribute(run_fwd_kernel<MODE, RW, ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)R::kBytes);
+  static OncePerDevice once;
+  const cudaError_t ready = once([] {
+    return cudaFuncSetAttribute(run_fwd_kernel<MODE, RW, ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)R::kBytes);
   });
   if (ready != cudaSuccess) return ready;
   const int tiles_x = (a.nx + R::kUse - 1) / R::kUse, tiles_y = (a.ny + kBlkCols - 1) / kBlkCols;
@@ -1813,11 +1797,10 @@ cudaError_t fwd_run(const BlkFwd& a, const FwdRun& r, int* err, cudaStream_t st)
 template <int RW, int ORDER>
 cudaError_t adj_run(const BlkAdj& a, const AdjRun& r, int* err, cudaStream_t st) {
   using R = RunTile<RW>;
-  static std::once_flag once;
-  static cudaError_t ready = cudaSuccess;
-  std::call_once(once, [] {
-    ready = cudaFuncSetAttribute(run_adj_kernel<RW, ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)R::kBytes);
+  static OncePerDevice once;
+  const cudaError_t ready = once([] {
+    return cudaFuncSetAttribute(run_adj_kernel<RW, ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)R::kBytes);
   });
   if (ready != cudaSuccess) return ready;
   const int tiles_x = (a.nx + R::kUse - 1) / R::kUse, tiles_y = (a.ny + kBlkCols - 1) / kBlkCols;
@@ -1829,10 +1812,9 @@ template <bool RUN>
 cudaError_t adj_f(const BlkAdj& a, const std::conditional_t<RUN, AdjRun, NoRun>& r, int* err, cudaStream_t st) {
   constexpr int W = kRunW, H = W - 2 * kH;
   constexpr size_t smem = (size_t)2 * 4 * W * kBox * 4 + 128;
-  static std::once_flag once;
-  static cudaError_t ready = cudaSuccess;
-  std::call_once(once, [] {
-    ready = cudaFuncSetAttribute(blk_adj_f_kernel<W, RUN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static OncePerDevice once;
+  const cudaError_t ready = once([] {
+    return cudaFuncSetAttribute(blk_adj_f_kernel<W, RUN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
   if (ready != cudaSuccess) return ready;
   const int tiles_x = (a.nx + H - 1) / H, tiles_y = (a.ny + kBlkCols - 1) / kBlkCols;
@@ -1843,7 +1825,7 @@ cudaError_t adj_f(const BlkAdj& a, const std::conditional_t<RUN, AdjRun, NoRun>&
                       ntiles, err);
   } else {
     return tracked_launch(kProfAdjoint, st, [&] {
-      launch_step_kernel(blk_adj_f_kernel<W, false>, dim3(ntiles < blk_sms() ? ntiles : blk_sms()), dim3(32 * W), smem,
+      launch_step_kernel(blk_adj_f_kernel<W, false>, dim3(ntiles < device_info().sms ? ntiles : device_info().sms), dim3(32 * W), smem,
                          st, a.chained != 0, a, r, tiles_x, tiles_y, ntiles, err);
     }, (double)a.S * a.nx * a.ny * (8.0 * a.T + 32.0 + 72.0));
   }
@@ -1970,12 +1952,8 @@ cudaError_t launch_blk_adj(int mode, const BlkAdj& a, int* err, cudaStream_t st)
 // planes.
 bool blk_run_fits(int mode, int geo, int nx, int ny, int S) {
   if (mode == kModeDField || (geo != kBlkFlat && geo != kBlkShort)) return false;
-  static const bool coop = [] {
-    int dev = 0, v = 0;
-    return cudaGetDevice(&dev) == cudaSuccess &&
-           cudaDeviceGetAttribute(&v, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && v != 0;
-  }();
-  return coop && S * blk_tiles(geo, nx, ny) <= (size_t)blk_sms();
+  const DeviceInfo d = device_info();
+  return d.cooperative && S * blk_tiles(geo, nx, ny) <= (size_t)d.sms;
 }
 
 cudaError_t launch_blk_fwd_run(int mode, const BlkFwd& a, const FwdRun& r, int* err, cudaStream_t st) {

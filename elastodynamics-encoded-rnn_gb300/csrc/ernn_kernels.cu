@@ -17,6 +17,22 @@
 
 namespace ernn {
 
+DeviceInfo device_info() {
+  static std::atomic<int> known[64];  // 0: not queried yet, else 2 SMs + cooperative
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return DeviceInfo{1, false};
+  int v = dev < 64 ? known[dev].load(std::memory_order_relaxed) : 0;
+  if (v == 0) {
+    int sms = 0, coop = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
+      return DeviceInfo{1, false};
+    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess) coop = 0;
+    v = 2 * sms + (coop != 0 ? 1 : 0);
+    if (dev < 64) known[dev].store(v, std::memory_order_relaxed);
+  }
+  return DeviceInfo{v / 2, (v & 1) != 0};
+}
+
 static std::atomic<uint64_t> g_launches{0};
 uint64_t launches() { return g_launches.load(std::memory_order_relaxed); }
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }

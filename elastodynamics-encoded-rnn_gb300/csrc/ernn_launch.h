@@ -2,6 +2,7 @@
 // kernels (ernn_kernels.cu).  Internal to the library.
 #pragma once
 
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 #include <functional>
@@ -86,6 +87,36 @@ cudaError_t launch_operator(int S, int nx, int ny, int mode, double h, const flo
                             const float* D, const float* rho, const float* ux, const float* uy,
                             const float* fx, const float* fy, float* Lux, float* Luy,
                             cudaStream_t st);
+
+// What the library keeps about a device it has run on.
+struct DeviceInfo {
+  int sms;           // at least 1
+  bool cooperative;  // cooperative launches
+};
+DeviceInfo device_info();  // of the current device; queried once per device
+
+// A step made once per device, such as raising a kernel's dynamic
+// shared-memory limit: the limit belongs to the device's copy of the kernel.
+// One object per kernel (a function-local static); threads may race to the
+// first call, whose step is then made more than once.  A failed step is tried
+// again by the next call.
+class OncePerDevice {
+ public:
+  template <class Fn>
+  cudaError_t operator()(Fn&& step) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const uint64_t bit = dev < 64 ? (uint64_t)1 << dev : 0;  // (later devices: every call)
+    if (done_.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    e = step();
+    if (e == cudaSuccess) done_.fetch_or(bit, std::memory_order_release);
+    return e;
+  }
+
+ private:
+  std::atomic<uint64_t> done_{0};
+};
 
 uint64_t launches();
 void count_launch();

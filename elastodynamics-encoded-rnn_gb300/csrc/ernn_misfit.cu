@@ -174,20 +174,9 @@ __global__ void __launch_bounds__(kMisfitThreads)
   }
 }
 
-int num_sms_cached() {
-  static int sms = [] {
-    int dev = 0, v = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      return 132;
-    return v;
-  }();
-  return sms;
-}
-
 // Blocks along a row and over rows: about four blocks per SM in all.
 dim3 grid_of(int64_t rows, int64_t len) {
-  const int64_t want = 4LL * num_sms_cached();
+  const int64_t want = 4LL * device_info().sms;
   int64_t gx = (len + kMisfitThreads * 4 - 1) / (kMisfitThreads * 4);
   gx = gx < 1 ? 1 : (gx > want ? want : gx);
   int64_t gy = want / gx;

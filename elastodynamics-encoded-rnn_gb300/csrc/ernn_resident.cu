@@ -1309,48 +1309,46 @@ size_t resident_smem_bytes(const ResCommon& c) {
 }
 
 // Raise the kernel's dynamic shared-memory limit to at least `smem` (once per
-// kernel and size; the limit only grows).
+// device, kernel and size; the limit only grows).
 static cudaError_t configure(const void* fn, size_t smem) {
+  struct Limit {
+    int dev;
+    const void* fn;
+    size_t smem;
+  };
   static std::mutex mu;
-  static std::vector<std::pair<const void*, size_t>> done;
+  static std::vector<Limit> done;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
   std::lock_guard<std::mutex> lock(mu);
-  for (auto& kv : done)
-    if (kv.first == fn && kv.second >= smem) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  for (auto& d : done)
+    if (d.dev == dev && d.fn == fn && d.smem >= smem) return cudaSuccess;
+  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
-  for (auto& kv : done)
-    if (kv.first == fn) { kv.second = smem; return cudaSuccess; }
-  done.push_back({fn, smem});
+  for (auto& d : done)
+    if (d.dev == dev && d.fn == fn) { d.smem = smem; return cudaSuccess; }
+  done.push_back({dev, fn, smem});
   return cudaSuccess;
-}
-
-static int sm_count() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
-      n = 1;
-  }
-  return n;
 }
 
 int resident_img_clusters(const ResCommon& c) {
   // IMG clusters per shot row of the grid: fill the SMs the FWD and LAM
   // clusters leave free, at least one, at most eight
-  const int free_sm = sm_count() - 2 * c.S * c.CL;
+  const int free_sm = device_info().sms - 2 * c.S * c.CL;
   int z = free_sm / (c.CL * c.S);
   if (z < 1) z = 1;
   if (z > 8) z = 8;
   return z;
 }
 
-// Feasibility answers per (kernel, cluster size, shared memory): the
+// Feasibility answers per (device, kernel, cluster size, shared memory): the
 // attribute and occupancy queries run once, so later calls (for example
 // during stream capture) make no CUDA runtime calls here.
 struct FeasKey {
+  int dev;
   bool dense;
   int CL;
   size_t smem;
@@ -1375,11 +1373,13 @@ bool resident_feasible(const ResCommon& c, bool dense) {
   if ((c.CL - 1) * c.R >= c.nx) return false;  // every CTA owns >= 1 row
   const size_t smem = resident_smem_bytes(c);
   if (smem > kResSmemLimit) return false;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
   std::lock_guard<std::mutex> lock(g_feas_mu);
   for (const auto& kv : g_feas)
-    if (kv.first.dense == dense && kv.first.CL == c.CL && kv.first.smem == smem) return kv.second;
+    if (kv.first.dev == dev && kv.first.dense == dense && kv.first.CL == c.CL && kv.first.smem == smem) return kv.second;
   const bool ok = feasible_uncached(c, dense, smem);
-  g_feas.push_back({FeasKey{dense, c.CL, smem}, ok});
+  g_feas.push_back({FeasKey{dev, dense, c.CL, smem}, ok});
   return ok;
 }
 

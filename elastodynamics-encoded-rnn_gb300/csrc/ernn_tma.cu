@@ -637,17 +637,6 @@ bool make_map(CUtensorMap* m, const float* base, int nx, int ny, int S, int bw, 
             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-int num_sms() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
-      n = 1;
-  }
-  return n;
-}
-
 // Tensor map over the degradation plane [nx][ny]: dims (ny, nx).
 bool make_map2(CUtensorMap* m, const float* base, int nx, int ny, int bw, int bh) {
   auto fn = encode_fn();
@@ -665,14 +654,12 @@ constexpr size_t kFwdSmem = 2 * (size_t)FwdLayout::kStage * 4 + 16 + 128;
 constexpr size_t kAdjSmem = (size_t)AdjLayout::kStages * AdjLayout::kStage * 4 + 8 * AdjLayout::kStages + 128;
 
 cudaError_t set_smem() {
-  static std::once_flag once;
-  static cudaError_t result = cudaSuccess;
-  std::call_once(once, [] {
+  static OncePerDevice once;
+  return once([] {
     const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    result = cudaFuncSetAttribute(tma_fwd_kernel, at, (int)kFwdSmem);
-    if (result == cudaSuccess) result = cudaFuncSetAttribute(tma_adj_kernel, at, (int)kAdjSmem);
+    const cudaError_t e = cudaFuncSetAttribute(tma_fwd_kernel, at, (int)kFwdSmem);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(tma_adj_kernel, at, (int)kAdjSmem);
   });
-  return result;
 }
 
 }  // namespace
@@ -740,7 +727,7 @@ cudaError_t launch_tma_fwd(const FwdStep& a, int* err, cudaStream_t st) {
   cudaError_t e = set_smem();
   if (e != cudaSuccess) return e;
   const int tiles_x = (a.nx + F::kTR - 1) / F::kTR, tiles_y = (a.ny + kTY - 1) / kTY;
-  const int grid = persistent_grid(a.S * tiles_x * tiles_y, num_sms() * F::kCtasPerSm);
+  const int grid = persistent_grid(a.S * tiles_x * tiles_y, device_info().sms * F::kCtasPerSm);
   return tracked_launch(kProfForward, st, [&] {
     launch_step_kernel(tma_fwd_kernel, dim3(grid), dim3(kThreads), kFwdSmem, st, false, a, cur_map, prev_map, tiles_x,
                        tiles_y, a.prev ? 1 : 0, err);
@@ -760,7 +747,7 @@ cudaError_t launch_tma_adj(const AdjStep& a, int* err, cudaStream_t st) {
   cudaError_t e = set_smem();
   if (e != cudaSuccess) return e;
   const int tiles_x = (a.nx + L::kTR - 1) / L::kTR, tiles_y = (a.ny + kTY - 1) / kTY;
-  const int grid = persistent_grid(a.S * tiles_x * tiles_y, num_sms() * L::kCtasPerSm);
+  const int grid = persistent_grid(a.S * tiles_x * tiles_y, device_info().sms * L::kCtasPerSm);
   return tracked_launch(kProfAdjoint, st, [&] {
     launch_step_kernel(tma_adj_kernel, dim3(grid), dim3(kThreads), kAdjSmem, st, false, a, cur_map, u_map, d_map,
                        tiles_x, tiles_y, a.u ? 1 : 0, err);

@@ -1,0 +1,89 @@
+"""The host side of the library on a CUDA runtime that only records
+(tests/abi_c/fake_cudart.c): what is launched, on which device, with which
+workspaces, and what happens when the runtime refuses.  Runs on the CPU; no
+kernel runs."""
+import ctypes
+import glob
+import os
+import shutil
+import subprocess
+
+import pytest
+
+import ernn_gb300 as E
+from conftest import ROOT
+
+TAPE, SCRATCH, DATA = 1 << 40, 1 << 41, 1 << 42  # addresses that are never dereferenced
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    gcc = shutil.which("gcc")
+    include = "/usr/local/cuda/include"
+    E.load_library()  # builds the objects where they are missing
+    objs = glob.glob(os.path.join(os.path.dirname(E._lib.library_path()), "*.o"))
+    if gcc is None or not os.path.exists(os.path.join(include, "cuda_runtime_api.h")) or not objs:
+        pytest.skip("gcc, the CUDA headers or the library's objects absent")
+    out = str(tmp_path_factory.mktemp("fake") / "libernn_fake.so")
+    subprocess.run([gcc, "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I", include,
+                    os.path.join(ROOT, "tests", "abi_c", "fake_cudart.c"), *objs, "-lstdc++", "-o", out], check=True)
+    lib = ctypes.CDLL(out)
+    for name, (res, args) in E._lib.SIGNATURES.items():
+        f = getattr(lib, name)
+        f.restype, f.argtypes = res, args
+    lib.fake_launch.restype = ctypes.c_char_p
+    lib.fake_memset.restype = ctypes.c_void_p
+    return lib
+
+
+def setup(lib, device=0, sms=152, refuse_cooperative=0, clusters=1):
+    lib.fake_set(device, sms, refuse_cooperative, clusters)
+    lib.fake_reset()
+
+
+def problem(**kw):
+    base = dict(nshots=1, nx=64, ny=48, nt=20, stride=1, mode=0, record=1, nrec=8, src_comp=1, src_bx=9, src_by=9,
+                ckpt_k=20, path=0, flags=0, h=1e-4, dt=5e-9)
+    base.update(kw)
+    return E._lib.ErnnProblem(*[base[f] for f, _ in E._lib.ErnnProblem._fields_])
+
+
+def call(lib, p, tape=TAPE, scratch=SCRATCH):
+    """ernn_forward and ernn_adjoint; their return codes."""
+    ptr = ctypes.c_void_p
+    ins = E._lib.ErnnInputs(*[ptr(DATA + (k << 36)) for k in range(7)])
+    nt, ns = lib.ernn_tape_bytes(ctypes.byref(p), 1), lib.ernn_adjoint_scratch_bytes(ctypes.byref(p))
+    a, b, c, d = (ptr(DATA + (k << 36)) for k in (8, 9, 10, 11))
+    return (lib.ernn_forward(ctypes.byref(p), ctypes.byref(ins), a, b, ptr(tape), nt, 1, None),
+            lib.ernn_adjoint(ctypes.byref(p), ctypes.byref(ins), a, b, ptr(tape), nt, ptr(scratch), ns, c, d, None))
+
+
+def launches(lib):
+    """(kernel, device, cooperative, grid, first bytes of the first argument) of every launch since setup."""
+    out = []
+    for i in range(lib.fake_launches()):
+        v, smem, arg = (ctypes.c_int * 5)(), ctypes.c_size_t(), (ctypes.c_ubyte * 96)()
+        name = lib.fake_launch(i, v, ctypes.byref(smem), arg).decode()
+        out.append((name, v[0], v[1], v[2], bytes(arg)))
+    return out
+
+
+@pytest.mark.parametrize("kw", [
+    dict(nx=61, ny=43), dict(nx=200, ny=243, nshots=4), dict(nx=300, ny=301, nshots=9), dict(path=3), dict(mode=1, ny=47),
+    dict(mode=1, path=3), dict(mode=2, ny=47), dict(nx=128, ny=128), dict(mode=2, nx=200, ny=243, nshots=4),
+])
+def test_every_device_of_a_process_gets_its_own_limits(lib, kw):
+    for device in (0, 1, 0, 2):
+        setup(lib, device)
+        assert call(lib, problem(**kw)) == (0, 0), device
+        assert lib.fake_launches() > 0 and all(l[1] == device for l in launches(lib))
+
+
+def test_grids_follow_the_device_they_run_on(lib):
+    p = problem(nx=300, ny=301, nshots=16)  # more tiles than either device has slots for
+    grid = {}
+    for device, sms in ((0, 152), (3, 40)):
+        setup(lib, device, sms)
+        assert call(lib, p) == (0, 0)
+        grid[device] = max(l[3] for l in launches(lib) if "blk_adj_kernel" in l[0])
+    assert grid == {0: 304, 3: 80}
