@@ -47,10 +47,14 @@ struct Plan {
 };
 
 // Grids that the plain per-step kernels took before the time-blocked ones:
-// odd rows, or a step of fewer than four 64 x 32 tiles per SM.
+// odd rows, or a step of fewer than four 64 x 32 tiles per SM of this part's
+// 152.  From sizes alone: the workspace plan and the choice of the tiled
+// per-step kernels (use_tiled), whose tables the plan makes room for, use the
+// same line on every device.
+constexpr size_t kTiledMinTiles = 4 * 152;
 inline bool plain_size(const ErnnProblem& p) {
   return p.path == ERNN_PATH_AUTO && !(p.flags & ERNN_FLAG_INSTANCES) &&
-         (p.ny % 4 != 0 || tma_tiles(p.nx, p.ny, p.nshots) < 608);
+         (p.ny % 4 != 0 || tma_tiles(p.nx, p.ny, p.nshots) < kTiledMinTiles);
 }
 
 // Problems of the time-blocked tile kernels, from sizes alone (the workspace
@@ -251,9 +255,8 @@ std::atomic<int32_t> g_last_path{ERNN_PATH_AUTO};
 
 // Tiled per-step kernels (degradation maps): requested (ERNN_PATH_TILED, an
 // error when the problem is not eligible) or chosen by ERNN_PATH_AUTO when
-// eligible and one step has at least four 64 x 32 tiles per SM.  They are
-// persistent (2-3 CTAs of 72-111 KB shared memory per SM, each streaming
-// several tiles).  Scalar problems of the tiled path get here only with a
+// eligible and no plain_size grid.  They are persistent (2-3 CTAs of 72-111
+// KB shared memory per SM, each streaming several tiles).  Scalar problems of the tiled path get here only with a
 // tape that is not on a 16-byte boundary: the plain kernels take those.
 int use_tiled(const ErnnProblem& p, int* tiled) {
   *tiled = 0;
@@ -263,11 +266,7 @@ int use_tiled(const ErnnProblem& p, int* tiled) {
     *tiled = ok;
     return ok || (p.mode == kModeScalar && p.ny % 4 == 0 && blk_available()) ? ERNN_OK : ERNN_ERR_UNSUPPORTED;
   }
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    return ERNN_ERR_CUDA;
-  *tiled = ok && tma_tiles(p.nx, p.ny, p.nshots) >= 4 * (size_t)sms;
+  *tiled = ok && !plain_size(p);
   return ERNN_OK;
 }
 

@@ -87,3 +87,24 @@ def test_grids_follow_the_device_they_run_on(lib):
         assert call(lib, p) == (0, 0)
         grid[device] = max(l[3] for l in launches(lib) if "blk_adj_kernel" in l[0])
     assert grid == {0: 304, 3: 80}
+
+
+@pytest.mark.parametrize("sms", [152, 132, 40])
+@pytest.mark.parametrize("kw", [
+    dict(mode=1, nx=960, ny=1216),             # 570 tiles of 64 x 32: the tiles of four steps
+    dict(mode=1, nx=1024, ny=1216),            # 608: the tiled per-step kernels
+    dict(mode=1, nx=1024, ny=1216, path=3), dict(mode=1, nx=961, ny=1215), dict(nx=960, ny=1216), dict(nx=960, ny=1215),
+])
+def test_work_areas_are_cleared_inside_the_buffers(lib, kw, sms):
+    """Also with a tape that is on no 16-byte boundary, which changes the
+    kernels but not the sizes that were asked for."""
+    p = problem(ckpt_k=7, **kw)
+    nt, ns = lib.ernn_tape_bytes(ctypes.byref(p), 1), lib.ernn_adjoint_scratch_bytes(ctypes.byref(p))
+    for tape, scratch in ((TAPE, SCRATCH), (TAPE + 8, SCRATCH + 8)):
+        setup(lib, 0, sms)
+        assert call(lib, p, tape, scratch) == (0, 0)
+        for i in range(lib.fake_memsets()):
+            n = ctypes.c_size_t()
+            a = lib.fake_memset(i, ctypes.byref(n))
+            inside = [lo <= a and a + n.value <= lo + size for lo, size in ((tape, nt), (scratch, ns))]
+            assert any(inside) or a >= DATA, (hex(a), n.value)
