@@ -57,6 +57,10 @@ inline bool plain_size(const ErnnProblem& p) {
          (p.ny % 4 != 0 || tma_tiles(p.nx, p.ny, p.nshots) < kTiledMinTiles);
 }
 
+inline bool cluster_fits(const ErnnProblem& p) {
+  return resident_fits(p.mode, p.nx, p.ny, p.record == kRecordReceivers ? p.nrec : 0);
+}
+
 // Problems of the time-blocked tile kernels, from sizes alone (the workspace
 // queries, the forward and the adjoint agree).
 //  - Instances, and scalar constants on the tiled path: all of them.
@@ -64,7 +68,11 @@ inline bool plain_size(const ErnnProblem& p) {
 //    spans 120 columns: narrower grids leave most lanes idle, the plain
 //    kernels take those); states of odd rows are padded to 16-byte rows.
 //    (16 x 941x41, 200 steps: 5.11 ms there, 4.98 here; 5 x 1000x41: 3.05, 2.52.)
-//    Where the cluster-resident path can run it comes first.
+//    Where the cluster-resident path fits it comes first (on a device that
+//    cannot schedule its clusters such a problem takes the plain kernels).
+//    Larger receiver arrays, and grids that no cluster size can hold, come
+//    here (us per iteration, plain -> here: 24 x 256^2 with 2000 receivers,
+//    60 steps, 3980 -> 1616; 64 x 128^2 with 1100, 100 steps, 3631 -> 2308).
 //  - A degradation map: grids of the plain kernels' size.  On larger ones the
 //    TMA-fed kernels of one step are faster (8 x 512^2: 29 against 33 us per
 //    forward and adjoint step): the map, u's rows and the running gradient
@@ -85,7 +93,7 @@ bool block_rule(const ErnnProblem& p) {
     const double cost = blk_cost(blk_geometry(p.mode, p.nx, p.ny, p.nshots), p.nx, p.ny, p.nshots);
     return plain_size(p) && (cost <= 10.0 || cost <= 6.0 + 31e-6 * p.nshots * p.nx * p.ny);
   }
-  return !resident_possible(p.mode, p.nx, p.ny);
+  return !cluster_fits(p);
 }
 
 // Upper bound of the tile-table entries of any placement of S instances on
@@ -150,7 +158,7 @@ Plan make_plan(const ErnnProblem& p) {
   // two recompute segments: the cluster-resident path recomputes segment j-1
   // while the adjoint consumes segment j
   // (one segment where that path cannot run)
-  const bool res = resident_possible(p.mode, p.nx, p.ny) && !pl.inst;
+  const bool res = cluster_fits(p) && !pl.inst;
   pl.s_seg = off; if (!pl.store_all) off += (size_t)(pl.block && !res ? 1 : 2) * pl.k * pl.state_bytes;
   // lam buffers of the resident reverse pass: two segments of kres steps,
   // only where that path can run
@@ -256,8 +264,10 @@ std::atomic<int32_t> g_last_path{ERNN_PATH_AUTO};
 // Tiled per-step kernels (degradation maps): requested (ERNN_PATH_TILED, an
 // error when the problem is not eligible) or chosen by ERNN_PATH_AUTO when
 // eligible and no plain_size grid.  They are persistent (2-3 CTAs of 72-111
-// KB shared memory per SM, each streaming several tiles).  Scalar problems of the tiled path get here only with a
-// tape that is not on a 16-byte boundary: the plain kernels take those.
+// KB shared memory per SM, each streaming several tiles).  Scalar problems get
+// here with a tape that is not on a 16-byte boundary, with rows below
+// kBlockMinCols cells, or on a device that cannot schedule the clusters of the
+// resident path: the plain kernels take those.
 int use_tiled(const ErnnProblem& p, int* tiled) {
   *tiled = 0;
   if (p.path == ERNN_PATH_STEP) return ERNN_OK;
@@ -273,8 +283,7 @@ int use_tiled(const ErnnProblem& p, int* tiled) {
 // Cluster-resident configuration: CL CTAs of R rows each.  Returns false when
 // the problem does not fit the path (mode, alignment, receivers, memory).
 bool pick_resident(const ErnnProblem& p, const ErnnInputs& in, Coef* coef, ResCommon& rc) {
-  if (!resident_possible(p.mode, p.nx, p.ny)) return false;  // (the plan reserved no lam buffers)
-  if (p.record == kRecordReceivers && p.nrec > kResMaxRec) return false;
+  if (!cluster_fits(p)) return false;  // (the plan reserved no lam buffers)
   rc.nx = p.nx; rc.ny = p.ny; rc.S = p.nshots; rc.nt = p.nt; rc.stride = p.stride;
   rc.nt_out = (p.nt + p.stride - 1) / p.stride;
   rc.coef = coef;
@@ -285,11 +294,9 @@ bool pick_resident(const ErnnProblem& p, const ErnnInputs& in, Coef* coef, ResCo
   rc.nrec = (p.record == kRecordReceivers) ? p.nrec : 0;
   rc.err = &coef->err;
   for (int CL = 16; CL >= 1; CL /= 2) {
-    if (CL > p.nx) continue;
     rc.CL = CL;
-    rc.R = (p.nx + CL - 1) / CL;
-    if ((CL - 1) * rc.R >= p.nx) continue;
-    if (resident_feasible(rc, p.record == kRecordFields)) return true;
+    rc.R = resident_rows(p.nx, CL);
+    if (rc.R > 0 && resident_feasible(rc, p.record == kRecordFields)) return true;
   }
   return false;
 }

@@ -1360,12 +1360,18 @@ static bool feasible_uncached(const ResCommon& c, bool dense, size_t smem);
 
 constexpr size_t kResSmemLimit = 220 * 1024;
 
-bool resident_possible(int mode, int nx, int ny) {
-  if (mode != kModeScalar || ny % 4 != 0 || nx < 1) return false;
+int resident_rows(int nx, int CL) {
+  const int R = (nx + CL - 1) / CL;
+  return (CL - 1) * R < nx ? R : 0;
+}
+
+bool resident_fits(int mode, int nx, int ny, int nrec) {
+  if (mode != kModeScalar || ny % 4 != 0 || nrec > kResMaxRec) return false;
   ResCommon c{};
   c.ny = ny;
-  c.R = (nx + 15) / 16;  // the most CTAs per cluster give the fewest rows per CTA
-  return resident_smem_bytes(c) <= kResSmemLimit;
+  for (int CL = 16; CL >= 1; CL /= 2)
+    if ((c.R = resident_rows(nx, CL)) > 0 && resident_smem_bytes(c) <= kResSmemLimit) return true;
+  return false;
 }
 
 bool resident_feasible(const ResCommon& c, bool dense) {

@@ -70,9 +70,12 @@ struct ResRoles {
 };
 
 size_t resident_smem_bytes(const ResCommon& c);
-// Whether any cluster size can hold a shot of this grid (the adjoint scratch
-// reserves the path's lam buffers only then).
-bool resident_possible(int mode, int nx, int ny);
+// Rows per CTA of a cluster of CL CTAs over nx rows; 0: not every CTA has one.
+int resident_rows(int nx, int CL);
+// Whether any cluster size can hold a shot of this grid with nrec receivers,
+// from sizes alone (the adjoint scratch reserves the path's lam buffers only
+// then, and the time-blocked kernels take the other grids).
+bool resident_fits(int mode, int nx, int ny, int nrec);
 bool resident_feasible(const ResCommon& c, bool dense);
 // IMG clusters along z for one launch (total IMG CTAs = this x S x CL)
 int resident_img_clusters(const ResCommon& c);

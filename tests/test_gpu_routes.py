@@ -9,7 +9,8 @@ import torch
 import ernn_gb300 as E
 from cases import random_case, rel
 from oracle import oracle as O
-from test_gpu_parity import DEV, to_geometry
+from test_gpu_block import run
+from test_gpu_parity import DEV, to_geometry, weights
 
 pytestmark = pytest.mark.gpu
 
@@ -56,3 +57,18 @@ def test_receivers_outside_the_grid_record_zeros(kw, path):
     shot, rec = np.nonzero(out)
     assert np.all(got[:, shot, :, rec] == 0) and np.all(want[:, shot, :, rec] == 0)
     assert np.all(np.isfinite(got)) and rel(got, want) <= 1e-5
+
+
+@pytest.mark.parametrize("kw", [
+    dict(nx=64, ny=64, S=2, nrec=1025),    # more receivers than a CTA of a cluster may own
+    dict(nx=128, ny=132, nrec=1500),
+    dict(nx=20, ny=1600, nrec=9),          # no cluster size whose CTAs all own rows and hold them
+])
+def test_problems_that_no_cluster_takes_run_on_tiles(kw):
+    case = random_case(nt=50, record=O.RECORD_RECEIVERS, **kw)
+    wx, wy = weights(case)
+    ax, ay, ag, used = run(case, wx, wy, E.PATH_AUTO, 12)
+    assert used == E.PATH_TILED
+    bx, by, bg, _ = run(case, wx, wy, E.PATH_STEP, 12)
+    assert np.array_equal(ax, bx) and np.array_equal(ay, by)
+    assert rel(ag, bg) <= 1e-5, rel(ag, bg)
