@@ -64,10 +64,12 @@ inline bool cluster_fits(const ErnnProblem& p) {
 // Problems of the time-blocked tile kernels, from sizes alone (the workspace
 // queries, the forward and the adjoint agree).
 //  - Instances, and scalar constants on the tiled path: all of them.
-//  - ERNN_PATH_AUTO takes rows of any length from kBlockMinCols up (a warp
-//    spans 120 columns: narrower grids leave most lanes idle, the plain
-//    kernels take those); states of odd rows are padded to 16-byte rows.
-//    (16 x 941x41, 200 steps: 5.11 ms there, 4.98 here; 5 x 1000x41: 3.05, 2.52.)
+//  - ERNN_PATH_AUTO takes rows of any length from kBlockMinCols up (16 x
+//    941x41, 200 steps, time-blocked tiles against plain kernels: 4.98 and
+//    5.11 ms; 5 x 1000x41: 2.52 and 3.05), shorter ones from the size at which
+//    one-step tiles used to take them (64 x 4000x36, 40 steps: 5.29 ms, 15.7
+//    with the plain kernels, 7.63 with those tiles; 4 x 5000x32: 0.75, 1.02
+//    and 1.25); states of odd rows are padded to 16-byte rows.
 //    Where the cluster-resident path fits it comes first (on a device that
 //    cannot schedule its clusters such a problem takes the plain kernels).
 //    Larger receiver arrays, and grids that no cluster size can hold, come
@@ -87,20 +89,23 @@ inline bool cluster_fits(const ErnnProblem& p) {
 bool block_rule(const ErnnProblem& p) {
   if (p.flags & ERNN_FLAG_INSTANCES) return true;
   if (p.path == ERNN_PATH_TILED) return p.mode == kModeScalar && p.ny % 4 == 0;
-  if (p.path != ERNN_PATH_AUTO || p.ny < kBlockMinCols) return false;
+  if (p.path != ERNN_PATH_AUTO) return false;
+  if (p.mode == kModeScalar) return (p.ny >= kBlockMinCols || !plain_size(p)) && !cluster_fits(p);
+  if (p.ny < kBlockMinCols) return false;
   if (p.mode == kModeFields) return (double)p.nshots * p.nx * p.ny <= kBlockMaxFields;
   if (p.mode == kModeDField) {
     const double cost = blk_cost(blk_geometry(p.mode, p.nx, p.ny, p.nshots), p.nx, p.ny, p.nshots);
     return plain_size(p) && (cost <= 10.0 || cost <= 6.0 + 31e-6 * p.nshots * p.nx * p.ny);
   }
-  return !cluster_fits(p);
+  return false;
 }
 
 // Upper bound of the tile-table entries of any placement of S instances on
 // an nx x ny canvas (each instance's tiling has at most one partial tile row
 // and column).
 inline size_t inst_table_bound(int nx, int ny, int S) {
-  return ((size_t)(nx + blk_tile_rows(kBlkTall) - 1) / blk_tile_rows(kBlkTall) + S) * ((size_t)(ny + kBlkCols - 1) / kBlkCols + S);
+  const BlkShape g = blk_shape(kBlkTall);
+  return ((size_t)(nx + g.rows - 1) / g.rows + S) * ((size_t)(ny + g.cols - 1) / g.cols + S);
 }
 
 Plan make_plan(const ErnnProblem& p) {
@@ -265,7 +270,7 @@ std::atomic<int32_t> g_last_path{ERNN_PATH_AUTO};
 // error when the problem is not eligible) or chosen by ERNN_PATH_AUTO when
 // eligible and no plain_size grid.  They are persistent (2-3 CTAs of 72-111
 // KB shared memory per SM, each streaming several tiles).  Scalar problems get
-// here with a tape that is not on a 16-byte boundary, with rows below
+// here with a tape that is not on a 16-byte boundary, with few rows below
 // kBlockMinCols cells, or on a device that cannot schedule the clusters of the
 // resident path: the plain kernels take those.
 int use_tiled(const ErnnProblem& p, int* tiled) {
@@ -434,8 +439,8 @@ int plan_instances(const ErnnProblem& p, const ErnnInstances* in, InstPlan* ip) 
   for (int k = 0; k < S; ++k) order[k] = k;
   std::stable_sort(order, order + S, [&](int u, int v) { return in->nt[u] > in->nt[v]; });
   ip->d.count = S;
-  ip->d.tile_rows = blk_tile_rows(kBlkTall);
-  ip->d.tile_cols = kBlkCols;
+  ip->d.tile_rows = blk_shape(kBlkTall).rows;
+  ip->d.tile_cols = blk_shape(kBlkTall).cols;
   ip->upto[0] = 0;
   for (int g = 0; g < S; ++g) {
     const int k = order[g];

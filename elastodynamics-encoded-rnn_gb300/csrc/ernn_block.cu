@@ -14,8 +14,9 @@
 // of the window; the columns beside a quad come by lane shuffles, rows of
 // other warps from shared memory (one CTA barrier per step).  The valid region
 // shrinks by one cell per step, so the outer quad and the outer four rows of
-// the tile are not stored: 120 columns x (W RW - 8) rows are.  Two CTAs per SM
-// (tall tiles): one loads its tile while the other computes.
+// the tile are not stored: 120 columns x (W RW - 8) rows are (on grids of at
+// most 128 or 64 columns a tile holds whole rows and has no halo columns).  Two
+// CTAs per SM (tall tiles): one loads its tile while the other computes.
 //
 // Measured (16 x 1024^2, us per launch of four steps against four launches of
 // the one-step kernels before): forward 173 against 264, adjoint 290 against
@@ -54,7 +55,7 @@ struct BTile {
 // The tiles first, first + step, ... of a CTA.  Grid: walked in (shot, row
 // block, column block) digits, an addition with carries per tile; instances:
 // entries of the tile table.
-template <bool INST, int H>
+template <bool INST, int H, int C = kBlkCols>
 struct BWalk {
   int t, step, shot, xt, yt, ds, dx, dy, tiles_x, tiles_y, nx, ny;
   __device__ __forceinline__ void init(int first, int step_, int tx, int ty, int nx_, int ny_) {
@@ -82,7 +83,7 @@ struct BWalk {
       return BTile{0, e.x, (int)((unsigned)e.y & 0xffffu), (int)((unsigned)e.y >> 16), (int)((unsigned)e.z & 0xffffu),
                    (int)((unsigned)e.z >> 16), (int)((unsigned)e.w & 0xffffu), (int)((unsigned)e.w >> 16)};
     } else {
-      return BTile{shot, shot, xt * H, yt * kBlkCols, 0, 0, nx, ny};
+      return BTile{shot, shot, xt * H, yt * C, 0, 0, nx, ny};
     }
   }
   __device__ __forceinline__ void next() {
@@ -179,19 +180,38 @@ __device__ __forceinline__ Coefs cell_coefs(const float* f, size_t n, size_t o, 
 // (2 c - p) + l
 __device__ __forceinline__ float leap(float c, float p, float l) { return fmaf(2.f, c, -p) + l; }
 
-// A CTA's tile: both levels of W RW rows of 128 columns, both components,
-// with a guard row on either side (read for rows that are never stored).
-template <int W, int RW>
+// A CTA's tile: both levels of its rows, both components, with a guard row on
+// either side (read for rows that are never stored).  A row takes L lanes, a
+// quad each, so a warp holds 32 / L shares of RW rows.  WHOLE: the tile's
+// columns are all the grid's (or instance's): no halo columns, zeros beside
+// the first and the last.
+template <int W_, int RW_, int L = 32, bool WHOLE = false>
 struct BlkTile {
-  static constexpr int kThreads = 32 * W;
-  static constexpr int kRows = W * RW;
+  static constexpr int kW = W_, kRW = RW_, kLanes = L, kShares = 32 / L;
+  static constexpr bool kWhole = WHOLE;
+  static constexpr int kThreads = 32 * W_;
+  static constexpr int kRows = W_ * RW_ * kShares;
+  static constexpr int kCols = 4 * L;
+  static constexpr int kHY = WHOLE ? 0 : kH;         // halo columns
   static constexpr int kUse = kRows - 2 * kH;        // rows stored
-  static constexpr int kPlane = kRows * kBox;        // floats of a component
+  static constexpr int kUseY = kCols - 2 * kHY;      // columns stored
+  static constexpr int kPlane = kRows * kCols;       // floats of a component
   static constexpr int kLevel = 2 * kPlane;
   static constexpr int kFloats = 2 * kLevel + 2 * kBox;
   static constexpr int kMeta = 16;
   static constexpr size_t kBytes = (size_t)(kFloats + kMeta) * 4 + 8 + 128;
+  static_assert(L == 32 || WHOLE, "shares of a warp: whole rows");
 };
+
+// Whether a condition holds for any / every share of the warp.
+template <class B>
+__device__ __forceinline__ bool any_share(bool c) {
+  return B::kShares == 1 ? c : __any_sync(kFull, c) != 0;
+}
+template <class B>
+__device__ __forceinline__ bool every_share(bool c) {
+  return B::kShares == 1 ? c : __all_sync(kFull, c) != 0;
+}
 
 template <bool V>
 struct BoolC {
@@ -207,6 +227,14 @@ __device__ __forceinline__ void mask_q(float (&v)[4], int n) {
 __device__ __forceinline__ Row load_row(const float* p) {  // a row of the tile at the lane's quad
   return row_of(q4(*reinterpret_cast<const float4*>(p)));
 }
+// The same for a tile of the kernels below; ql: the lane's quad in its row.
+template <class B>
+__device__ __forceinline__ Row load_row(const float* p, int ql) {
+  if constexpr (!B::kWhole) return load_row(p);
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  const float l = __shfl_up_sync(kFull, v.w, 1, B::kLanes), r = __shfl_down_sync(kFull, v.x, 1, B::kLanes);
+  return Row{{ql > 0 ? l : 0.f, v.x, v.y, v.z, v.w, ql < B::kLanes - 1 ? r : 0.f}};
+}
 
 // Rows of a warp's share that lie in [lo, hi) of the tile, as bits.
 template <int RW>
@@ -218,11 +246,10 @@ __device__ __forceinline__ uint32_t rows_in(int rr0, int lo, int hi) {
 
 // Zeroes the tile's cells outside its instance's region (on a canvas they
 // belong to other instances), or all of a level that is a zero state.
-template <int W, int RW>
+template <class B>
 __device__ __forceinline__ void clear_cells(float* lev, bool all, const BTile& t) {
-  using B = BlkTile<W, RW>;
   for (int e = threadIdx.x; e < B::kPlane / 4; e += B::kThreads) {
-    const int gi = t.x0 - kH + (e >> 5), gj = t.y0 - kH + 4 * (e & 31);
+    const int gi = t.x0 - kH + e / B::kLanes, gj = t.y0 - B::kHY + 4 * (e % B::kLanes);
     if (!all && gi >= t.xs && gi < t.xe && gj >= t.ys && gj < t.ye) continue;
     const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
     *reinterpret_cast<float4*>(lev + 4 * e) = z;
@@ -233,38 +260,36 @@ __device__ __forceinline__ void clear_cells(float* lev, bool all, const BTile& t
 // Both levels of a tile into shared memory: c (u^i, or lam^{m+1}) and p (the
 // level before it); a level that is not used is zero.  Every thread calls it;
 // the tile is complete after the caller's next CTA barrier.
-template <int W, int RW, bool INST>
+template <class B, bool INST>
 __device__ __forceinline__ void load_tile(float* lev0, float* lev1, const CUtensorMap* cm, const CUtensorMap* pm,
                                           bool has_c, bool has_p, bool use_c, bool use_p, const BTile& t, int k,
                                           uint64_t* bar, PipeGuard* guard, int* err) {
-  using B = BlkTile<W, RW>;
   const uint32_t bytes = (uint32_t)((has_c ? B::kLevel : 0) + (has_p ? B::kLevel : 0)) * 4u;
   if (bytes != 0) {
     if (threadIdx.x == 0 && !pipe_failed(guard)) {
       pipe_issued(guard, k);
       fence_async();
       bar_expect(bar, bytes);
-      if (has_c) tma_load3(lev0, cm, t.y0 - kH, t.x0 - kH, 2 * t.plane, bar);
-      if (has_p) tma_load3(lev1, pm, t.y0 - kH, t.x0 - kH, 2 * t.plane, bar);
+      if (has_c) tma_load3(lev0, cm, t.y0 - B::kHY, t.x0 - kH, 2 * t.plane, bar);
+      if (has_p) tma_load3(lev1, pm, t.y0 - B::kHY, t.x0 - kH, 2 * t.plane, bar);
     }
     bar_wait_ok(bar, (uint32_t)k & 1u, err, guard);
   }
-  if (INST || !use_c) clear_cells<W, RW>(lev0, !use_c, t);
-  if (INST || !use_p) clear_cells<W, RW>(lev1, !use_p, t);
+  if (INST || !use_c) clear_cells<B>(lev0, !use_c, t);
+  if (INST || !use_p) clear_cells<B>(lev1, !use_p, t);
 }
 
 // ----------------------------------------------------------------- forward
 // Per-cell modes: FIELDS keeps the constants of the thread's cells in registers
 // for the launch (one row per thread); DFIELD reads the weights 1 - D of a row
 // one row ahead.
-template <int MODE, int W, int RW, bool INST, int ORDER, int CTAS>
-__global__ void __launch_bounds__(32 * W, CTAS)
+template <int MODE, class B, bool INST, int ORDER, int CTAS>
+__global__ void __launch_bounds__(B::kThreads, CTAS)
     blk_fwd_kernel(const BlkFwd a, const __grid_constant__ CUtensorMap cur_map,
                    const __grid_constant__ CUtensorMap prev_map, int tiles_x, int tiles_y, int ntiles, int* err) {
   extern __shared__ float sm_raw[];
   float* sm = aligned128(sm_raw);
-  using B = BlkTile<W, RW>;
-  constexpr int NT = B::kThreads;
+  constexpr int NT = B::kThreads, RW = B::kRW, kCols = B::kCols;
   float* lev0 = sm + kBox;  // (a guard row before and after the levels)
   float* lev1 = lev0 + B::kLevel;
   float* meta = sm + B::kFloats;
@@ -284,13 +309,14 @@ __global__ void __launch_bounds__(32 * W, CTAS)
   }
   // (zeros: what rows without a neighbour read stays finite)
   if (tid < kBox) sm[tid] = sm[B::kFloats - kBox + tid] = 0.f;
-  BWalk<INST, B::kUse> walk;
+  BWalk<INST, B::kUse, B::kUseY> walk;
   walk.init((int)blockIdx.x, (int)gridDim.x, tiles_x, tiles_y, nx, ny);
   __syncthreads();
   grid_dep_wait();  // the states of the previous launch are complete from here on
 
-  const int rr0 = w * RW;  // first row of the warp in the tile
-  const int o0 = rr0 * kBox + 4 * lane;
+  const int ql = lane % B::kLanes;                           // the lane's quad of its rows
+  const int rr0 = (w * B::kShares + lane / B::kLanes) * RW;  // the first of them in the tile
+  const int o0 = rr0 * kCols + 4 * ql;
   for (int k = 0; walk.t < ntiles; ++k, walk.next()) {
     const BTile tile = walk.tile(a.inst);
     // per-tile scalars: coefficients, amplitudes of the steps, source origin
@@ -301,15 +327,17 @@ __global__ void __launch_bounds__(32 * W, CTAS)
         meta[lane] = a.src_signal[(size_t)tile.inst * a.nt + a.i + lane - 8] * K->kappa;
       if (lane >= 12 && lane < 14 && has_src) meta[lane] = __int_as_float(a.src_origin[2 * tile.inst + lane - 12]);
     }
-    load_tile<W, RW, INST>(lev0, lev1, &cur_map, &prev_map, a.cur != nullptr, a.prev != nullptr, a.cur != nullptr,
-                           a.prev != nullptr, tile, k, bar, &guard, err);
+    load_tile<B, INST>(lev0, lev1, &cur_map, &prev_map, a.cur != nullptr, a.prev != nullptr, a.cur != nullptr,
+                       a.prev != nullptr, tile, k, bar, &guard, err);
     __syncthreads();
-    const int gj = tile.y0 - kH + 4 * lane, gi0 = tile.x0 - kH + rr0;
+    const int gj = tile.y0 - B::kHY + 4 * ql, gi0 = tile.x0 - kH + rr0;
     // cells of the quad inside the region's columns; rows of the warp inside
     // its rows, and those this lane stores
     const int nq = gj >= tile.ys ? max(0, min(4, tile.ye - gj)) : 0;
     const uint32_t region = rows_in<RW>(rr0, tile.xs - tile.x0 + kH, tile.xe - tile.x0 + kH);
-    const uint32_t stored = lane >= 1 && lane <= 30 && nq > 0 ? region & rows_in<RW>(rr0, kH, B::kRows - kH) : 0u;
+    const uint32_t stored = (B::kWhole || (ql >= 1 && ql <= B::kLanes - 2)) && nq > 0
+                                ? region & rows_in<RW>(rr0, kH, B::kRows - kH)
+                                : 0u;
     const Coefs ks = coefs_in(meta, nq > 0);
     Coefs kc[MODE == kModeFields ? 4 : 1];
     if constexpr (MODE == kModeFields) {
@@ -332,8 +360,8 @@ __global__ void __launch_bounds__(32 * W, CTAS)
     };
     const int ox = __float_as_int(meta[12]), oy = __float_as_int(meta[13]);
     const bool src = has_src && tile.x0 - kH < ox + a.bx && tile.x0 - kH + B::kRows > ox &&
-                     tile.y0 - kH < oy + a.by && tile.y0 - kH + kBox > oy;
-    const bool ragged = ((tile.ye - tile.ys) & 3) != 0 && tile.y0 - kH + kBox > tile.ye;
+                     tile.y0 - B::kHY < oy + a.by && tile.y0 - B::kHY + kCols > oy;
+    const bool ragged = ((tile.ye - tile.ys) & 3) != 0 && tile.y0 - B::kHY + kCols > tile.ye;
     const int2 recs = a.rec_tile != nullptr ? a.rec_tile[walk.t] : make_int2(0, 0);
     int T = a.T;
     if (INST) T = min(T, a.inst.box[2 * tile.inst + 1].z - a.i);
@@ -343,8 +371,8 @@ __global__ void __launch_bounds__(32 * W, CTAS)
       for (int r = 0; r < RW; ++r)
         if ((stored >> r) & 1u) {
           float* o = a.out[0] + off + (ptrdiff_t)r * a.pitch;
-          *reinterpret_cast<float4*>(o) = *reinterpret_cast<const float4*>(lev0 + o0 + r * kBox);
-          *reinterpret_cast<float4*>(o + Np) = *reinterpret_cast<const float4*>(lev0 + B::kPlane + o0 + r * kBox);
+          *reinterpret_cast<float4*>(o) = *reinterpret_cast<const float4*>(lev0 + o0 + r * kCols);
+          *reinterpret_cast<float4*>(o + Np) = *reinterpret_cast<const float4*>(lev0 + B::kPlane + o0 + r * kCols);
         }
     }
     for (int t = 1; t <= T; ++t) {
@@ -359,8 +387,8 @@ __global__ void __launch_bounds__(32 * W, CTAS)
         constexpr bool PLAIN = decltype(plain)::value;
         [[maybe_unused]] float wn[4], wv[4];
         if constexpr (MODE == kModeDField) weights(0, wn);
-        Row t0 = load_row(c0 - kBox), t1 = load_row(c0 + B::kPlane - kBox);
-        Row m0 = load_row(c0), m1 = load_row(c0 + B::kPlane);
+        Row t0 = load_row<B>(c0 - kCols, ql), t1 = load_row<B>(c0 + B::kPlane - kCols, ql);
+        Row m0 = load_row<B>(c0, ql), m1 = load_row<B>(c0 + B::kPlane, ql);
 #pragma unroll
         for (int r = 0; r < RW; ++r) {
           if constexpr (MODE == kModeDField) {
@@ -368,10 +396,10 @@ __global__ void __launch_bounds__(32 * W, CTAS)
             for (int q = 0; q < 4; ++q) wv[q] = wn[q];
             if (r + 1 < RW) weights(r + 1, wn);
           }
-          const Row b0 = load_row(c0 + (r + 1) * kBox), b1 = load_row(c0 + B::kPlane + (r + 1) * kBox);
+          const Row b0 = load_row<B>(c0 + (r + 1) * kCols, ql), b1 = load_row<B>(c0 + B::kPlane + (r + 1) * kCols, ql);
           if (PLAIN || ((region >> r) & 1u)) {  // (rows outside the region stay zero)
-            const float4 pv0 = *reinterpret_cast<const float4*>(p0 + r * kBox);
-            const float4 pv1 = *reinterpret_cast<const float4*>(p0 + B::kPlane + r * kBox);
+            const float4 pv0 = *reinterpret_cast<const float4*>(p0 + r * kCols);
+            const float4 pv1 = *reinterpret_cast<const float4*>(p0 + B::kPlane + r * kCols);
             const float q0[4] = {pv0.x, pv0.y, pv0.z, pv0.w}, q1[4] = {pv1.x, pv1.y, pv1.z, pv1.w};
             float v0[4], v1[4];
 #pragma unroll
@@ -408,8 +436,8 @@ __global__ void __launch_bounds__(32 * W, CTAS)
               mask_q(v1, nq);
             }
             const float4 n0 = make_float4(v0[0], v0[1], v0[2], v0[3]), n1 = make_float4(v1[0], v1[1], v1[2], v1[3]);
-            *reinterpret_cast<float4*>(p0 + r * kBox) = n0;
-            *reinterpret_cast<float4*>(p0 + B::kPlane + r * kBox) = n1;
+            *reinterpret_cast<float4*>(p0 + r * kCols) = n0;
+            *reinterpret_cast<float4*>(p0 + B::kPlane + r * kCols) = n1;
             if ((st >> r) & 1u) {
               *reinterpret_cast<float4*>(out0) = n0;
               *reinterpret_cast<float4*>(out1) = n1;
@@ -435,8 +463,8 @@ __global__ void __launch_bounds__(32 * W, CTAS)
         }
       };
       // (warps none of whose rows a later step reads have nothing to do)
-      if (region != 0 && rows_in<RW>(rr0, t, B::kRows - t) != 0) {
-        if (region == (1u << RW) - 1u && !src && !ragged && !dense) rows(BoolC<true>{});
+      if (any_share<B>(region != 0 && rows_in<RW>(rr0, t, B::kRows - t) != 0)) {
+        if (every_share<B>(region == (1u << RW) - 1u) && !src && !ragged && !dense) rows(BoolC<true>{});
         else rows(BoolC<false>{});
       }
       __syncthreads();  // u^{i+t} is complete; its receivers are read beside the next step
@@ -445,8 +473,8 @@ __global__ void __launch_bounds__(32 * W, CTAS)
         const size_t o = ((size_t)tile.inst * a.nt_out + frame) * a.nrec;
         for (int e = tid; e < recs.y; e += NT) {
           const int2 v = a.rec_ent[recs.x + e];
-          const int rr = v.x / kBox, cc = v.x % kBox;
-          if (rr < kH || rr >= B::kRows - kH || cc < kH || cc >= kBox - kH) continue;  // another tile's
+          const int rr = v.x / kCols, cc = v.x % kCols;
+          if (rr < kH || rr >= B::kRows - kH || cc < B::kHY || cc >= kCols - B::kHY) continue;  // another tile's
           a.rec_x[o + v.y] = lv[v.x];
           a.rec_y[o + v.y] = lv[B::kPlane + v.x];
         }
@@ -535,20 +563,19 @@ __device__ __forceinline__ void image(float (&acc)[6], float ux, float uy, const
 // form sum_cells u . (dA/dC_k lam) (the second differences with zero ghosts
 // are symmetric), which needs u^m only at the cell itself, read from global
 // memory one row ahead.
-template <int W, int RW, bool INST, int ORDER, int CTAS>
-__global__ void __launch_bounds__(32 * W, CTAS)
+template <class B, bool INST, int ORDER, int CTAS>
+__global__ void __launch_bounds__(B::kThreads, CTAS)
     blk_adj_kernel(const BlkAdj a, const __grid_constant__ CUtensorMap cur_map,
                    const __grid_constant__ CUtensorMap prev_map, int tiles_x, int tiles_y, int ntiles, int* err) {
   extern __shared__ float sm_raw[];
   float* sm = aligned128(sm_raw);
-  using B = BlkTile<W, RW>;
-  constexpr int NT = B::kThreads;
+  constexpr int NT = B::kThreads, RW = B::kRW, kCols = B::kCols;
   float* lev0 = sm + kBox;
   float* lev1 = lev0 + B::kLevel;
   float* meta = sm + B::kFloats;
   uint64_t* bar = reinterpret_cast<uint64_t*>(meta + B::kMeta);
   __shared__ PipeGuard guard;
-  __shared__ float2 red[W][6];
+  __shared__ float2 red[B::kW][6];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int nx = a.nx, ny = a.ny;
   const size_t N = (size_t)nx * ny, Np = (size_t)nx * a.pitch;
@@ -567,7 +594,7 @@ __global__ void __launch_bounds__(32 * W, CTAS)
   const int t_end = per_shot ? (int)((long long)(b + 1) * ntiles / nb) : ntiles;
   // (zeros: what rows without a neighbour read stays finite)
   if (tid < kBox) sm[tid] = sm[B::kFloats - kBox + tid] = 0.f;
-  BWalk<INST, B::kUse> walk;
+  BWalk<INST, B::kUse, B::kUseY> walk;
   walk.init(per_shot ? (int)((long long)b * ntiles / nb) : b, per_shot ? 1 : nb, tiles_x, tiles_y, nx, ny);
   __syncthreads();
   grid_dep_wait();  // the states of the previous launch are complete from here on
@@ -578,12 +605,13 @@ __global__ void __launch_bounds__(32 * W, CTAS)
   // are split over launches), FP64 across warps and launches.
   float hi[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, lo[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   auto flush = [&](int shot) {  // CTA-uniform
-    flush_sums<W>(hi, lo, red, a.partials + (per_shot ? (size_t)shot * kTiledRowsPerShot + b : (size_t)b) * 8);
+    flush_sums<B::kW>(hi, lo, red, a.partials + (per_shot ? (size_t)shot * kTiledRowsPerShot + b : (size_t)b) * 8);
   };
   int acc_shot = -1;
 
-  const int rr0 = w * RW;  // first row of the warp in the tile
-  const int o0 = rr0 * kBox + 4 * lane;
+  const int ql = lane % B::kLanes;                           // the lane's quad of its rows
+  const int rr0 = (w * B::kShares + lane / B::kLanes) * RW;  // the first of them in the tile
+  const int o0 = rr0 * kCols + 4 * ql;
   for (int k = 0; walk.t < t_end; ++k, walk.next()) {
     const BTile tile = walk.tile(a.inst);
     if (per_shot && tile.inst != acc_shot) {
@@ -594,16 +622,18 @@ __global__ void __launch_bounds__(32 * W, CTAS)
     // imaging pairs are m <= steps - 1
     const int steps = INST ? min(a.inst.box[2 * tile.inst + 1].z, a.nt) : a.nt;
     if (w == 0 && lane < 8) meta[lane] = (&(a.coef + (size_t)tile.inst * a.coef_stride)->k11)[lane];
-    load_tile<W, RW, INST>(lev0, lev1, &cur_map, &prev_map, a.cur != nullptr, a.prev != nullptr,
-                           a.cur != nullptr && steps >= a.m_hi + 1, a.prev != nullptr && steps >= a.m_hi + 2, tile, k,
-                           bar, &guard, err);
+    load_tile<B, INST>(lev0, lev1, &cur_map, &prev_map, a.cur != nullptr, a.prev != nullptr,
+                       a.cur != nullptr && steps >= a.m_hi + 1, a.prev != nullptr && steps >= a.m_hi + 2, tile, k, bar,
+                       &guard, err);
     __syncthreads();
-    const int gj = tile.y0 - kH + 4 * lane, gi0 = tile.x0 - kH + rr0;
+    const int gj = tile.y0 - B::kHY + 4 * ql, gi0 = tile.x0 - kH + rr0;
     const int nq = gj >= tile.ys ? max(0, min(4, tile.ye - gj)) : 0;
     const uint32_t region = rows_in<RW>(rr0, tile.xs - tile.x0 + kH, tile.xe - tile.x0 + kH);
-    const uint32_t stored = lane >= 1 && lane <= 30 && nq > 0 ? region & rows_in<RW>(rr0, kH, B::kRows - kH) : 0u;
+    const uint32_t stored = (B::kWhole || (ql >= 1 && ql <= B::kLanes - 2)) && nq > 0
+                                ? region & rows_in<RW>(rr0, kH, B::kRows - kH)
+                                : 0u;
     const Coefs ks = coefs_in(meta, nq > 0);
-    const bool ragged = ((tile.ye - tile.ys) & 3) != 0 && tile.y0 - kH + kBox > tile.ye;
+    const bool ragged = ((tile.ye - tile.ys) & 3) != 0 && tile.y0 - B::kHY + kCols > tile.ye;
     const int2 recs = a.rec_tile != nullptr ? a.rec_tile[walk.t] : make_int2(0, 0);
     const ptrdiff_t off = (ptrdiff_t)tile.plane * 2 * (ptrdiff_t)Np + (ptrdiff_t)gi0 * a.pitch + gj;
     for (int t = max(1, a.m_hi - steps + 1); t <= a.T; ++t) {
@@ -648,17 +678,17 @@ __global__ void __launch_bounds__(32 * W, CTAS)
         };
         float4 ux4, uy4, nx4, ny4;
         load_u(0, nx4, ny4);
-        Row t0 = load_row(c0 - kBox), t1 = load_row(c0 + B::kPlane - kBox);
-        Row m0 = load_row(c0), m1 = load_row(c0 + B::kPlane);
+        Row t0 = load_row<B>(c0 - kCols, ql), t1 = load_row<B>(c0 + B::kPlane - kCols, ql);
+        Row m0 = load_row<B>(c0, ql), m1 = load_row<B>(c0 + B::kPlane, ql);
 #pragma unroll
         for (int r = 0; r < RW; ++r) {
           ux4 = nx4;
           uy4 = ny4;
           if (r + 1 < RW) load_u(r + 1, nx4, ny4);
-          const Row b0 = load_row(c0 + (r + 1) * kBox), b1 = load_row(c0 + B::kPlane + (r + 1) * kBox);
+          const Row b0 = load_row<B>(c0 + (r + 1) * kCols, ql), b1 = load_row<B>(c0 + B::kPlane + (r + 1) * kCols, ql);
           if (PLAIN || ((region >> r) & 1u)) {  // (rows outside the region stay zero)
-            const float4 pv0 = *reinterpret_cast<const float4*>(p0 + r * kBox);
-            const float4 pv1 = *reinterpret_cast<const float4*>(p0 + B::kPlane + r * kBox);
+            const float4 pv0 = *reinterpret_cast<const float4*>(p0 + r * kCols);
+            const float4 pv1 = *reinterpret_cast<const float4*>(p0 + B::kPlane + r * kCols);
             const float q0[4] = {pv0.x, pv0.y, pv0.z, pv0.w}, q1[4] = {pv1.x, pv1.y, pv1.z, pv1.w};
             const float ux[4] = {ux4.x, ux4.y, ux4.z, ux4.w}, uy[4] = {uy4.x, uy4.y, uy4.z, uy4.w};
             float v0[4], v1[4];
@@ -685,8 +715,8 @@ __global__ void __launch_bounds__(32 * W, CTAS)
               mask_q(v1, nq);
             }
             const float4 n0 = make_float4(v0[0], v0[1], v0[2], v0[3]), n1 = make_float4(v1[0], v1[1], v1[2], v1[3]);
-            *reinterpret_cast<float4*>(p0 + r * kBox) = n0;
-            *reinterpret_cast<float4*>(p0 + B::kPlane + r * kBox) = n1;
+            *reinterpret_cast<float4*>(p0 + r * kCols) = n0;
+            *reinterpret_cast<float4*>(p0 + B::kPlane + r * kCols) = n1;
             if ((st >> r) & 1u) {
               *reinterpret_cast<float4*>(out0) = n0;
               *reinterpret_cast<float4*>(out1) = n1;
@@ -697,8 +727,8 @@ __global__ void __launch_bounds__(32 * W, CTAS)
           t0 = m0; t1 = m1; m0 = b0; m1 = b1;
         }
       };
-      if (region != 0 && rows_in<RW>(rr0, t, B::kRows - t) != 0) {
-        if (region == (1u << RW) - 1u && !ragged && !dense) rows(BoolC<true>{});
+      if (any_share<B>(region != 0 && rows_in<RW>(rr0, t, B::kRows - t) != 0)) {
+        if (every_share<B>(region == (1u << RW) - 1u) && !ragged && !dense) rows(BoolC<true>{});
         else rows(BoolC<false>{});
         fold_sums(hi, lo, acc);
       }
@@ -707,10 +737,10 @@ __global__ void __launch_bounds__(32 * W, CTAS)
         add_residuals(gs);
         if (out != nullptr) {
           for (int e = tid; e < recs.y; e += NT) {
-            const int c = a.rec_ent[recs.x + e].x, rr = c / kBox, cc = c % kBox;
-            if (rr < kH || rr >= B::kRows - kH || cc < kH || cc >= kBox - kH) continue;  // another tile's
+            const int c = a.rec_ent[recs.x + e].x, rr = c / kCols, cc = c % kCols;
+            if (rr < kH || rr >= B::kRows - kH || cc < B::kHY || cc >= kCols - B::kHY) continue;  // another tile's
             float* o = out + (ptrdiff_t)tile.plane * 2 * (ptrdiff_t)Np + (ptrdiff_t)(tile.x0 - kH + rr) * a.pitch +
-                       (tile.y0 - kH + cc);
+                       (tile.y0 - B::kHY + cc);
             o[0] = lp[c];
             o[Np] = lp[B::kPlane + c];
           }
@@ -1204,8 +1234,8 @@ __global__ void __launch_bounds__(32 * W, CTAS)
   for (int k = 0; walk.t < ntiles; ++k, walk.next()) {
     const BTile tile = walk.tile(a.inst);
     const int2 recs = a.rec_tile != nullptr ? a.rec_tile[walk.t] : make_int2(0, 0);
-    load_tile<W, RW, false>(lev0, lev1, &cur_map, &prev_map, a.cur != nullptr, a.prev != nullptr, a.cur != nullptr,
-                            a.prev != nullptr, tile, k, bar, &guard, err);
+    load_tile<B, false>(lev0, lev1, &cur_map, &prev_map, a.cur != nullptr, a.prev != nullptr, a.cur != nullptr,
+                        a.prev != nullptr, tile, k, bar, &guard, err);
     __syncthreads();
     const int gj = tile.y0 - kH + 4 * lane, gi0 = tile.x0 - kH + rr0;
     const int nq = gj >= 0 ? max(0, min(4, ny - gj)) : 0;
@@ -1597,7 +1627,8 @@ __global__ void inst_table_kernel(const InstDesc d, int4* __restrict__ tiles, in
 // grid is in no tile: the counting kernel writes its nt_out frames (zeros).
 struct RecPlace {  // the tiles (at most 2 x 2) around a cell
   int x0, x1, y0, y1, base, tiles_y, oi, oj;
-  __device__ __forceinline__ bool find(int idx, int s, int nx, int ny, int H, int tiles_x, int ty, const int4* box) {
+  __device__ __forceinline__ bool find(int idx, int s, int nx, int ny, const BlkShape& g, int tiles_x, int ty,
+                                       const int4* box) {
     if (idx < 0 || (int64_t)idx >= (int64_t)nx * ny) return false;  // out of range: ignored
     int gi = idx / ny, gj = idx - gi * ny;
     if (box != nullptr) {
@@ -1607,23 +1638,23 @@ struct RecPlace {  // the tiles (at most 2 x 2) around a cell
       gj -= r.y;
       base = m.x;
       tiles_y = m.y;
-      tiles_x = (r.z - r.x + H - 1) / H;
+      tiles_x = (r.z - r.x + g.rows - 1) / g.rows;
     } else {
       base = s * tiles_x * ty;
       tiles_y = ty;
     }
     oi = gi + kH;
-    oj = gj + kH;
-    x1 = min(oi / H, tiles_x - 1);
-    x0 = max((oi - (H + 2 * kH) + H) / H, 0);  // first tile whose last row reaches the cell
-    y1 = min(oj / kBlkCols, tiles_y - 1);
-    y0 = max((oj - kBox + kBlkCols) / kBlkCols, 0);
+    oj = gj + g.hy;
+    x1 = min(oi / g.rows, tiles_x - 1);
+    x0 = max((oi - 2 * kH) / g.rows, 0);  // first tile whose last row reaches the cell
+    y1 = min(oj / g.cols, tiles_y - 1);
+    y0 = max((oj - 2 * g.hy) / g.cols, 0);
     return true;
   }
 };
 
 template <bool FILL>
-__global__ void rec_tiles_kernel(const int32_t* __restrict__ rec_idx, int S, int nrec, int nx, int ny, int H,
+__global__ void rec_tiles_kernel(const int32_t* __restrict__ rec_idx, int S, int nrec, int nx, int ny, const BlkShape g,
                                  int tiles_x, int tiles_y, const int4* __restrict__ box, int* __restrict__ count,
                                  int2* __restrict__ tile, int2* __restrict__ ent, float* __restrict__ tr_x,
                                  float* __restrict__ tr_y, int nt_out) {
@@ -1631,7 +1662,7 @@ __global__ void rec_tiles_kernel(const int32_t* __restrict__ rec_idx, int S, int
   if (e >= S * nrec) return;
   const int s = e / nrec;
   RecPlace p;
-  if (!p.find(rec_idx[e], s, nx, ny, H, tiles_x, tiles_y, box)) {
+  if (!p.find(rec_idx[e], s, nx, ny, g, tiles_x, tiles_y, box)) {
     if (!FILL && tr_x != nullptr)
       for (int k = 0; k < nt_out; ++k) {
         const size_t o = ((size_t)s * nt_out + k) * nrec + (e - s * nrec);
@@ -1639,12 +1670,13 @@ __global__ void rec_tiles_kernel(const int32_t* __restrict__ rec_idx, int S, int
       }
     return;
   }
+  const int width = g.cols + 2 * g.hy;
   for (int xt = p.x0; xt <= p.x1; ++xt)
     for (int yt = p.y0; yt <= p.y1; ++yt) {
-      const int rr = p.oi - xt * H, cc = p.oj - yt * kBlkCols;
-      if (rr < 0 || rr >= H + 2 * kH || cc < 0 || cc >= kBox) continue;
+      const int rr = p.oi - xt * g.rows, cc = p.oj - yt * g.cols;
+      if (rr < 0 || rr >= g.rows + 2 * kH || cc < 0 || cc >= width) continue;
       const int t = p.base + xt * p.tiles_y + yt;
-      if (FILL) ent[tile[t].x + atomicAdd(&tile[t].y, 1)] = make_int2(rr * kBox + cc, e - s * nrec);
+      if (FILL) ent[tile[t].x + atomicAdd(&tile[t].y, 1)] = make_int2(rr * width + cc, e - s * nrec);
       else atomicAdd(&count[t], 1);
     }
 }
@@ -1686,55 +1718,53 @@ bool blk_map(CUtensorMap* m, const float* base, int nx, int ny, int pitch, int S
             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int MODE, int W, int RW, int CTAS, bool INST, int ORDER>
+template <int MODE, class B, int CTAS, bool INST, int ORDER>
 cudaError_t fwd_t(const BlkFwd& a, int* err, cudaStream_t st) {
-  using B = BlkTile<W, RW>;
   constexpr size_t smem = B::kBytes;
   static OncePerDevice once;
   const cudaError_t ready = once([] {
-    return cudaFuncSetAttribute(blk_fwd_kernel<MODE, W, RW, INST, ORDER, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return cudaFuncSetAttribute(blk_fwd_kernel<MODE, B, INST, ORDER, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
   if (ready != cudaSuccess) return ready;
   const int planes = INST ? 1 : a.S;
   const float* any = a.cur ? a.cur : a.out[a.T];  // (a level that is zero is not loaded)
   CUtensorMap cm, pm;
-  if (!blk_map(&cm, any, a.nx, a.ny, a.pitch, planes, kBox, B::kRows) ||
-      !blk_map(&pm, a.prev ? a.prev : any, a.nx, a.ny, a.pitch, planes, kBox, B::kRows))
+  if (!blk_map(&cm, any, a.nx, a.ny, a.pitch, planes, B::kCols, B::kRows) ||
+      !blk_map(&pm, a.prev ? a.prev : any, a.nx, a.ny, a.pitch, planes, B::kCols, B::kRows))
     return cudaErrorNotSupported;
-  const int tiles_x = (a.nx + B::kUse - 1) / B::kUse, tiles_y = (a.ny + kBlkCols - 1) / kBlkCols;
+  const int tiles_x = (a.nx + B::kUse - 1) / B::kUse, tiles_y = (a.ny + B::kUseY - 1) / B::kUseY;
   const int ntiles = INST ? a.inst.ntiles : a.S * tiles_x * tiles_y;
   const int grid = ntiles < CTAS * device_info().sms ? ntiles : CTAS * device_info().sms;
-  const double cells = INST ? (double)ntiles * B::kUse * kBlkCols : (double)a.S * a.nx * a.ny;
+  const double cells = INST ? (double)ntiles * B::kUse * B::kUseY : (double)a.S * a.nx * a.ny;
   int stores = 0;
   for (int t = 0; t <= a.T; ++t) stores += a.out[t] != nullptr ? 1 : 0;
   return tracked_launch(kProfForward, st, [&] {
-    launch_step_kernel(blk_fwd_kernel<MODE, W, RW, INST, ORDER, CTAS>, dim3(grid), dim3(32 * W), smem, st, a.chained != 0, a, cm, pm,
+    launch_step_kernel(blk_fwd_kernel<MODE, B, INST, ORDER, CTAS>, dim3(grid), dim3(B::kThreads), smem, st, a.chained != 0, a, cm, pm,
                        tiles_x, tiles_y, ntiles, err);
   }, cells * 8.0 * (stores + (a.cur ? 1 : 0) + (a.prev ? 1 : 0)));
 }
 
-template <int W, int RW, int CTAS, bool INST, int ORDER>
+template <class B, int CTAS, bool INST, int ORDER>
 cudaError_t adj_t(const BlkAdj& a, int* err, cudaStream_t st) {
-  using B = BlkTile<W, RW>;
   constexpr size_t smem = B::kBytes;
   static OncePerDevice once;
   const cudaError_t ready = once([] {
-    return cudaFuncSetAttribute(blk_adj_kernel<W, RW, INST, ORDER, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return cudaFuncSetAttribute(blk_adj_kernel<B, INST, ORDER, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
   if (ready != cudaSuccess) return ready;
   const int planes = INST ? 1 : a.S;
   const float* any = a.cur ? a.cur : a.out_last;  // (a level that is zero is not loaded)
   CUtensorMap cm, pm;
-  if (!blk_map(&cm, any, a.nx, a.ny, a.pitch, planes, kBox, B::kRows) ||
-      !blk_map(&pm, a.prev ? a.prev : any, a.nx, a.ny, a.pitch, planes, kBox, B::kRows))
+  if (!blk_map(&cm, any, a.nx, a.ny, a.pitch, planes, B::kCols, B::kRows) ||
+      !blk_map(&pm, a.prev ? a.prev : any, a.nx, a.ny, a.pitch, planes, B::kCols, B::kRows))
     return cudaErrorNotSupported;
-  const int tiles_x = (a.nx + B::kUse - 1) / B::kUse, tiles_y = (a.ny + kBlkCols - 1) / kBlkCols;
+  const int tiles_x = (a.nx + B::kUse - 1) / B::kUse, tiles_y = (a.ny + B::kUseY - 1) / B::kUseY;
   const int ntiles = INST ? a.inst.ntiles : a.S * tiles_x * tiles_y;
   const int all = CTAS * device_info().sms, slots = all < kTiledRowsPerShot ? all : kTiledRowsPerShot;  // a partial row each
   const int grid = ntiles < slots ? ntiles : slots;
-  const double cells = INST ? (double)ntiles * B::kUse * kBlkCols : (double)a.S * a.nx * a.ny;
+  const double cells = INST ? (double)ntiles * B::kUse * B::kUseY : (double)a.S * a.nx * a.ny;
   return tracked_launch(kProfAdjoint, st, [&] {
-    launch_step_kernel(blk_adj_kernel<W, RW, INST, ORDER, CTAS>, dim3(grid), dim3(32 * W), smem, st, a.chained != 0, a, cm, pm,
+    launch_step_kernel(blk_adj_kernel<B, INST, ORDER, CTAS>, dim3(grid), dim3(B::kThreads), smem, st, a.chained != 0, a, cm, pm,
                        tiles_x, tiles_y, ntiles, err);
   }, cells * 8.0 * (a.T + (a.T > 1 ? 2 : 1) + (a.cur ? 1 : 0) + (a.prev ? 1 : 0)));
 }
@@ -1841,14 +1871,28 @@ cudaError_t adj_f(const BlkAdj& a, const std::conditional_t<RUN, AdjRun, NoRun>&
 // of 32 rows stored, and kBlkFlat: sixteen warps of one row, 8 of 16 stored,
 // whose tiles take a half and a quarter as long, for grids that would leave
 // SMs idle.
-int blk_tile_rows(int geo) {
-  const int rows[] = {8 * 6, 16 * 2, 16, 8 * 5, 8 * 4};
-  return rows[geo] - 2 * kH;
+// kBlkRow128 and kBlkRow64: grids of at most 128 or 64 columns, whose rows a
+// tile holds whole: the tall tile without halo columns, and with two rows
+// side by side in a warp (96 rows, 88 stored).  With 120-column tiles most
+// lanes would be idle there, or a second tile hold a few columns: us per
+// forward and adjoint step, one-step tiles / 120-column tiles / these: 64 x
+// 4000x40 194 / 243 / 131, 64 x 4000x64 217 / 247 / 139, 30 x 3000x124
+// 160 / 183 / 113.
+BlkShape blk_shape(int geo) {
+  switch (geo) {
+    case kBlkShort: return {16 * 2 - 2 * kH, kBlkCols, kH};
+    case kBlkFlat: return {16 - 2 * kH, kBlkCols, kH};
+    case kBlkTall5: return {8 * 5 - 2 * kH, kBlkCols, kH};
+    case kBlkTall4: return {8 * 4 - 2 * kH, kBlkCols, kH};
+    case kBlkRow128: return {8 * 6 - 2 * kH, 128, 0};
+    case kBlkRow64: return {8 * 6 * 2 - 2 * kH, 64, 0};
+    default: return {8 * 6 - 2 * kH, kBlkCols, kH};
+  }
 }
 
 size_t blk_tiles(int geo, int nx, int ny) {
-  const int h = blk_tile_rows(geo);
-  return (size_t)((nx + h - 1) / h) * ((ny + kBlkCols - 1) / kBlkCols);
+  const BlkShape g = blk_shape(geo);
+  return (size_t)((nx + g.rows - 1) / g.rows) * ((ny + g.cols - 1) / g.cols);
 }
 
 // The geometry whose waves of tiles take the least time: us per wave on 152
@@ -1857,15 +1901,16 @@ size_t blk_tiles(int geo, int nx, int ny) {
 // sizes alone, as the workspace layout depends on it.
 double blk_cost(int geo, int nx, int ny, int S) {
   const double sms = 152.0, tiles = S * (double)blk_tiles(geo, nx, ny);
-  if (geo == kBlkTall) return tiles <= sms ? 21.0 : 20.0 * std::ceil(tiles / (2.0 * sms));
+  if (blk_shape(geo).hy == 0 && ny > blk_shape(geo).cols) return HUGE_VAL;  // not the whole row
+  if (geo == kBlkTall || geo == kBlkRow128 || geo == kBlkRow64) return tiles <= sms ? 21.0 : 20.0 * std::ceil(tiles / (2.0 * sms));
   if (geo == kBlkTall5 || geo == kBlkTall4) return (geo == kBlkTall5 ? 17.3 : 14.6) * std::ceil(tiles / (2.0 * sms));
   return (geo == kBlkShort ? 9.4 : 5.0) * std::ceil(tiles / sms);
 }
 
 int blk_geometry(int mode, int nx, int ny, int S) {
   int best = kBlkTall;
-  // (the five- and four-row tiles: scalar constants)
-  for (int geo : {kBlkShort, kBlkFlat, kBlkTall5, kBlkTall4})
+  // (the five- and four-row tiles, and those of whole rows: scalar constants)
+  for (int geo : {kBlkShort, kBlkFlat, kBlkTall5, kBlkTall4, kBlkRow128, kBlkRow64})
     if ((mode == kModeScalar || geo < kBlkTall5) && blk_cost(geo, nx, ny, S) < blk_cost(best, nx, ny, S)) best = geo;
   return best;
 }
@@ -1884,7 +1929,7 @@ size_t blk_rec_bytes(size_t ntiles, int S, int nrec) {
 cudaError_t launch_rec_tiles(int geo, const int32_t* rec_idx, int S, int nrec, int nx, int ny, const int4* box,
                              size_t ntiles, void* ws, const int2** tile, const int2** ent, float* tr_x, float* tr_y,
                              int nt_out, cudaStream_t st) {
-  const int H = blk_tile_rows(geo);
+  const BlkShape g = blk_shape(geo);
   int* count = static_cast<int*>(ws);
   int2* tl = reinterpret_cast<int2*>(static_cast<char*>(ws) + (ntiles + 2) / 2 * 8);
   int2* en = tl + ntiles;
@@ -1892,17 +1937,17 @@ cudaError_t launch_rec_tiles(int geo, const int32_t* rec_idx, int S, int nrec, i
   *ent = en;
   cudaError_t e = cudaMemsetAsync(count, 0, (ntiles + 1) * sizeof(int), st);
   if (e != cudaSuccess) return e;
-  const int n = S * nrec, tx = (nx + H - 1) / H, ty = (ny + kBlkCols - 1) / kBlkCols;
+  const int n = S * nrec, tx = (nx + g.rows - 1) / g.rows, ty = (ny + g.cols - 1) / g.cols;
   const int nt = (int)ntiles;
   e = tracked_launch(kProfOther, st, [&] {
-    rec_tiles_kernel<false><<<(n + 255) / 256, 256, 0, st>>>(rec_idx, S, nrec, nx, ny, H, tx, ty, box, count, tl, en, tr_x,
+    rec_tiles_kernel<false><<<(n + 255) / 256, 256, 0, st>>>(rec_idx, S, nrec, nx, ny, g, tx, ty, box, count, tl, en, tr_x,
                                                              tr_y, nt_out);
   });
   if (e != cudaSuccess) return e;
   e = tracked_launch(kProfOther, st, [&] { rec_base_kernel<<<(nt + 255) / 256, 256, 0, st>>>(count, nt, tl); });
   if (e != cudaSuccess) return e;
   return tracked_launch(kProfOther, st, [&] {
-    rec_tiles_kernel<true><<<(n + 255) / 256, 256, 0, st>>>(rec_idx, S, nrec, nx, ny, H, tx, ty, box, count, tl, en, tr_x,
+    rec_tiles_kernel<true><<<(n + 255) / 256, 256, 0, st>>>(rec_idx, S, nrec, nx, ny, g, tx, ty, box, count, tl, en, tr_x,
                                                             tr_y, nt_out);
   });
 }
@@ -1910,28 +1955,32 @@ cudaError_t launch_rec_tiles(int geo, const int32_t* rec_idx, int S, int nrec, i
 namespace {
 template <int MODE, int ORDER>
 cudaError_t fwd_geo(const BlkFwd& a, int* err, cudaStream_t st) {
-  if (a.geo == kBlkFlat) return fwd_t<MODE, 16, 1, 1, false, ORDER>(a, err, st);
-  if (a.geo == kBlkShort) return fwd_t<MODE, 16, 2, 1, false, ORDER>(a, err, st);
+  if (a.geo == kBlkFlat) return fwd_t<MODE, BlkTile<16, 1>, 1, false, ORDER>(a, err, st);
+  if (a.geo == kBlkShort) return fwd_t<MODE, BlkTile<16, 2>, 1, false, ORDER>(a, err, st);
   if constexpr (MODE == kModeScalar) {
-    if (a.geo == kBlkTall5) return fwd_t<MODE, 8, 5, 2, false, ORDER>(a, err, st);
-    if (a.geo == kBlkTall4) return fwd_t<MODE, 8, 4, 2, false, ORDER>(a, err, st);
+    if (a.geo == kBlkTall5) return fwd_t<MODE, BlkTile<8, 5>, 2, false, ORDER>(a, err, st);
+    if (a.geo == kBlkTall4) return fwd_t<MODE, BlkTile<8, 4>, 2, false, ORDER>(a, err, st);
+    if (a.geo == kBlkRow128) return fwd_t<MODE, BlkTile<8, 6, 32, true>, 2, false, ORDER>(a, err, st);
+    if (a.geo == kBlkRow64) return fwd_t<MODE, BlkTile<8, 6, 16, true>, 2, false, ORDER>(a, err, st);
   }
-  return fwd_t<MODE, 8, 6, 2, false, ORDER>(a, err, st);
+  return fwd_t<MODE, BlkTile<8, 6>, 2, false, ORDER>(a, err, st);
 }
 
 template <int ORDER>
 cudaError_t adj_geo(const BlkAdj& a, int* err, cudaStream_t st) {
-  if (a.geo == kBlkFlat) return adj_t<16, 1, 1, false, ORDER>(a, err, st);
-  if (a.geo == kBlkShort) return adj_t<16, 2, 1, false, ORDER>(a, err, st);
-  if (a.geo == kBlkTall5) return adj_t<8, 5, 2, false, ORDER>(a, err, st);
-  if (a.geo == kBlkTall4) return adj_t<8, 4, 2, false, ORDER>(a, err, st);
-  return adj_t<8, 6, 2, false, ORDER>(a, err, st);
+  if (a.geo == kBlkFlat) return adj_t<BlkTile<16, 1>, 1, false, ORDER>(a, err, st);
+  if (a.geo == kBlkShort) return adj_t<BlkTile<16, 2>, 1, false, ORDER>(a, err, st);
+  if (a.geo == kBlkTall5) return adj_t<BlkTile<8, 5>, 2, false, ORDER>(a, err, st);
+  if (a.geo == kBlkTall4) return adj_t<BlkTile<8, 4>, 2, false, ORDER>(a, err, st);
+  if (a.geo == kBlkRow128) return adj_t<BlkTile<8, 6, 32, true>, 2, false, ORDER>(a, err, st);
+  if (a.geo == kBlkRow64) return adj_t<BlkTile<8, 6, 16, true>, 2, false, ORDER>(a, err, st);
+  return adj_t<BlkTile<8, 6>, 2, false, ORDER>(a, err, st);
 }
 }  // namespace
 
 cudaError_t launch_blk_fwd(int mode, const BlkFwd& a, int* err, cudaStream_t st) {
-  if (a.inst.tiles != nullptr) return fwd_t<kModeScalar, 8, 6, 2, true, kOrderTiled>(a, err, st);
-  if (mode == kModeFields) return fwd_t<kModeFields, 16, 1, 1, false, kOrderFields>(a, err, st);
+  if (a.inst.tiles != nullptr) return fwd_t<kModeScalar, BlkTile<8, 6>, 2, true, kOrderTiled>(a, err, st);
+  if (mode == kModeFields) return fwd_t<kModeFields, BlkTile<16, 1>, 1, false, kOrderFields>(a, err, st);
   if (mode == kModeDField) return fwd_geo<kModeDField, kOrderPlain>(a, err, st);
   return a.plain_order ? fwd_geo<kModeScalar, kOrderPlain>(a, err, st) : fwd_geo<kModeScalar, kOrderTiled>(a, err, st);
 }
@@ -1943,7 +1992,7 @@ cudaError_t launch_blk_adj(int mode, const BlkAdj& a, int* err, cudaStream_t st)
     if (a.geo == kBlkShort) return adj_d_t<16, 2, 1>(a, err, st);
     return adj_d_t<8, 6, 2>(a, err, st);
   }
-  if (a.inst.tiles != nullptr) return adj_t<8, 6, 2, true, kOrderTiled>(a, err, st);
+  if (a.inst.tiles != nullptr) return adj_t<BlkTile<8, 6>, 2, true, kOrderTiled>(a, err, st);
   return a.plain_order ? adj_geo<kOrderPlain>(a, err, st) : adj_geo<kOrderTiled>(a, err, st);
 }
 

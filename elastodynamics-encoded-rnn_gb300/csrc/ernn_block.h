@@ -110,12 +110,16 @@ bool blk_run_fits(int mode, int geo, int nx, int ny, int S);
 cudaError_t launch_blk_fwd_run(int mode, const BlkFwd& a, const FwdRun& r, int* err, cudaStream_t st);
 cudaError_t launch_blk_adj_run(int mode, const BlkAdj& a, const AdjRun& r, int* err, cudaStream_t st);
 
-// Tile geometry of a grid problem (instances: kBlkTall), rows it stores,
-// tiles of an nx x ny grid.
-constexpr int kBlkTall = 0, kBlkShort = 1, kBlkFlat = 2, kBlkTall5 = 3, kBlkTall4 = 4;
+// Tile geometry of a grid problem (instances: kBlkTall), tiles of an nx x ny
+// grid.
+constexpr int kBlkTall = 0, kBlkShort = 1, kBlkFlat = 2, kBlkTall5 = 3, kBlkTall4 = 4, kBlkRow128 = 5, kBlkRow64 = 6;
+struct BlkShape {
+  int rows, cols;  // that a tile stores
+  int hy;          // halo columns on either side; 0: the tile holds whole rows
+};
+BlkShape blk_shape(int geo);
 int blk_geometry(int mode, int nx, int ny, int S);
 double blk_cost(int geo, int nx, int ny, int S);  // us of a launch of four steps (scalar constants)
-int blk_tile_rows(int geo);
 size_t blk_tiles(int geo, int nx, int ny);
 // Partial-sum rows reserved per shot with per-shot constants (an adjoint grid
 // never exceeds this many CTAs).

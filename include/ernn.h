@@ -58,15 +58,16 @@ enum {
 enum {
   ERNN_PATH_AUTO = 0,     /* cluster-resident when the problem fits, else time-blocked
                              tiles (scalar constants and constant planes with rows of
-                             any length from 40 cells; degradation maps of moderate
-                             size), else tiled or per-step launches */
+                             any length from 40 cells, large scalar problems with
+                             shorter ones; degradation maps of moderate size), else
+                             tiled or per-step launches */
   ERNN_PATH_STEP = 1,     /* one fused kernel launch per time step (any size, any mode) */
   ERNN_PATH_RESIDENT = 2, /* one thread-block cluster per shot holds the state in
                              distributed shared memory for all steps (scalar constants,
                              ny % 4 == 0, state small enough); ERNN_ERR_UNSUPPORTED otherwise */
   ERNN_PATH_TILED = 3     /* persistent CTAs that stream tiles through TMA loads, ny %
-                             4 == 0: scalar constants in time-blocked tiles of 120
-                             columns, up to four steps per launch; a degradation map
+                             4 == 0: scalar constants in time-blocked tiles, up to
+                             four steps per launch; a degradation map
                              in 64 x 32 tiles, one launch per step.
                              ERNN_ERR_UNSUPPORTED otherwise */
 };

@@ -72,3 +72,53 @@ def test_problems_that_no_cluster_takes_run_on_tiles(kw):
     bx, by, bg, _ = run(case, wx, wy, E.PATH_STEP, 12)
     assert np.array_equal(ax, bx) and np.array_equal(ay, by)
     assert rel(ag, bg) <= 1e-5, rel(ag, bg)
+
+
+# Grids whose rows one tile holds: 88 rows of at most 64 columns, 40 of at most 128.
+ROWS64 = [(88, 41, 153), (89, 63, 120), (97, 61, 120), (177, 43, 95), (180, 57, 62)]
+ROWS128 = [(40, 121, 153), (41, 127, 153), (180, 125, 31), (121, 123, 40)]
+
+
+@pytest.mark.parametrize("nx,ny,S", ROWS64 + ROWS128)
+@pytest.mark.parametrize("record,nrec", [(O.RECORD_FIELDS, 0), (O.RECORD_RECEIVERS, 200)])
+@pytest.mark.parametrize("nt,ckpt_k", [(22, None), (27, 6)])
+def test_narrow_odd_grids(nx, ny, S, record, nrec, nt, ckpt_k):
+    """The plain kernels' rounding order: bit for bit."""
+    case = random_case(nx=nx, ny=ny, nt=nt, S=S, record=record, nrec=nrec, stride=1 + nt % 2, src_comp=nx % 2)
+    wx, wy = weights(case)
+    ax, ay, ag, used = run(case, wx, wy, E.PATH_AUTO, ckpt_k)
+    assert used == E.PATH_TILED
+    bx, by, bg, _ = run(case, wx, wy, E.PATH_STEP, ckpt_k)
+    assert np.array_equal(ax, bx) and np.array_equal(ay, by)
+    assert rel(ag, bg) <= 1e-5, rel(ag, bg)
+
+
+@pytest.mark.parametrize("nx,ny,S,path", [
+    (5000, 32, 4, E.PATH_AUTO), (4000, 36, 5, E.PATH_AUTO),      # rows below 40 cells, 608 tiles of 64 x 32
+    (20000, 4, 1, E.PATH_TILED), (4500, 64, 5, E.PATH_AUTO),
+    (300, 8, 40, E.PATH_TILED), (177, 60, 95, E.PATH_TILED), (89, 64, 120, E.PATH_TILED),
+    (180, 124, 31, E.PATH_TILED), (41, 128, 160, E.PATH_TILED),
+])
+@pytest.mark.parametrize("per_shot", [False, True])
+def test_narrow_grids_of_whole_quads(nx, ny, S, path, per_shot):
+    """The tiled rounding order: equal to the plain kernels' to FP32 rounding
+    over 30 steps (2^-24 a step and term, as between the two orders before)."""
+    case = random_case(nx=nx, ny=ny, nt=30, S=S, record=O.RECORD_RECEIVERS, nrec=150, stride=2)
+    case.rec_idx[:, 0] = case.src_origin[:, 0].clip(0, nx - 1) * ny + case.src_origin[:, 1].clip(0, ny - 1)
+    wx, wy = weights(case)
+    got = []
+    for pth in (path, E.PATH_STEP):
+        geom = to_geometry(case, 7, pth)
+        C = torch.tensor(case.C, dtype=torch.float32, device=DEV)
+        rho = torch.tensor(case.rho, dtype=torch.float32, device=DEV)
+        if per_shot:
+            C = C[None] * (1 + 0.05 * torch.arange(S, device=DEV)[:, None] / S)
+            rho = rho.reshape(1).repeat(S)
+        C.requires_grad_(True)
+        ux, uy = E.propagate(C, rho, geom)
+        assert E.load_library().ernn_last_path() == (E.PATH_TILED if pth == path else E.PATH_STEP)
+        ((ux.double() * torch.as_tensor(wx, device=DEV)).sum() + (uy.double() * torch.as_tensor(wy, device=DEV)).sum()).backward()
+        got.append((ux.detach().cpu().numpy(), uy.detach().cpu().numpy(), C.grad.double().cpu().numpy()))
+    for a, b in zip(*got):
+        assert np.any(b != 0) and rel(a, b) <= 1e-5, rel(a, b)
+
