@@ -1897,13 +1897,18 @@ size_t blk_tiles(int geo, int nx, int ny) {
 
 // The geometry whose waves of tiles take the least time: us per wave on 152
 // SMs, mean of a forward and an adjoint launch of four steps (measured at
-// one shot of 301^2 and 512^2, three of 501 x 389, eight of 640 x 720).  From
-// sizes alone, as the workspace layout depends on it.
+// one shot of 301^2 and 512^2, three of 501 x 389, eight of 640 x 720; low
+// grids: 100 to 500 shots of 1 to 16 rows and 4000 to 8000 columns).  From sizes
+// alone, as the workspace layout depends on it.
 double blk_cost(int geo, int nx, int ny, int S) {
   const double sms = 152.0, tiles = S * (double)blk_tiles(geo, nx, ny);
   if (blk_shape(geo).hy == 0 && ny > blk_shape(geo).cols) return HUGE_VAL;  // not the whole row
   if (geo == kBlkTall || geo == kBlkRow128 || geo == kBlkRow64) return tiles <= sms ? 21.0 : 20.0 * std::ceil(tiles / (2.0 * sms));
-  if (geo == kBlkTall5 || geo == kBlkTall4) return (geo == kBlkTall5 ? 17.3 : 14.6) * std::ceil(tiles / (2.0 * sms));
+  if (geo == kBlkTall5) return 17.3 * std::ceil(tiles / (2.0 * sms));
+  // (a grid lower than the tile leaves warps idle and takes as much less time:
+  // 4.3 us a wave at one row, 7.1 at 8, 8.4 at 16)
+  if (geo == kBlkTall4)
+    return 14.6 * (nx < 24 ? 0.4 + 0.6 * nx / 24.0 : 1.0) * std::ceil(tiles / (2.0 * sms));
   return (geo == kBlkShort ? 9.4 : 5.0) * std::ceil(tiles / sms);
 }
 

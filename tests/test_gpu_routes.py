@@ -74,15 +74,17 @@ def test_problems_that_no_cluster_takes_run_on_tiles(kw):
     assert rel(ag, bg) <= 1e-5, rel(ag, bg)
 
 
-# Grids whose rows one tile holds: 88 rows of at most 64 columns, 40 of at most 128.
+# Grids whose rows one tile holds: 88 rows of at most 64 columns, 40 of at most
+# 128; grids lower than a tile's 24 rows.
 ROWS64 = [(88, 41, 153), (89, 63, 120), (97, 61, 120), (177, 43, 95), (180, 57, 62)]
 ROWS128 = [(40, 121, 153), (41, 127, 153), (180, 125, 31), (121, 123, 40)]
+LOW = [(1, 1601, 22), (4, 1501, 25), (8, 241, 70), (23, 365, 50)]
 
 
-@pytest.mark.parametrize("nx,ny,S", ROWS64 + ROWS128)
+@pytest.mark.parametrize("nx,ny,S", ROWS64 + ROWS128 + LOW)
 @pytest.mark.parametrize("record,nrec", [(O.RECORD_FIELDS, 0), (O.RECORD_RECEIVERS, 200)])
 @pytest.mark.parametrize("nt,ckpt_k", [(22, None), (27, 6)])
-def test_narrow_odd_grids(nx, ny, S, record, nrec, nt, ckpt_k):
+def test_narrow_and_low_odd_grids(nx, ny, S, record, nrec, nt, ckpt_k):
     """The plain kernels' rounding order: bit for bit."""
     case = random_case(nx=nx, ny=ny, nt=nt, S=S, record=record, nrec=nrec, stride=1 + nt % 2, src_comp=nx % 2)
     wx, wy = weights(case)
@@ -121,4 +123,3 @@ def test_narrow_grids_of_whole_quads(nx, ny, S, path, per_shot):
         got.append((ux.detach().cpu().numpy(), uy.detach().cpu().numpy(), C.grad.double().cpu().numpy()))
     for a, b in zip(*got):
         assert np.any(b != 0) and rel(a, b) <= 1e-5, rel(a, b)
-
