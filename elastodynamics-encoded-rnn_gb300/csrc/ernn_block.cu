@@ -227,10 +227,10 @@ __device__ __forceinline__ void mask_q(float (&v)[4], int n) {
 __device__ __forceinline__ Row load_row(const float* p) {  // a row of the tile at the lane's quad
   return row_of(q4(*reinterpret_cast<const float4*>(p)));
 }
-// The same for a tile of the kernels below; ql: the lane's quad in its row.
+// A row of a tile of whole rows, whose ends have zeros beside them; ql: the
+// lane's quad in its row.
 template <class B>
-__device__ __forceinline__ Row load_row(const float* p, int ql) {
-  if constexpr (!B::kWhole) return load_row(p);
+__device__ __forceinline__ Row whole_row(const float* p, int ql) {
   const float4 v = *reinterpret_cast<const float4*>(p);
   const float l = __shfl_up_sync(kFull, v.w, 1, B::kLanes), r = __shfl_down_sync(kFull, v.x, 1, B::kLanes);
   return Row{{ql > 0 ? l : 0.f, v.x, v.y, v.z, v.w, ql < B::kLanes - 1 ? r : 0.f}};
@@ -385,10 +385,14 @@ __global__ void __launch_bounds__(B::kThreads, CTAS)
       const uint32_t st = a.out[t] != nullptr ? stored : 0u;
       auto rows = [&](auto plain) {
         constexpr bool PLAIN = decltype(plain)::value;
+        auto row_at = [&](const float* p) {  // a row of the tile at the lane's quad
+          if constexpr (B::kWhole) return whole_row<B>(p, ql);
+          else return row_of(q4(*reinterpret_cast<const float4*>(p)));
+        };
         [[maybe_unused]] float wn[4], wv[4];
         if constexpr (MODE == kModeDField) weights(0, wn);
-        Row t0 = load_row<B>(c0 - kCols, ql), t1 = load_row<B>(c0 + B::kPlane - kCols, ql);
-        Row m0 = load_row<B>(c0, ql), m1 = load_row<B>(c0 + B::kPlane, ql);
+        Row t0 = row_at(c0 - kCols), t1 = row_at(c0 + B::kPlane - kCols);
+        Row m0 = row_at(c0), m1 = row_at(c0 + B::kPlane);
 #pragma unroll
         for (int r = 0; r < RW; ++r) {
           if constexpr (MODE == kModeDField) {
@@ -396,7 +400,7 @@ __global__ void __launch_bounds__(B::kThreads, CTAS)
             for (int q = 0; q < 4; ++q) wv[q] = wn[q];
             if (r + 1 < RW) weights(r + 1, wn);
           }
-          const Row b0 = load_row<B>(c0 + (r + 1) * kCols, ql), b1 = load_row<B>(c0 + B::kPlane + (r + 1) * kCols, ql);
+          const Row b0 = row_at(c0 + (r + 1) * kCols), b1 = row_at(c0 + B::kPlane + (r + 1) * kCols);
           if (PLAIN || ((region >> r) & 1u)) {  // (rows outside the region stay zero)
             const float4 pv0 = *reinterpret_cast<const float4*>(p0 + r * kCols);
             const float4 pv1 = *reinterpret_cast<const float4*>(p0 + B::kPlane + r * kCols);
@@ -667,6 +671,10 @@ __global__ void __launch_bounds__(B::kThreads, CTAS)
       float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       auto rows = [&](auto plain) {
         constexpr bool PLAIN = decltype(plain)::value;
+        auto row_at = [&](const float* p) {  // a row of the tile at the lane's quad
+          if constexpr (B::kWhole) return whole_row<B>(p, ql);
+          else return row_of(q4(*reinterpret_cast<const float4*>(p)));
+        };
         auto load_u = [&](int r, float4& x, float4& y) {
           x = y = make_float4(0.f, 0.f, 0.f, 0.f);
           if ((im >> r) & 1u) {
@@ -678,14 +686,14 @@ __global__ void __launch_bounds__(B::kThreads, CTAS)
         };
         float4 ux4, uy4, nx4, ny4;
         load_u(0, nx4, ny4);
-        Row t0 = load_row<B>(c0 - kCols, ql), t1 = load_row<B>(c0 + B::kPlane - kCols, ql);
-        Row m0 = load_row<B>(c0, ql), m1 = load_row<B>(c0 + B::kPlane, ql);
+        Row t0 = row_at(c0 - kCols), t1 = row_at(c0 + B::kPlane - kCols);
+        Row m0 = row_at(c0), m1 = row_at(c0 + B::kPlane);
 #pragma unroll
         for (int r = 0; r < RW; ++r) {
           ux4 = nx4;
           uy4 = ny4;
           if (r + 1 < RW) load_u(r + 1, nx4, ny4);
-          const Row b0 = load_row<B>(c0 + (r + 1) * kCols, ql), b1 = load_row<B>(c0 + B::kPlane + (r + 1) * kCols, ql);
+          const Row b0 = row_at(c0 + (r + 1) * kCols), b1 = row_at(c0 + B::kPlane + (r + 1) * kCols);
           if (PLAIN || ((region >> r) & 1u)) {  // (rows outside the region stay zero)
             const float4 pv0 = *reinterpret_cast<const float4*>(p0 + r * kCols);
             const float4 pv1 = *reinterpret_cast<const float4*>(p0 + B::kPlane + r * kCols);
