@@ -102,7 +102,7 @@ bool block_rule(const ErnnProblem& p) {
 
 // Upper bound of the tile-table entries of any placement of S instances on
 // an nx x ny canvas (each instance's tiling has at most one partial tile row
-// and column).
+// and column; tiles of whole rows are fewer).
 inline size_t inst_table_bound(int nx, int ny, int S) {
   const BlkShape g = blk_shape(kBlkTall);
   return ((size_t)(nx + g.rows - 1) / g.rows + S) * ((size_t)(ny + g.cols - 1) / g.cols + S);
@@ -401,6 +401,7 @@ int resident_adjoint(const ErnnProblem& p, const Plan& pl, ResCommon& rc, const 
 // by decreasing step count; upto[g] = tiles of the first g of that order.
 struct InstPlan {
   InstDesc d;
+  int geo;  // tiles: kBlkTall, or kBlkRow64 where every instance fits its columns
   int upto[kMaxInstances + 1];
   // tiles of forward (or recompute) step i: instances with nt > i
   int fwd_tiles(int i) const {
@@ -439,8 +440,18 @@ int plan_instances(const ErnnProblem& p, const ErnnInstances* in, InstPlan* ip) 
   for (int k = 0; k < S; ++k) order[k] = k;
   std::stable_sort(order, order + S, [&](int u, int v) { return in->nt[u] > in->nt[v]; });
   ip->d.count = S;
-  ip->d.tile_rows = blk_shape(kBlkTall).rows;
-  ip->d.tile_cols = blk_shape(kBlkTall).cols;
+  // Tiles of whole rows where they save a wave of tiles (256 instances of 300 x
+  // 32, 60 steps: 5.66 -> 3.52 ms).
+  size_t tall = 0, rows = 0;
+  bool narrow = true;
+  for (int k = 0; k < S; ++k) {
+    tall += blk_tiles(kBlkTall, in->nx[k], in->ny[k]);
+    rows += blk_tiles(kBlkRow64, in->nx[k], in->ny[k]);
+    narrow = narrow && in->ny[k] <= blk_shape(kBlkRow64).cols;
+  }
+  ip->geo = narrow && (rows + 303) / 304 < (tall + 303) / 304 ? kBlkRow64 : kBlkTall;
+  ip->d.tile_rows = blk_shape(ip->geo).rows;
+  ip->d.tile_cols = blk_shape(ip->geo).cols;
   ip->upto[0] = 0;
   for (int g = 0; g < S; ++g) {
     const int k = order[g];
@@ -451,7 +462,7 @@ int plan_instances(const ErnnProblem& p, const ErnnInstances* in, InstPlan* ip) 
     ip->d.ny[g] = in->ny[k];
     ip->d.nt[g] = in->nt[k];
     ip->d.base[g] = ip->upto[g];
-    ip->upto[g + 1] = ip->upto[g] + (int)blk_tiles(kBlkTall, in->nx[k], in->ny[k]);
+    ip->upto[g + 1] = ip->upto[g] + (int)blk_tiles(ip->geo, in->nx[k], in->ny[k]);
   }
   return ERNN_OK;
 }
@@ -468,10 +479,11 @@ inline float* free_state(float* const pool[4], const float* x, const float* y, c
   return nullptr;
 }
 
-BlkFwd base_blk_fwd(const ErnnProblem& p, const Plan& pl, const ErnnInputs& in, const Coef* coef, const InstTiles& it) {
+BlkFwd base_blk_fwd(const ErnnProblem& p, const Plan& pl, const ErnnInputs& in, const InstPlan* ip, const Coef* coef,
+                    const InstTiles& it) {
   BlkFwd a;
   std::memset(&a, 0, sizeof(a));
-  a.geo = pl.geo;
+  a.geo = ip != nullptr ? ip->geo : pl.geo;
   a.plain_order = plain_size(p) ? 1 : 0;
   a.nx = p.nx; a.ny = p.ny; a.pitch = pl.pitch; a.S = p.nshots; a.nt = p.nt;
   a.nt_out = pl.nt_out; a.record = p.record; a.nrec = p.nrec;
@@ -587,9 +599,9 @@ struct PassRunner {
 // leaves behind.
 int block_forward(const ErnnProblem& p, const Plan& pl, const ErnnInputs& in, const InstPlan* ip, InstTiles itab,
                   Coef* coef, float* out_ux, float* out_uy, void* tape, int with_tape, cudaStream_t st) {
-  BlkFwd a = base_blk_fwd(p, pl, in, coef, itab);
+  BlkFwd a = base_blk_fwd(p, pl, in, ip, coef, itab);
   if (p.record == kRecordReceivers)
-    ERNN_CUDA(launch_rec_tiles(pl.geo, in.rec_idx, p.nshots, p.nrec, p.nx, p.ny, itab.box, block_tiles(p, pl, ip),
+    ERNN_CUDA(launch_rec_tiles(a.geo, in.rec_idx, p.nshots, p.nrec, p.nx, p.ny, itab.box, block_tiles(p, pl, ip),
                                at(tape, pl.t_rec), &a.rec_tile, &a.rec_ent, out_ux, out_uy, pl.nt_out, st));
   a.rec_x = out_ux;
   a.rec_y = out_uy;
@@ -638,17 +650,17 @@ int block_forward(const ErnnProblem& p, const Plan& pl, const ErnnInputs& in, co
 int block_adjoint(const ErnnProblem& p, const Plan& pl, const ErnnInputs& in, const InstPlan* ip, InstTiles itab,
                   Coef* coef, const float* g_ux, const float* g_uy, void* tape, void* scratch, double* partials,
                   cudaStream_t st) {
-  BlkFwd a = base_blk_fwd(p, pl, in, coef, itab);
+  BlkFwd a = base_blk_fwd(p, pl, in, ip, coef, itab);
   BlkAdj b;
   std::memset(&b, 0, sizeof(b));
-  b.geo = pl.geo;
+  b.geo = a.geo;
   b.plain_order = a.plain_order;
   b.nx = p.nx; b.ny = p.ny; b.pitch = pl.pitch; b.S = p.nshots; b.nt = p.nt;
   b.u_stride = pl.state_bytes / sizeof(float);
   b.g_x = g_ux; b.g_y = g_uy;
   b.stride = p.stride; b.nt_out = pl.nt_out; b.record = p.record; b.nrec = p.nrec;
   if (p.record == kRecordReceivers)
-    ERNN_CUDA(launch_rec_tiles(pl.geo, in.rec_idx, p.nshots, p.nrec, p.nx, p.ny, itab.box, block_tiles(p, pl, ip),
+    ERNN_CUDA(launch_rec_tiles(a.geo, in.rec_idx, p.nshots, p.nrec, p.nx, p.ny, itab.box, block_tiles(p, pl, ip),
                                at(scratch, pl.s_rec), &b.rec_tile, &b.rec_ent, nullptr, nullptr, 0, st));
   b.coef = coef;
   b.coef_stride = a.coef_stride;

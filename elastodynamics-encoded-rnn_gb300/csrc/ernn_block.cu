@@ -1992,7 +1992,9 @@ cudaError_t adj_geo(const BlkAdj& a, int* err, cudaStream_t st) {
 }  // namespace
 
 cudaError_t launch_blk_fwd(int mode, const BlkFwd& a, int* err, cudaStream_t st) {
-  if (a.inst.tiles != nullptr) return fwd_t<kModeScalar, BlkTile<8, 6>, 2, true, kOrderTiled>(a, err, st);
+  if (a.inst.tiles != nullptr)
+    return a.geo == kBlkRow64 ? fwd_t<kModeScalar, BlkTile<8, 6, 16, true>, 2, true, kOrderTiled>(a, err, st)
+                              : fwd_t<kModeScalar, BlkTile<8, 6>, 2, true, kOrderTiled>(a, err, st);
   if (mode == kModeFields) return fwd_t<kModeFields, BlkTile<16, 1>, 1, false, kOrderFields>(a, err, st);
   if (mode == kModeDField) return fwd_geo<kModeDField, kOrderPlain>(a, err, st);
   return a.plain_order ? fwd_geo<kModeScalar, kOrderPlain>(a, err, st) : fwd_geo<kModeScalar, kOrderTiled>(a, err, st);
@@ -2005,7 +2007,9 @@ cudaError_t launch_blk_adj(int mode, const BlkAdj& a, int* err, cudaStream_t st)
     if (a.geo == kBlkShort) return adj_d_t<16, 2, 1>(a, err, st);
     return adj_d_t<8, 6, 2>(a, err, st);
   }
-  if (a.inst.tiles != nullptr) return adj_t<BlkTile<8, 6>, 2, true, kOrderTiled>(a, err, st);
+  if (a.inst.tiles != nullptr)
+    return a.geo == kBlkRow64 ? adj_t<BlkTile<8, 6, 16, true>, 2, true, kOrderTiled>(a, err, st)
+                              : adj_t<BlkTile<8, 6>, 2, true, kOrderTiled>(a, err, st);
   return a.plain_order ? adj_geo<kOrderPlain>(a, err, st) : adj_geo<kOrderTiled>(a, err, st);
 }
 

@@ -110,8 +110,8 @@ bool blk_run_fits(int mode, int geo, int nx, int ny, int S);
 cudaError_t launch_blk_fwd_run(int mode, const BlkFwd& a, const FwdRun& r, int* err, cudaStream_t st);
 cudaError_t launch_blk_adj_run(int mode, const BlkAdj& a, const AdjRun& r, int* err, cudaStream_t st);
 
-// Tile geometry of a grid problem (instances: kBlkTall), tiles of an nx x ny
-// grid.
+// Tile geometry of a grid problem (instances: kBlkTall or kBlkRow64), tiles of
+// an nx x ny grid.
 constexpr int kBlkTall = 0, kBlkShort = 1, kBlkFlat = 2, kBlkTall5 = 3, kBlkTall4 = 4, kBlkRow128 = 5, kBlkRow64 = 6;
 struct BlkShape {
   int rows, cols;  // that a tile stores

@@ -7,10 +7,11 @@ import pytest
 import torch
 
 import ernn_gb300 as E
-from cases import random_case, rel
+from cases import DT, H, RHO, random_case, rel
 from oracle import oracle as O
 from test_gpu_block import run
-from test_gpu_parity import DEV, to_geometry, weights
+from test_gpu_instances import _canvas, _instances, _run_canvas, _run_single, _weights
+from test_gpu_parity import DEV, GRAD_TOL, to_geometry, weights
 
 pytestmark = pytest.mark.gpu
 
@@ -123,3 +124,29 @@ def test_narrow_grids_of_whole_quads(nx, ny, S, path, per_shot):
         got.append((ux.detach().cpu().numpy(), uy.detach().cpu().numpy(), C.grad.double().cpu().numpy()))
     for a, b in zip(*got):
         assert np.any(b != 0) and rel(a, b) <= 1e-5, rel(a, b)
+
+
+@pytest.mark.parametrize("ckpt_k", [None, 6])
+def test_canvas_of_narrow_instances(ckpt_k):
+    """Instances whose rows one tile holds (two waves of 40-row tiles, one of
+    whole-row tiles): each one's traces as if run alone, bit for bit, its
+    gradient against the 64-bit oracle (alone it has other tiles, and with
+    them other FP32 partial sums)."""
+    rng = np.random.default_rng(2)
+    specs = [(int(rng.integers(180, 330)), 4 * int(rng.integers(2, 17)), int(rng.integers(9, 30))) for _ in range(70)]
+    specs[:4] = [(176, 64, 30), (177, 60, 29), (88, 8, 9), (8, 64, 17)]
+    insts = _instances(specs)
+    geom = _canvas(insts, ckpt_k)
+    wx, wy = _weights(insts, geom.nt)
+    cx, cy, cg = _run_canvas(insts, geom, wx, wy)
+    for k, d in enumerate(insts):
+        nt = d["nt"]
+        sx, sy, sg = _run_single(d, wx[k:k + 1, :nt], wy[k:k + 1, :nt], ckpt_k)
+        assert np.array_equal(cx[k, :nt], sx) and np.array_equal(cy[k, :nt], sy), k
+        assert not np.any(cx[k, nt:]) and not np.any(cy[k, nt:])
+        case = O.Case(d["nx"], d["ny"], nt, H, DT, RHO, d["C"], d["sig"][None].astype(np.float64),
+                      d["smap"][None].astype(np.float64), np.array([d["org"]], np.int32), record=O.RECORD_RECEIVERS,
+                      rec_idx=d["rec"][None])
+        gC, _ = O.adjoint(case, O.forward(case, "f64", keep_states=True)[2], wx[k:k + 1, :nt], wy[k:k + 1, :nt], "f64")
+        assert rel(cg[k], gC) <= GRAD_TOL and rel(sg, gC) <= GRAD_TOL, (k, rel(cg[k], gC), rel(sg, gC))
+
