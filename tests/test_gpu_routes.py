@@ -150,3 +150,20 @@ def test_canvas_of_narrow_instances(ckpt_k):
         gC, _ = O.adjoint(case, O.forward(case, "f64", keep_states=True)[2], wx[k:k + 1, :nt], wy[k:k + 1, :nt], "f64")
         assert rel(cg[k], gC) <= GRAD_TOL and rel(sg, gC) <= GRAD_TOL, (k, rel(cg[k], gC), rel(sg, gC))
 
+
+@pytest.mark.parametrize("nx,ny,S", [(61, 127, 1), (200, 243, 3)])  # passes of one launch; a launch per pass
+@pytest.mark.parametrize("nrec", [1, 40, 511, 513, 1100])
+def test_constant_planes_with_receivers_crowded_on_a_tile(nx, ny, S, nrec):
+    """Around the 512 threads of a tile's CTA, on both sides of tile edges
+    (rows 8 k, column 120), two receivers on one cell among them."""
+    case = random_case(nx=nx, ny=ny, nt=20, S=S, mode=O.MODE_FIELDS, record=O.RECORD_RECEIVERS, nrec=nrec)
+    cells = np.array([i * ny + j for j in range(60, 127) for i in range(5, 27)])
+    case.rec_idx[:] = np.random.default_rng(nrec).permutation(cells)[:nrec]
+    case.rec_idx[:, -1] = case.rec_idx[:, 0]
+    wx, wy = weights(case)
+    ax, ay, ag, used = run(case, wx, wy, E.PATH_AUTO, 6)
+    assert used == E.PATH_TILED
+    bx, by, bg, _ = run(case, wx, wy, E.PATH_STEP, 6)
+    assert np.array_equal(ax, bx) and np.array_equal(ay, by)
+    assert rel(ag, bg) <= 1e-5, rel(ag, bg)
+
