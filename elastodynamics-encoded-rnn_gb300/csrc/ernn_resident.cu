@@ -837,6 +837,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const ResCommo
       const int32_t idx = c.rec_idx[(size_t)shot * c.nrec + r];
       if (idx < 0 || (size_t)idx >= N) {  // out of range: no source in the adjoint, zeros in the traces
         if (is_fwd && f.tr_x && rank == 0)
+#pragma unroll 1
           for (int k = 0; k < c.nt_out; ++k) {
             const size_t o = ((size_t)shot * c.nt_out + k) * c.nrec + r;
             f.tr_x[o] = f.tr_y[o] = 0.f;
