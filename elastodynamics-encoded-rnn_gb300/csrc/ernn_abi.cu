@@ -61,6 +61,29 @@ inline bool cluster_fits(const ErnnProblem& p) {
   return resident_fits(p.mode, p.nx, p.ny, p.record == kRecordReceivers ? p.nrec : 0);
 }
 
+// Estimates of a forward and an adjoint step of the per-cell modes, us: here
+// by waves of tiles, in the plain kernels by the cells of their blocks (columns
+// to 32, rows to 8).  Fitted to 48 grids of each mode, 17 thousand to 1.8
+// million cells, 9 to 20000 rows; us there -> here on either side of the line:
+//   constant planes  1 x 3000x240 34.0 -> 18.5, 16 x 250^2 39.3 -> 37.0, 20 x
+//     130^2 19.1 -> 18.9; 300 x 50^2 41.6 -> 47.0, 120 x 64^2 22.1 -> 25.5
+//   degradation map  7 x 301^2 20.1 -> 14.8, 1 x 700x701 14.9 -> 14.1; 10 x
+//     200x201 14.3 -> 14.7, 8 x 500x121 16.1 -> 18.6, 7 x 563x51 10.2 -> 14.5
+struct StepUs {
+  double block, plain;
+};
+StepUs per_cell_step_us(const ErnnProblem& p) {
+  const bool fields = p.mode == kModeFields;
+  const int geo = fields ? kBlkFlat : blk_geometry(p.mode, p.nx, p.ny, p.nshots);
+  const double slots = geo == kBlkTall ? 304.0 : 152.0;
+  const double waves = std::ceil(p.nshots * (double)blk_tiles(geo, p.nx, p.ny) / slots);
+  const double M = 1e-6 * p.nshots * ((p.nx + 7) / 8 * 8.0) * ((p.ny + 31) / 32 * 32.0);
+  const bool small = step_rows(p.nx, p.ny, p.nshots) == 8;
+  if (fields) return {1.0 + 3.35 * waves, small ? 8.0 + 26.0 * M : 16.0 + 24.0 * M};
+  return {1.0 + (geo == kBlkTall ? 17.0 : geo == kBlkShort ? 6.8 : 4.1) * waves,
+          small ? 6.3 + 17.0 * M : 6.5 + 18.4 * M};
+}
+
 // Problems of the time-blocked tile kernels, from sizes alone (the workspace
 // queries, the forward and the adjoint agree).
 //  - Instances, and scalar constants on the tiled path: all of them.
@@ -79,25 +102,18 @@ inline bool cluster_fits(const ErnnProblem& p) {
 //    TMA-fed kernels of one step are faster (8 x 512^2: 29 against 33 us per
 //    forward and adjoint step): the map, u's rows and the running gradient
 //    are read at every step either way, here from L2 by the threads.
-//    Tiles that a narrow grid leaves half empty cost more than the plain
-//    kernels' step: a forward and an adjoint step take about 2 us + 0.7 of
-//    the cost of the launch here, 6 us + 20 us per million cells there
-//    (measured, us per iteration, plain -> here: 7 x 563x51 1516 -> 2022, 7 x
-//    595x72 2684 -> 2721, 8 x 98x560 3267 -> 2644, 1 x 563x51 1468 -> 1055).
-//  - Six constant planes: up to kBlockMaxFields cells, where launches set the
-//    time (301^2: 36.1 against 21.9 ms per 4001-step iteration).
+//  - Six constant planes: up to kBlockMaxFields cells.
+//    Both per-cell modes where a step takes less here than with the plain
+//    kernels (per_cell_step_us).
 bool block_rule(const ErnnProblem& p) {
   if (p.flags & ERNN_FLAG_INSTANCES) return true;
   if (p.path == ERNN_PATH_TILED) return p.mode == kModeScalar && p.ny % 4 == 0;
   if (p.path != ERNN_PATH_AUTO) return false;
   if (p.mode == kModeScalar) return (p.ny >= kBlockMinCols || !plain_size(p)) && !cluster_fits(p);
   if (p.ny < kBlockMinCols) return false;
-  if (p.mode == kModeFields) return (double)p.nshots * p.nx * p.ny <= kBlockMaxFields;
-  if (p.mode == kModeDField) {
-    const double cost = blk_cost(blk_geometry(p.mode, p.nx, p.ny, p.nshots), p.nx, p.ny, p.nshots);
-    return plain_size(p) && (cost <= 10.0 || cost <= 6.0 + 31e-6 * p.nshots * p.nx * p.ny);
-  }
-  return false;
+  if (p.mode == kModeFields ? (double)p.nshots * p.nx * p.ny > kBlockMaxFields : !plain_size(p)) return false;
+  const StepUs us = per_cell_step_us(p);
+  return us.block <= us.plain;
 }
 
 // Upper bound of the tile-table entries of any placement of S instances on

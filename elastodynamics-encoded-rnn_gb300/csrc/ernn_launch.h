@@ -65,6 +65,7 @@ struct AdjStep {
   int chained;  // previous launch on the stream is a step kernel of the same loop
 };
 
+int step_rows(int nx, int ny, int S);  // rows of a block of the plain kernels: 32, or 8 on small grids
 dim3 step_grid(int nx, int ny, int S);
 
 // ncoef coefficient blocks from C[6 ncoef] and rho[ncoef].

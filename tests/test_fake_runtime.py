@@ -108,3 +108,20 @@ def test_work_areas_are_cleared_inside_the_buffers(lib, kw, sms):
             a = lib.fake_memset(i, ctypes.byref(n))
             inside = [lo <= a and a + n.value <= lo + size for lo, size in ((tape, nt), (scratch, ns))]
             assert any(inside) or a >= DATA, (hex(a), n.value)
+
+
+@pytest.mark.parametrize("mode,S,nx,ny,tiles", [
+    # grids measured on either side of the line between plain and time-blocked kernels
+    (2, 1, 301, 301, True), (2, 20, 130, 130, True), (2, 16, 250, 250, True), (2, 1, 3000, 240, True),
+    (2, 1, 4000, 42, True), (2, 40, 130, 130, True), (2, 100, 9, 1000, True), (2, 1, 1000, 1000, True),
+    (2, 300, 50, 50, False), (2, 120, 64, 64, False), (2, 1, 8000, 61, False), (2, 1, 20000, 48, False),
+    (1, 1, 301, 301, True), (1, 7, 301, 301, True), (1, 1, 700, 701, True), (1, 30, 130, 130, True),
+    (1, 40, 17, 1001, True), (1, 8, 98, 560, True), (1, 300, 40, 41, True), (1, 2, 512, 512, True),
+    (1, 8, 500, 121, False), (1, 1, 8000, 61, False), (1, 6, 2000, 123, False), (1, 300, 24, 121, False),
+    (1, 10, 200, 201, False), (1, 7, 563, 51, False),
+])
+def test_per_cell_modes_take_the_kernels_measured_faster(lib, mode, S, nx, ny, tiles):
+    setup(lib)
+    assert call(lib, problem(mode=mode, nshots=S, nx=nx, ny=ny)) == (0, 0)
+    assert lib.ernn_last_path() == (E.PATH_TILED if tiles else E.PATH_STEP)
+
