@@ -175,6 +175,22 @@ def peaks():
     return 6800.0, "fallback"
 
 
+def kernel_names(path, mode, steps_per_launch):
+    """Kernels of the forward and the adjoint time loop on a kernel path
+    (ernn_last_path) for "scalar" constants, a "damage" map or constant
+    "fields".  On the tiled path the adjoint's steps per launch tell one-step
+    tiles (1), time-blocked tiles (up to 4) and runs of them (more) apart."""
+    if path != 3:
+        return {2: {"forward": "resident_kernel", "adjoint": "resident_kernel"}}.get(
+            path, {"forward": "fwd_step_kernel", "adjoint": "adj_step_kernel"})
+    if mode == "damage" and steps_per_launch < 1.5:
+        return {"forward": "tma_fwd_kernel", "adjoint": "tma_adj_kernel"}
+    run = steps_per_launch > 4
+    return {"forward": "run_fwd_kernel" if run else "blk_fwd_kernel",
+            "adjoint": {"fields": "blk_adj_f_kernel", "damage": "blk_adj_d_kernel"}.get(
+                mode, "run_adj_kernel" if run else "blk_adj_kernel")}
+
+
 def profiled_traffic(kernel, workload):
     """DRAM bytes per launch of `kernel` from the committed ncu summary, or None."""
     path = os.path.join(ROOT, "profiles", f"{kernel}_{workload}.txt")
@@ -448,10 +464,8 @@ def run_ernn(args, dist):
     achieved = alg_bytes / (per_launch_ms * 1e-3) / 1e9
     peak, peak_kind = peaks()
     used = int(lib.ernn_last_path())
-    kernel_name = {E.PATH_RESIDENT: {"forward": "resident_kernel", "adjoint": "resident_kernel"},
-                   E.PATH_TILED: {"forward": "tma_fwd_kernel", "adjoint": "tma_adj_kernel"} if w.D_true is not None
-                   else {"forward": "blk_fwd_kernel", "adjoint": "blk_adj_kernel"}}.get(
-        used, {"forward": "fwd_step_kernel", "adjoint": "adj_step_kernel"})[cls]
+    mode = "fields" if w.extra.get("fields") else "damage" if w.D_true is not None else "scalar"
+    kernel_name = kernel_names(used, mode, w.nt / max(prof["adjoint"][1], 1))[cls]
     traffic = profiled_traffic(kernel_name, args.workload)
     state_mb = w.nshots * 2 * w.nx * w.ny * 4 / 2**20
     l2_note = ("working set (three state levels) is L2-resident at this size; bytes are algorithmic"

@@ -538,7 +538,8 @@ struct PassRunner {
 
   PassRunner(const ErnnProblem& p, const Plan& pl, const InstPlan* ip, int* flags_, int* err_, cudaStream_t st_)
       : mode(p.mode), err(err_), st(st_), flags(flags_) {
-    on = ip == nullptr && launch_overlap() && (p.mode != kModeScalar || plain_size(p)) &&
+    // (the setting alone: a profiled call makes the launches of an unprofiled one)
+    on = ip == nullptr && launch_overlap_setting() && (p.mode != kModeScalar || plain_size(p)) &&
          blk_run_fits(p.mode, pl.geo, p.nx, p.ny, p.nshots);
     f.n = r.n = 0;
   }

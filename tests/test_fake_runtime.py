@@ -125,3 +125,20 @@ def test_per_cell_modes_take_the_kernels_measured_faster(lib, mode, S, nx, ny, t
     assert call(lib, problem(mode=mode, nshots=S, nx=nx, ny=ny)) == (0, 0)
     assert lib.ernn_last_path() == (E.PATH_TILED if tiles else E.PATH_STEP)
 
+
+
+@pytest.mark.parametrize("kw,mode", [
+    (dict(nx=61, ny=43, nt=200), "scalar"), (dict(nx=300, ny=301, nshots=9, nt=20), "scalar"),
+    (dict(nx=61, ny=43, mode=2, nt=200), "fields"), (dict(nx=200, ny=243, nshots=4, mode=2), "fields"),
+    (dict(nx=61, ny=43, mode=1), "damage"), (dict(nx=1024, ny=1216, mode=1), "damage"),
+    (dict(nx=128, ny=128), "scalar"), (dict(nx=61, ny=33), "scalar"), (dict(nx=61, ny=33, mode=1), "damage"),
+])
+def test_bench_names_the_kernels_that_run(lib, kw, mode):
+    import bench
+    setup(lib)
+    p = problem(**{**kw, "ckpt_k": kw.get("nt", 20)})
+    assert call(lib, p) == (0, 0)
+    loop = [l[0] for l in launches(lib) if any(k in l[0] for k in ("blk_", "run_", "tma_", "step_kernel", "resident"))]
+    adjoint = [l for l in loop if "adj" in l]
+    names = bench.kernel_names(lib.ernn_last_path(), mode, p.nt / max(len(adjoint), 1))
+    assert any(names["forward"] in l for l in loop) and any(names["adjoint"] in l for l in loop), (names, set(loop))

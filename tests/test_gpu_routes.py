@@ -167,3 +167,26 @@ def test_constant_planes_with_receivers_crowded_on_a_tile(nx, ny, S, nrec):
     assert np.array_equal(ax, bx) and np.array_equal(ay, by)
     assert rel(ag, bg) <= 1e-5, rel(ag, bg)
 
+
+@pytest.mark.parametrize("mode", [O.MODE_SCALAR, O.MODE_FIELDS])
+def test_the_profiler_times_the_launches_of_an_unprofiled_call(mode):
+    """Passes that share a launch share it under the profiler too."""
+    case = random_case(nx=61, ny=243, nt=120, mode=mode, record=O.RECORD_RECEIVERS, nrec=12)
+    wx, wy = weights(case)
+    lib = E.load_library()
+
+    def launches():
+        n = lib.ernn_launch_count()
+        run(case, wx, wy, E.PATH_AUTO, None)
+        return lib.ernn_launch_count() - n
+    plain = launches()
+    E._lib.profile(True)
+    try:
+        profiled = launches()
+        torch.cuda.synchronize()
+        prof = E._lib.profile_read()
+    finally:
+        E._lib.profile(False)
+    assert profiled == plain
+    # 120 steps are 30 passes of four: two launches each way
+    assert prof["forward"][1] == 2 and prof["adjoint"][1] == 2
