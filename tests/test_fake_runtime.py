@@ -127,6 +127,41 @@ def test_per_cell_modes_take_the_kernels_measured_faster(lib, mode, S, nx, ny, t
 
 
 
+class Pass(ctypes.Structure):
+    """The first fields of BlkFwd and BlkAdj (out: of BlkAdj the last two levels)."""
+    _fields_ = [(n, ctypes.c_int32) for n in ("geo", "plain_order", "nx", "ny", "pitch", "S", "nt", "step", "T")] + [
+        ("cur", ctypes.c_uint64), ("prev", ctypes.c_uint64), ("out", ctypes.c_uint64 * 2)]
+
+
+@pytest.mark.parametrize("mode", [0, 2])
+@pytest.mark.parametrize("nt,ckpt_k", [(30, 30), (205, 205), (205, 103), (97, 9)])
+def test_refused_cooperative_launches_become_a_launch_per_pass(lib, mode, nt, ckpt_k):
+    """The passes of a refused run, in order, with the states they read and
+    write: those of a call that never tries runs."""
+    p = problem(nx=61, ny=243, mode=mode, nt=nt, ckpt_k=ckpt_k)
+
+    def passes(**kw):
+        setup(lib, **kw)
+        assert call(lib, p) == (0, 0)
+        out = []
+        for name, _, coop, _, arg in launches(lib):
+            assert not coop
+            if "blk_" in name:
+                a = Pass.from_buffer_copy(arg)
+                out.append((name, a.step, a.T, a.cur, a.prev, a.out[0], a.out[1]))
+        return out
+    refused = passes(refuse_cooperative=1)
+    lib.ernn_set_launch_overlap(0)
+    try:
+        apart = passes()
+    finally:
+        lib.ernn_set_launch_overlap(1)
+    assert refused == apart and len(apart) >= 2 * (nt // 4)
+    setup(lib)
+    assert call(lib, p) == (0, 0)
+    assert any(coop for _, _, coop, _, _ in launches(lib))  # (they are runs where the runtime takes them)
+
+
 @pytest.mark.parametrize("kw,mode", [
     (dict(nx=61, ny=43, nt=200), "scalar"), (dict(nx=300, ny=301, nshots=9, nt=20), "scalar"),
     (dict(nx=61, ny=43, mode=2, nt=200), "fields"), (dict(nx=200, ny=243, nshots=4, mode=2), "fields"),

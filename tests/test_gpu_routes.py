@@ -11,7 +11,7 @@ from cases import DT, H, RHO, random_case, rel
 from oracle import oracle as O
 from test_gpu_block import run
 from test_gpu_instances import _canvas, _instances, _run_canvas, _run_single, _weights
-from test_gpu_parity import DEV, GRAD_TOL, to_geometry, weights
+from test_gpu_parity import DEV, FWD_TOL, GRAD_TOL, run_oracle, to_geometry, weights
 
 pytestmark = pytest.mark.gpu
 
@@ -166,6 +166,36 @@ def test_constant_planes_with_receivers_crowded_on_a_tile(nx, ny, S, nrec):
     bx, by, bg, _ = run(case, wx, wy, E.PATH_STEP, 6)
     assert np.array_equal(ax, bx) and np.array_equal(ay, by)
     assert rel(ag, bg) <= 1e-5, rel(ag, bg)
+
+
+# Grids on the 40-row tiles, around multiples of 40 rows and 120 columns.
+@pytest.mark.parametrize("mode,nx,ny,S", [
+    (O.MODE_SCALAR, 80, 129, 51), (O.MODE_SCALAR, 161, 131, 26), (O.MODE_SCALAR, 79, 241, 34),
+    (O.MODE_DFIELD, 81, 361, 24), (O.MODE_DFIELD, 121, 243, 24), (O.MODE_DFIELD, 241, 361, 9),
+])
+@pytest.mark.parametrize("record,nrec", [(O.RECORD_FIELDS, 0), (O.RECORD_RECEIVERS, 150)])
+@pytest.mark.parametrize("nt,ckpt_k", [(17, None), (23, 6)])
+def test_forty_row_tiles(mode, nx, ny, S, record, nrec, nt, ckpt_k):
+    case = random_case(nx=nx, ny=ny, nt=nt, S=S, mode=mode, record=record, nrec=nrec, stride=1 + nt % 2, src_comp=nx % 2)
+    wx, wy = weights(case)
+    ax, ay, ag, used = run(case, wx, wy, E.PATH_AUTO, ckpt_k)
+    assert used == E.PATH_TILED
+    bx, by, bg, _ = run(case, wx, wy, E.PATH_STEP, ckpt_k)
+    assert np.array_equal(ax, bx) and np.array_equal(ay, by)
+    assert rel(ag, bg) <= 1e-5, rel(ag, bg)
+
+
+@pytest.mark.parametrize("mode", [O.MODE_DFIELD, O.MODE_FIELDS])
+@pytest.mark.parametrize("nx,ny", [(8, 120), (25, 121), (41, 243), (40, 119)])
+@pytest.mark.parametrize("record,nrec", [(O.RECORD_FIELDS, 0), (O.RECORD_RECEIVERS, 60)])
+def test_per_cell_modes_vs_fp64_oracle_at_tile_edges(mode, nx, ny, record, nrec):
+    case = random_case(nx=nx, ny=ny, nt=45, S=2, mode=mode, record=record, nrec=nrec)
+    wx, wy = weights(case)
+    ax, ay, ag, used = run(case, wx, wy, E.PATH_AUTO, 11)
+    assert used == E.PATH_TILED
+    ox, oy, og = run_oracle(case, wx, wy)
+    assert rel(ax, ox) <= FWD_TOL and rel(ay, oy) <= FWD_TOL
+    assert rel(ag, og) <= GRAD_TOL, rel(ag, og)
 
 
 @pytest.mark.parametrize("mode", [O.MODE_SCALAR, O.MODE_FIELDS])
