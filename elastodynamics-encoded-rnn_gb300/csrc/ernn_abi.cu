@@ -35,7 +35,7 @@ struct Plan {
   size_t t_coef, t_A, t_B, t_store, t_total_tape, t_total_notape;
   // adjoint scratch
   size_t s_coef, s_LA, s_LB, s_seg, s_lbuf, s_gacc, s_part, s_tflags, s_total;
-  // instances on a canvas: tile table (tape and scratch), a zero state (scratch)
+  // instances on a canvas: tile table (tape and scratch)
   bool inst;
   size_t inst_bytes, t_inst, s_inst;
   // time-blocked tile kernels: the problem is theirs (given aligned buffers),
@@ -520,8 +520,8 @@ size_t block_tiles(const ErnnProblem& p, const Plan& pl, const InstPlan* ip) {
 
 // Passes collected into runs (one cooperative launch each) where the tiles fit
 // the chip, one per SM; otherwise every pass is a launch.  Measured, a launch
-// per pass -> runs: 301^2 dense 4.64 -> 3.92 ms, 512^2 traces 5.27 -> 4.05,
-// 301^2 constant planes 21.9 -> 17.0.  (52-row tiles for grids of up to 1 M
+// per pass -> runs: 301^2 dense 4.69 -> 3.91 ms, 512^2 traces 5.23 -> 4.05,
+// 301^2 constant planes 18.3 -> 17.1.  (52-row tiles for grids of up to 1 M
 // cells, 12 warps of five rows: 3 x 501x389 8.27 -> 8.60 ms, left out.)
 struct PassRunner {
   int mode;

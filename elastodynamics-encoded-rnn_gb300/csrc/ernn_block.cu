@@ -496,6 +496,10 @@ __global__ void __launch_bounds__(B::kThreads, CTAS)
 // than a step of a small tile), and each exchange halves the values a lane
 // still carries: 4 + 2 + 1 additions leave one value in every group of four
 // lanes, two more sum it over the group.
+// (The per-step kernels add warps and steps in FP64.  The same sums over steps
+// and lanes in FP64 here gave the same gradients, in float32, on the five timed
+// scalar cases and eight drawn ones, and passes of 1.04 to 1.27 times the time.
+// The pair of 96 random terms was their exact sum in each of 400 trials.)
 template <int W>
 __device__ __forceinline__ void flush_sums(float (&hi)[6], float (&lo)[6], float2 (*red)[6], double* row) {
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -769,8 +773,9 @@ __global__ void __launch_bounds__(B::kThreads, CTAS)
 // four columns of them; rows beside another warp's go through shared memory
 // (one barrier per step), and between passes a CTA waits only for the tiles
 // around it, by a flag per tile that counts passes, and reloads its halo.
-// A neighbour is at most one pass ahead, and a pass never writes the states
-// that the pass before it has read.
+// A pass writes the two states, of four, that the pass before it has read; the
+// tiles around it that read them have counted that pass before it starts, so a
+// neighbour is at most one pass ahead.
 // Measured, us per pass of four steps, forward / adjoint: 301^2 (8-row tiles)
 // 6.0 / 7.5 against 7.5 / 11 with a launch each, 512^2 (24-row tiles) 7.0 /
 // 11.1 against 9.4 / 14.  Without waiting for neighbours, halo loads and
@@ -1636,7 +1641,8 @@ __global__ void __launch_bounds__(32 * W, 1)
 
 // ------------------------------------------------------- instance tiles
 // Block b writes the tiles of instance d.id[b] (entry base[b] + xt * tiles_y
-// + yt for the tile at rows x0 + 16 xt, columns y0 + 64 yt) and its box.
+// + yt for the tile at rows x0 + tile_rows xt, columns y0 + tile_cols yt) and
+// its box.
 __global__ void inst_table_kernel(const InstDesc d, int4* __restrict__ tiles, int4* __restrict__ box) {
   const int b = blockIdx.x;
   const int k = d.id[b];

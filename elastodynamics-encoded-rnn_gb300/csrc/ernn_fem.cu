@@ -387,7 +387,10 @@ FemStencil fem_stencil(const ErnnFemProblem& p) {
 // field per (levels / nodes across) (61^2, 120^2, 200^2, 301^2 nodes, 430 to
 // 2001 levels), and the two kernels' frames part by as much: up to this line
 // by 1.6e-5 at most in what was measured.  Longer runs on small grids keep the
-// element form, and with it their frames.
+// element form, and with it their frames, at three to five times the time
+// (100^2 nodes, 700 and 701 levels: 0.84 and 2.36 ms; 200^2, 1400 and 1401:
+// 1.67 and 8.35): the line is where the frames stay the same to 2e-5, not where
+// the kernels cross.
 constexpr int kFemCrossings = 7;
 inline bool fem_block_rule(const ErnnFemProblem& p) {
   return p.nt <= (int64_t)kFemCrossings * (p.nx < p.ny ? p.nx : p.ny);

@@ -84,8 +84,9 @@ enum {
    * a rectangular region of the canvas with its own constants (C nshots x 6,
    * rho nshots, as ERNN_FLAG_SHOT_CONSTANTS), source (src_signal nshots x nt,
    * src_map, src_origin in canvas cells), receivers (rec_idx: canvas cell
-   * indices; one outside its instance's region records zeros) and step count; nt is the largest step count.  SCALAR mode,
-   * RECORD_RECEIVERS, tiled kernels (ERNN_PATH_AUTO or _TILED). */
+   * indices; one outside its instance's region records zeros) and step count;
+   * nt is the largest step count.  SCALAR mode, RECORD_RECEIVERS, tiled kernels
+   * (ERNN_PATH_AUTO or _TILED). */
   ERNN_FLAG_INSTANCES = 2,
   /* Accepted and without effect: the tiled kernels choose their tiles from
    * the grid (it once chose 64 x 32 over 64 x 16 tiles). */
