@@ -3,7 +3,6 @@
 workspaces, and what happens when the runtime refuses.  Runs on the CPU; no
 kernel runs."""
 import ctypes
-import glob
 import os
 import shutil
 import subprocess
@@ -21,8 +20,9 @@ def lib(tmp_path_factory):
     gcc = shutil.which("gcc")
     include = "/usr/local/cuda/include"
     E.load_library()  # builds the objects where they are missing
-    objs = glob.glob(os.path.join(os.path.dirname(E._lib.library_path()), "*.o"))
-    if gcc is None or not os.path.exists(os.path.join(include, "cuda_runtime_api.h")) or not objs:
+    out_dir = os.path.dirname(E._lib.library_path())
+    objs = [os.path.join(out_dir, os.path.basename(f)[:-3] + ".o") for f in E._lib._build.sources()]
+    if gcc is None or not os.path.exists(os.path.join(include, "cuda_runtime_api.h")) or not all(map(os.path.exists, objs)):
         pytest.skip("gcc, the CUDA headers or the library's objects absent")
     out = str(tmp_path_factory.mktemp("fake") / "libernn_fake.so")
     subprocess.run([gcc, "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I", include,
