@@ -61,27 +61,41 @@ inline bool cluster_fits(const ErnnProblem& p) {
   return resident_fits(p.mode, p.nx, p.ny, p.record == kRecordReceivers ? p.nrec : 0);
 }
 
-// Estimates of a forward and an adjoint step of the per-cell modes, us: here
-// by waves of tiles, in the plain kernels by the cells of their blocks (columns
-// to 32, rows to 8).  Fitted to 48 grids of each mode, 17 thousand to 1.8
-// million cells, 9 to 20000 rows; us there -> here on either side of the line:
-//   constant planes  1 x 3000x240 34.0 -> 18.5, 16 x 250^2 39.3 -> 37.0, 20 x
-//     130^2 19.1 -> 18.9; 300 x 50^2 41.6 -> 47.0, 120 x 64^2 22.1 -> 25.5
-//   degradation map  7 x 301^2 20.1 -> 14.8, 1 x 700x701 14.9 -> 14.1; 10 x
+// Estimates of the time that the per-cell modes take a step, us: here by waves
+// of tiles, in the plain kernels by the cells of their blocks (columns to 32,
+// rows to 8).  Fitted to some 50 grids of each mode, 17 thousand to 1.8 million
+// cells, 9 to 20000 rows; us there -> here on either side of the line:
+//   constant planes, every state kept: 1 x 3000x240 34.0 -> 18.5, 16 x 250^2
+//     39.3 -> 37.0, 20 x 130^2 19.1 -> 18.9; 300 x 50^2 41.6 -> 47.0, 120 x 64^2
+//     22.1 -> 25.5; checkpoints (every 13 steps: the forward counts twice, and
+//     segments end launches early) 8 x 301^2 46.2 -> 32.4; 16 x 250^2 50.3 ->
+//     54.9; forward alone 8 x 301^2 9.6 -> 7.9; 16 x 250^2 10.6 -> 13.0
+//   degradation map: 7 x 301^2 20.1 -> 14.8, 1 x 700x701 14.9 -> 14.1; 10 x
 //     200x201 14.3 -> 14.7, 8 x 500x121 16.1 -> 18.6, 7 x 563x51 10.2 -> 14.5
-struct StepUs {
-  double block, plain;
-};
-StepUs per_cell_step_us(const ErnnProblem& p) {
-  const bool fields = p.mode == kModeFields;
-  const int geo = fields ? kBlkFlat : blk_geometry(p.mode, p.nx, p.ny, p.nshots);
-  const double slots = geo == kBlkTall ? 304.0 : 152.0;
-  const double waves = std::ceil(p.nshots * (double)blk_tiles(geo, p.nx, p.ny) / slots);
-  const double M = 1e-6 * p.nshots * ((p.nx + 7) / 8 * 8.0) * ((p.ny + 31) / 32 * 32.0);
-  const bool small = step_rows(p.nx, p.ny, p.nshots) == 8;
-  if (fields) return {1.0 + 3.35 * waves, small ? 8.0 + 26.0 * M : 16.0 + 24.0 * M};
-  return {1.0 + (geo == kBlkTall ? 17.0 : geo == kBlkShort ? 6.8 : 4.1) * waves,
-          small ? 6.3 + 17.0 * M : 6.5 + 18.4 * M};
+//     (the same line with checkpoints, within 2 %)
+enum class Pass { kForward, kBoth };
+bool per_cell_tiles(const ErnnProblem& p, Pass pass) {
+  const bool small = step_rows(p.nx, p.ny, p.nshots) == 8;  // blocks of the plain kernels
+  const double rows = (p.nx + 7) / 8 * 8.0, cols = (p.ny + 31) / 32 * 32.0;
+  double M = 1e-6 * p.nshots * rows * cols;
+  if (p.mode == kModeDField) {
+    const int geo = blk_geometry(p.mode, p.nx, p.ny, p.nshots);
+    const double w = std::ceil(p.nshots * (double)blk_tiles(geo, p.nx, p.ny) / (geo == kBlkTall ? 304.0 : 152.0));
+    return 1.0 + (geo == kBlkTall ? 17.0 : geo == kBlkShort ? 6.8 : 4.1) * w <=
+           (small ? 6.3 + 17.0 * M : 6.5 + 18.4 * M);
+  }
+  const double tiles = p.nshots * (double)blk_tiles(kBlkFlat, p.nx, p.ny);
+  if (tiles <= 152.0) return true;  // a run: half the time of the plain kernels
+  // (a twentieth of a wave is lost in the wave before it)
+  const double w = std::ceil(tiles / 152.0 - 0.05);
+  double fwd = 0.9 + 1.07 * w, adj = 0.4 + 2.25 * w;
+  if (p.ny <= 48 && p.nx > 64) fwd *= 0.94, adj *= 0.88;  // (half the sectors of a row)
+  if (!small) M *= 0.5 + 0.5 * ((p.ny + 7) / 8 * 8.0) / cols;  // (a block's idle columns cost half)
+  const double fwd_plain = small ? 2.1 + 9.0 * M : 2.0 + 8.4 * M, adj_plain = small ? 4.2 + 20.0 * M : 14.0 + 15.6 * M;
+  if (pass == Pass::kForward) return fwd <= fwd_plain;
+  if (p.ckpt_k >= p.nt) return fwd + adj <= fwd_plain + adj_plain;
+  const double whole = std::ceil(p.ckpt_k / (double)kBlkSteps) * kBlkSteps / p.ckpt_k;
+  return (2.0 * fwd + adj) * (0.5 + 0.5 * whole) <= 2.0 * fwd_plain + adj_plain;
 }
 
 // Problems of the time-blocked tile kernels, from sizes alone (the workspace
@@ -103,8 +117,9 @@ StepUs per_cell_step_us(const ErnnProblem& p) {
 //    forward and adjoint step): the map, u's rows and the running gradient
 //    are read at every step either way, here from L2 by the threads.
 //  - Six constant planes: up to kBlockMaxFields cells.
-//    Both per-cell modes where a step takes less here than with the plain
-//    kernels (per_cell_step_us).
+//    Both per-cell modes where a forward and an adjoint step take less here
+//    than with the plain kernels (per_cell_tiles); a forward without a tape of
+//    constant planes asks for its own time (forward_impl).
 bool block_rule(const ErnnProblem& p) {
   if (p.flags & ERNN_FLAG_INSTANCES) return true;
   if (p.path == ERNN_PATH_TILED) return p.mode == kModeScalar && p.ny % 4 == 0;
@@ -112,8 +127,7 @@ bool block_rule(const ErnnProblem& p) {
   if (p.mode == kModeScalar) return (p.ny >= kBlockMinCols || !plain_size(p)) && !cluster_fits(p);
   if (p.ny < kBlockMinCols) return false;
   if (p.mode == kModeFields ? (double)p.nshots * p.nx * p.ny > kBlockMaxFields : !plain_size(p)) return false;
-  const StepUs us = per_cell_step_us(p);
-  return us.block <= us.plain;
+  return per_cell_tiles(p, Pass::kBoth);
 }
 
 // Upper bound of the tile-table entries of any placement of S instances on
@@ -832,7 +846,8 @@ static int forward_impl(const ErnnProblem* p, const ErnnInputs* in, const InstPl
   ERNN_CUDA(launch_coef(p->mode, in->C, in->rho, p->h, p->dt, coef, st, pl.ncoef));
 
   InstTiles itab{nullptr, nullptr, 0};
-  const bool block = pl.block && al16(tape) && blk_available();
+  const bool block = pl.block && al16(tape) && blk_available() &&
+                     (with_tape != 0 || p->mode != kModeFields || per_cell_tiles(*p, Pass::kForward));
   if (ip != nullptr) {
     // instances: the time-blocked kernels over the tile table only, which
     // read and write a state inside the instances' regions alone; trace

@@ -127,6 +127,27 @@ def test_per_cell_modes_take_the_kernels_measured_faster(lib, mode, S, nx, ny, t
 
 
 
+@pytest.mark.parametrize("S,nx,ny,kept,ckpt,alone", [
+    # constant planes: every state kept, checkpoints every 13 steps, forward alone (True: tiles)
+    (8, 301, 301, True, True, True), (1, 1000, 1000, True, True, True), (1, 301, 301, True, True, True),
+    (16, 250, 250, True, False, False), (20, 130, 130, True, False, False), (3, 2245, 136, False, False, False),
+    (2, 3000, 44, True, False, False), (300, 50, 50, False, False, False),
+])
+def test_constant_planes_ask_for_what_a_call_runs(lib, S, nx, ny, kept, ckpt, alone):
+    names = {True: E.PATH_TILED, False: E.PATH_STEP}
+    setup(lib)
+    for k, want in ((26, kept), (13, ckpt)):
+        assert call(lib, problem(mode=2, nshots=S, nx=nx, ny=ny, nt=26, ckpt_k=k)) == (0, 0)
+        assert lib.ernn_last_path() == names[want], k
+    p = problem(mode=2, nshots=S, nx=nx, ny=ny, nt=26, ckpt_k=26)
+    ptr = ctypes.c_void_p
+    ins = E._lib.ErnnInputs(*[ptr(DATA + (k << 36)) for k in range(7)])
+    n = lib.ernn_tape_bytes(ctypes.byref(p), 0)
+    assert lib.ernn_forward(ctypes.byref(p), ctypes.byref(ins), ptr(DATA + (8 << 36)), ptr(DATA + (9 << 36)), ptr(TAPE), n, 0,
+                            None) == 0
+    assert lib.ernn_last_path() == names[alone]
+
+
 class Pass(ctypes.Structure):
     """The first fields of BlkFwd and BlkAdj (out: of BlkAdj the last two levels)."""
     _fields_ = [(n, ctypes.c_int32) for n in ("geo", "plain_order", "nx", "ny", "pitch", "S", "nt", "step", "T")] + [
